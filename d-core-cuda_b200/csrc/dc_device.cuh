@@ -44,6 +44,9 @@ struct EngineCtl {
     // polled by idle warps
     alignas(128) unsigned error;
     unsigned err_where;
+    unsigned long long step_word;  // (step number << 32) | level, see "Steps without a barrier"
+    unsigned worked;               // last step of which an item was kept by the warp that found it
+    unsigned log_used;             // corner records written (the log's ranges have holes)
     unsigned phase_done;    // set by whoever brings outstanding to 0
     // work queue (monotone within one phase)
     alignas(128) unsigned q_head;
@@ -66,6 +69,8 @@ struct EngineCtl {
     alignas(128) unsigned t_head;  // next ticket
     alignas(128) unsigned t_tail;  // next slot to reserve
     alignas(128) int outstanding;  // unfinished producers + pushed, unfinished items
+    alignas(128) unsigned long long t_work;    // steps without a barrier: both in one word
+    alignas(128) unsigned long long next_low;  // (step << 32) | (2^31 - 1 - least next level)
     alignas(128) unsigned rc_cur[2];  // remaining-list sizes per peel instance
     PadU rc_next[2];        // next level's remaining-list sizes (appended by every warp)
     int maxv[2];            // largest value per peel instance
@@ -526,6 +531,244 @@ __device__ __forceinline__ bool tq_take_warp_lazy(EngineCtl* c, TicketQueue q, u
         }
     }
     return tq_take_warp(c, q, ticket, item);
+}
+
+// ---------------------------------------------------------------------------
+// Steps without a barrier.  A step (level or row) is over when every block has
+// reported its seeding and every item is finished; no warp works on it any
+// more then, so the one that finished last prepares the next step itself and
+// publishes it in step_word, and the others, which wait for items, see the
+// word change and start it.  Nothing arrives at a barrier: a grid barrier per
+// step cost its arrival and release round trips on top of the queue's own
+// termination (an empty step took 16-17 us with 296 blocks).
+//   - t_work holds the queue's tail (low 33 bits) and the number of unfinished
+//     producers and items (high 31 bits) in one word: a push is one atomic,
+//     and the count can never lag behind the items it covers
+//   - counters that belong to a step carry its number, so none is reset
+//     between steps
+//   - one warp of each block polls the step word and passes it on through
+//     shared memory (2,368 pollers of one line kept its L2 slice busy for
+//     longer than the light steps last)
+//   - a warp keeps its ticket from one step to the next (a ticket dropped by
+//     one warp while another advances the step would lose an item), and items
+//     carry their step: a warp that finds an item of a newer step in its slot
+//     has not started that step yet and leaves the item there until it has
+// Memory order: acquire loads and acquire atomics cost no more than relaxed
+// ones here (327 and 528 clocks), a fence costs 280-900 clocks, so readers
+// acquire, and a writer fences once, between its value and whatever makes
+// another warp look at it.  Counters are only changed by atomics whose result
+// is used: they are performed in L2, where every reader reads, before
+// anything that follows from the result.
+// ---------------------------------------------------------------------------
+constexpr int kWorkShift = 33;
+
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+// Makes the program wait for an atomic's result: it is performed then.
+__device__ __forceinline__ void used_result(unsigned long long a, unsigned long long b = 0) {
+    asm volatile("{ .reg .b64 t; add.s64 t, %0, %1; }" ::"l"(a), "l"(b) : "memory");
+}
+
+__device__ __forceinline__ int step_level(unsigned long long w) { return (int)(uint32_t)w; }
+__device__ __forceinline__ unsigned step_number(unsigned long long w) { return (unsigned)(w >> 32); }
+// 9 bits above 32 bits of payload and 22 of detail; the top bit stays 0, so
+// no item equals kEmptyItem
+__device__ __forceinline__ unsigned long long step_tag(unsigned long long w) { return ((w >> 32) & 0x1FFull) << 54; }
+
+constexpr unsigned long long kStopWord = ~0ull;  // the block leaves (error or wait limit)
+constexpr int kNoBound = 0x7FFFFFFF;
+
+// Shared state of a block.
+struct StepBlock {
+    unsigned long long word;  // the step word as the polling warp saw it last
+    unsigned done;            // warps that finished their seeding share
+    int bound;                // least next level they found
+};
+// All threads, at kernel start.
+__device__ __forceinline__ void step_block_init(StepBlock* b, const EngineCtl* c) {
+    if (threadIdx.x == 0) {
+        b->word = ld_acquire(&c->step_word);
+        b->done = 0;
+        b->bound = kNoBound;
+    }
+    __syncthreads();
+}
+__device__ __forceinline__ unsigned long long step_block_word(const StepBlock* b) {
+    return *reinterpret_cast<const volatile unsigned long long*>(&b->word);
+}
+
+// One thread: n producers or items of step `word` are finished; the last one
+// advances the step.  next(c, level, worked, bound): the next level.
+template <typename Next>
+__device__ __forceinline__ void step_finish(EngineCtl* c, int n, unsigned long long word, const Next& next) {
+    const unsigned long long old = atomicAdd(&c->t_work, 0ull - ((unsigned long long)n << kWorkShift));
+    if ((old >> kWorkShift) != (unsigned long long)n) return;
+    const unsigned step = step_number(word);
+    const unsigned tail = (unsigned)old;
+    const unsigned tail0 = ld_vol(&c->trace_tail0);
+    const unsigned long long low = *reinterpret_cast<const volatile unsigned long long*>(&c->next_low);
+    const bool worked = tail != tail0 || ld_vol(&c->worked) == step;
+    const int bound = (unsigned)(low >> 32) == step ? kNoBound - (int)(uint32_t)low : kNoBound;
+    const int level = next(c, step_level(word), worked, bound);
+    if (c->trace) {
+        const unsigned long long now = gtimer();
+        const unsigned st = step - 1;
+        if (st < c->trace_cap) {
+            c->trace[8 * st + 1] = now;
+            c->trace[8 * st + 2] = tail - tail0;
+            c->trace[8 * st + 3] = now;
+        }
+        if (st + 1 < c->trace_cap) {
+            c->trace[8 * (st + 1)] = now;
+            c->trace[8 * (st + 1) + 6] = ~0ull;
+        }
+    }
+    c->step = (int)step;
+    c->trace_tail0 = tail;
+    atomicAdd(&c->t_work, (unsigned long long)gridDim.x << kWorkShift);
+    __threadfence();
+    *reinterpret_cast<volatile unsigned long long*>(&c->step_word) =
+        ((unsigned long long)(step + 1) << 32) | (unsigned long long)(uint32_t)level;
+}
+
+// Converged warp: its seeding share of the step is done; bound (any lane's):
+// no level below it can have work that this warp saw.  The last warp of a
+// block reports the block.
+template <typename Next>
+__device__ __forceinline__ void step_seeded(EngineCtl* c, StepBlock* b, int bound, unsigned long long word,
+                                            bool tracing, const Next& next) {
+    bound = __reduce_min_sync(0xFFFFFFFFu, bound);
+    if ((threadIdx.x & 31u) == 0) {
+        if (bound != kNoBound) atomicMin(&b->bound, bound);
+        __threadfence_block();
+        if (atomicAdd(&b->done, 1u) == (blockDim.x >> 5) - 1) {
+            b->done = 0;
+            __threadfence_block();
+            const int m = atomicExch(&b->bound, kNoBound);
+            const unsigned step = step_number(word);
+            if (tracing && step - 1 < c->trace_cap) atomicMax(&c->trace[8 * (step - 1) + 5], gtimer());
+            if (m != kNoBound)
+                used_result(atomicMax(&c->next_low, ((unsigned long long)step << 32) | (unsigned long long)(kNoBound - m)));
+            step_finish(c, 1, word, next);
+        }
+    }
+    __syncwarp();
+}
+
+// Converged warp, while the step is being seeded: an item kept by the warp
+// counts like a queued one, and the step has work.
+__device__ __forceinline__ void step_count_kept(EngineCtl* c, unsigned long long word) {
+    if ((threadIdx.x & 31u) == 0) {
+        const unsigned long long a = atomicAdd(&c->t_work, 1ull << kWorkShift);
+        const unsigned o = atomicMax(&c->worked, step_number(word));
+        used_result(a, o);
+    }
+    __syncwarp();
+}
+
+// Start of a step in the optional trace (one thread per block).
+__device__ __forceinline__ void trace_wake(EngineCtl* c, unsigned long long word) {
+    const unsigned st = step_number(word) - 1;
+    if (st < c->trace_cap) {
+        const unsigned long long now = gtimer();
+        atomicMax(&c->trace[8 * st + 4], now);
+        atomicMin(&c->trace[8 * st + 6], now);
+    }
+}
+
+// Converged warp: reserves `total` slots for items (lane 0's value counts);
+// returns the first one's number on every lane.
+__device__ __forceinline__ unsigned step_reserve(EngineCtl* c, unsigned total) {
+    unsigned base = 0;
+    if ((threadIdx.x & 31u) == 0)
+        base = (unsigned)atomicAdd(&c->t_work, ((unsigned long long)total << kWorkShift) | total);
+    return __shfl_sync(0xFFFFFFFFu, base, 0);
+}
+__device__ __forceinline__ void step_put(TicketQueue q, unsigned at, unsigned long long item) {
+    *reinterpret_cast<volatile unsigned long long*>(&q.slots[at & q.mask]) = item;
+}
+// Converged warp: lanes with pred push one item each.
+__device__ __forceinline__ void step_push(EngineCtl* c, TicketQueue q, bool pred, unsigned long long item) {
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, pred);
+    if (!m) return;
+    const unsigned base = step_reserve(c, __popc(m));
+    if (pred) step_put(q, base + __popc(m & ((1u << (threadIdx.x & 31u)) - 1u)), item);
+}
+
+// Converged warp: the next item (kTakeItem, *item), or the start of the next
+// step (kTakeStep, *word updated), or kTakeStop after an error.  *pending
+// (lane 0): items this warp finished and has not counted off; they are
+// counted off before the warp waits.
+enum : int { kTakeItem = 1, kTakeStep = 2, kTakeStop = 3 };
+template <typename Next>
+__device__ __forceinline__ int step_take(EngineCtl* c, TicketQueue q, StepBlock* b, unsigned* ticket,
+                                         unsigned long long* item, int* pending, unsigned long long* word,
+                                         const Next& next) {
+    const unsigned lane = threadIdx.x & 31u;
+    unsigned long long it = kEmptyItem, w = *word;
+    int state = 0;
+    if (lane == 0) {
+        const bool poller = threadIdx.x == 0;
+        if (*ticket == kNoTicket) *ticket = atomicAdd(&c->t_head, 1u);
+        unsigned long long* s = &q.slots[*ticket & q.mask];
+        const unsigned long long tag = step_tag(w) >> 54;
+        it = ld_acquire(s);
+        if (it == kEmptyItem && *pending > 0) {
+            step_finish(c, *pending, w, next);
+            *pending = 0;
+        }
+        unsigned long long t0 = 0, seen = 0;
+        unsigned spins = 0;
+        while ((it >> 54) != tag) {
+            if (poller) {
+                w = ld_acquire(&c->step_word);
+                if ((++spins & 15u) == 0) {
+                    // the limit bounds a wait without progress: while the
+                    // step's other warps still push or finish items the clock
+                    // restarts
+                    const unsigned long long tw = *reinterpret_cast<volatile unsigned long long*>(&c->t_work);
+                    if (ld_vol(&c->error)) {
+                        w = kStopWord;
+                    } else if (spins == 64 || tw != seen) {
+                        seen = tw;
+                        t0 = gtimer();
+                    } else if (spins > 64 && gtimer() - t0 > wait_limit(c)) {
+                        set_dev_error(c, DC_DEV_ERR_TIMEOUT, 5);
+                        w = kStopWord;
+                    }
+                }
+                if (w != *word) *reinterpret_cast<volatile unsigned long long*>(&b->word) = w;
+            } else {
+                w = step_block_word(b);
+                ++spins;
+            }
+            if (w != *word) break;
+            if (spins > 8) __nanosleep(poller ? 20 : spins > 128 ? 64 : 20);
+            it = ld_acquire(s);
+        }
+        if ((it >> 54) == tag) {
+            *reinterpret_cast<volatile unsigned long long*>(s) = kEmptyItem;
+            *ticket = kNoTicket;
+            state = kTakeItem;
+        } else {
+            state = w == kStopWord ? kTakeStop : kTakeStep;
+        }
+    }
+    state = __shfl_sync(0xFFFFFFFFu, state, 0);
+    if (state == kTakeItem) it = __shfl_sync(0xFFFFFFFFu, it, 0);
+    else w = __shfl_sync(0xFFFFFFFFu, w, 0);
+    *item = it;
+    *word = w;
+    return state;
 }
 
 // Idle-wait helper for the drain loops: returns false once the phase has made

@@ -253,29 +253,11 @@ __device__ __forceinline__ void block_producer_done(EngineCtl* c, unsigned* s_cn
     __syncwarp();
 }
 
-// Per-vertex queue state for the transition drain:
-//   0 idle, 1 queued, 2 being evaluated, 3 being evaluated and re-run
-//   requested.  A vertex is never evaluated by two warps at once, and a
-//   request that lands during an evaluation re-queues the vertex when that
-//   evaluation ends.  Returns true when the caller must push the vertex.
-__device__ __forceinline__ bool mark_request(uint32_t* m, EngineCtl* c) {
-    unsigned s = ld_vol(m);
-    for (int it = 0; it < 1024; ++it) {
-        if (s == 0u) {
-            unsigned o = atomicCAS(m, 0u, 1u);
-            if (o == 0u) return true;
-            s = o;
-        } else if (s == 2u) {
-            unsigned o = atomicCAS(m, 2u, 3u);
-            if (o == 2u) return false;
-            s = o;
-        } else {
-            return false;
-        }
-    }
-    set_dev_error(c, DC_DEV_ERR_TIMEOUT, 21);
-    return false;
-}
+// Per-vertex queue state for the transition drain: bit 0 = requested, bit 1
+// = being evaluated.  A vertex is never evaluated by two warps at once, and a
+// request that lands during an evaluation re-queues the vertex when that
+// evaluation ends.  Returns true when the caller must push the vertex.
+__device__ __forceinline__ bool mark_request(uint32_t* m) { return atomicOr(m, 1u) == 0u; }
 
 // ---------------------------------------------------------------------------
 // fused peel, ticket queue, chunked items
@@ -582,23 +564,12 @@ struct Trans2Params {
     EngineCtl* ctl;
 };
 
+// Next row (run by the warp that finished the step): after a row that needed
+// no work, jump to the first row whose leaving set or seed set can be
+// non-empty (the step's bound).
 struct TransHook {
-    unsigned nworkers;
-    int K;
-    int K0;
-    __device__ void operator()(EngineCtl* c) const {
-        // next row: after a row that needed no work, jump to the first row
-        // whose leaving set or seed set can be non-empty (next_min)
-        if (c->step < 0) c->level = K0;
-        else if (c->t_tail == c->trace_tail0) c->level = max(c->level + 1, c->next_min);
-        else c->level = c->level + 1;
-        c->next_min = K + 1;
-        trace_step_end(c);
-        c->t_tail = c->t_head;
-        c->trace_tail0 = c->t_tail;
-        c->outstanding = (int)nworkers;
-        c->phase_done = 0;
-        __threadfence();
+    __device__ __forceinline__ int operator()(const EngineCtl*, int row, bool worked, int bound) const {
+        return worked ? row + 1 : max(row + 1, bound);
     }
 };
 
@@ -667,24 +638,23 @@ __global__ void k_counters_init(uint32_t V, const uint32_t* out_off, const int32
 // Converged warp: when the warp holds no item of its own yet (*keep ==
 // kNoKeep), it keeps the first request of the lowest requesting lane to
 // evaluate next itself instead of queueing it: the link from a drop to the
-// neighbour's evaluation skips the queue's publish and take.  The kept item
-// counts as outstanding like a queued one.
+// neighbour's evaluation skips the queue's publish and take.
 constexpr uint32_t kNoKeep = 0xFFFFFFFFu;
 // Requests of a lane: bit r of *req set = u[r] is requested (r < 4); the
 // items stay in registers (no dynamically indexed array).
 __device__ __forceinline__ uint32_t first_requested(unsigned req, const uint32_t u[4]) {
     return (req & 1u) ? u[0] : (req & 2u) ? u[1] : (req & 4u) ? u[2] : u[3];
 }
-__device__ __forceinline__ void keep_one(EngineCtl* c, uint32_t* keep, unsigned* req, const uint32_t u[4]) {
-    if (*keep != kNoKeep) return;
-    const unsigned lane = threadIdx.x & 31u;
+// Returns true (on every lane) when an item was kept.
+__device__ __forceinline__ bool keep_one(uint32_t* keep, unsigned* req, const uint32_t u[4]) {
+    if (*keep != kNoKeep) return false;
     const unsigned m = __ballot_sync(0xFFFFFFFFu, *req != 0u);
-    if (!m) return;
+    if (!m) return false;
     const unsigned src = __ffs(m) - 1;
     const uint32_t item = __shfl_sync(0xFFFFFFFFu, first_requested(*req, u), src);
-    if (lane == src) *req &= *req - 1u;  // drop the kept request
-    if (lane == 0) atomicAdd(&c->outstanding, 1);
+    if ((threadIdx.x & 31u) == src) *req &= *req - 1u;  // drop the kept request
     *keep = item;
+    return true;
 }
 
 // ---- vectorised list passes of the row kernel ----------------------------
@@ -714,10 +684,13 @@ __device__ __forceinline__ int last_value(const int x[4], int b, int last) {
     return __shfl_sync(0xFFFFFFFFu, sel4(x, r & 3), r >> 2);
 }
 
-// hist_pass2 with 16-byte id loads (same bins, counts and stopping rule).
+// Counts the neighbours at each value of [lo, hi] (both lists) into the bins
+// bo / bi; values above hi are not counted (the caller carries them).  On
+// kmax-sorted lists a list ends at its first neighbour outside C_j.  Returns
+// the entries read.
 __device__ __forceinline__ int hist_pass2v(const int32_t* cur, const uint32_t* onbr, uint32_t oo, int no,
-                                           const uint32_t* inbr, uint32_t io, int ni, int lo, int hi, bool first,
-                                           bool sorted, int* bo, int* bi) {
+                                           const uint32_t* inbr, uint32_t io, int ni, int lo, int hi, bool sorted,
+                                           int* bo, int* bi) {
     const unsigned lane = threadIdx.x & 31u;
     const int so = (int)(oo & 3u), si = (int)(io & 3u), endo = so + no, endi = si + ni;
     int to = 0, ti = 0, entries = 0;
@@ -737,10 +710,10 @@ __device__ __forceinline__ int hist_pass2v(const int32_t* cur, const uint32_t* o
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             int x = co[q];
-            to += first ? (x >= hi) : (x == hi);
+            to += (x == hi);
             if (x >= lo && x < hi) atomicAdd(&bo[x - lo], 1);
             x = ci[q];
-            ti += first ? (x >= hi) : (x == hi);
+            ti += (x == hi);
             if (x >= lo && x < hi) atomicAdd(&bi[x - lo], 1);
         }
         if (!doneo) {
@@ -769,11 +742,12 @@ __device__ __forceinline__ int hist_pass2v(const int32_t* cur, const uint32_t* o
 }
 
 // Converged warp: each lane pushes items_a[r] for bits r of ma and items_b[r]
-// for bits r of mb (r < 4), one reservation for the warp.
-__device__ __forceinline__ void tq_push_warp_mask8(EngineCtl* c, TicketQueue q, unsigned ma, const uint32_t items_a[4],
-                                                   unsigned mb, const uint32_t items_b[4]) {
+// for bits r of mb (r < 4) with the step's tag, one reservation for the warp.
+__device__ __forceinline__ void step_push_mask8(EngineCtl* c, TicketQueue q, unsigned ma, const uint32_t items_a[4],
+                                                   unsigned mb, const uint32_t items_b[4], unsigned long long tag) {
     const unsigned lane = threadIdx.x & 31u;
     const unsigned cnt = __popc(ma) + __popc(mb);
+    if (!__any_sync(0xFFFFFFFFu, cnt != 0u)) return;
     unsigned x = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -781,85 +755,256 @@ __device__ __forceinline__ void tq_push_warp_mask8(EngineCtl* c, TicketQueue q, 
         if (lane >= (unsigned)o) x += y;
     }
     const unsigned total = __shfl_sync(0xFFFFFFFFu, x, 31);
-    if (total == 0) return;
-    unsigned base = 0;
-    if (lane == 0) {
-        atomicAdd(&c->outstanding, (int)total);
-        base = atomicAdd(&c->t_tail, total);
-    }
-    base = __shfl_sync(0xFFFFFFFFu, base, 0) + (x - cnt);
-    if (cnt) __threadfence();
+    unsigned base = step_reserve(c, total) + (x - cnt);
 #pragma unroll
     for (unsigned r = 0; r < 4; ++r)
-        if (ma & (1u << r)) *(volatile unsigned long long*)&q.slots[(base + __popc(ma & ((1u << r) - 1u))) & q.mask] =
-            (unsigned long long)items_a[r];
+        if (ma & (1u << r)) step_put(q, base + __popc(ma & ((1u << r) - 1u)), (unsigned long long)items_a[r] | tag);
     base += __popc(ma);
 #pragma unroll
     for (unsigned r = 0; r < 4; ++r)
-        if (mb & (1u << r)) *(volatile unsigned long long*)&q.slots[(base + __popc(mb & ((1u << r) - 1u))) & q.mask] =
-            (unsigned long long)items_b[r];
+        if (mb & (1u << r)) step_put(q, base + __popc(mb & ((1u << r) - 1u)), (unsigned long long)items_b[r] | tag);
 }
 
-// recount_pass over both lists at once with 16-byte id loads: counts the
-// neighbours with value >= nv into *cnt_o / *cnt_i (this lane's share) and
-// takes x's support away from the neighbours whose level lies in (nv, cap]
-// (out-neighbours lose a unit of cnt_in, in-neighbours one of cnt_out); a
-// step's counter decrements are all issued before any result is used.
-// Stops like hist_pass2v.  Returns the entries read.
-__device__ __forceinline__ int recount_pass2v(const Trans2Params& p, EngineCtl* c, uint32_t oo, int no, uint32_t io,
-                                              int ni, int nv, int cap, int j, int* cnt_o, int* cnt_i,
-                                              uint32_t* keep) {
-    const unsigned lane = threadIdx.x & 31u;
-    const int so = (int)(oo & 3u), si = (int)(io & 3u), endo = so + no, endi = si + ni;
+// Both lists of a vertex and the ids of their first window.
+struct RowLists {
+    uint32_t oo, io;  // list starts
+    int no, ni;       // lengths
+    uint32_t uo[4], ui[4];
+};
+
+// The lists never change while the kernel runs: read through the read-only
+// path, so that the loads may be issued ahead of fences.
+__device__ __forceinline__ RowLists row_lists(const Trans2Params& p, uint32_t x) {
+    RowLists L;
+    L.oo = __ldg(p.out_off + x);
+    L.io = __ldg(p.in_off + x);
+    L.no = __ldg(p.out_len + x);
+    L.ni = __ldg(p.in_len + x);
+    load_ids4(p.out_nbr, L.oo, (int)(L.oo & 3u) + L.no, 0, L.no > 0, L.uo);
+    load_ids4(p.in_nbr, L.io, (int)(L.io & 3u) + L.ni, 0, L.ni > 0, L.ui);
+    return L;
+}
+
+// Values of the window's four entries of this lane (-1 outside the list).
+__device__ __forceinline__ void gather4(const int32_t* cur, const uint32_t u[4], int b, int start, int end,
+                                        bool active, int v[4]) {
+    const int t0 = b + 4 * (int)(threadIdx.x & 31u);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = (active && t0 + q >= start && t0 + q < end) ? ld_vol(&cur[u[q]]) : -1;
+}
+
+// Counts, over both lists, the neighbours at each of the kThr values cap,
+// cap - 1, .. (a drop is rarely larger), this lane's share in go / gi.  The
+// next window's ids are in flight while a window's values are gathered, so a
+// step of 128 entries per list costs one memory latency.  Returns the entries
+// read.
+constexpr int kThr = 4;
+__device__ __forceinline__ int count_pass(const Trans2Params& p, const RowLists& L, int cap, int go[kThr],
+                                          int gi[kThr]) {
+    const int so = (int)(L.oo & 3u), si = (int)(L.io & 3u), endo = so + L.no, endi = si + L.ni;
+    uint32_t uo[4], ui[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        uo[q] = L.uo[q];
+        ui[q] = L.ui[q];
+    }
+#pragma unroll
+    for (int r = 0; r < kThr; ++r) go[r] = gi[r] = 0;
+    bool ao = L.no > 0, ai = L.ni > 0;
     int entries = 0;
-    bool doneo = no <= 0, donei = ni <= 0;
-    for (int b = 0; !(doneo && donei); b += 128) {
-        uint32_t uo[4], ui[4];
-        load_ids4(p.out_nbr, oo, endo, b, !doneo, uo);
-        load_ids4(p.in_nbr, io, endi, b, !donei, ui);
-        const int t0 = b + 4 * (int)lane;
-        int co[4], ci[4];
+    for (int b = 0; ao || ai; b += 128) {
+        int vo[4], vi[4];
+        gather4(p.cur, uo, b, so, endo, ao, vo);
+        gather4(p.cur, ui, b, si, endi, ai, vi);
+        entries += (ao ? min(128, endo - b) : 0) + (ai ? min(128, endi - b) : 0);
+        ao = ao && b + 128 < endo;
+        ai = ai && b + 128 < endi;
+        load_ids4(p.out_nbr, L.oo, endo, b + 128, ao, uo);
+        load_ids4(p.in_nbr, L.io, endi, b + 128, ai, ui);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int t = t0 + q;
-            co[q] = (!doneo && t >= so && t < endo) ? ld_vol(&p.cur[uo[q]]) : -1;
-            ci[q] = (!donei && t >= si && t < endi) ? ld_vol(&p.cur[ui[q]]) : -1;
-        }
-        int oldo[4], oldi[4];
+        for (int q = 0; q < 4; ++q)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            *cnt_o += (co[q] >= nv);
-            *cnt_i += (ci[q] >= nv);
-            oldo[q] = (co[q] > nv && co[q] <= cap) ? atomicSub(&p.cnt_in[uo[q]], 1) : 0x7FFFFFFF;
-            oldi[q] = (ci[q] > nv && ci[q] <= cap) ? atomicSub(&p.cnt_out[ui[q]], 1) : 0x7FFFFFFF;
-        }
-        unsigned ro = 0, ri = 0;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (oldo[q] != 0x7FFFFFFF && oldo[q] - 1 < j && mark_request(&p.mark[uo[q]], c)) ro |= 1u << q;
-            if (oldi[q] != 0x7FFFFFFF && oldi[q] - 1 < ci[q] && mark_request(&p.mark[ui[q]], c)) ri |= 1u << q;
-        }
-        keep_one(c, keep, &ro, uo);
-        keep_one(c, keep, &ri, ui);
-        tq_push_warp_mask8(c, p.q, ro, uo, ri, ui);
-        if (!doneo) {
-            const int last = min(b + 127, endo - 1);
-            entries += last + 1 - max(b, so);
-            const int lv = last_value(co, b, last);
-            if (b + 128 >= endo || (p.sorted && lv == -1)) doneo = true;
-        }
-        if (!donei) {
-            const int last = min(b + 127, endi - 1);
-            entries += last + 1 - max(b, si);
-            const int lv = last_value(ci, b, last);
-            if (b + 128 >= endi || (p.sorted && lv == -1)) donei = true;
-        }
+            for (int r = 0; r < kThr; ++r) {
+                go[r] += vo[q] >= cap - r;
+                gi[r] += vi[q] >= cap - r;
+            }
+        // kmax-sorted lists end at the first neighbour outside C_j
+        if (p.sorted && ao && __shfl_sync(0xFFFFFFFFu, vo[3], 31) == -1) ao = false;
+        if (p.sorted && ai && __shfl_sync(0xFFFFFFFFu, vi[3], 31) == -1) ai = false;
     }
     return entries;
 }
 
+// One pass over both lists of x after its value fell from cap to nv: counts
+// the neighbours with value >= nv into *cnt_o / *cnt_i (this lane's share)
+// and takes x's support away from the neighbours whose level lies in
+// (nv, cap] (out-neighbours lose a unit of cnt_in, in-neighbours one of
+// cnt_out), requesting those that fall below what they need.  The next
+// window's values and the ids after it are in flight while a window's
+// decrements return.  kLeave: x leaves C_j (nv = 0, cap = its old value); the
+// requests kept are counted as outstanding, and *lmin bounds the next row
+// that can need work.  Returns the entries read.
+template <bool kLeave>
+__device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, const RowLists& L, int nv, int cap,
+                                         int j, unsigned long long word, int* cnt_o, int* cnt_i, uint32_t* keep,
+                                         int* pending, int* lmin) {
+    const int so = (int)(L.oo & 3u), si = (int)(L.io & 3u), endo = so + L.no, endi = si + L.ni;
+    bool ao = L.no > 0, ai = L.ni > 0;
+    if (!ao && !ai) return 0;
+    int entries = 0;
+    uint32_t uo[4], ui[4], no[4], ni[4];
+    int vo[4], vi[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        uo[q] = L.uo[q];
+        ui[q] = L.ui[q];
+    }
+    gather4(p.cur, uo, 0, so, endo, ao, vo);
+    gather4(p.cur, ui, 0, si, endi, ai, vi);
+    load_ids4(p.out_nbr, L.oo, endo, 128, ao, no);
+    load_ids4(p.in_nbr, L.io, endi, 128, ai, ni);
+    for (int b = 0;; b += 128) {
+        entries += (ao ? min(128, endo - b) : 0) + (ai ? min(128, endi - b) : 0);
+        bool mo = ao && b + 128 < endo, mi = ai && b + 128 < endi;
+        if (p.sorted && mo && __shfl_sync(0xFFFFFFFFu, vo[3], 31) == -1) mo = false;
+        if (p.sorted && mi && __shfl_sync(0xFFFFFFFFu, vi[3], 31) == -1) mi = false;
+        int oldo[4], oldi[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (!kLeave) {
+                *cnt_o += vo[q] >= nv;
+                *cnt_i += vi[q] >= nv;
+            }
+            oldo[q] = (vo[q] > nv && vo[q] <= cap) ? atomicSub(&p.cnt_in[uo[q]], 1) : 0x7FFFFFFF;
+            oldi[q] = (vi[q] > nv && vi[q] <= cap) ? atomicSub(&p.cnt_out[ui[q]], 1) : 0x7FFFFFFF;
+        }
+        int wo[4], wi[4];
+        gather4(p.cur, no, b + 128, so, endo, mo, wo);
+        gather4(p.cur, ni, b + 128, si, endi, mi, wi);
+        unsigned ro = 0, ri = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (oldo[q] - 1 < j) ro |= 1u << q;
+            else if (kLeave) *lmin = min(*lmin, oldo[q]);
+            if (oldi[q] != 0x7FFFFFFF && oldi[q] - 1 < vi[q]) ri |= 1u << q;
+        }
+        if (__any_sync(0xFFFFFFFFu, (ro | ri) != 0u)) {
+            unsigned so_[4], si_[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                so_[q] = (ro >> q) & 1u ? atomicOr(&p.mark[uo[q]], 1u) : 1u;
+                si_[q] = (ri >> q) & 1u ? atomicOr(&p.mark[ui[q]], 1u) : 1u;
+            }
+            ro = ri = 0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (so_[q] == 0u) ro |= 1u << q;
+                if (si_[q] == 0u) ri |= 1u << q;
+            }
+            if (keep_one(keep, &ro, uo) || keep_one(keep, &ri, ui)) {
+                if (kLeave) step_count_kept(c, word);
+                else --*pending;  // the item being finished pays for the kept one
+            }
+            step_push_mask8(c, p.q, ro, uo, ri, ui, step_tag(word));
+        }
+        if (!mo && !mi) break;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            uo[q] = no[q];
+            ui[q] = ni[q];
+            vo[q] = wo[q];
+            vi[q] = wi[q];
+        }
+        load_ids4(p.out_nbr, L.oo, endo, b + 256, mo, no);
+        load_ids4(p.in_nbr, L.io, endi, b + 256, mi, ni);
+        ao = mo;
+        ai = mi;
+    }
+    return entries;
+}
+
+// The value of x when it fell more than kThr - 1 below cap: windows of kWin
+// values below hi, histograms in shared memory; carry_o / carry_i = counts
+// above hi.  Counts at the value found go to *c_o / *c_i.
+__device__ __forceinline__ int window_value(const Trans2Params& p, const RowLists& L, int j, int hi, int carry_o,
+                                            int carry_i, int* ho, int* hi_, int* c_o, int* c_i, int* entries) {
+    const unsigned lane = threadIdx.x & 31u;
+    for (;;) {
+        int lo = max(0, hi - (kWin - 1));
+        ho[lane] = 0;
+        ho[lane + 32] = 0;
+        hi_[lane] = 0;
+        hi_[lane + 32] = 0;
+        __syncwarp();
+        *entries += hist_pass2v(p.cur, p.out_nbr, L.oo, L.no, p.in_nbr, L.io, L.ni, lo, hi, p.sorted != 0, ho, hi_);
+        __syncwarp();
+        int b0 = 2 * lane, b1 = 2 * lane + 1;
+        int o0 = ho[b0], o1 = ho[b1], i0 = hi_[b0], i1 = hi_[b1];
+        int po = o0 + o1, pi = i0 + i1;
+        int so = po, si = pi;
+#pragma unroll
+        for (int s = 1; s < 32; s <<= 1) {
+            int yo = __shfl_down_sync(0xFFFFFFFFu, so, s);
+            int yi = __shfl_down_sync(0xFFFFFFFFu, si, s);
+            if (lane + s < 32) {
+                so += yo;
+                si += yi;
+            }
+        }
+        int cum_o1 = carry_o + (so - po) + o1, cum_i1 = carry_i + (si - pi) + i1;
+        int cum_o0 = cum_o1 + o0, cum_i0 = cum_i1 + i0;
+        int L0 = lo + b0, L1 = lo + b1;
+        bool ok1 = (L1 <= hi) && cum_o1 >= L1 && cum_i1 >= j;
+        bool ok0 = (L0 <= hi) && cum_o0 >= L0 && cum_i0 >= j;
+        unsigned m1 = __ballot_sync(0xFFFFFFFFu, ok1), m0 = __ballot_sync(0xFFFFFFFFu, ok0);
+        int t1 = m1 ? 31 - __clz(m1) : -1, t0 = m0 ? 31 - __clz(m0) : -1;
+        int best = -1, bt = 0, bodd = 0;
+        if (t1 >= 0) {
+            best = lo + 2 * t1 + 1;
+            bt = t1;
+            bodd = 1;
+        }
+        if (t0 >= 0 && lo + 2 * t0 > best) {
+            best = lo + 2 * t0;
+            bt = t0;
+            bodd = 0;
+        }
+        if (best >= 0) {
+            int xo = bodd ? cum_o1 : cum_o0, xi = bodd ? cum_i1 : cum_i0;
+            *c_o = __shfl_sync(0xFFFFFFFFu, xo, bt);
+            *c_i = __shfl_sync(0xFFFFFFFFu, xi, bt);
+            return best;
+        }
+        carry_o += __shfl_sync(0xFFFFFFFFu, so, 0);
+        carry_i += __shfl_sync(0xFFFFFFFFu, si, 0);
+        if (lo == 0) {  // unreachable for members of C_j
+            *c_o = carry_o;
+            *c_i = carry_i;
+            return 0;
+        }
+        hi = lo - 1;
+        __syncwarp();
+    }
+}
+
+// Corner records a warp takes from the log at a time.
+static constexpr unsigned kLogChunk = 8;
+
+// Latency-bound: a row's changes run through dependent evaluations (one row
+// of R-MAT 20 takes 480 us for 178 evaluations), so what counts is the number
+// of memory round trips and fences from one vertex's drop to the next one's
+// evaluation.  Hence: the static data of a vertex is loaded while its mark is
+// set, its value and counters come with it, the new value is found with
+// register counters at the four highest candidates (the shared-memory
+// histogram only for larger drops), a corner record's place is in hand before
+// the drop, one fence stands between the new value (with its record) and the
+// neighbours' values, a request is one atomicOr, a warp keeps one of the items
+// it requests, and rows advance without a grid barrier.  Together: rows
+// 1..kmax of R-MAT 18 / 20 / 22 in one launch 16.5 / 25.8 / 53.5 -> 9.6 / 17.6 /
+// 38.5 ms, ER 10,000 / 100,000 0.71 -> 0.39 ms.  80 registers for three
+// blocks per SM (64 spill); one to four blocks measure within 7 %.
 #ifndef DC_TRANS2_MIN_BLOCKS
-#define DC_TRANS2_MIN_BLOCKS 4
+#define DC_TRANS2_MIN_BLOCKS 3
 #endif
 __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans2Params p) {
     const unsigned lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
@@ -868,265 +1013,216 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
     EngineCtl* c = p.ctl;
     __shared__ int s_ho[kWarpsPerBlock][kWin];
     __shared__ int s_hi[kWarpsPerBlock][kWin];
-    int* ho = s_ho[wib];
-    int* hi_ = s_hi[wib];
-    TransHook hook{gridDim.x, p.Kstop, p.K0};
-    unsigned long long my_evals = 0, my_drops = 0, my_entries = 0;
+    __shared__ StepBlock s_step;
+    const bool tracing = c->trace != nullptr;
+    // failure-detection tests: this block never reports, the others' waits run out
+    if (c->test_skip_block && (int)blockIdx.x == c->test_skip_block - 1) return;
+    const TransHook next;
+    unsigned my_evals = 0, my_drops = 0, my_log = 0;
+    unsigned long long my_entries = 0;
     unsigned ticket = kNoTicket;
-    __shared__ unsigned s_prod;
-    if (threadIdx.x == 0) s_prod = 0;
-    if (!grid_sync_hook(c, hook)) return;
-
+    unsigned long long log_at = 0;  // lane 0: the records of the warp's chunk
+    unsigned log_left = 0;
+    step_block_init(&s_step, c);
+    unsigned long long word = step_block_word(&s_step);
     int jprev = p.preleft ? p.K0 : 0;  // row currently held in cur
     bool seed_out = p.preleft != 0;
     for (;;) {
-        const int j = ld_vol(&c->level);
-        if (j > p.Kstop) break;
+        const int j = step_level(word);
+        if (word == kStopWord || j > p.Kstop) break;
+        const unsigned long long tag = step_tag(word);
+        if (tracing && threadIdx.x == 0) trace_wake(c, word);
+        uint32_t keep = kNoKeep;
+        int pending = 0;
         // rows jprev+1 .. j-1 equal row jprev; vertices with kmax in
         // [jprev, j-1] leave now (all but those with kmax == j-1 have value 0)
-        const uint32_t vj = p.ck[j], vprev = p.ck[jprev];
+        const uint32_t vj = __ldg(p.ck + j), vprev = __ldg(p.ck + jprev);
         // ---- vertices leaving C_j: value -1; neighbours they supported lose one count
-        int lmin = 0x7FFFFFFF;  // bound on the next row that can need work (see hook)
-        for (uint32_t i = vj + gwarp; i < vprev; i += nwarps) {
-            uint32_t x = p.order ? p.order[i] : i;
-            int a = ld_vol(&p.cur[x]);
-            __syncwarp();
-            if (lane == 0) {
-                atomicExch(&p.cur[x], -1);
-                __threadfence();
+        int bound = kNoBound;  // on the next row that can need work
+        // spread over all warps; a warp's share (up to 32 at a time) is cleared
+        // with one fence, and the next one's lists are loaded while one's are read
+        const uint32_t share = vprev > vj ? min(32u, (vprev - vj + nwarps - 1) / nwarps) : 1u;
+        for (uint32_t base = vj + gwarp * share; base < vprev; base += nwarps * share) {
+            const uint32_t i = base + lane;
+            uint32_t xl = 0;
+            int al = 0;
+            if (lane < share && i < vprev) {
+                xl = p.order ? __ldg(p.order + i) : i;
+                al = ld_vol(&p.cur[xl]);
+                *(volatile int32_t*)&p.cur[xl] = -1;
             }
-            __syncwarp();
-            if (a < 1) continue;
+            unsigned m = __ballot_sync(0xFFFFFFFFu, al >= 1);
+            if (!m) continue;
+            RowLists L = row_lists(p, __shfl_sync(0xFFFFFFFFu, xl, __ffs(m) - 1));
             __threadfence();
-            uint32_t o = p.out_off[x];
-            int n = p.out_len[x];
-            for (int b = 0; b < n; b += 32) {
-                bool req = false;
-                uint32_t z = 0;
-                int cz = -1;
-                if (b + (int)lane < n) {
-                    z = p.out_nbr[o + b + lane];
-                    cz = ld_vol(&p.cur[z]);
-                    if (cz >= 1 && cz <= a) {
-                        int old = atomicSub(&p.cnt_in[z], 1);
-                        if (old - 1 < j) req = mark_request(&p.mark[z], c);
-                        else lmin = min(lmin, min(old - 1, p.kmax[z]) + 1);
-                    }
-                }
-                tq_push_warp(c, p.q, req, z);
-                int last = min(31, n - 1 - b);
-                if (p.sorted && __shfl_sync(0xFFFFFFFFu, cz, last) == -1) break;
-            }
-            o = p.in_off[x];
-            n = p.in_len[x];
-            for (int b = 0; b < n; b += 32) {
-                bool req = false;
-                uint32_t y = 0;
-                int cy = -1;
-                if (b + (int)lane < n) {
-                    y = p.in_nbr[o + b + lane];
-                    cy = ld_vol(&p.cur[y]);
-                    if (cy >= 1 && cy <= a) {
-                        int old = atomicSub(&p.cnt_out[y], 1);
-                        req = (old - 1 < cy) && mark_request(&p.mark[y], c);
-                    }
-                }
-                tq_push_warp(c, p.q, req, y);
-                int last = min(31, n - 1 - b);
-                if (p.sorted && __shfl_sync(0xFFFFFFFFu, cy, last) == -1) break;
+            while (m) {
+                const int a = __shfl_sync(0xFFFFFFFFu, al, __ffs(m) - 1);
+                const RowLists cur_l = L;
+                m &= m - 1u;
+                if (m) L = row_lists(p, __shfl_sync(0xFFFFFFFFu, xl, __ffs(m) - 1));
+                drop_pass<true>(p, c, cur_l, 0, a, j, word, nullptr, nullptr, &keep, &pending, &bound);
             }
         }
-#pragma unroll
-        for (int s = 16; s; s >>= 1) lmin = min(lmin, __shfl_xor_sync(0xFFFFFFFFu, lmin, s));
-        if (lane == 0 && lmin != 0x7FFFFFFF) atomicMin(&c->next_min, lmin);
         // ---- seeds: members whose in-count at their own level is below j;
         // the least min(cnt_in, kmax) + 1 of the others bounds the next row
         // that can need work
-        int jmin = 0x7FFFFFFF;
         for (uint32_t base = gwarp * 32; base < vj; base += nwarps * 32) {
-            uint32_t i = base + lane;
-            bool req = false;
+            const uint32_t i = base + lane;
+            unsigned req = 0;
             uint32_t v = 0;
             if (i < vj) {
-                v = p.order ? p.order[i] : i;
-                const int cv = ld_vol(&p.cur[v]);
+                v = p.order ? __ldg(p.order + i) : i;
+                const int cv = ld_vol(&p.cur[v]), ci = ld_vol(&p.cnt_in[v]);
+                const int co = seed_out ? ld_vol(&p.cnt_out[v]) : 0x7FFFFFFF;
+                const int km = __ldg(p.kmax + v);
                 if (cv >= 1) {
-                    int ci = ld_vol(&p.cnt_in[v]);
-                    if (ci < j || (seed_out && ld_vol(&p.cnt_out[v]) < cv)) req = mark_request(&p.mark[v], c);
-                    else jmin = min(jmin, min(ci, p.kmax[v]) + 1);
+                    if (ci < j || co < cv) req = mark_request(&p.mark[v]) ? 1u : 0u;
+                    else bound = min(bound, min(ci, km) + 1);
                 }
             }
-            tq_push_warp(c, p.q, req, v);
+            if (__any_sync(0xFFFFFFFFu, req != 0u)) {
+                const uint32_t u[4] = {v, 0u, 0u, 0u};
+                if (keep_one(&keep, &req, u)) step_count_kept(c, word);
+                step_push(c, p.q, req != 0u, (unsigned long long)v | tag);
+            }
         }
-#pragma unroll
-        for (int s = 16; s; s >>= 1) jmin = min(jmin, __shfl_xor_sync(0xFFFFFFFFu, jmin, s));
-        if (lane == 0 && jmin != 0x7FFFFFFF) atomicMin(&c->next_min, jmin);
-        block_producer_done(c, &s_prod);
+        step_seeded(c, &s_step, bound, word, tracing, next);
 
         // ---- drain: the warp's kept item first, else the queue; finished
         // items are counted off in batches (before the warp waits)
-        unsigned long long item;
-        uint32_t keep = kNoKeep;
-        unsigned done_pending = 0;
+        unsigned long long item = 0;
+        int state = kTakeItem;
         for (;;) {
+            uint32_t x;
             if (keep != kNoKeep) {
-                item = keep;
+                x = keep;
                 keep = kNoKeep;
-            } else if (!tq_take_warp_lazy(c, p.q, &ticket, &item, &done_pending)) {
-                break;
+            } else {
+                state = step_take(c, p.q, &s_step, &ticket, &item, &pending, &word, next);
+                if (state != kTakeItem) break;
+                x = (uint32_t)item;
             }
-            const uint32_t x = (uint32_t)item;
-            if (lane == 0) {
-                atomicExch(&p.mark[x], 2u);
-                __threadfence();
-            }
-            __syncwarp();
+            // the mark says "being evaluated" before any neighbour is read (a
+            // request made before it belongs to a drop that is seen below, one
+            // made after it has x evaluated again); a decrement that lands
+            // between the counter snapshot and the mark only makes the counter
+            // too low, which costs an evaluation
+            unsigned mk = 0;
+            if (lane == 0) mk = atomicExch(&p.mark[x], 2u);
             const int cap = ld_vol(&p.cur[x]);
-            if (p.kmax[x] < j || cap < 1) {
-                if (lane == 0) {
-                    atomicExch(&p.mark[x], 0u);
-                    ++done_pending;
-                }
+            const int s0o = ld_vol(&p.cnt_out[x]), s0i = ld_vol(&p.cnt_in[x]);
+            const int stamp = ld_vol(&p.stamp[x]);
+            const uint32_t logidx = ld_vol(&p.logidx[x]);
+            const int km = __ldg(p.kmax + x);
+            const RowLists L = row_lists(p, x);
+            if (lane == 0) used_result(mk, ld_acquire(&p.mark[x]));
+            __syncwarp();
+            if (km < j || cap < 1) {
+                if (lane == 0) atomicExch(&p.mark[x], 0u);
+                ++pending;
                 continue;
             }
-            int s0o = 0, s0i = 0;
-            if (lane == 0) {
-                s0o = ld_vol(&p.cnt_out[x]);
-                s0i = ld_vol(&p.cnt_in[x]);
-            }
-            __threadfence();
-            const uint32_t oo = p.out_off[x], io = p.in_off[x];
-            const unsigned long long ev_entries0 = my_entries;
-            // ---- new value from windowed histograms
-            int carry_o = 0, carry_i = 0, hi = cap, nv = -1, c_o = 0, c_i = 0;
-            bool first = true;
-            for (;;) {
-                int lo = max(0, hi - (kWin - 1));
-                ho[lane] = 0;
-                ho[lane + 32] = 0;
-                hi_[lane] = 0;
-                hi_[lane + 32] = 0;
-                __syncwarp();
-                my_entries += hist_pass2v(p.cur, p.out_nbr, oo, p.out_len[x], p.in_nbr, io, p.in_len[x], lo, hi, first,
-                                          p.sorted != 0, ho, hi_);
-                __syncwarp();
-                int b0 = 2 * lane, b1 = 2 * lane + 1;
-                int o0 = ho[b0], o1 = ho[b1], i0 = hi_[b0], i1 = hi_[b1];
-                int po = o0 + o1, pi = i0 + i1;
-                int so = po, si = pi;
+            // ---- new value
+            int c_o = 0, c_i = 0, nv = -1, entries;
+            {
+                int go[kThr], gi[kThr];
+                entries = count_pass(p, L, cap, go, gi);
 #pragma unroll
-                for (int s = 1; s < 32; s <<= 1) {
-                    int yo = __shfl_down_sync(0xFFFFFFFFu, so, s);
-                    int yi = __shfl_down_sync(0xFFFFFFFFu, si, s);
-                    if (lane + s < 32) {
-                        so += yo;
-                        si += yi;
+                for (int r = 0; r < kThr; ++r) {
+                    go[r] = __reduce_add_sync(0xFFFFFFFFu, go[r]);
+                    gi[r] = __reduce_add_sync(0xFFFFFFFFu, gi[r]);
+                }
+#pragma unroll
+                for (int r = kThr - 1; r >= 0; --r)
+                    if (cap - r >= 0 && go[r] >= cap - r && gi[r] >= j) {
+                        nv = cap - r;
+                        c_o = go[r];
+                        c_i = gi[r];
+                    }
+                if (nv < 0) {
+                    if (cap >= kThr) {
+                        nv = window_value(p, L, j, cap - kThr, go[kThr - 1], gi[kThr - 1], s_ho[wib], s_hi[wib], &c_o,
+                                          &c_i, &entries);
+                    } else {  // unreachable for members of C_j
+                        nv = 0;
                     }
                 }
-                int cum_o1 = carry_o + (so - po) + o1, cum_i1 = carry_i + (si - pi) + i1;
-                int cum_o0 = cum_o1 + o0, cum_i0 = cum_i1 + i0;
-                int L0 = lo + b0, L1 = lo + b1;
-                bool ok1 = (L1 <= hi) && cum_o1 >= L1 && cum_i1 >= j;
-                bool ok0 = (L0 <= hi) && cum_o0 >= L0 && cum_i0 >= j;
-                unsigned m1 = __ballot_sync(0xFFFFFFFFu, ok1), m0 = __ballot_sync(0xFFFFFFFFu, ok0);
-                int t1 = m1 ? 31 - __clz(m1) : -1, t0 = m0 ? 31 - __clz(m0) : -1;
-                int best = -1, bt = 0, bodd = 0;
-                if (t1 >= 0) {
-                    best = lo + 2 * t1 + 1;
-                    bt = t1;
-                    bodd = 1;
-                }
-                if (t0 >= 0 && lo + 2 * t0 > best) {
-                    best = lo + 2 * t0;
-                    bt = t0;
-                    bodd = 0;
-                }
-                if (best >= 0) {
-                    int xo = bodd ? cum_o1 : cum_o0, xi = bodd ? cum_i1 : cum_i0;
-                    c_o = __shfl_sync(0xFFFFFFFFu, xo, bt);
-                    c_i = __shfl_sync(0xFFFFFFFFu, xi, bt);
-                    nv = best;
-                    break;
-                }
-                carry_o += __shfl_sync(0xFFFFFFFFu, so, 0);
-                carry_i += __shfl_sync(0xFFFFFFFFu, si, 0);
-                first = false;
-                if (lo == 0) {  // unreachable for members of C_j
-                    nv = 0;
-                    c_o = carry_o;
-                    c_i = carry_i;
-                    break;
-                }
-                hi = lo - 1;
-                __syncwarp();
             }
             ++my_evals;
-            if (c->trace && lane == 0) {
-                int st = ld_vol(&c->step);
-                if (st >= 0 && (unsigned)st < c->trace_cap)
-                    atomicMax(&c->trace[8 * st + 7], (unsigned long long)(my_entries - ev_entries0));
-            }
             if (nv < cap) {
                 ++my_drops;
                 if (lane == 0) {
-                    atomicExch(&p.cur[x], nv);
-                    __threadfence();
-                    if (p.stamp[x] != j) {
-                        unsigned long long li = atomicAdd(&c->log_count, 1u);
-                        if (li < p.log_cap) {
+                    // the value and its corner record
+                    unsigned long long li = logidx;
+                    const bool fresh = stamp != j;
+                    if (fresh) {
+                        if (!log_left) {
+                            log_at = atomicAdd(&c->log_count, kLogChunk);
+                            log_left = kLogChunk;
+                        }
+                        li = log_at++;
+                        --log_left;
+                        ++my_log;
+                    }
+                    if (li < p.log_cap) {
+                        if (fresh) {
                             p.stamp[x] = j;
                             p.logidx[x] = (uint32_t)li;
                             p.log_v[li] = x;
                             p.log_k[li] = j;
-                            p.log_l[li] = nv;
-                        } else {
-                            set_dev_error(c, DC_DEV_ERR_CAPACITY, 20);
                         }
+                        p.log_l[li] = nv;
                     } else {
-                        p.log_l[p.logidx[x]] = nv;
+                        set_dev_error(c, DC_DEV_ERR_CAPACITY, 20);
                     }
+                    *(volatile int32_t*)&p.cur[x] = nv;
                 }
                 __syncwarp();
                 __threadfence();
                 // recount at nv after the write, and take x's support away
-                // from neighbours whose level lies in (nv, cap]
+                // from neighbours whose level lies in (nv, cap]: out-neighbours
+                // hold x in cnt_in, in-neighbours in cnt_out
                 c_o = 0;
                 c_i = 0;
-                // out-neighbours z hold x in cnt_in; in-neighbours y hold x in cnt_out
-                my_entries += recount_pass2v(p, c, oo, p.out_len[x], io, p.in_len[x], nv, cap, j, &c_o, &c_i, &keep);
-#pragma unroll
-                for (int s = 16; s; s >>= 1) {
-                    c_o += __shfl_xor_sync(0xFFFFFFFFu, c_o, s);
-                    c_i += __shfl_xor_sync(0xFFFFFFFFu, c_i, s);
-                }
+                entries += drop_pass<false>(p, c, L, nv, cap, j, word, &c_o, &c_i, &keep, &pending, nullptr);
+                c_o = __reduce_add_sync(0xFFFFFFFFu, c_o);
+                c_i = __reduce_add_sync(0xFFFFFFFFu, c_i);
             }
-            bool requeue = false;
+            my_entries += (unsigned)entries;
+            if (tracing && lane == 0 && step_number(word) - 1 < c->trace_cap)
+                atomicMax(&c->trace[8 * (step_number(word) - 1) + 7], (unsigned long long)entries);
+            unsigned again = 0;
             if (lane == 0) {
-                int no = atomicAdd(&p.cnt_out[x], c_o - s0o) + (c_o - s0o);
-                int ni = atomicAdd(&p.cnt_in[x], c_i - s0i) + (c_i - s0i);
-                bool stable = nv < 1 || (no >= nv && ni >= j);
-                __threadfence();
-                if (!stable) {
-                    atomicExch(&p.mark[x], 1u);
-                    requeue = true;
-                } else {
-                    unsigned o = atomicCAS(&p.mark[x], 2u, 0u);
-                    if (o == 3u) {
-                        atomicExch(&p.mark[x], 1u);
-                        requeue = true;
-                    }
+                const int no = atomicAdd(&p.cnt_out[x], c_o - s0o) + (c_o - s0o);
+                const int ni = atomicAdd(&p.cnt_in[x], c_i - s0i) + (c_i - s0i);
+                const bool stable = nv < 1 || (no >= nv && ni >= j);
+                // released once the counters are; requested meanwhile or
+                // unstable: evaluated again
+                if (!stable || atomicCAS(&p.mark[x], 2u, 0u) == 3u) {
+                    used_result(atomicExch(&p.mark[x], 1u));
+                    again = 1u;
                 }
             }
-            tq_push_warp(c, p.q, requeue, x);
-            if (lane == 0) ++done_pending;
+            if (__shfl_sync(0xFFFFFFFFu, again, 0)) {
+                if (keep == kNoKeep) {
+                    keep = x;  // at once: still the item being finished
+                    continue;
+                }
+                step_push(c, p.q, lane == 0, (unsigned long long)x | tag);
+            }
+            ++pending;
         }
+        if (state == kTakeStop) break;
         jprev = j;
         seed_out = false;
-        if (!grid_sync_hook(c, hook)) break;
     }
     if (lane == 0) {
-        atomicAdd(&c->evals, my_evals);
-        atomicAdd(&c->drops, my_drops);
+        // unused records of the last chunk are void
+        for (; log_left; --log_left, ++log_at)
+            if (log_at < p.log_cap) p.log_k[log_at] = -1;
+        atomicAdd(&c->log_used, my_log);
+        atomicAdd(&c->evals, (unsigned long long)my_evals);
+        atomicAdd(&c->drops, (unsigned long long)my_drops);
         atomicAdd(&c->edges_scanned, my_entries);
     }
 }
@@ -2021,14 +2117,14 @@ int ensure_tring(dc_graph* h, uint64_t need) {
 // once the queue counters sit on separate lines (the autotuner refines it).
 static constexpr int kDefaultBlocksPerSm = 2;
 
-static int persistent_grid(dc_graph* h, const void* fn, int bps, int* blocks) {
+static int persistent_grid(dc_graph* h, const void* fn, int bps, int* blocks, int share = 1) {
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, 0);
     if (e != cudaSuccess || per_sm < 1)
         return set_error(DC_ERR_CUDA, "occupancy query failed (%s)", cudaGetErrorString(e));
     if (bps <= 0) bps = h->blocks_per_sm > 0 ? h->blocks_per_sm : kDefaultBlocksPerSm;
-    per_sm = std::min(per_sm, bps);
-    *blocks = per_sm * h->geom.sms;
+    // launches that share the SMs get an equal part of the resident blocks each
+    *blocks = std::max(1, std::min(bps * h->geom.sms, per_sm * h->geom.sms / share));
     return DC_OK;
 }
 
@@ -2068,12 +2164,19 @@ int persistent_enqueue(dc_graph* h, const void* fn, void** args, const char* nam
     return DC_OK;
 }
 
+// First step of a kernel whose steps advance without a barrier.
+struct FirstStep {
+    int level;
+};
+
 // Initialises a control block (on stream st) and launches a persistent
 // kernel there without waiting.  The handle's own block carries the trace.
+// first: the kernel's first step (nullptr: it starts with a grid barrier);
+// share: the launch is one of that many which run at the same time.
 static int persistent_launch(dc_graph* h, const void* fn, void** args, const char* name, EngineCtl* ctl,
-                             cudaStream_t st, int bps) {
+                             cudaStream_t st, int bps, const FirstStep* first = nullptr, int share = 1) {
     int blocks = 0;
-    if (int rc = persistent_grid(h, fn, bps, &blocks)) return rc;
+    if (int rc = persistent_grid(h, fn, bps, &blocks, share)) return rc;
     const bool own = ctl == h->ctl;
     EngineCtl* initp = &h->ctl_init;
     for (int i = 0; i < kMaxRowSegments - 1; ++i)
@@ -2082,6 +2185,11 @@ static int persistent_launch(dc_graph* h, const void* fn, void** args, const cha
     memset(&init, 0, sizeof(init));
     init.step = -1;
     init.wait_ns = h->wait_ns;
+    if (first) {
+        init.step = 0;
+        init.t_work = (unsigned long long)blocks << kWorkShift;
+        init.step_word = (1ull << 32) | (unsigned long long)(uint32_t)first->level;
+    }
     if (own) {
         init.trace = h->trace_dev;
         init.trace_cap = h->trace_cap;
@@ -2248,8 +2356,9 @@ int run_peel(dc_graph* h, int which, const int32_t* member, int32_t k, int32_t* 
 }
 
 // Skyline from row 0 and the corner logs of the last run of rows: the
-// first segment's nlog entries at the log's start and the other segments'
-// ranges (h->seg_off / seg_n, voided entries skipped).
+// first segment's nlog entries at the log's start (h->log_used of them
+// records, the others void) and the other segments' ranges (h->seg_off /
+// seg_n, void entries skipped).
 int build_skyline_from_log(dc_graph* h, uint64_t nlog) {
     Scratch* s = h->scratch;
     Decomp& d = h->d;
@@ -2261,7 +2370,7 @@ int build_skyline_from_log(dc_graph* h, uint64_t nlog) {
     if (nlog) {
         lo[nr] = 0;
         n[nr++] = nlog;
-        total += nlog;
+        total += h->log_used;
     }
     for (int i = 0; i < h->nseg_extra; ++i)
         if (h->seg_n[i]) {
@@ -2421,10 +2530,10 @@ __global__ void k_len_to_u64e(uint32_t V, const int32_t* len, unsigned long long
         out[i] = (unsigned long long)len[i];
 }
 
-// corner records of the relabeled run back to original ids
-__global__ void k_unlabel_log(uint64_t n, const uint32_t* order, uint32_t* log_v) {
+// corner records of the relabeled run back to original ids (void ones hold none)
+__global__ void k_unlabel_log(uint64_t n, const uint32_t* order, uint32_t* log_v, const int32_t* log_k) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        log_v[i] = order[log_v[i]];
+        if (log_k[i] >= 0) log_v[i] = order[log_v[i]];
 }
 
 // Builds the relabeled graph (s->order must hold the kmax order of the
@@ -2499,6 +2608,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     Scratch* s = h->scratch;
     const uint32_t V = g.V;
     *nlog_out = 0;
+    h->log_used = 0;
     h->nseg_extra = 0;
     cudaEventRecord(h->ev[2], h->stream);
     if (s->ck_cap < (uint32_t)K + 2) {
@@ -2547,22 +2657,11 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
             if (c >= 1 && c < Kstop && (nseg == 1 || c > cut[nseg - 2])) cut[nseg++ - 1] = c;
         }
     cut[nseg - 1] = Kstop;
-    int seg_bps = h->rows_bps;
-    if (nseg > 1) {
-        // every segment's blocks must be resident together for their grid barriers
-        int per_sm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_trans2, kThreads, 0) != cudaSuccess)
-            per_sm = 0;
-        while (nseg > 1 && per_sm / nseg < 1) {
-            cut[nseg - 2] = Kstop;
-            --nseg;
-        }
-        const int want = seg_bps > 0 ? seg_bps : (h->blocks_per_sm > 0 ? h->blocks_per_sm : kDefaultBlocksPerSm);
-        if (nseg > 1) seg_bps = std::min(want, per_sm / nseg);
-    }
     // log ranges: [off[i], off[i] + cap[i]) per segment
     uint64_t off[kMaxRowSegments] = {}, capn[kMaxRowSegments] = {};
-    uint64_t lc = bound + 1;
+    // records every warp of the largest grid may leave unused in its last chunk
+    const uint64_t spare = (uint64_t)kLogChunk * kWarpsPerBlock * 8 * h->geom.sms / nseg;
+    uint64_t lc = bound + 1 + spare;
     if (nseg > 1) {
         SegBounds sb;
         sb.n = nseg;
@@ -2579,7 +2678,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
         lc = 0;
         for (int i = 0; i < nseg; ++i) {
             off[i] = lc;
-            capn[i] = bs[i] + 1;
+            capn[i] = bs[i] + 1 + spare;
             lc += capn[i];
         }
     }
@@ -2691,7 +2790,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
         }
     }
     uint64_t nlog = 0;
-    uint64_t nseg_log[kMaxRowSegments] = {};
+    uint64_t nseg_log[kMaxRowSegments] = {}, nseg_used[kMaxRowSegments] = {};
     unsigned long long voids[kMaxRowSegments] = {};
     cudaEventRecord(h->ev[3], h->stream);
     if (tp[0].Kstop >= tp[0].K0) {
@@ -2706,7 +2805,8 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
             args[i][0] = &tp[i];
             EngineCtl* ctl = i == 0 ? h->ctl : s->seg[i - 1].ctl;
             cudaStream_t st = i == 0 ? h->stream : s->seg[i - 1].stream;
-            rc = persistent_launch(h, (const void*)k_trans2, args[i], kNames[i], ctl, st, seg_bps);
+            const FirstStep first{tp[i].K0};
+            rc = persistent_launch(h, (const void*)k_trans2, args[i], kNames[i], ctl, st, h->rows_bps, &first, nseg);
             if (rc == DC_OK) ++launched;
         }
         h->stat_evals = h->stat_drops = h->stat_entries = 0;
@@ -2720,12 +2820,14 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
                 continue;
             }
             nseg_log[i] = hc.log_count;
+            nseg_used[i] = hc.log_used;
             h->stat_evals += hc.evals;
             h->stat_drops += hc.drops;
             h->stat_entries += hc.edges_scanned;
         }
         if (rc) return rc;
         nlog = nseg_log[0];
+        h->log_used = nseg_used[0];
         if (nseg > 1) {
             DC_CUDA(cudaMemsetAsync(acc, 0, nseg * sizeof(unsigned long long), h->stream));
             for (int i = 1; i < nseg; ++i) {
@@ -2747,7 +2849,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
             for (int i = 1; i < nseg; ++i) {
                 h->seg_off[i - 1] = off[i];
                 h->seg_n[i - 1] = nseg_log[i];
-                h->seg_void[i - 1] = voids[i];
+                h->seg_void[i - 1] = nseg_log[i] - nseg_used[i] + voids[i];
             }
         }
         if (relabel)  // corner records back to original ids (the seam check above compares relabeled state)
@@ -2755,7 +2857,8 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
                 if (nseg_log[i]) {
                     ++g_launches;
                     k_unlabel_log<<<grid_for(h, nseg_log[i]), kThreads, 0, h->stream>>>(nseg_log[i], s->order,
-                                                                                       s->log_v + off[i]);
+                                                                                       s->log_v + off[i],
+                                                                                       s->log_k + off[i]);
                 }
     }
     cudaEventRecord(h->ev[4], h->stream);

@@ -126,6 +126,7 @@ struct dc_graph {
     // corner logs of the segments after the first from the last run:
     // [seg_off[i], seg_off[i] + seg_n[i]), seg_void[i] entries voided (row k < 0)
     int nseg_extra = 0;
+    uint64_t log_used = 0;  // records of the first segment's log (its other entries are void)
     uint64_t seg_off[dc::kMaxRowSegments - 1] = {}, seg_n[dc::kMaxRowSegments - 1] = {},
              seg_void[dc::kMaxRowSegments - 1] = {};
     uint64_t stat_evals = 0, stat_drops = 0, stat_entries = 0;
