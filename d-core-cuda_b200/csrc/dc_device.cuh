@@ -29,9 +29,10 @@ constexpr int kMinSplitRows = 32;   // runs of fewer rows are never split
 struct alignas(128) PadU {
     unsigned v;
 };
-struct alignas(128) PadI {
-    int v;
+struct alignas(128) PadW {
+    unsigned long long v;
 };
+constexpr int kStepWords = 8;  // copies of the step word, each block polls one
 
 // The counters every warp hits (ticket head and tail, the outstanding count,
 // the barrier) and the flags idle warps poll (phase_done, error) each sit in
@@ -44,7 +45,6 @@ struct EngineCtl {
     // polled by idle warps
     alignas(128) unsigned error;
     unsigned err_where;
-    unsigned long long step_word;  // (step number << 32) | level, see "Steps without a barrier"
     unsigned worked;               // last step of which an item was kept by the warp that found it
     unsigned log_used;             // corner records written (the log's ranges have holes)
     unsigned phase_done;    // set by whoever brings outstanding to 0
@@ -69,7 +69,12 @@ struct EngineCtl {
     alignas(128) unsigned t_head;  // next ticket
     alignas(128) unsigned t_tail;  // next slot to reserve
     alignas(128) int outstanding;  // unfinished producers + pushed, unfinished items
+    PadW step_word[kStepWords];                // (step number << 32) | level, see "Steps without a barrier"
     alignas(128) unsigned long long t_work;    // steps without a barrier: both in one word
+    alignas(128) unsigned bag_tail;            // fused peel: vertices put into bags
+    int peel_list[2];       // per peel: remaining vertices in rem0 / rem1, or all (-1)
+    int peel_compact[2];    // the level writes the list anew
+    unsigned removed[2];    // removed since it was written
     alignas(128) unsigned long long next_low;  // (step << 32) | (2^31 - 1 - least next level)
     alignas(128) unsigned rc_cur[2];  // remaining-list sizes per peel instance
     PadU rc_next[2];        // next level's remaining-list sizes (appended by every warp)
@@ -77,8 +82,6 @@ struct EngineCtl {
     int step;               // level / transition index
     unsigned nworkers;      // producers per phase (warps in the grid)
     int level;              // current level / row of the persistent loop
-    int next_min;           // smallest level / row a skipped step may jump to
-    PadI minkey[2];         // per peel instance: least peeling degree kept by the scan
     // optional per-step timing trace: 8 words per step
     //   [0] %globaltimer at step start, [1] when its work ran out,
     //   [2] queue items of the step, [3] %globaltimer at the closing barrier,
@@ -546,9 +549,9 @@ __device__ __forceinline__ bool tq_take_warp_lazy(EngineCtl* c, TicketQueue q, u
 //     and the count can never lag behind the items it covers
 //   - counters that belong to a step carry its number, so none is reset
 //     between steps
-//   - one warp of each block polls the step word and passes it on through
-//     shared memory (2,368 pollers of one line kept its L2 slice busy for
-//     longer than the light steps last)
+//   - one warp of each block polls one of the copies of the step word and
+//     passes it on through shared memory (2,368 pollers of one line kept its
+//     L2 slice busy for longer than the light steps last)
 //   - a warp keeps its ticket from one step to the next (a ticket dropped by
 //     one warp while another advances the step would lose an item), and items
 //     carry their step: a warp that finds an item of a newer step in its slot
@@ -592,13 +595,17 @@ struct StepBlock {
     unsigned long long word;  // the step word as the polling warp saw it last
     unsigned done;            // warps that finished their seeding share
     int bound;                // least next level they found
+    unsigned worked;          // one of them found work that is not in the queue
+    unsigned count[2];        // fused peel: vertices they removed
 };
 // All threads, at kernel start.
 __device__ __forceinline__ void step_block_init(StepBlock* b, const EngineCtl* c) {
     if (threadIdx.x == 0) {
-        b->word = ld_acquire(&c->step_word);
+        b->word = ld_acquire(&c->step_word[blockIdx.x % kStepWords].v);
         b->done = 0;
         b->bound = kNoBound;
+        b->worked = 0;
+        b->count[0] = b->count[1] = 0;
     }
     __syncthreads();
 }
@@ -636,28 +643,36 @@ __device__ __forceinline__ void step_finish(EngineCtl* c, int n, unsigned long l
     c->trace_tail0 = tail;
     atomicAdd(&c->t_work, (unsigned long long)gridDim.x << kWorkShift);
     __threadfence();
-    *reinterpret_cast<volatile unsigned long long*>(&c->step_word) =
-        ((unsigned long long)(step + 1) << 32) | (unsigned long long)(uint32_t)level;
+    const unsigned long long w = ((unsigned long long)(step + 1) << 32) | (unsigned long long)(uint32_t)level;
+#pragma unroll
+    for (int i = 0; i < kStepWords; ++i) *reinterpret_cast<volatile unsigned long long*>(&c->step_word[i].v) = w;
 }
 
 // Converged warp: its seeding share of the step is done; bound (any lane's):
-// no level below it can have work that this warp saw.  The last warp of a
-// block reports the block.
+// no level below it can have work that this warp saw; worked: it found work
+// (queued items say so by themselves).  The last warp of a block reports the
+// block.
 template <typename Next>
-__device__ __forceinline__ void step_seeded(EngineCtl* c, StepBlock* b, int bound, unsigned long long word,
-                                            bool tracing, const Next& next) {
+__device__ __forceinline__ void step_seeded(EngineCtl* c, StepBlock* b, int bound, bool worked,
+                                            unsigned long long word, bool tracing, const Next& next) {
     bound = __reduce_min_sync(0xFFFFFFFFu, bound);
     if ((threadIdx.x & 31u) == 0) {
         if (bound != kNoBound) atomicMin(&b->bound, bound);
+        if (worked) atomicOr(&b->worked, 1u);
         __threadfence_block();
         if (atomicAdd(&b->done, 1u) == (blockDim.x >> 5) - 1) {
             b->done = 0;
             __threadfence_block();
             const int m = atomicExch(&b->bound, kNoBound);
             const unsigned step = step_number(word);
+            unsigned long long r = 0;
+            if (atomicExch(&b->worked, 0u)) r = atomicMax(&c->worked, step);
+            for (int i = 0; i < 2; ++i)
+                if (const unsigned k = atomicExch(&b->count[i], 0u)) r += atomicAdd(&c->removed[i], k);
             if (tracing && step - 1 < c->trace_cap) atomicMax(&c->trace[8 * (step - 1) + 5], gtimer());
             if (m != kNoBound)
-                used_result(atomicMax(&c->next_low, ((unsigned long long)step << 32) | (unsigned long long)(kNoBound - m)));
+                r += atomicMax(&c->next_low, ((unsigned long long)step << 32) | (unsigned long long)(kNoBound - m));
+            used_result(r);
             step_finish(c, 1, word, next);
         }
     }
@@ -730,7 +745,7 @@ __device__ __forceinline__ int step_take(EngineCtl* c, TicketQueue q, StepBlock*
         unsigned spins = 0;
         while ((it >> 54) != tag) {
             if (poller) {
-                w = ld_acquire(&c->step_word);
+                w = ld_acquire(&c->step_word[blockIdx.x % kStepWords].v);
                 if ((++spins & 15u) == 0) {
                     // the limit bounds a wait without progress: while the
                     // step's other warps still push or finish items the clock
@@ -752,7 +767,7 @@ __device__ __forceinline__ int step_take(EngineCtl* c, TicketQueue q, StepBlock*
                 ++spins;
             }
             if (w != *word) break;
-            if (spins > 8) __nanosleep(poller ? 20 : spins > 128 ? 64 : 20);
+            if (!poller) __nanosleep(spins > 16 ? 200 : 100);
             it = ld_acquire(s);
         }
         if ((it >> 54) == tag) {

@@ -106,42 +106,17 @@ __device__ unsigned long long block_excl_scan64(unsigned long long x, unsigned l
     return res;
 }
 
-// Block-wide reservation for the peel's scans: every thread of the block
-// contributes nk entries to append to a list (counter *list_ctr) and ni queue
-// items; thread 0 reserves both ranges with one atomic each (the items'
-// outstanding count is raised before their slots can be filled) and every
-// thread gets its own offsets.  All threads of the block must call it.
-__device__ __forceinline__ void block_reserve(EngineCtl* c, unsigned* list_ctr, unsigned nk, unsigned ni,
-                                              unsigned* keep_off, unsigned* item_off) {
-    __shared__ unsigned s_kb, s_ib;
+// Block-wide append: threads with pred get consecutive positions of a list
+// (counter *ctr), one atomic per block.  All threads of the block call it.
+__device__ __forceinline__ unsigned block_append(unsigned* ctr, bool pred) {
+    __shared__ unsigned s_base;
     unsigned long long tot;
-    const unsigned long long ex = block_excl_scan64(((unsigned long long)nk << 32) | ni, &tot);
-    if (threadIdx.x == 0) {
-        const unsigned tk = (unsigned)(tot >> 32), ti = (unsigned)tot;
-        s_kb = tk ? atomicAdd(list_ctr, tk) : 0u;
-        s_ib = 0;
-        if (ti) {
-            atomicAdd(&c->outstanding, (int)ti);
-            s_ib = atomicAdd(&c->t_tail, ti);
-        }
-    }
+    const unsigned long long ex = block_excl_scan64(pred ? 1ull : 0ull, &tot);
+    if (threadIdx.x == 0) s_base = tot ? atomicAdd(ctr, (unsigned)tot) : 0u;
     __syncthreads();
-    *keep_off = s_kb + (unsigned)(ex >> 32);
-    *item_off = s_ib + (unsigned)ex;
+    const unsigned pos = s_base + (unsigned)ex;
     __syncthreads();
-}
-
-// Block-wide minimum, one global atomicMin per block (all threads call it).
-__device__ __forceinline__ void block_atomic_min(int* dst, int x) {
-    __shared__ int s_m;
-    if (threadIdx.x == 0) s_m = 0x7FFFFFFF;
-    __syncthreads();
-#pragma unroll
-    for (int o = 16; o; o >>= 1) x = min(x, __shfl_xor_sync(0xFFFFFFFFu, x, o));
-    if ((threadIdx.x & 31u) == 0 && x != 0x7FFFFFFF) atomicMin(&s_m, x);
-    __syncthreads();
-    if (threadIdx.x == 0 && s_m != 0x7FFFFFFF) atomicMin(dst, s_m);
-    __syncthreads();
+    return pos;
 }
 
 // ---------------------------------------------------------------------------
@@ -233,26 +208,6 @@ __global__ void k_scatter_edges(uint64_t E, const uint32_t* src, const uint32_t*
 // ---------------------------------------------------------------------------
 static constexpr int kWin = 64;
 
-// The last warp of a block to finish its seeding share reports the block as
-// one producer (outstanding counts blocks, not warps: far fewer atomics on
-// the shared counter per step).
-__device__ __forceinline__ void block_producer_done(EngineCtl* c, unsigned* s_cnt) {
-    __syncwarp();
-    if ((threadIdx.x & 31u) == 0) {
-        __threadfence();
-        unsigned o = atomicAdd(s_cnt, 1u);
-        if (o == (blockDim.x >> 5) - 1) {
-            *s_cnt = 0;
-            if (c->trace) {
-                int st = ld_vol(&c->step);
-                if (st >= 0 && (unsigned)st < c->trace_cap) atomicMax(&c->trace[8 * st + 5], gtimer());
-            }
-            tq_finish(c, 1);
-        }
-    }
-    __syncwarp();
-}
-
 // Per-vertex queue state for the transition drain: bit 0 = requested, bit 1
 // = being evaluated.  A vertex is never evaluated by two warps at once, and a
 // request that lands during an evaluation re-queues the vertex when that
@@ -260,7 +215,7 @@ __device__ __forceinline__ void block_producer_done(EngineCtl* c, unsigned* s_cn
 __device__ __forceinline__ bool mark_request(uint32_t* m) { return atomicOr(m, 1u) == 0u; }
 
 // ---------------------------------------------------------------------------
-// fused peel, ticket queue, chunked items
+// fused peel
 // ---------------------------------------------------------------------------
 struct PeelInst {
     const uint32_t* a_off;
@@ -281,249 +236,460 @@ struct PeelInst {
 struct Peel2Params {
     uint32_t V;
     int ninst;
-    unsigned chunk;  // adjacency entries per queue item
+    unsigned chunk;  // a list longer than 4 chunks is split into items of that size
     PeelInst in[2];
+    uint32_t* bag;  // [2 V] vertices handed to other warps
     TicketQueue q;
     EngineCtl* ctl;
 };
 
-__device__ __forceinline__ unsigned long long peel_item(uint32_t v, unsigned ch, int inst) {
-    return (unsigned long long)v | ((unsigned long long)ch << 32) | ((unsigned long long)inst << 63);
-}
+// Queue items: a removed vertex (piece 0: its taker queues the other pieces of
+// a long list), a further piece of a long list, or a bag of up to 32 removed
+// vertices (start in the bag array, count).
+constexpr unsigned long long kPeelInst = 1ull << 32, kPeelBag = 1ull << 33;
+constexpr int kPeelDetail = 34;  // 20 bits: piece or count
+// Vertices in a warp's stack and in the bags carry their instance in the top
+// bit (2^31 vertices would not fit the device: the scratch alone takes 88
+// bytes per vertex).
+constexpr uint32_t kPeelTop = 0x80000000u;
+constexpr int kPeelEnd = 0x7FFFFFFF;  // level: nothing remains
 
-__device__ __forceinline__ unsigned peel_nitems(const PeelInst& I, uint32_t x, unsigned CH) {
-    unsigned len = (unsigned)(I.k > 0 ? I.a_len[x] : 0) + (unsigned)I.b_len[x];
-    return (len + CH - 1) / CH;
+constexpr unsigned kPeelStack = 384;   // vertices in a warp's stack
+// 256 and 96 or 384 entries measure the same within 1 %.
+constexpr unsigned kPeelBatch = 512;   // entries a warp starts on at a time
+constexpr unsigned kPeelShare = 192;   // entries a warp keeps for itself when others wait
+
+// Entries per item of a list of len entries (piece numbers have 20 bits).
+__device__ __forceinline__ unsigned peel_unit(unsigned chunk, unsigned len) {
+    unsigned u = 4 * chunk;
+    while (len > ((unsigned long long)u << 20)) u <<= 1;
+    return u;
 }
 
 struct PeelHook {
     int ninst;
-    unsigned nworkers;
-    __device__ void operator()(EngineCtl* c) const {
-        // next level: a level whose scan found nothing to remove changed no
-        // degree, so the following levels up to the least degree kept are
-        // empty too and are skipped
-        if (c->step < 0) {
-            c->level = 0;
-        } else if (c->t_tail == c->trace_tail0) {
-            int m = 0x7FFFFFFF;
-            for (int i = 0; i < ninst; ++i)
-                if (c->rc_next[i].v) m = min(m, c->minkey[i].v);
-            c->level = max(c->level + 1, m == 0x7FFFFFFF ? c->level + 1 : m);
-        } else {
-            c->level = c->level + 1;
-        }
+    __device__ __forceinline__ int operator()(EngineCtl* c, int level, bool worked, int bound) const {
         for (int i = 0; i < ninst; ++i) {
-            c->rc_cur[i] = c->rc_next[i].v;
-            c->rc_next[i].v = 0;
-            c->minkey[i].v = 0x7FFFFFFF;
+            unsigned n = ld_vol(&c->rc_cur[i]);
+            if (ld_vol(&c->peel_compact[i])) {
+                n = ld_vol(&c->rc_next[i].v);
+                c->rc_cur[i] = n;
+                c->rc_next[i].v = 0;
+                c->peel_list[i] = ld_vol(&c->peel_list[i]) == 0 ? 1 : 0;
+                c->removed[i] = 0;
+                c->peel_compact[i] = 0;
+            } else {
+                // the list is written anew once a quarter of it is gone
+                c->peel_compact[i] = 4ull * ld_vol(&c->removed[i]) > n;
+            }
         }
-        trace_step_end(c);
-        c->t_tail = c->t_head;
-        c->trace_tail0 = c->t_tail;
-        c->outstanding = (int)nworkers;
-        c->phase_done = 0;
+        // a level whose scan found nothing to remove changed no degree: the
+        // levels up to the least degree kept are empty too
+        return worked ? level + 1 : bound == kNoBound ? kPeelEnd : max(level + 1, bound);
+    }
+};
+// Run by the last block to finish the initialisation.
+struct PeelStart {
+    int ninst;
+    uint32_t V;
+    bool member;
+    __device__ void operator()(EngineCtl* c) const {
+        for (int i = 0; i < ninst; ++i) {
+            c->rc_cur[i] = member ? c->rc_next[i].v : V;
+            c->rc_next[i].v = 0;
+            c->peel_list[i] = member ? 0 : -1;
+            c->peel_compact[i] = 1;
+        }
         __threadfence();
     }
 };
 
-// Converged warp: when the warp holds no item of its own (*keep empty), it
-// keeps the first of the items the lowest lane with *cnt > 0 is about to push
-// (*first, then *first + chunk step for the rest) to process next itself; the
-// kept item counts as outstanding like a queued one.
-__device__ __forceinline__ void keep_first_item(EngineCtl* c, unsigned long long* keep, unsigned* cnt,
-                                                unsigned long long* first) {
-    if (*keep != kEmptyItem) return;
-    const unsigned lane = threadIdx.x & 31u;
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, *cnt > 0);
-    if (!m) return;
-    const unsigned src = __ffs(m) - 1;
-    const unsigned long long it = __shfl_sync(0xFFFFFFFFu, *first, src);
-    if (lane == src) {
-        *first += 1ull << 32;  // next chunk of the same vertex
-        --*cnt;
+// One warp's part of the peel: removed vertices wait on the warp's own stack
+// in shared memory, and what it cannot hold or others can start on at once
+// goes to them through the queue.
+template <bool kBoth>
+struct PeelWarp {
+    const Peel2Params& p;
+    EngineCtl* c;
+    uint32_t* stack;
+    unsigned n;  // vertices on the stack (the same on every lane)
+    int L;
+    unsigned long long tag;
+    unsigned peeled0, peeled1;  // this warp's removals not reported yet, per peel
+    int maxv0, maxv1;           // last level with one
+
+    // nb bags of sz (<= 32) vertices each from the stack's top to the queue.
+    __device__ void spill(unsigned nb, unsigned sz) {
+        const unsigned lane = threadIdx.x & 31u, total = nb * sz;
+        unsigned at = 0;
+        if (lane == 0) at = atomicAdd(&c->bag_tail, total);
+        at = __shfl_sync(0xFFFFFFFFu, at, 0);
+        n -= total;
+        __syncwarp();
+        for (unsigned k = lane; k < total; k += 32) *(volatile uint32_t*)&p.bag[at + k] = stack[n + k];
+        __threadfence();
+        __syncwarp();
+        const unsigned base = step_reserve(c, nb);
+        for (unsigned k = lane; k < nb; k += 32)
+            step_put(p.q, base + k, (unsigned long long)(at + k * sz) | kPeelBag |
+                                        ((unsigned long long)sz << kPeelDetail) | tag);
     }
-    if (lane == 0) atomicAdd(&c->outstanding, 1);
-    *keep = it;
-}
+
+    // A vertex's lists end to end: the constraint list, if any, then the other.
+    struct List {
+        unsigned len, la;      // entries in all, entries of the constraint list
+        uint32_t aoff, boff;   // starts
+    };
+    __device__ __forceinline__ List list_of(uint32_t v, int i) const {
+        const PeelInst& I0 = p.in[0];
+        const PeelInst& I1 = p.in[1];
+        List l{0u, 0u, 0u, 0u};
+        l.len = (unsigned)__ldg((i ? I1.b_len : I0.b_len) + v);
+        l.boff = __ldg((i ? I1.b_off : I0.b_off) + v);
+        if (kBoth) {
+            l.la = (unsigned)__ldg((i ? I1.a_len : I0.a_len) + v);
+            l.aoff = __ldg((i ? I1.a_off : I0.a_off) + v);
+            l.len += l.la;
+        }
+        return l;
+    }
+
+    // Lanes with cnt > 0 hold the entries [e0, e0 + cnt) of a vertex's lists
+    // (instance i): all of them are spread over the warp's lanes, four in
+    // flight per lane; every entry takes one from its neighbour's degree.
+    __device__ void entries(const List& l, int i, unsigned e0, unsigned cnt) {
+        const unsigned lane = threadIdx.x & 31u;
+        const unsigned incl = warp_incl_scan(cnt);
+        const unsigned T = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        const PeelInst& I0 = p.in[0];
+        const PeelInst& I1 = p.in[1];
+        // entry of t: rel + t; rel and the bases may be "negative", so the sums
+        // with t are taken in 32 bits before they index anything
+        const unsigned rel = e0 - (incl - cnt);
+        const unsigned la = l.la, abase = l.aoff, bbase = l.boff + rel - la;
+        for (unsigned t0 = 0; t0 < T; t0 += 128) {
+            if (n > kPeelStack - 128) spill(4, 32);
+            uint32_t u[4];
+            int io[4], old[4];
+            bool isa[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const unsigned t = t0 + 32 * r + lane;
+                unsigned o = 0;
+#pragma unroll
+                for (unsigned s = 16; s; s >>= 1)
+                    if (__shfl_sync(0xFFFFFFFFu, incl, o + s - 1) <= t) o += s;
+                o = min(o, 31u);
+                const unsigned bb = __shfl_sync(0xFFFFFFFFu, bbase, o);
+                io[r] = __shfl_sync(0xFFFFFFFFu, i, o);
+                isa[r] = false;
+                if (kBoth) {
+                    const unsigned ab = __shfl_sync(0xFFFFFFFFu, abase, o), re = __shfl_sync(0xFFFFFFFFu, rel, o);
+                    isa[r] = re + t < __shfl_sync(0xFFFFFFFFu, la, o);
+                    if (isa[r] && t < T) u[r] = __ldg((io[r] ? I1.a_nbr : I0.a_nbr) + (ab + re + t));
+                }
+                if (!isa[r]) u[r] = t < T ? __ldg((io[r] ? I1.b_nbr : I0.b_nbr) + (bb + t)) : 0u;
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const unsigned t = t0 + 32 * r + lane;
+                old[r] = 0x80000000;
+                if (t < T)
+                    old[r] = atomicSub(isa[r] ? (io[r] ? I1.cdeg : I0.cdeg) + u[r] : (io[r] ? I1.key : I0.key) + u[r], 1);
+            }
+            bool any = false;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int lim = isa[r] ? (io[r] ? I1.k : I0.k) : L + 1;
+                old[r] = (t0 + 32 * r + lane < T && old[r] == lim) ? 1 : 0;
+                any |= old[r] != 0;
+            }
+            if (__any_sync(0xFFFFFFFFu, any)) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r)
+                    if (old[r]) old[r] = atomicCAS((io[r] ? I1.val : I0.val) + u[r], -1, L) == -1 ? 1 : 0;
+#pragma unroll
+                for (int r = 0; r < 4; ++r) take_removed(old[r] != 0, u[r], io[r]);
+            }
+        }
+    }
+
+    // Converged warp: lanes with pred add vertex v to the stack.
+    __device__ __forceinline__ void take_removed(bool pred, uint32_t v, int i) {
+        const unsigned lane = threadIdx.x & 31u;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, pred);
+        if (!m) return;
+        if (pred) stack[n + __popc(m & ((1u << lane) - 1u))] = v | (i ? kPeelTop : 0u);
+        n += __popc(m);
+        const unsigned m1 = __ballot_sync(0xFFFFFFFFu, pred && i != 0);
+        peeled0 += __popc(m & ~m1);
+        peeled1 += __popc(m1);
+        if (m & ~m1) maxv0 = L;
+        if (m1) maxv1 = L;
+    }
+
+    // Converged warp: the pieces after the first of the long lists (lanes with
+    // len > unit) go to the queue.
+    __device__ void push_pieces(uint32_t v, int i, unsigned len, unsigned unit) {
+        const unsigned lane = threadIdx.x & 31u;
+        unsigned m = __ballot_sync(0xFFFFFFFFu, len > unit);
+        while (m) {
+            const unsigned o = __ffs(m) - 1;
+            m &= m - 1u;
+            const uint32_t x = __shfl_sync(0xFFFFFFFFu, v, o);
+            const int ix = __shfl_sync(0xFFFFFFFFu, i, o);
+            const unsigned l = __shfl_sync(0xFFFFFFFFu, len, o), un = __shfl_sync(0xFFFFFFFFu, unit, o);
+            const unsigned more = (l - 1) / un;
+            const unsigned base = step_reserve(c, more);
+            for (unsigned k = lane; k < more; k += 32)
+                step_put(p.q, base + k, (unsigned long long)x | (ix ? kPeelInst : 0ull) |
+                                            ((unsigned long long)(k + 1) << kPeelDetail) | tag);
+        }
+    }
+
+    // nb vertices from the stack's top to the queue, one item each.
+    __device__ void give(unsigned nb) {
+        n -= nb;
+        const unsigned base = step_reserve(c, nb);
+        for (unsigned k = threadIdx.x & 31u; k < nb; k += 32) {
+            const uint32_t e = stack[n + k];
+            step_put(p.q, base + k, (unsigned long long)(e & ~kPeelTop) | ((e & kPeelTop) ? kPeelInst : 0ull) | tag);
+        }
+    }
+
+    // Works off the stack, 32 vertices at a time from its top (fewer when
+    // their lists are long).  What remains is shared once it is more than a
+    // moment's work and warps wait: one vertex each while they last, else
+    // bags of 32.  (Sharing by the number of vertices alone left one warp with
+    // 2.8 ms of long lists in one level of R-MAT 22.)
+    __device__ void drain() {
+        const unsigned lane = threadIdx.x & 31u;
+        while (n) {
+            __syncwarp();
+            const bool has = lane < n;
+            const uint32_t e = has ? stack[n - 1 - lane] : 0u;
+            const uint32_t v = e & ~kPeelTop;
+            const int i = e >> 31;
+            List l{0u, 0u, 0u, 0u};
+            if (has) l = list_of(v, i);
+            const unsigned unit = peel_unit(p.chunk, l.len);
+            unsigned cnt = min(l.len, unit);
+            const unsigned before = warp_incl_scan(cnt) - cnt;
+            const bool mine = has && before < kPeelBatch;
+            const unsigned m = __popc(__ballot_sync(0xFFFFFFFFu, mine));
+            const unsigned total = __shfl_sync(0xFFFFFFFFu, before + cnt, m - 1);
+            n -= m;
+            __syncwarp();
+            if (!mine) cnt = l.len = 0;
+            push_pieces(v, i, l.len, unit);
+            entries(l, i, 0u, cnt);
+            __syncwarp();
+            if (n > 1 && (unsigned long long)n * total > (unsigned long long)kPeelShare * m) {
+                const int idle = (int)(ld_vol(&c->t_head) -
+                                       (unsigned)*reinterpret_cast<volatile unsigned long long*>(&c->t_work));
+                const unsigned own = max(1u, kPeelShare * m / max(total, 1u));
+                if (idle > 0 && n > own) {
+                    const unsigned more = n - own;
+                    if (more <= 32 || (unsigned)idle >= more) give(min((unsigned)idle, more));
+                    else spill(min((unsigned)idle, more / 32), 32);
+                }
+            }
+        }
+        __syncwarp();
+    }
+
+    // A queue item.
+    __device__ void item(unsigned long long it) {
+        const unsigned lane = threadIdx.x & 31u;
+        const unsigned detail = (unsigned)(it >> kPeelDetail) & 0xFFFFFu;
+        uint32_t v = (uint32_t)it;
+        int i = (it & kPeelInst) ? 1 : 0;
+        unsigned e0 = 0, cnt = 0, unit = 1;
+        List l{0u, 0u, 0u, 0u};
+        if (it & kPeelBag) {
+            if (lane < detail) {
+                const uint32_t e = ld_vol(&p.bag[v + lane]);
+                v = e & ~kPeelTop;
+                i = e >> 31;
+                l = list_of(v, i);
+                unit = peel_unit(p.chunk, l.len);
+                cnt = min(l.len, unit);
+            }
+            push_pieces(v, i, l.len, unit);
+        } else {
+            if (lane == 0) {
+                l = list_of(v, i);
+                unit = peel_unit(p.chunk, l.len);
+                e0 = detail * unit;
+                cnt = min(unit, l.len - e0);
+            }
+            if (!detail) push_pieces(v, i, l.len, unit);
+        }
+        __syncwarp();
+        entries(l, i, e0, cnt);
+        drain();
+    }
+};
 
 // Up to two independent peels advance level by level in one grid: the kmax
 // pass (peeling in-degree, swapInOut + KListInplace(k = 0), main.cu:218-220)
 // and row 0 (peeling out-degree), or two rows of the per-row method.  Level
 // L of each peel removes every remaining vertex whose peeling degree is at
 // most L (scan, main.cu:37-56) and the cascade that follows (process,
-// main.cu:100-135) with value L.  Work items are (vertex, chunk of its
-// adjacency), so hub lists spread over many warps.
+// main.cu:100-135) with value L.
+//
+// Bound by latency in the light levels and, with one queue item per removed
+// vertex, by the queue's same-address atomics in the heavy ones (2.5 ns per
+// item, 4 M items in 14 levels of R-MAT 22).  So a removed vertex stays with
+// the warp that removed it, on a stack in shared memory; 32 of them are worked
+// off together, their lists laid end to end over the lanes with four entries
+// in flight per lane; the queue carries only the pieces of long lists and
+// vertices that waiting warps can start on.  Levels advance without a grid
+// barrier.  The remaining vertices' list is scanned once per level for both
+// peels together and written anew only when a quarter of it is gone.
+// kBoth: the instances have a constraint list too (rows k >= 1).
 #ifndef DC_PEEL_MIN_BLOCKS
 #define DC_PEEL_MIN_BLOCKS 4
 #endif
+template <bool kBoth>
 __global__ void __launch_bounds__(kThreads, DC_PEEL_MIN_BLOCKS) k_peel2(Peel2Params p) {
     const unsigned lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
     const unsigned gwarp = blockIdx.x * kWarpsPerBlock + wib;
     const unsigned nwarps = gridDim.x * kWarpsPerBlock;
     EngineCtl* c = p.ctl;
-    const unsigned CH = p.chunk;
-    PeelHook hook{p.ninst, gridDim.x};
-    __shared__ unsigned s_prod;
-    if (threadIdx.x == 0) s_prod = 0;
-    __syncthreads();
+    __shared__ uint32_t s_stack[kWarpsPerBlock][kPeelStack];
+    __shared__ StepBlock s_step;
+    const bool tracing = c->trace != nullptr;
 
-    // ---- init (remaining lists appended block by block: one atomic per block chunk)
+    // ---- init
     for (int i = 0; i < p.ninst; ++i) {
         const PeelInst& I = p.in[i];
         for (uint64_t base = (uint64_t)blockIdx.x * kThreads; base < p.V; base += (uint64_t)gridDim.x * kThreads) {
-            uint64_t vi = base + threadIdx.x;
-            bool ok = vi < p.V, in = false;
-            uint32_t v = (uint32_t)vi;
-            if (ok) {
-                in = !I.member || I.member[v] >= I.k;
-                if (!in) {
-                    I.val[v] = 0;
-                } else {
+            const uint64_t vi = base + threadIdx.x;
+            const uint32_t v = (uint32_t)vi;
+            if (!kBoth) {
+                if (vi < p.V) {
                     I.val[v] = -1;
-                    int kd = 0, cd = 0;
-                    if (!I.member) {
-                        kd = I.a_len[v];
-                    } else {
-                        uint32_t o = I.a_off[v], e = o + (uint32_t)I.a_len[v];
-                        for (; o < e; ++o) kd += (I.member[I.a_nbr[o]] >= I.k);
-                        o = I.b_off[v];
-                        e = o + (uint32_t)I.b_len[v];
-                        for (; o < e; ++o) cd += (I.member[I.b_nbr[o]] >= I.k);
-                    }
-                    I.key[v] = kd;
-                    I.cdeg[v] = cd;
+                    I.key[v] = __ldg(I.a_len + v);
                 }
+                continue;
             }
-            unsigned pos, unused;
-            block_reserve(c, &c->rc_next[i].v, (ok && in) ? 1u : 0u, 0u, &pos, &unused);
-            if (ok && in) I.rem0[pos] = v;
+            const bool in = vi < p.V && I.member[v] >= I.k;
+            if (vi < p.V && !in) I.val[v] = 0;
+            if (in) {
+                I.val[v] = -1;
+                int kd = 0, cd = 0;
+                uint32_t o = I.a_off[v], e = o + (uint32_t)I.a_len[v];
+                for (; o < e; ++o) kd += (I.member[I.a_nbr[o]] >= I.k);
+                o = I.b_off[v];
+                e = o + (uint32_t)I.b_len[v];
+                for (; o < e; ++o) cd += (I.member[I.b_nbr[o]] >= I.k);
+                I.key[v] = kd;
+                I.cdeg[v] = cd;
+            }
+            const unsigned pos = block_append(&c->rc_next[i].v, in);
+            if (in) I.rem0[pos] = v;
         }
     }
-    if (!grid_sync_hook(c, hook)) return;
+    if (!grid_sync_hook(c, PeelStart{p.ninst, p.V, kBoth})) return;
 
+    const PeelHook next{p.ninst};
+    PeelWarp<kBoth> w{p, c, s_stack[wib], 0u, 0, 0ull, 0u, 0u, 0, 0};
     unsigned ticket = kNoTicket;
-    for (int it = 0;; ++it) {
-        const int L = ld_vol(&c->level);
-        bool any_left = false;
-        for (int i = 0; i < p.ninst; ++i) any_left |= ld_vol(&c->rc_cur[i]) != 0u;
-        if (!any_left) break;
-        unsigned pushed_mask = 0;
-        // ---- scan remaining lists
-        for (int i = 0; i < p.ninst; ++i) {
-            const PeelInst& I = p.in[i];
-            const unsigned n_rem = ld_vol(&c->rc_cur[i]);
-            const uint32_t* rc = (it & 1) ? I.rem1 : I.rem0;
-            uint32_t* rn = (it & 1) ? I.rem0 : I.rem1;
-            // block-cooperative: the kept vertices and the pushed items of a
-            // chunk of blockDim vertices take one reservation per block
-            // (kSeedPer vertices per thread and step)
-            constexpr int kSeedPer = 1;  // measured: four per thread was slower (18.3 -> 19.2 ms)
-            int kmin = 0x7FFFFFFF;
-            for (unsigned base = blockIdx.x * kThreads * kSeedPer; base < n_rem;
-                 base += gridDim.x * kThreads * kSeedPer) {
-                uint32_t vv[kSeedPer];
-                unsigned cnt[kSeedPer];
-                unsigned keepm = 0, nk = 0, ni = 0;
-                bool pushed = false;
+    step_block_init(&s_step, c);
+    unsigned long long word = step_block_word(&s_step);
+    for (;;) {
+        const int L = step_level(word);
+        if (word == kStopWord || L == kPeelEnd) break;
+        if (tracing && threadIdx.x == 0) trace_wake(c, word);
+        w.L = L;
+        w.tag = step_tag(word);
+        int pending = 0;
+        int bound = kNoBound;
+        // ---- scan of the remaining vertices, both peels together
+        unsigned nr[2] = {0, 0};
+        bool compact[2] = {false, false};
+        const uint32_t* from[2] = {nullptr, nullptr};
+        uint32_t* to[2] = {nullptr, nullptr};
+        bool wrote = false;
 #pragma unroll
-                for (int r = 0; r < kSeedPer; ++r) {
-                    const unsigned idx = base + r * kThreads + threadIdx.x;
-                    const bool ok = idx < n_rem;
-                    const uint32_t v = ok ? rc[idx] : 0;
-                    bool keep = false, push = false;
-                    if (ok && ld_vol(&I.val[v]) == -1) {
-                        int kv = ld_vol(&I.key[v]);
-                        if (kv <= L) {
-                            push = atomicCAS(&I.val[v], -1, L) == -1;
-                        } else {
-                            keep = true;
-                            kmin = min(kmin, kv);
-                        }
-                    }
-                    vv[r] = v;
-                    cnt[r] = push ? peel_nitems(I, v, CH) : 0u;
-                    keepm |= keep ? 1u << r : 0u;
-                    nk += keep ? 1u : 0u;
-                    ni += cnt[r];
-                    pushed |= push;
-                }
-                unsigned kpos, ipos;
-                block_reserve(c, &c->rc_next[i].v, nk, ni, &kpos, &ipos);
-                if (ni) __threadfence();
+        for (int i = 0; i < 2; ++i) {
+            if (i >= p.ninst) continue;
+            const int l = ld_vol(&c->peel_list[i]);
+            nr[i] = ld_vol(&c->rc_cur[i]);
+            compact[i] = ld_vol(&c->peel_compact[i]) != 0;
+            from[i] = l < 0 ? nullptr : l == 0 ? p.in[i].rem0 : p.in[i].rem1;
+            to[i] = l == 0 ? p.in[i].rem1 : p.in[i].rem0;
+        }
+        const unsigned before = w.peeled0 + w.peeled1;
+        for (uint64_t base = 0; base < max(nr[0], nr[1]); base += 64ull * nwarps) {
+            uint32_t v[4];
+            int val[4], key[4];
 #pragma unroll
-                for (int r = 0; r < kSeedPer; ++r) {
-                    if (keepm & (1u << r)) rn[kpos++] = vv[r];
-                    for (unsigned j = 0; j < cnt[r]; ++j) {
-                        volatile unsigned long long* sl = &p.q.slots[(ipos++) & p.q.mask];
-                        *sl = peel_item(vv[r], j, i);
+            for (int r = 0; r < 4; ++r) {
+                const int i = r >> 1;
+                const uint64_t idx = base + (uint64_t)(r & 1) * 32u * nwarps + 32u * gwarp + lane;
+                v[r] = 0xFFFFFFFFu;
+                if (idx < nr[i]) v[r] = from[i] ? ld_vol(from[i] + idx) : (uint32_t)idx;
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const PeelInst& I = p.in[r >> 1];
+                val[r] = 0;
+                key[r] = 0;
+                if (v[r] != 0xFFFFFFFFu) {
+                    val[r] = ld_vol(&I.val[v[r]]);
+                    key[r] = ld_vol(&I.key[v[r]]);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (val[r] == -1) {
+                    if (key[r] <= L) val[r] = atomicCAS(&p.in[r >> 1].val[v[r]], -1, L) == -1 ? -2 : 0;
+                    else bound = min(bound, key[r]);
+                }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (compact[i]) {
+                    const unsigned m0 = __ballot_sync(0xFFFFFFFFu, val[2 * i] == -1);
+                    const unsigned m1 = __ballot_sync(0xFFFFFFFFu, val[2 * i + 1] == -1);
+                    if (m0 | m1) {
+                        unsigned at = 0;
+                        if (lane == 0) at = atomicAdd(&c->rc_next[i].v, (unsigned)(__popc(m0) + __popc(m1)));
+                        at = __shfl_sync(0xFFFFFFFFu, at, 0);
+                        const unsigned below = (1u << lane) - 1u;
+                        if (val[2 * i] == -1) to[i][at + __popc(m0 & below)] = v[2 * i];
+                        if (val[2 * i + 1] == -1) to[i][at + __popc(m0) + __popc(m1 & below)] = v[2 * i + 1];
+                        wrote = true;
                     }
                 }
-                if (__any_sync(0xFFFFFFFFu, pushed)) pushed_mask |= 1u << i;
+                w.take_removed(val[2 * i] == -2, v[2 * i], i);
+                w.take_removed(val[2 * i + 1] == -2, v[2 * i + 1], i);
             }
-            block_atomic_min(&c->minkey[i].v, kmin);
+            if (w.n > kPeelStack - 128) w.drain();
         }
-        block_producer_done(c, &s_prod);
-        // ---- drain the cascade: the warp's kept item first, else the queue;
-        // finished items are counted off in batches (before the warp waits)
-        unsigned long long item;
-        unsigned long long pkeep = kEmptyItem;
-        unsigned done_pending = 0;
-        for (;;) {
-            if (pkeep != kEmptyItem) {
-                item = pkeep;
-                pkeep = kEmptyItem;
-            } else if (!tq_take_warp_lazy(c, p.q, &ticket, &item, &done_pending)) {
-                break;
-            }
-            const int i = (int)(item >> 63);
-            const uint32_t x = (uint32_t)item;
-            const unsigned ch = (unsigned)((item >> 32) & 0x7FFFFFFFull);
-            const PeelInst& I = p.in[i];
-            const unsigned la = (unsigned)(I.k > 0 ? I.a_len[x] : 0);
-            const unsigned len = la + (unsigned)I.b_len[x];
-            const unsigned e0 = ch * CH, e1 = min(len, e0 + CH);
-            const uint32_t ao = I.a_off[x], bo = I.b_off[x];
-            bool pushed = false;
-            for (unsigned base = e0; base < e1; base += 64) {
-                // two entries per lane, both atomics issued before either result is used
-                unsigned ea = base + lane, eb = base + 32 + lane;
-                int olda = 0, oldb = 0;
-                uint32_t ua = 0, ub = 0;
-                bool isa_a = false, isa_b = false;
-                if (ea < e1) {
-                    isa_a = ea < la;
-                    ua = isa_a ? I.a_nbr[ao + ea] : I.b_nbr[bo + (ea - la)];
-                }
-                if (eb < e1) {
-                    isa_b = eb < la;
-                    ub = isa_b ? I.a_nbr[ao + eb] : I.b_nbr[bo + (eb - la)];
-                }
-                if (ea < e1) olda = atomicSub(isa_a ? &I.cdeg[ua] : &I.key[ua], 1);
-                if (eb < e1) oldb = atomicSub(isa_b ? &I.cdeg[ub] : &I.key[ub], 1);
-                bool pa = ea < e1 && (isa_a ? olda == I.k : olda == L + 1) && ld_vol(&I.val[ua]) == -1 &&
-                          atomicCAS(&I.val[ua], -1, L) == -1;
-                bool pb = eb < e1 && (isa_b ? oldb == I.k : oldb == L + 1) && ld_vol(&I.val[ub]) == -1 &&
-                          atomicCAS(&I.val[ub], -1, L) == -1;
-                unsigned cnta = pa ? peel_nitems(I, ua, CH) : 0u;
-                unsigned long long fa = peel_item(ua, 0, i);
-                keep_first_item(c, &pkeep, &cnta, &fa);
-                tq_push_warp_multi(c, p.q, cnta, fa, 1ull << 32);
-                unsigned cntb = pb ? peel_nitems(I, ub, CH) : 0u;
-                unsigned long long fb = peel_item(ub, 0, i);
-                keep_first_item(c, &pkeep, &cntb, &fb);
-                tq_push_warp_multi(c, p.q, cntb, fb, 1ull << 32);
-                pushed |= __any_sync(0xFFFFFFFFu, pa || pb);
-            }
-            if (pushed) pushed_mask |= 1u << i;
-            __syncwarp();
-            if (lane == 0) ++done_pending;
-        }
+        const bool worked = w.peeled0 + w.peeled1 != before;
+        w.drain();
+        // removals counted so far (those of queue items follow in a later level)
         if (lane == 0) {
-            for (int i = 0; i < p.ninst; ++i)
-                if (pushed_mask & (1u << i)) atomicMax(&c->maxv[i], L);
+            if (w.peeled0) atomicAdd(&s_step.count[0], w.peeled0);
+            if (w.peeled1) atomicAdd(&s_step.count[1], w.peeled1);
         }
-        if (!grid_sync_hook(c, hook)) return;
+        w.peeled0 = w.peeled1 = 0;
+        if (wrote) __threadfence();
+        step_seeded(c, &s_step, bound, worked, word, tracing, next);
+        // ---- the queue
+        unsigned long long item = 0;
+        int state;
+        while ((state = step_take(c, p.q, &s_step, &ticket, &item, &pending, &word, next)) == kTakeItem) {
+            w.item(item);
+            ++pending;
+        }
+        if (state == kTakeStop) break;
+    }
+    if (lane == 0) {
+        if (w.maxv0) atomicMax(&c->maxv[0], w.maxv0);
+        if (w.maxv1) atomicMax(&c->maxv[1], w.maxv1);
     }
 }
 
@@ -568,7 +734,7 @@ struct Trans2Params {
 // no work, jump to the first row whose leaving set or seed set can be
 // non-empty (the step's bound).
 struct TransHook {
-    __device__ __forceinline__ int operator()(const EngineCtl*, int row, bool worked, int bound) const {
+    __device__ __forceinline__ int operator()(EngineCtl*, int row, bool worked, int bound) const {
         return worked ? row + 1 : max(row + 1, bound);
     }
 };
@@ -1086,7 +1252,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 step_push(c, p.q, req != 0u, (unsigned long long)v | tag);
             }
         }
-        step_seeded(c, &s_step, bound, word, tracing, next);
+        step_seeded(c, &s_step, bound, false, word, tracing, next);
 
         // ---- drain: the warp's kept item first, else the queue; finished
         // items are counted off in batches (before the warp waits)
@@ -2164,11 +2330,6 @@ int persistent_enqueue(dc_graph* h, const void* fn, void** args, const char* nam
     return DC_OK;
 }
 
-// First step of a kernel whose steps advance without a barrier.
-struct FirstStep {
-    int level;
-};
-
 // Initialises a control block (on stream st) and launches a persistent
 // kernel there without waiting.  The handle's own block carries the trace.
 // first: the kernel's first step (nullptr: it starts with a grid barrier);
@@ -2188,7 +2349,7 @@ static int persistent_launch(dc_graph* h, const void* fn, void** args, const cha
     if (first) {
         init.step = 0;
         init.t_work = (unsigned long long)blocks << kWorkShift;
-        init.step_word = (1ull << 32) | (unsigned long long)(uint32_t)first->level;
+        for (auto& w : init.step_word) w.v = (1ull << 32) | (unsigned long long)(uint32_t)first->level;
     }
     if (own) {
         init.trace = h->trace_dev;
@@ -2236,8 +2397,9 @@ static int finish_persistent(dc_graph* h, EngineCtl* ctl, cudaStream_t st, const
 }
 
 // Launches a persistent kernel, waits, and converts its device status.
-int run_persistent(dc_graph* h, const void* fn, void** args, const char* name, EngineCtl* out, int bps) {
-    if (int rc = persistent_launch(h, fn, args, name, h->ctl, h->stream, bps)) return rc;
+int run_persistent(dc_graph* h, const void* fn, void** args, const char* name, EngineCtl* out, int bps,
+                   const FirstStep* first) {
+    if (int rc = persistent_launch(h, fn, args, name, h->ctl, h->stream, bps, first)) return rc;
     return finish_persistent(h, h->ctl, h->stream, name, out);
 }
 
@@ -2318,7 +2480,8 @@ int run_peel2(dc_graph* h, int ninst, const PeelInst* inst, int32_t* maxv) {
     Scratch* s = h->scratch;
     DevGraph& g = h->g;
     const unsigned chunk = h->peel_chunk ? h->peel_chunk : 64;
-    uint64_t need = 2ull * g.V + 2ull * (g.out_cap + g.in_cap) / chunk + (uint64_t)h->geom.sms * 64 + 4096;
+    // bags (at least 8 of the 2 V vertices each) and pieces of long lists
+    uint64_t need = 2ull * g.V + 2ull * (g.out_cap + g.in_cap) / (4ull * chunk) + (uint64_t)h->geom.sms * 64 + 4096;
     if (int rc = ensure_tring(h, need)) return rc;
     Peel2Params p;
     p.V = g.V;
@@ -2326,12 +2489,15 @@ int run_peel2(dc_graph* h, int ninst, const PeelInst* inst, int32_t* maxv) {
     p.chunk = chunk;
     p.in[0] = inst[0];
     p.in[1] = ninst > 1 ? inst[1] : inst[0];
+    p.bag = (uint32_t*)s->tmp64;  // V + 2 words of 8 bytes; no scan runs meanwhile
     p.q.slots = s->tring;
     p.q.mask = (unsigned)(s->tring_cap - 1);
     p.ctl = h->ctl;
     void* args[] = {&p};
     EngineCtl hc;
-    if (int rc = run_persistent(h, (const void*)k_peel2, args, "peel", &hc, h->peel_bps)) return rc;
+    const void* fn = inst[0].member ? (const void*)k_peel2<true> : (const void*)k_peel2<false>;
+    const FirstStep first{0};
+    if (int rc = run_persistent(h, fn, args, "peel", &hc, h->peel_bps, &first)) return rc;
     for (int i = 0; i < ninst; ++i) maxv[i] = hc.maxv[i];
     return DC_OK;
 }

@@ -24,6 +24,11 @@ struct RowSegment {
     cudaEvent_t ev[2] = {nullptr, nullptr};
 };
 
+// First step of a kernel whose steps advance without a barrier.
+struct FirstStep {
+    int level;
+};
+
 struct Scratch {
     uint32_t cap_V = 0;
     int32_t* key = nullptr;      // [V] peeling degree / cnt_in
@@ -182,7 +187,8 @@ int ensure_tring(dc_graph* h, uint64_t need);
 // synchronised) converted to DC_* codes.
 int check_ctl_on(EngineCtl* ctl, cudaStream_t st, EngineCtl* hc, const char* what);
 // bps: blocks per SM for this kernel (0 = the handle's blocks_per_sm, else 2).
-int run_persistent(dc_graph* h, const void* fn, void** args, const char* name, EngineCtl* out, int bps = 0);
+int run_persistent(dc_graph* h, const void* fn, void** args, const char* name, EngineCtl* out, int bps = 0,
+                   const FirstStep* first = nullptr);
 // Capture-safe forms (no host memory, no waiting): a control block reset by a
 // kernel, and a persistent launch after such a reset.
 int ctl_init_enqueue(dc_graph* h, EngineCtl* ctl, cudaStream_t st);
