@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(kThreads, DC_PEEL_MIN_BLOCKS) k_peel2(Peel2Par
 // incremental rows with exact support counters
 // ---------------------------------------------------------------------------
 struct Trans2Params {
-    uint32_t V;
+    uint32_t n;  // vertices with state: V, or |C_K0| of the relabeled graph (ids from n on are outside C_K0)
     const uint32_t* out_off;
     int32_t* out_len;
     uint32_t* out_nbr;
@@ -739,8 +739,8 @@ struct TransHook {
     }
 };
 
-// Starting values of a run of rows that starts at row a: row 0 inside C_a,
-// -1 (left) outside.
+// Starting values of a run of rows that starts at row a on the handle's own
+// graph: row 0 inside C_a, -1 (left) outside.
 __global__ void k_preleft_cur(uint32_t V, const int32_t* kmax, const int32_t* row0, int32_t a, int32_t* cur) {
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
         cur[v] = kmax[v] >= a ? row0[v] : -1;
@@ -748,36 +748,41 @@ __global__ void k_preleft_cur(uint32_t V, const int32_t* kmax, const int32_t* ro
 
 // This lane's share of #{entries u of list a[0..n) : cur[u] >= cv}, 128
 // entries per warp step; on kmax-sorted lists (sorted != 0) the count stops
-// after the step whose last entry has cur == -1 (outside C_a: so is every
-// later entry).
-__device__ __forceinline__ int count_at_least(const int32_t* cur, const uint32_t* a, int n, int cv, int sorted) {
+// after the step whose last entry is outside C_a (cur == -1, or an id from
+// `ids` on: so is every later entry).
+__device__ __forceinline__ int count_at_least(const int32_t* cur, uint32_t ids, const uint32_t* a, int n, int cv,
+                                              int sorted) {
     const unsigned lane = threadIdx.x & 31u;
     int c = 0;
     for (int b = 0; b < n; b += 128) {
+        uint32_t u[4];
         int x[4];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int e = b + 32 * r + (int)lane;
-            x[r] = e < n ? cur[a[e]] : -1;
-            c += (x[r] >= cv);
+            u[r] = e < n ? a[e] : ids;
         }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) x[r] = u[r] < ids ? cur[u[r]] : -1;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) c += (x[r] >= cv);
         if (sorted && b + 128 < n && __shfl_sync(0xFFFFFFFFu, x[3], 31) == -1) break;
     }
     return c;
 }
 
-// Counters of v against every neighbour, at v's starting value (vertices
-// with a value below 1 get zero counts: they are never evaluated and no
-// counter includes them).  On kmax-sorted lists (sorted != 0) a list ends at
-// its first neighbour outside C_a: cur holds -1 there and for every later
-// entry, which counts nothing.
-__global__ void k_counters_init(uint32_t V, const uint32_t* out_off, const int32_t* out_len, const uint32_t* out_nbr,
+// Counters of the first n vertices against every neighbour, at the vertex's
+// starting value (vertices with a value below 1 get zero counts: they are
+// never evaluated and no counter includes them).  On kmax-sorted lists
+// (sorted != 0) a list ends at its first neighbour outside C_a, which counts
+// nothing.
+__global__ void k_counters_init(uint32_t n, const uint32_t* out_off, const int32_t* out_len, const uint32_t* out_nbr,
                                 const uint32_t* in_off, const int32_t* in_len, const uint32_t* in_nbr,
                                 const int32_t* cur, int32_t* cnt_out, int32_t* cnt_in, int sorted) {
     const unsigned lane = threadIdx.x & 31u;
     const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t v = gw; v < V; v += nw) {
+    for (uint64_t v = gw; v < n; v += nw) {
         int cv = cur[v];
         int co = 0, ci = 0;
         if (cv < 1) {  // never evaluated, never counted: no support needed
@@ -787,13 +792,10 @@ __global__ void k_counters_init(uint32_t V, const uint32_t* out_off, const int32
             }
             continue;
         }
-        co = count_at_least(cur, out_nbr + out_off[v], out_len[v], cv, sorted);
-        ci = count_at_least(cur, in_nbr + in_off[v], in_len[v], cv, sorted);
-#pragma unroll
-        for (int s = 16; s; s >>= 1) {
-            co += __shfl_xor_sync(0xFFFFFFFFu, co, s);
-            ci += __shfl_xor_sync(0xFFFFFFFFu, ci, s);
-        }
+        co = count_at_least(cur, n, out_nbr + out_off[v], out_len[v], cv, sorted);
+        ci = count_at_least(cur, n, in_nbr + in_off[v], in_len[v], cv, sorted);
+        co = __reduce_add_sync(0xFFFFFFFFu, co);
+        ci = __reduce_add_sync(0xFFFFFFFFu, ci);
         if (lane == 0) {
             cnt_out[v] = co;
             cnt_in[v] = ci;
@@ -854,7 +856,7 @@ __device__ __forceinline__ int last_value(const int x[4], int b, int last) {
 // bo / bi; values above hi are not counted (the caller carries them).  On
 // kmax-sorted lists a list ends at its first neighbour outside C_j.  Returns
 // the entries read.
-__device__ __forceinline__ int hist_pass2v(const int32_t* cur, const uint32_t* onbr, uint32_t oo, int no,
+__device__ __forceinline__ int hist_pass2v(const int32_t* cur, uint32_t ids, const uint32_t* onbr, uint32_t oo, int no,
                                            const uint32_t* inbr, uint32_t io, int ni, int lo, int hi, bool sorted,
                                            int* bo, int* bi) {
     const unsigned lane = threadIdx.x & 31u;
@@ -870,8 +872,8 @@ __device__ __forceinline__ int hist_pass2v(const int32_t* cur, const uint32_t* o
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const int t = t0 + q;
-            co[q] = (!doneo && t >= so && t < endo) ? ld_vol(&cur[uo[q]]) : -1;
-            ci[q] = (!donei && t >= si && t < endi) ? ld_vol(&cur[ui[q]]) : -1;
+            co[q] = (!doneo && t >= so && t < endo && uo[q] < ids) ? ld_vol(&cur[uo[q]]) : -1;
+            ci[q] = (!donei && t >= si && t < endi && ui[q] < ids) ? ld_vol(&cur[ui[q]]) : -1;
         }
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -951,12 +953,14 @@ __device__ __forceinline__ RowLists row_lists(const Trans2Params& p, uint32_t x)
     return L;
 }
 
-// Values of the window's four entries of this lane (-1 outside the list).
-__device__ __forceinline__ void gather4(const int32_t* cur, const uint32_t u[4], int b, int start, int end,
-                                        bool active, int v[4]) {
+// Values of the window's four entries of this lane (-1 outside the list, and
+// for ids from `ids` on).
+__device__ __forceinline__ void gather4(const int32_t* cur, uint32_t ids, const uint32_t u[4], int b, int start,
+                                        int end, bool active, int v[4]) {
     const int t0 = b + 4 * (int)(threadIdx.x & 31u);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = (active && t0 + q >= start && t0 + q < end) ? ld_vol(&cur[u[q]]) : -1;
+    for (int q = 0; q < 4; ++q)
+        v[q] = (active && t0 + q >= start && t0 + q < end && u[q] < ids) ? ld_vol(&cur[u[q]]) : -1;
 }
 
 // Counts, over both lists, the neighbours at each of the kThr values cap,
@@ -980,8 +984,8 @@ __device__ __forceinline__ int count_pass(const Trans2Params& p, const RowLists&
     int entries = 0;
     for (int b = 0; ao || ai; b += 128) {
         int vo[4], vi[4];
-        gather4(p.cur, uo, b, so, endo, ao, vo);
-        gather4(p.cur, ui, b, si, endi, ai, vi);
+        gather4(p.cur, p.n, uo, b, so, endo, ao, vo);
+        gather4(p.cur, p.n, ui, b, si, endi, ai, vi);
         entries += (ao ? min(128, endo - b) : 0) + (ai ? min(128, endi - b) : 0);
         ao = ao && b + 128 < endo;
         ai = ai && b + 128 < endi;
@@ -1025,8 +1029,8 @@ __device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, co
         uo[q] = L.uo[q];
         ui[q] = L.ui[q];
     }
-    gather4(p.cur, uo, 0, so, endo, ao, vo);
-    gather4(p.cur, ui, 0, si, endi, ai, vi);
+    gather4(p.cur, p.n, uo, 0, so, endo, ao, vo);
+    gather4(p.cur, p.n, ui, 0, si, endi, ai, vi);
     load_ids4(p.out_nbr, L.oo, endo, 128, ao, no);
     load_ids4(p.in_nbr, L.io, endi, 128, ai, ni);
     for (int b = 0;; b += 128) {
@@ -1045,8 +1049,8 @@ __device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, co
             oldi[q] = (vi[q] > nv && vi[q] <= cap) ? atomicSub(&p.cnt_out[ui[q]], 1) : 0x7FFFFFFF;
         }
         int wo[4], wi[4];
-        gather4(p.cur, no, b + 128, so, endo, mo, wo);
-        gather4(p.cur, ni, b + 128, si, endi, mi, wi);
+        gather4(p.cur, p.n, no, b + 128, so, endo, mo, wo);
+        gather4(p.cur, p.n, ni, b + 128, si, endi, mi, wi);
         unsigned ro = 0, ri = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -1102,7 +1106,7 @@ __device__ __forceinline__ int window_value(const Trans2Params& p, const RowList
         hi_[lane] = 0;
         hi_[lane + 32] = 0;
         __syncwarp();
-        *entries += hist_pass2v(p.cur, p.out_nbr, L.oo, L.no, p.in_nbr, L.io, L.ni, lo, hi, p.sorted != 0, ho, hi_);
+        *entries += hist_pass2v(p.cur, p.n, p.out_nbr, L.oo, L.no, p.in_nbr, L.io, L.ni, lo, hi, p.sorted != 0, ho, hi_);
         __syncwarp();
         int b0 = 2 * lane, b1 = 2 * lane + 1;
         int o0 = ho[b0], o1 = ho[b1], i0 = hi_[b0], i1 = hi_[b1];
@@ -2102,6 +2106,8 @@ uint64_t device_footprint(const dc_graph* h) {
         b += 4ull * s->ck_cap + 12 * s->log_cap + 8 * s->tring_cap;
         b += 4 * (s->w_out_cap + s->w_in_cap);
         if (s->kmax_old) b += 8 * n;
+        for (const RowSegment& sg : s->seg)
+            b += (sg.cur ? 24 * ((uint64_t)sg.cap_V + 1) : 0) + 8 * sg.tring_cap + (sg.ctl ? sizeof(EngineCtl) : 0);
         if (s->pos) b += 4 * 7 * ((uint64_t)s->r_cap_V + 1);     // relabeled graph: ids, kmax, row 0, offsets, lengths
         if (s->r_nbr_alloc[0]) b += 2 * 4 * (s->r_cap + 7);     // its lists
     }
@@ -2403,16 +2409,23 @@ int run_persistent(dc_graph* h, const void* fn, void** args, const char* name, E
     return finish_persistent(h, h->ctl, h->stream, name, out);
 }
 
-// State of row segment i + 1 (seg[i]), sized for V vertices.
-static int ensure_segment(dc_graph* h, int i, uint32_t V) {
-    Scratch* s = h->scratch;
-    RowSegment& g = s->seg[i];
+// Stream, events and control block of row segment i + 1 (seg[i]).
+static int ensure_segment_stream(dc_graph* h, int i) {
+    RowSegment& g = h->scratch->seg[i];
     if (!g.stream) {
         DC_CUDA(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
         for (auto& e : g.ev) DC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     if (!g.ctl && dmalloc(h->stream, &g.ctl, 1)) return DC_ERR_NOMEM;
-    if (g.cap_V < V || !g.cur) {
+    return DC_OK;
+}
+
+// State of row segment i + 1 for the n vertices of its first row's core (ids
+// below n of the relabeled graph), with an eighth of headroom.
+static int ensure_segment(dc_graph* h, int i, uint32_t n) {
+    if (int rc = ensure_segment_stream(h, i)) return rc;
+    RowSegment& g = h->scratch->seg[i];
+    if (g.cap_V < n || !g.cur) {
         dfree(h->stream, g.cur);
         dfree(h->stream, g.cnt_out);
         dfree(h->stream, g.cnt_in);
@@ -2420,13 +2433,13 @@ static int ensure_segment(dc_graph* h, int i, uint32_t V) {
         dfree(h->stream, g.stamp);
         dfree(h->stream, g.logidx);
         g.cap_V = 0;
-        const uint64_t n = (uint64_t)V + 1;
-        if (dmalloc(h->stream, &g.cur, n) || dmalloc(h->stream, &g.cnt_out, n) || dmalloc(h->stream, &g.cnt_in, n) ||
-            dmalloc(h->stream, &g.mark, n) || dmalloc(h->stream, &g.stamp, n) || dmalloc(h->stream, &g.logidx, n))
+        const uint64_t m = (uint64_t)n + n / 8 + 1;
+        if (dmalloc(h->stream, &g.cur, m) || dmalloc(h->stream, &g.cnt_out, m) || dmalloc(h->stream, &g.cnt_in, m) ||
+            dmalloc(h->stream, &g.mark, m) || dmalloc(h->stream, &g.stamp, m) || dmalloc(h->stream, &g.logidx, m))
             return DC_ERR_NOMEM;
-        g.cap_V = V;
+        g.cap_V = (uint32_t)std::min<uint64_t>(m - 1, 0xFFFFFFFFull);
     }
-    uint64_t need = 2ull * V + (uint64_t)h->geom.sms * 64 + 4096, cap = 1024;
+    uint64_t need = 2ull * n + (uint64_t)h->geom.sms * 64 + 4096, cap = 1024;
     while (cap < need) cap <<= 1;
     if (g.tring_cap < cap || !g.tring) {
         dfree(h->stream, g.tring);
@@ -2438,8 +2451,8 @@ static int ensure_segment(dc_graph* h, int i, uint32_t V) {
     return DC_OK;
 }
 
-// Allocates the state of the row segments the handle's cuts ask for, so
-// that no later run of rows allocates it (maintenance batches included).
+// Creates the streams of the row segments the handle's cuts ask for (their
+// state is sized for the graph's cores by the first run that uses them).
 int prepare_row_segments(dc_graph* h) {
     const uint32_t V = h->g.V;
     if (!V) return DC_OK;
@@ -2448,8 +2461,7 @@ int prepare_row_segments(dc_graph* h) {
     if (!n) return DC_OK;
     if (int rc = ensure_scratch(h, V)) return rc;
     for (int i = 0; i < n; ++i)
-        if (int rc = ensure_segment(h, i, V)) return rc;
-    DC_CUDA(cudaStreamSynchronize(h->stream));
+        if (int rc = ensure_segment_stream(h, i)) return rc;
     return DC_OK;
 }
 
@@ -2808,20 +2820,49 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     DC_CUDA(cudaMemcpyAsync(hist, start.data(), sizeof(uint32_t) * ((size_t)K + 2), cudaMemcpyHostToDevice, h->stream));
     ++g_launches;
     k_order_scatter<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, d.kmax_v, hist, s->order);
-    // a run from row 1 (a full decomposition, or rows 1..R of a maintenance
-    // batch) may be split in row segments run concurrently: segment 0 (rows
+    // The graph the row kernel reads: where sorting is allowed, the graph
+    // relabeled in kmax order with kmax-sorted lists (C_k a prefix of the
+    // ids); else the handle's own lists (kmax-sorted when they still are from
+    // an earlier run) with C_k listed by `order`.
+    const bool relabel = allow_sort && allow_relabel && K + 1 <= kSortBigBins;
+    // a run from row 1 on the relabeled graph (a full decomposition, or rows
+    // 1..R of a maintenance batch) may be split in row segments run concurrently: segment 0 (rows
     // 1..cut[0]) on the handle's stream, segment i (rows cut[i-1]+1..cut[i],
     // starting there from row 0) on seg[i-1]'s stream, each with its own
-    // state and its own range of the corner log; runs of fewer than
-    // kMinSplitRows rows stay whole
+    // state (for the vertices of its first row's core: the ids below |C_a|)
+    // and its own range of the corner log; runs of fewer than kMinSplitRows
+    // rows stay whole
     const int32_t k0 = std::max(1, K0);
     int32_t cut[kMaxRowSegments];
     int nseg = 1;
-    if (k0 == 1 && Kstop >= kMinSplitRows)
-        for (int i = 0; i < kMaxRowSegments - 1 && h->rows_split[i] > 0; ++i) {
-            const int32_t c = (int32_t)((int64_t)K * h->rows_split[i] / 1000);
+    if (relabel && k0 == 1 && Kstop >= kMinSplitRows) {
+        int32_t split[kMaxRowSegments - 1] = {};
+        for (int i = 0; i < kMaxRowSegments - 1; ++i)
+            split[i] = (int32_t)((int64_t)K * (h->auto_cuts ? (i + 1) * 1000 / kMaxRowSegments : h->rows_split[i]) / 1000);
+        if (h->auto_cuts) {
+            // Cuts of a handle whose launch shapes were never set: equal runs
+            // of rows, where the core a run starts from is small.  A run's
+            // start costs a pass over its first core's lists and a refinement
+            // from row 0 there: with skewed degrees (|C_k| a few per cent of
+            // |C_1| at the first cut) eight runs at a time take the rows from
+            // 3.46 / 8.92 / 34.2 ms to 1.30 / 3.66 / 19.6 (R-MAT 17 / 18 / 22,
+            // the best of 13 sets of cuts 1.27 / 3.23 / 18.1); where every
+            // vertex is in almost every core (ER, 100 edges per vertex) the
+            // same cuts take them from 3.6 to 11.0 ms.  Hence a quarter of
+            // |C_1| at most for a run's core, half of it for all together
+            // (which also bounds the runs' state).
+            uint64_t sum = 0;
+            for (int i = kMaxRowSegments - 2; i >= 0; --i) {
+                const uint64_t m = split[i] >= 1 && split[i] < Kstop ? ck[split[i] + 1] : 0;
+                if (4 * m > ck[1] || 2 * (sum + m) > ck[1]) split[i] = 0;
+                else sum += m;
+            }
+        }
+        for (int i = 0; i < kMaxRowSegments - 1; ++i) {
+            const int32_t c = split[i];
             if (c >= 1 && c < Kstop && (nseg == 1 || c > cut[nseg - 2])) cut[nseg++ - 1] = c;
         }
+    }
     cut[nseg - 1] = Kstop;
     // log ranges: [off[i], off[i] + cap[i]) per segment
     uint64_t off[kMaxRowSegments] = {}, capn[kMaxRowSegments] = {};
@@ -2859,12 +2900,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
         s->log_cap = cap;
     }
     if (nseg == 1) capn[0] = s->log_cap;
-    // The graph the row kernel reads: where sorting is allowed, the graph
-    // relabeled in kmax order with kmax-sorted lists (C_k a prefix of the
-    // ids); else the handle's own lists (kmax-sorted when they still are from
-    // an earlier run) with C_k listed by `order`.
     int sorted = 0;
-    const bool relabel = allow_sort && allow_relabel && K + 1 <= kSortBigBins;
     const uint32_t *G_out_off = g.out_off, *G_in_off = g.in_off, *G_order = s->order;
     int32_t *G_out_len = g.out_len, *G_in_len = g.in_len;
     uint32_t *G_out_nbr = g.out_nbr, *G_in_nbr = g.in_nbr;
@@ -2888,20 +2924,27 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     // inside C_a with the vertices outside already left (for a = 1 those of
     // kmax 0), so the run's first step has no leaving pass
     auto start_state = [&](cudaStream_t st, int32_t a, int32_t* cur, int32_t* co, int32_t* ci, uint32_t* mark,
-                           int32_t* stamp) -> int {
+                           uint64_t n_mark, int32_t* stamp) -> int {
+        const uint32_t n = relabel ? ck[std::min(a, K + 1)] : V;
+        DC_CUDA(cudaMemsetAsync(mark, 0, sizeof(uint32_t) * n_mark, st));
+        if (!n) return DC_OK;
+        if (relabel) {
+            DC_CUDA(cudaMemcpyAsync(cur, G_row0, 4ull * n, cudaMemcpyDeviceToDevice, st));
+        } else {
+            ++g_launches;
+            k_preleft_cur<<<grid_for(h, n), kThreads, 0, st>>>(n, G_kmax, G_row0, a, cur);
+        }
         ++g_launches;
-        k_preleft_cur<<<grid_for(h, V), kThreads, 0, st>>>(V, G_kmax, G_row0, a, cur);
-        ++g_launches;
-        k_counters_init<<<grid_for(h, (uint64_t)V * 32), kThreads, 0, st>>>(
-            V, G_out_off, G_out_len, G_out_nbr, G_in_off, G_in_len, G_in_nbr, cur, co, ci, sorted);
-        DC_CUDA(cudaMemsetAsync(mark, 0, sizeof(uint32_t) * V, st));
-        DC_CUDA(cudaMemsetAsync(stamp, 0xFF, sizeof(int32_t) * V, st));
+        k_counters_init<<<grid_for(h, (uint64_t)n * 32), kThreads, 0, st>>>(
+            n, G_out_off, G_out_len, G_out_nbr, G_in_off, G_in_len, G_in_nbr, cur, co, ci, sorted);
+        DC_CUDA(cudaMemsetAsync(stamp, 0xFF, sizeof(int32_t) * n, st));
         return DC_OK;
     };
-    if (int rc = start_state(h->stream, k0, s->cur, s->cnt_out, s->key, s->mark, s->stamp)) return rc;
+    if (int rc = start_state(h->stream, k0, s->cur, s->cnt_out, s->key, s->mark, V, s->stamp))
+        return rc;  // (the marks of all V vertices: the local core update expects them clear)
     if (int rc = ensure_tring(h, 2ull * V + (uint64_t)h->geom.sms * 64 + 4096)) return rc;
     Trans2Params tp[kMaxRowSegments];
-    tp[0].V = V;
+    tp[0].n = relabel ? ck[std::min(k0, K + 1)] : V;
     tp[0].out_off = G_out_off; tp[0].out_len = G_out_len; tp[0].out_nbr = G_out_nbr;
     tp[0].in_off = G_in_off; tp[0].in_len = G_in_len; tp[0].in_nbr = G_in_nbr;
     tp[0].kmax = G_kmax;
@@ -2926,17 +2969,19 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     tp[0].q.mask = (unsigned)(s->tring_cap - 1);
     tp[0].ctl = h->ctl;
     for (int i = 1; i < nseg; ++i)
-        if (int rc = ensure_segment(h, i - 1, V)) return rc;
+        if (int rc = ensure_segment(h, i - 1, ck[cut[i - 1] + 1])) return rc;
     if (nseg > 1) {
         // the other segments start once the shared preparation is done
         DC_CUDA(cudaEventRecord(s->seg[0].ev[0], h->stream));
         for (int i = 1; i < nseg; ++i) {
             RowSegment& sg = s->seg[i - 1];
             DC_CUDA(cudaStreamWaitEvent(sg.stream, s->seg[0].ev[0], 0));
-            if (int rc = start_state(sg.stream, cut[i - 1] + 1, sg.cur, sg.cnt_out, sg.cnt_in, sg.mark, sg.stamp))
+            const uint32_t t_n = ck[cut[i - 1] + 1];
+            if (int rc = start_state(sg.stream, cut[i - 1] + 1, sg.cur, sg.cnt_out, sg.cnt_in, sg.mark, t_n, sg.stamp))
                 return rc;
             Trans2Params& t = tp[i];
             t = tp[0];
+            t.n = t_n;
             t.K0 = cut[i - 1] + 1;
             t.preleft = 1;
             t.Kstop = cut[i];

@@ -123,6 +123,7 @@ struct dc_graph {
     // full decompositions: rows cut after kmax * rows_split[i] / 1000 for
     // each nonzero entry (ascending), segments run concurrently
     int rows_split[dc::kMaxRowSegments - 1] = {};
+    bool auto_cuts = true;  // launch shapes never set: cuts by the rule in rows_from_row0
     // corner logs of the segments after the first from the last run:
     // [seg_off[i], seg_off[i] + seg_n[i]), seg_void[i] entries voided (row k < 0)
     int nseg_extra = 0;

@@ -1014,7 +1014,7 @@ static int recompute_rows(dc_graph* h, int32_t R, int32_t Knew, int32_t lmax) {
     const uint32_t V = h->g.V;
     MT_CUDA(cudaMemcpyAsync(s->row0, d.row0, 4ull * V, cudaMemcpyDeviceToDevice, h->stream));
     uint64_t nlog = 0;
-    int rc = rows_from_row0(h, Knew, R, R > 48, &nlog, 1, false);
+    int rc = rows_from_row0(h, Knew, R, R > 48, &nlog, 1);
     if (rc != DC_OK) return rc;
     // the old skyline stays readable while rows 0..R are assembled in
     // spare slot 0 and merged into spare slot 1; then the merged one is

@@ -106,6 +106,10 @@ uint64_t footprint_bound(uint64_t V, uint64_t E, uint64_t sms) {
     b += 16 * (2 * V + 2 * cap / 32 + sms * 64 + 4096);
     b += 8 * E + 2 * 4 * cap;
     b += 4 * 7 * (V + 1) + 2 * 4 * ((E + 8) + (E + 8) / 8 + 7);  // the row kernel's relabeled graph
+    // row segments: state of at most V / 2 vertices together (27 bytes each)
+    // and their ticket rings (powers of two), control blocks, the log's spare
+    // records
+    b += 30 * V + (3ull << 20);
     return b + (1ull << 20);
 }
 

@@ -431,18 +431,21 @@ int dc_set_trace(dc_graph* g, uint32_t max_steps, dc_trace_fn fn, void* user);
 int dc_set_launch(dc_graph* g, int blocks_per_sm);
 
 /* Launch shapes of the persistent kernels: blocks per SM of the fused peel
- * and of the row kernel, and adjacency entries per peel work item.  No
+ * and of the row kernel, and a quarter of the adjacency entries per peel work item.  No
  * counterpart in the reference (its launches are fixed at <<<256, 1024>>>,
  * src/common.h:32-33).  Any setting gives identical results. */
 typedef struct dc_tuning {
     int32_t peel_blocks_per_sm; /* 1..8 (capped by occupancy) */
     int32_t rows_blocks_per_sm; /* 1..8 (capped by occupancy) */
-    int32_t peel_chunk;         /* power of two, 16..4096 */
+    int32_t peel_chunk;         /* power of two, 16..4096: a list of more than four
+                                   chunks is split into items of four */
     /* Row segments of a full decomposition: each nonzero s cuts rows 1..kmax
      * after row kmax*s/1000, and the segments run as concurrent launches
      * (each one after the first starts from row 0 inside its first row's
      * core).  Nonzero entries are strictly ascending in 1..999 and precede
-     * the zeros; all zero = one launch.  Segments share the SMs: each gets
+     * the zeros; all zero = one launch.  (On a handle whose shapes were never
+     * set the engine cuts into up to eight equal runs where the cores shrink
+     * fast enough for that to pay.)  Segments share the SMs: each gets
      * at most 1/n of the row kernel's resident blocks. */
     int32_t rows_split_permille[7];
 } dc_tuning;
