@@ -97,8 +97,90 @@ __global__ void k_del_validate(uint32_t n, const uint32_t* du, const uint32_t* d
     }
 }
 
+// Deletions of a host-driven batch, in two kernels: a warp per deleted entry
+// finds it in its list (k_del_find), then a warp per list closes the holes
+// (k_del_close).  One warp per list that searched the list once per deletion
+// took 48 ms for a hub's share of 125,000 deletions (R-MAT 22).
+constexpr uint32_t kDeleted = 0xFFFFFFFFu;  // no vertex id: ids are below V
+
+// Warp per deleted entry t of the grouped deletions (gof[t] = its list's
+// vertex): claims one occurrence of gnbr[t] and leaves its position in the
+// list in pos[t].  Duplicate edges claim different occurrences.
+__global__ void k_del_find(uint32_t n, const uint32_t* gof, const uint32_t* gnbr, const uint32_t* off,
+                           const int32_t* len, uint32_t* nbr, uint32_t* pos, EngineCtl* c) {
+    const unsigned lane = threadIdx.x & 31u;
+    const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t t = gw; t < n; t += nw) {
+        const uint32_t v = gof[t], x = gnbr[t];
+        uint32_t* a = nbr + off[v];
+        const int m = len[v];
+        int at = -1;
+        for (int b = 0; b < m && at < 0; b += 128) {
+            uint32_t w[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int e = b + 32 * r + (int)lane;
+                w[r] = e < m ? ld_vol(&a[e]) : 0xFFFFFFFFu;
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                unsigned hit = __ballot_sync(0xFFFFFFFFu, w[r] == x);
+                while (hit && at < 0) {
+                    const int e = b + 32 * r + __ffs(hit) - 1;
+                    hit &= hit - 1u;
+                    unsigned got = 0;
+                    if (lane == 0) got = atomicCAS(&a[e], x, kDeleted) == x;
+                    if (__shfl_sync(0xFFFFFFFFu, got, 0)) at = e;
+                }
+            }
+        }
+        if (lane == 0) {
+            pos[t] = (uint32_t)at;
+            if (at < 0) set_dev_error(c, DC_DEV_ERR_NOTFOUND, 31);
+        }
+    }
+}
+
+// Warp per list with deletions [goff[g], goff[g+1]): the k-th hole among the
+// entries that stay takes the k-th live entry of the part that goes.  pos and
+// gnbr (the live entries) are overwritten.
+__global__ void k_del_close(uint32_t ngroups, const uint32_t* gvert, const uint32_t* goff, uint32_t* gnbr,
+                            const uint32_t* off, int32_t* len, uint32_t* nbr, uint32_t* pos, const EngineCtl* c) {
+    const bool undo = ld_vol(&c->error) != 0u;  // an entry was not found: the lists stay as they were
+    const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t g = gw; g < ngroups; g += nw) {
+        const uint32_t v = gvert[g], t0 = goff[g], m = goff[g + 1] - t0;
+        uint32_t* a = nbr + off[v];
+        if (undo) {
+            for (uint32_t k = lane; k < m; k += 32)
+                if (pos[t0 + k] != 0xFFFFFFFFu) a[pos[t0 + k]] = gnbr[t0 + k];
+            continue;
+        }
+        const uint32_t n = (uint32_t)len[v] - m;  // entries that stay
+        uint32_t holes = 0, live = 0;
+        for (uint32_t b = 0; b < m; b += 32) {
+            const uint32_t q = b + lane < m ? pos[t0 + b + lane] : n;
+            const uint32_t w = b + lane < m ? a[n + b + lane] : kDeleted;
+            const unsigned mh = __ballot_sync(0xFFFFFFFFu, q < n), ml = __ballot_sync(0xFFFFFFFFu, w != kDeleted);
+            if (q < n) pos[t0 + holes + __popc(mh & below)] = q;
+            if (w != kDeleted) gnbr[t0 + live + __popc(ml & below)] = w;
+            holes += __popc(mh);
+            live += __popc(ml);
+            __syncwarp();
+        }
+        for (uint32_t k = lane; k < holes; k += 32) a[pos[t0 + k]] = gnbr[t0 + k];
+        if (lane == 0) len[v] = (int32_t)n;
+        __syncwarp();
+    }
+}
+
 // Warp per list: removes the listed neighbours (one occurrence each, in
-// order) by swapping with the last live entry.  All deletions of one list
+// order) by swapping with the last live entry.  For captured batches (at most
+// 1,536 deletions, mostly one per list), where one kernel per side is
+// shorter than two.  All deletions of one list
 // are in one group, so no two warps touch the same list.
 // run: nullptr, or a device flag that must be nonzero for the kernel to act
 // (a captured batch skips its updates when the batch failed validation).
@@ -828,19 +910,29 @@ static int apply_deletions(dc_graph* h, const NetBatch& nb) {
         std::vector<uint32_t> gvert, goff, gnbr;
         if (side == 0) group_by(nb.del_u, nb.del_v, nb.del_n, gvert, goff, gnbr);
         else group_by(nb.del_v, nb.del_u, nb.del_n, gvert, goff, gnbr);
-        uint32_t *d_gv = nullptr, *d_go = nullptr, *d_gn = nullptr;
-        if ((rc = upload(h, &d_gv, gvert)) || (rc = upload(h, &d_go, goff)) || (rc = upload(h, &d_gn, gnbr))) {
+        std::vector<uint32_t> gof(gnbr.size());
+        for (size_t q = 0; q + 1 < goff.size(); ++q)
+            for (uint32_t t = goff[q]; t < goff[q + 1]; ++t) gof[t] = gvert[q];
+        uint32_t *d_gv = nullptr, *d_go = nullptr, *d_gn = nullptr, *d_gof = nullptr, *d_pos = nullptr;
+        auto release = [&]() {
             mt_free(h->stream, d_gv); mt_free(h->stream, d_go); mt_free(h->stream, d_gn);
+            mt_free(h->stream, d_gof); mt_free(h->stream, d_pos);
+        };
+        if ((rc = upload(h, &d_gv, gvert)) || (rc = upload(h, &d_go, goff)) || (rc = upload(h, &d_gn, gnbr)) ||
+            (rc = upload(h, &d_gof, gof)) || (rc = mt_malloc(h->stream, &d_pos, gnbr.size()))) {
+            release();
             return rc;
         }
-        ++g_launches;
-        k_del_apply<<<mgrid(h, gvert.size() * 32), kMThreads, 0, h->stream>>>(
-            (uint32_t)gvert.size(), d_gv, d_go, d_gn, side == 0 ? g.out_off : g.in_off,
-            side == 0 ? g.out_len : g.in_len, side == 0 ? g.out_nbr : g.in_nbr, h->ctl, nullptr);
+        const uint32_t* off = side == 0 ? g.out_off : g.in_off;
+        int32_t* len = side == 0 ? g.out_len : g.in_len;
+        uint32_t* nbr = side == 0 ? g.out_nbr : g.in_nbr;
+        g_launches += 2;
+        k_del_find<<<mgrid(h, gnbr.size() * 32), kMThreads, 0, h->stream>>>((uint32_t)gnbr.size(), d_gof, d_gn, off,
+                                                                            len, nbr, d_pos, h->ctl);
+        k_del_close<<<mgrid(h, gvert.size() * 32), kMThreads, 0, h->stream>>>(
+            (uint32_t)gvert.size(), d_gv, d_go, d_gn, off, len, nbr, d_pos, h->ctl);
         cudaError_t e = cudaStreamSynchronize(h->stream);
-        mt_free(h->stream, d_gv);
-        mt_free(h->stream, d_go);
-        mt_free(h->stream, d_gn);
+        release();
         if (e != cudaSuccess) return set_error(DC_ERR_CUDA, "deletion apply: %s", cudaGetErrorString(e));
     }
     rc = check_ctl(h, &hc, "dc_maintain: deletion apply");
