@@ -650,8 +650,7 @@ extern "C" int dc_set_tuning(dc_graph* h, const dc_tuning* t) {
     h->peel_chunk = (unsigned)t->peel_chunk;
     for (int i = 0; i < kCuts; ++i) h->rows_split[i] = t->rows_split_permille[i];
     h->auto_cuts = false;
-    API_CUDA(cudaSetDevice(h->device));
-    return prepare_row_segments(h);
+    return DC_OK;
 }
 
 // Smallest largest-segment cost over ncut cuts taken from the grid: best[j][i]

@@ -22,7 +22,8 @@ constexpr unsigned DC_DEV_ERR_NOTFOUND = 16u; // delete of an absent edge
 
 constexpr uint32_t kEmptySlot = 0xFFFFFFFFu;
 constexpr unsigned long long kWaitNs = 4000000000ull;  // default limit of one wait: 4 s
-constexpr int kMaxRowSegments = 8;  // concurrent launches a full run of rows may split into
+constexpr int kMaxRowSegments = 8;  // runs the rows' cuts (dc_tuning) may ask for
+constexpr int kRowGroups = 8;       // groups of blocks that work on runs of rows at the same time
 constexpr int kMinSplitRows = 32;   // runs of fewer rows are never split
 
 // A counter on a 128-byte line of its own.
@@ -614,7 +615,8 @@ __device__ __forceinline__ unsigned long long step_block_word(const StepBlock* b
 }
 
 // One thread: n producers or items of step `word` are finished; the last one
-// advances the step.  next(c, level, worked, bound): the next level.
+// advances the step.  next(c, level, worked, bound): the next level;
+// next.blocks: the blocks that work on the steps.
 template <typename Next>
 __device__ __forceinline__ void step_finish(EngineCtl* c, int n, unsigned long long word, const Next& next) {
     const unsigned long long old = atomicAdd(&c->t_work, 0ull - ((unsigned long long)n << kWorkShift));
@@ -641,7 +643,7 @@ __device__ __forceinline__ void step_finish(EngineCtl* c, int n, unsigned long l
     }
     c->step = (int)step;
     c->trace_tail0 = tail;
-    atomicAdd(&c->t_work, (unsigned long long)gridDim.x << kWorkShift);
+    atomicAdd(&c->t_work, (unsigned long long)next.blocks << kWorkShift);
     __threadfence();
     const unsigned long long w = ((unsigned long long)(step + 1) << 32) | (unsigned long long)(uint32_t)level;
 #pragma unroll

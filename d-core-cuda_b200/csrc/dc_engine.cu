@@ -268,6 +268,7 @@ __device__ __forceinline__ unsigned peel_unit(unsigned chunk, unsigned len) {
 
 struct PeelHook {
     int ninst;
+    unsigned blocks;
     __device__ __forceinline__ int operator()(EngineCtl* c, int level, bool worked, int bound) const {
         for (int i = 0; i < ninst; ++i) {
             unsigned n = ld_vol(&c->rc_cur[i]);
@@ -593,7 +594,7 @@ __global__ void __launch_bounds__(kThreads, DC_PEEL_MIN_BLOCKS) k_peel2(Peel2Par
     }
     if (!grid_sync_hook(c, PeelStart{p.ninst, p.V, kBoth})) return;
 
-    const PeelHook next{p.ninst};
+    const PeelHook next{p.ninst, gridDim.x};
     PeelWarp<kBoth> w{p, c, s_stack[wib], 0u, 0, 0ull, 0u, 0u, 0, 0};
     unsigned ticket = kNoTicket;
     step_block_init(&s_step, c);
@@ -696,8 +697,38 @@ __global__ void __launch_bounds__(kThreads, DC_PEEL_MIN_BLOCKS) k_peel2(Peel2Par
 // ---------------------------------------------------------------------------
 // incremental rows with exact support counters
 // ---------------------------------------------------------------------------
+// State of a group of blocks that works on a run of rows: the vertices of the
+// run's first core (the ids below |C_a| of the relabeled graph), or all.
+struct RowGroup {
+    int32_t* cur;
+    int32_t* cnt_out;  // #{u in N_out(v) : cur[u] >= cur[v]}  (never above the truth)
+    int32_t* cnt_in;   // #{w in N_in(v)  : cur[w] >= cur[v]}
+    uint32_t* mark;
+    int32_t* stamp;
+    uint32_t* logidx;
+    TicketQueue q;
+    EngineCtl* ctl;
+};
+
+// What the groups share (device memory).
+struct RowPlan {
+    PadW span[kRowGroups];  // (last row << 32) | current row of each group's run; 0: none
+    struct alignas(128) Own {
+        unsigned long long t_row;  // start of the current row
+        unsigned row_ns;           // what the last row took
+        int lo;                    // first row of the run to start
+        unsigned flush_n, flush_off;  // values of the finished run's last row to leave in the seam array
+        unsigned spare_n, spare_off;  // place in the seam array that an attempt to take rows over did not use
+        int from;                     // group whose values the run to start begins with (-1: row 0)
+        unsigned ready;               // the group's values belong to its run
+        unsigned readers;             // groups about to copy its values
+    } own[kRowGroups];
+    alignas(128) unsigned seam_tail;
+    alignas(128) unsigned log_count;
+    unsigned long long voids;
+};
+
 struct Trans2Params {
-    uint32_t n;  // vertices with state: V, or |C_K0| of the relabeled graph (ids from n on are outside C_K0)
     const uint32_t* out_off;
     int32_t* out_len;
     uint32_t* out_nbr;
@@ -705,37 +736,170 @@ struct Trans2Params {
     int32_t* in_len;
     uint32_t* in_nbr;
     const int32_t* kmax;
+    const int32_t* row0;
     int32_t K;
-    int32_t K0;     // first row to compute; cur holds row 0 (K0 > 1 jumps straight to row K0)
-    // preleft: cur already holds -1 for the vertices outside C_K0 and the
-    // counters ignore them, so the first row has no leaving set and seeds
-    // every member whose out-count is below its value as well (the host
-    // always starts runs this way; 0 = the leaving pass removes them)
-    int preleft;
+    int32_t K0;     // first row to compute; group 0's cur holds row 0 inside C_K0, -1 outside
     int32_t Kstop;  // last row to compute (rows above stay untouched)
+    uint32_t n;     // vertices group 0 has state for
     int sorted;     // lists ordered by neighbour kmax, descending
     const uint32_t* order;  // C_k = order[0 .. ck[k]); nullptr: the graph is relabeled, C_k = ids 0 .. ck[k]-1
     const uint32_t* ck;
-    int32_t* cur;
-    int32_t* cnt_out;  // #{u in N_out(v) : cur[u] >= cur[v]}  (never above the truth)
-    int32_t* cnt_in;   // #{w in N_in(v)  : cur[w] >= cur[v]}
-    uint32_t* mark;
-    int32_t* stamp;
-    uint32_t* logidx;
     uint32_t* log_v;
     int32_t* log_k;
     int32_t* log_l;
     unsigned long long log_cap;
-    TicketQueue q;
-    EngineCtl* ctl;
+    // groups (1: no plan, one run)
+    int n_groups;
+    unsigned first_block[kRowGroups + 1];
+    RowGroup g[kRowGroups];
+    RowPlan* plan;
+    int32_t run_min;    // least first row a run may have (its core fits the groups' state)
+    uint32_t* seam_of;  // [K + 2] 1 + place in `seam` of the values of row k - 1, where a run starts at row k
+    int32_t* seam;
+    unsigned seam_cap;
 };
 
-// Next row (run by the warp that finished the step): after a row that needed
-// no work, jump to the first row whose leaving set or seed set can be
-// non-empty (the step's bound).
-struct TransHook {
-    __device__ __forceinline__ int operator()(EngineCtl*, int row, bool worked, int bound) const {
-        return worked ? row + 1 : max(row + 1, bound);
+// Levels of the row kernel's steps other than rows.
+constexpr int kRowsEnd = 0x7FFFFFFF;  // the group leaves
+constexpr int kRowsInit = -1;         // start values of the group's next run
+constexpr int kRowsCount = -2;        // its counters
+constexpr int kRowsWait = -3;         // nothing to take over yet
+
+// Next step of a group (run by the warp that finished the step).  After a row
+// that needed no work the run jumps to the first row whose leaving set or
+// seed set can be non-empty (the step's bound).  A group whose run is over
+// takes over the upper half of what another group has left: the costs of rows
+// differ by orders of magnitude and cluster just below the values of k where
+// the core collapses, so no fixed cut balances them (eight equal runs of
+// R-MAT 22 took 0.006 to 17.8 ms each, 71 ms together).  It begins with the
+// other group's values as they are: values only fall, within a row and from
+// row to row, so any of them bounds the later row's from above (from row 0
+// the first row of such a run took up to 8 ms).
+struct RowsNext {
+    const Trans2Params& p;
+    int gid;
+    unsigned blocks;
+
+    __device__ int operator()(EngineCtl*, int level, bool worked, int bound) const {
+        const int r = worked ? level + 1 : max(level + 1, bound);
+        if (p.n_groups == 1) return r > p.Kstop ? kRowsEnd : r;
+        RowPlan* pl = p.plan;
+        RowPlan::Own& own = pl->own[gid];
+        const unsigned long long now = gtimer();
+        if (level == kRowsInit) {  // the values are copied
+            own.flush_n = 0;
+            if (own.from >= 0) used_result(atomicSub(&pl->own[own.from].readers, 1u));
+            return kRowsCount;
+        }
+        if (level == kRowsCount) {
+            own.t_row = now;
+            own.row_ns = 0;
+            __threadfence();
+            *(volatile unsigned*)&own.ready = 1u;
+            return ld_vol(&own.lo);
+        }
+        bool flush = false;
+        if (level > 0) {
+            unsigned long long s = ld_acquire(&pl->span[gid].v);
+            for (;;) {  // ends: others only shorten the run
+                const int stop = (int)(s >> 32);
+                const unsigned long long to = r > stop ? 0ull : ((unsigned long long)stop << 32) | (unsigned)r;
+                const unsigned long long o = atomicCAS(&pl->span[gid].v, s, to);
+                if (o != s) {
+                    s = o;
+                    continue;
+                }
+                if (to) {
+                    const unsigned long long t = *(volatile unsigned long long*)&own.t_row;
+                    if (t) *(volatile unsigned*)&own.row_ns = (unsigned)min(now - t, 0xFFFFFFFFull);
+                    *(volatile unsigned long long*)&own.t_row = now;
+                    return r;
+                }
+                // the run is over: the run that starts at stop + 1 needs its last row's values
+                *(volatile unsigned*)&own.ready = 0u;
+                __threadfence();
+                if (stop < p.Kstop) {
+                    own.flush_n = __ldg(p.ck + stop + 1);
+                    own.flush_off = ld_vol(p.seam_of + stop + 1) - 1u;
+                    flush = true;
+                }
+                break;
+            }
+        } else {
+            own.flush_n = 0;
+        }
+        bool any = false;
+        // (a group that others still copy from keeps its values)
+        const bool busy = ld_acquire(&own.readers) != 0u;
+        for (int attempt = 0; attempt < 4; ++attempt) {
+            int best = -1, best_start = 0;
+            unsigned long long best_s = 0, best_score = 0;
+            any = false;
+            for (int h = 0; h < p.n_groups; ++h) {
+                const unsigned long long s = h == gid ? 0ull : ld_acquire(&pl->span[h].v);
+                if (!s) continue;
+                any = true;
+                const int row = (int)(uint32_t)s, stop = (int)(s >> 32), left = stop - row;
+                const int start = max(row + 1 + left / 2, p.run_min);
+                if (left < 2 || start > stop || ld_vol(p.seam_of + start)) continue;
+                // worth it when what is left there takes longer than the start
+                // of a run (a pass over its core's lists, about 10 ns per
+                // vertex); a row takes as long as the last one or the current
+                // one so far
+                unsigned long long ns = 100000ull;
+                if (ld_vol(&pl->own[h].ready)) {
+                    const unsigned long long t = *(volatile unsigned long long*)&pl->own[h].t_row;
+                    ns = max((unsigned long long)ld_vol(&pl->own[h].row_ns), t && now > t ? now - t : 0ull);
+                }
+                const unsigned long long score = (unsigned long long)left * ns;
+                if (score > best_score && score > 40000ull + 10ull * __ldg(p.ck + start)) {
+                    best = h;
+                    best_start = start;
+                    best_s = s;
+                    best_score = score;
+                }
+            }
+            if (best < 0 || busy) break;
+            const unsigned n = __ldg(p.ck + best_start);
+            if (own.spare_n < n) {
+                if (ld_vol(&pl->seam_tail) + (unsigned long long)n > p.seam_cap) break;
+                own.spare_off = atomicAdd(&pl->seam_tail, n);
+                if (own.spare_off + (unsigned long long)n > p.seam_cap) {
+                    own.spare_n = 0;
+                    break;
+                }
+                own.spare_n = n;
+            }
+            // the seam is there, and the other group knows that its values
+            // are wanted, before its run is shortened
+            if (atomicCAS(p.seam_of + best_start, 0u, own.spare_off + 1u) != 0u) continue;
+            used_result(atomicAdd(&pl->own[best].readers, 1u));
+            __threadfence();
+            const unsigned long long stop = best_s >> 32;
+            for (int again = 0; again < 8; ++again) {  // the other group may move on meanwhile
+                const unsigned long long o = atomicCAS(
+                    &pl->span[best].v, best_s, ((unsigned long long)(best_start - 1) << 32) | (best_s & 0xFFFFFFFFull));
+                if (o == best_s) {
+                    own.from = ld_acquire(&pl->own[best].ready) ? best : -1;
+                    if (own.from < 0) used_result(atomicSub(&pl->own[best].readers, 1u));
+                    own.spare_n = 0;
+                    own.lo = best_start;
+                    *(volatile unsigned long long*)&pl->span[gid].v = (stop << 32) | (unsigned)best_start;
+                    return kRowsInit;
+                }
+                if ((o >> 32) != stop || (int)(uint32_t)o >= best_start) break;
+                best_s = o;
+            }
+            used_result(atomicExch(p.seam_of + best_start, 0u));
+            used_result(atomicSub(&pl->own[best].readers, 1u));
+        }
+        if (flush) return kRowsWait;  // leaves the values first
+        // nothing to wait for, or a group that stopped on an error
+        for (int h = 0; h < p.n_groups; ++h)
+            if (ld_vol(&p.g[h].ctl->error)) any = false;
+        if (!any) return kRowsEnd;
+        __nanosleep(10000);
+        return kRowsWait;
     }
 };
 
@@ -744,63 +908,6 @@ struct TransHook {
 __global__ void k_preleft_cur(uint32_t V, const int32_t* kmax, const int32_t* row0, int32_t a, int32_t* cur) {
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
         cur[v] = kmax[v] >= a ? row0[v] : -1;
-}
-
-// This lane's share of #{entries u of list a[0..n) : cur[u] >= cv}, 128
-// entries per warp step; on kmax-sorted lists (sorted != 0) the count stops
-// after the step whose last entry is outside C_a (cur == -1, or an id from
-// `ids` on: so is every later entry).
-__device__ __forceinline__ int count_at_least(const int32_t* cur, uint32_t ids, const uint32_t* a, int n, int cv,
-                                              int sorted) {
-    const unsigned lane = threadIdx.x & 31u;
-    int c = 0;
-    for (int b = 0; b < n; b += 128) {
-        uint32_t u[4];
-        int x[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-            const int e = b + 32 * r + (int)lane;
-            u[r] = e < n ? a[e] : ids;
-        }
-#pragma unroll
-        for (int r = 0; r < 4; ++r) x[r] = u[r] < ids ? cur[u[r]] : -1;
-#pragma unroll
-        for (int r = 0; r < 4; ++r) c += (x[r] >= cv);
-        if (sorted && b + 128 < n && __shfl_sync(0xFFFFFFFFu, x[3], 31) == -1) break;
-    }
-    return c;
-}
-
-// Counters of the first n vertices against every neighbour, at the vertex's
-// starting value (vertices with a value below 1 get zero counts: they are
-// never evaluated and no counter includes them).  On kmax-sorted lists
-// (sorted != 0) a list ends at its first neighbour outside C_a, which counts
-// nothing.
-__global__ void k_counters_init(uint32_t n, const uint32_t* out_off, const int32_t* out_len, const uint32_t* out_nbr,
-                                const uint32_t* in_off, const int32_t* in_len, const uint32_t* in_nbr,
-                                const int32_t* cur, int32_t* cnt_out, int32_t* cnt_in, int sorted) {
-    const unsigned lane = threadIdx.x & 31u;
-    const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t v = gw; v < n; v += nw) {
-        int cv = cur[v];
-        int co = 0, ci = 0;
-        if (cv < 1) {  // never evaluated, never counted: no support needed
-            if (lane == 0) {
-                cnt_out[v] = 0;
-                cnt_in[v] = 0;
-            }
-            continue;
-        }
-        co = count_at_least(cur, n, out_nbr + out_off[v], out_len[v], cv, sorted);
-        ci = count_at_least(cur, n, in_nbr + in_off[v], in_len[v], cv, sorted);
-        co = __reduce_add_sync(0xFFFFFFFFu, co);
-        ci = __reduce_add_sync(0xFFFFFFFFu, ci);
-        if (lane == 0) {
-            cnt_out[v] = co;
-            cnt_in[v] = ci;
-        }
-    }
 }
 
 // Converged warp: when the warp holds no item of its own yet (*keep ==
@@ -825,31 +932,23 @@ __device__ __forceinline__ bool keep_one(uint32_t* keep, unsigned* req, const ui
     return true;
 }
 
-// ---- vectorised list passes of the row kernel ----------------------------
-// A list is read with 16-byte id loads: the list at element offset o of its
-// array, length n, is covered by the virtual indices t in [o & 3, (o & 3) + n)
-// of the 16-byte aligned window starting at o - (o & 3); lane l takes the
-// four ids at t = b + 4 l .. b + 4 l + 3 of the step starting at b (128
-// entries per list and step), so eight neighbour values per lane (both
-// lists) are gathered in flight at once.  The adjacency arrays are 16-byte
-// aligned and padded so that the last window of the last list stays inside.
-__device__ __forceinline__ void load_ids4(const uint32_t* nbr, uint32_t o, int end, int b, bool active, uint32_t u[4]) {
-    const int t0 = b + 4 * (int)(threadIdx.x & 31u);
-    uint4 w = make_uint4(0u, 0u, 0u, 0u);
-    if (active && t0 < end) w = *reinterpret_cast<const uint4*>(nbr + (o - (o & 3u)) + t0);
-    u[0] = w.x;
-    u[1] = w.y;
-    u[2] = w.z;
-    u[3] = w.w;
+// ---- list passes of the row kernel ----------------------------------------
+// Lists are read in windows of 128 entries, four per lane (entries b + lane,
+// b + 32 + lane, ..): neighbouring lanes hold neighbouring entries, and with
+// lists in id order their values share cache lines -- in the dense cores,
+// where the work is, 32 consecutive neighbours lie in a few lines, so a
+// window's gathers and decrements take a fraction of the transactions that
+// 32 scattered ones would.  Ids past the list's end read as 0xFFFFFFFF, which
+// is outside every id range.
+__device__ __forceinline__ void load_ids4(const uint32_t* nbr, uint32_t o, int n, int b, bool active, uint32_t u[4]) {
+    const int e = b + (int)(threadIdx.x & 31u);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) u[q] = (active && e + 32 * q < n) ? __ldg(nbr + o + (uint32_t)(e + 32 * q)) : 0xFFFFFFFFu;
 }
-
-__device__ __forceinline__ int sel4(const int x[4], int q) { return q == 0 ? x[0] : q == 1 ? x[1] : q == 2 ? x[2] : x[3]; }
-
-// Value of the step's last entry (virtual index last >= b) for the early stop
-// on kmax-sorted lists.
-__device__ __forceinline__ int last_value(const int x[4], int b, int last) {
-    const int r = last - b;
-    return __shfl_sync(0xFFFFFFFFu, sel4(x, r & 3), r >> 2);
+// Values of a window's four entries of this lane (-1 for ids from `ids` on).
+__device__ __forceinline__ void gather4(const int32_t* cur, uint32_t ids, const uint32_t u[4], int v[4]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) v[q] = u[q] < ids ? ld_vol(&cur[u[q]]) : -1;
 }
 
 // Counts the neighbours at each value of [lo, hi] (both lists) into the bins
@@ -860,48 +959,30 @@ __device__ __forceinline__ int hist_pass2v(const int32_t* cur, uint32_t ids, con
                                            const uint32_t* inbr, uint32_t io, int ni, int lo, int hi, bool sorted,
                                            int* bo, int* bi) {
     const unsigned lane = threadIdx.x & 31u;
-    const int so = (int)(oo & 3u), si = (int)(io & 3u), endo = so + no, endi = si + ni;
     int to = 0, ti = 0, entries = 0;
-    bool doneo = no <= 0, donei = ni <= 0;
-    for (int b = 0; !(doneo && donei); b += 128) {
+    bool ao = no > 0, ai = ni > 0;
+    for (int b = 0; ao || ai; b += 128) {
         uint32_t uo[4], ui[4];
-        load_ids4(onbr, oo, endo, b, !doneo, uo);
-        load_ids4(inbr, io, endi, b, !donei, ui);
-        const int t0 = b + 4 * (int)lane;
-        int co[4], ci[4];
+        int vo[4], vi[4];
+        load_ids4(onbr, oo, no, b, ao, uo);
+        load_ids4(inbr, io, ni, b, ai, ui);
+        gather4(cur, ao ? ids : 0u, uo, vo);
+        gather4(cur, ai ? ids : 0u, ui, vi);
+        entries += (ao ? min(128, no - b) : 0) + (ai ? min(128, ni - b) : 0);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const int t = t0 + q;
-            co[q] = (!doneo && t >= so && t < endo && uo[q] < ids) ? ld_vol(&cur[uo[q]]) : -1;
-            ci[q] = (!donei && t >= si && t < endi && ui[q] < ids) ? ld_vol(&cur[ui[q]]) : -1;
+            to += vo[q] == hi;
+            ti += vi[q] == hi;
+            if (vo[q] >= lo && vo[q] < hi) atomicAdd(&bo[vo[q] - lo], 1);
+            if (vi[q] >= lo && vi[q] < hi) atomicAdd(&bi[vi[q] - lo], 1);
         }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            int x = co[q];
-            to += (x == hi);
-            if (x >= lo && x < hi) atomicAdd(&bo[x - lo], 1);
-            x = ci[q];
-            ti += (x == hi);
-            if (x >= lo && x < hi) atomicAdd(&bi[x - lo], 1);
-        }
-        if (!doneo) {
-            const int last = min(b + 127, endo - 1);
-            entries += last + 1 - max(b, so);
-            const int lv = last_value(co, b, last);
-            if (b + 128 >= endo || (sorted && lv == -1)) doneo = true;
-        }
-        if (!donei) {
-            const int last = min(b + 127, endi - 1);
-            entries += last + 1 - max(b, si);
-            const int lv = last_value(ci, b, last);
-            if (b + 128 >= endi || (sorted && lv == -1)) donei = true;
-        }
+        ao = ao && b + 128 < no;
+        ai = ai && b + 128 < ni;
+        if (sorted && ao && __shfl_sync(0xFFFFFFFFu, vo[3], 31) == -1) ao = false;
+        if (sorted && ai && __shfl_sync(0xFFFFFFFFu, vi[3], 31) == -1) ai = false;
     }
-#pragma unroll
-    for (int s = 16; s; s >>= 1) {
-        to += __shfl_xor_sync(0xFFFFFFFFu, to, s);
-        ti += __shfl_xor_sync(0xFFFFFFFFu, ti, s);
-    }
+    to = __reduce_add_sync(0xFFFFFFFFu, to);
+    ti = __reduce_add_sync(0xFFFFFFFFu, ti);
     if (lane == 0) {
         if (to) atomicAdd(&bo[hi - lo], to);
         if (ti) atomicAdd(&bi[hi - lo], ti);
@@ -948,30 +1029,20 @@ __device__ __forceinline__ RowLists row_lists(const Trans2Params& p, uint32_t x)
     L.io = __ldg(p.in_off + x);
     L.no = __ldg(p.out_len + x);
     L.ni = __ldg(p.in_len + x);
-    load_ids4(p.out_nbr, L.oo, (int)(L.oo & 3u) + L.no, 0, L.no > 0, L.uo);
-    load_ids4(p.in_nbr, L.io, (int)(L.io & 3u) + L.ni, 0, L.ni > 0, L.ui);
+    load_ids4(p.out_nbr, L.oo, L.no, 0, true, L.uo);
+    load_ids4(p.in_nbr, L.io, L.ni, 0, true, L.ui);
     return L;
 }
 
-// Values of the window's four entries of this lane (-1 outside the list, and
-// for ids from `ids` on).
-__device__ __forceinline__ void gather4(const int32_t* cur, uint32_t ids, const uint32_t u[4], int b, int start,
-                                        int end, bool active, int v[4]) {
-    const int t0 = b + 4 * (int)(threadIdx.x & 31u);
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-        v[q] = (active && t0 + q >= start && t0 + q < end && u[q] < ids) ? ld_vol(&cur[u[q]]) : -1;
-}
-
-// Counts, over both lists, the neighbours at each of the kThr values cap,
+// Counts, over both lists, the neighbours at each of the T values cap,
 // cap - 1, .. (a drop is rarely larger), this lane's share in go / gi.  The
 // next window's ids are in flight while a window's values are gathered, so a
 // step of 128 entries per list costs one memory latency.  Returns the entries
 // read.
 constexpr int kThr = 4;
-__device__ __forceinline__ int count_pass(const Trans2Params& p, const RowLists& L, int cap, int go[kThr],
-                                          int gi[kThr]) {
-    const int so = (int)(L.oo & 3u), si = (int)(L.io & 3u), endo = so + L.no, endi = si + L.ni;
+template <int T>
+__device__ __forceinline__ int count_pass(const Trans2Params& p, const int32_t* cur, uint32_t ids, const RowLists& L,
+                                          int cap, int go[T], int gi[T]) {
     uint32_t uo[4], ui[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -979,22 +1050,22 @@ __device__ __forceinline__ int count_pass(const Trans2Params& p, const RowLists&
         ui[q] = L.ui[q];
     }
 #pragma unroll
-    for (int r = 0; r < kThr; ++r) go[r] = gi[r] = 0;
+    for (int r = 0; r < T; ++r) go[r] = gi[r] = 0;
     bool ao = L.no > 0, ai = L.ni > 0;
     int entries = 0;
     for (int b = 0; ao || ai; b += 128) {
         int vo[4], vi[4];
-        gather4(p.cur, p.n, uo, b, so, endo, ao, vo);
-        gather4(p.cur, p.n, ui, b, si, endi, ai, vi);
-        entries += (ao ? min(128, endo - b) : 0) + (ai ? min(128, endi - b) : 0);
-        ao = ao && b + 128 < endo;
-        ai = ai && b + 128 < endi;
-        load_ids4(p.out_nbr, L.oo, endo, b + 128, ao, uo);
-        load_ids4(p.in_nbr, L.io, endi, b + 128, ai, ui);
+        gather4(cur, ao ? ids : 0u, uo, vo);
+        gather4(cur, ai ? ids : 0u, ui, vi);
+        entries += (ao ? min(128, L.no - b) : 0) + (ai ? min(128, L.ni - b) : 0);
+        ao = ao && b + 128 < L.no;
+        ai = ai && b + 128 < L.ni;
+        load_ids4(p.out_nbr, L.oo, L.no, b + 128, ao, uo);
+        load_ids4(p.in_nbr, L.io, L.ni, b + 128, ai, ui);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
 #pragma unroll
-            for (int r = 0; r < kThr; ++r) {
+            for (int r = 0; r < T; ++r) {
                 go[r] += vo[q] >= cap - r;
                 gi[r] += vi[q] >= cap - r;
             }
@@ -1003,6 +1074,29 @@ __device__ __forceinline__ int count_pass(const Trans2Params& p, const RowLists&
         if (p.sorted && ai && __shfl_sync(0xFFFFFFFFu, vi[3], 31) == -1) ai = false;
     }
     return entries;
+}
+
+// Counters of the first run's vertices against every neighbour, at the
+// vertex's starting value in group 0's cur (vertices with a value below 1 get
+// zero counts: they are never evaluated and no counter includes them).
+__global__ void k_counters_init(Trans2Params p) {
+    const unsigned lane = threadIdx.x & 31u;
+    const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    const RowGroup& G = p.g[0];
+    for (uint64_t v = gw; v < p.n; v += nw) {
+        int go[1] = {0}, gi[1] = {0};
+        const int cv = ld_vol(&G.cur[v]);
+        if (cv >= 1) {
+            count_pass<1>(p, G.cur, p.n, row_lists(p, (uint32_t)v), cv, go, gi);
+            go[0] = __reduce_add_sync(0xFFFFFFFFu, go[0]);
+            gi[0] = __reduce_add_sync(0xFFFFFFFFu, gi[0]);
+        }
+        if (lane == 0) {
+            G.cnt_out[v] = go[0];
+            G.cnt_in[v] = gi[0];
+        }
+    }
 }
 
 // One pass over both lists of x after its value fell from cap to nv: counts
@@ -1015,10 +1109,9 @@ __device__ __forceinline__ int count_pass(const Trans2Params& p, const RowLists&
 // requests kept are counted as outstanding, and *lmin bounds the next row
 // that can need work.  Returns the entries read.
 template <bool kLeave>
-__device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, const RowLists& L, int nv, int cap,
+__device__ __forceinline__ int drop_pass(const Trans2Params& p, const RowGroup& G, uint32_t ids, const RowLists& L, int nv, int cap,
                                          int j, unsigned long long word, int* cnt_o, int* cnt_i, uint32_t* keep,
                                          int* pending, int* lmin) {
-    const int so = (int)(L.oo & 3u), si = (int)(L.io & 3u), endo = so + L.no, endi = si + L.ni;
     bool ao = L.no > 0, ai = L.ni > 0;
     if (!ao && !ai) return 0;
     int entries = 0;
@@ -1029,13 +1122,13 @@ __device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, co
         uo[q] = L.uo[q];
         ui[q] = L.ui[q];
     }
-    gather4(p.cur, p.n, uo, 0, so, endo, ao, vo);
-    gather4(p.cur, p.n, ui, 0, si, endi, ai, vi);
-    load_ids4(p.out_nbr, L.oo, endo, 128, ao, no);
-    load_ids4(p.in_nbr, L.io, endi, 128, ai, ni);
+    gather4(G.cur, ids, uo, vo);
+    gather4(G.cur, ids, ui, vi);
+    load_ids4(p.out_nbr, L.oo, L.no, 128, ao, no);
+    load_ids4(p.in_nbr, L.io, L.ni, 128, ai, ni);
     for (int b = 0;; b += 128) {
-        entries += (ao ? min(128, endo - b) : 0) + (ai ? min(128, endi - b) : 0);
-        bool mo = ao && b + 128 < endo, mi = ai && b + 128 < endi;
+        entries += (ao ? min(128, L.no - b) : 0) + (ai ? min(128, L.ni - b) : 0);
+        bool mo = ao && b + 128 < L.no, mi = ai && b + 128 < L.ni;
         if (p.sorted && mo && __shfl_sync(0xFFFFFFFFu, vo[3], 31) == -1) mo = false;
         if (p.sorted && mi && __shfl_sync(0xFFFFFFFFu, vi[3], 31) == -1) mi = false;
         int oldo[4], oldi[4];
@@ -1045,12 +1138,12 @@ __device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, co
                 *cnt_o += vo[q] >= nv;
                 *cnt_i += vi[q] >= nv;
             }
-            oldo[q] = (vo[q] > nv && vo[q] <= cap) ? atomicSub(&p.cnt_in[uo[q]], 1) : 0x7FFFFFFF;
-            oldi[q] = (vi[q] > nv && vi[q] <= cap) ? atomicSub(&p.cnt_out[ui[q]], 1) : 0x7FFFFFFF;
+            oldo[q] = (vo[q] > nv && vo[q] <= cap) ? atomicSub(&G.cnt_in[uo[q]], 1) : 0x7FFFFFFF;
+            oldi[q] = (vi[q] > nv && vi[q] <= cap) ? atomicSub(&G.cnt_out[ui[q]], 1) : 0x7FFFFFFF;
         }
         int wo[4], wi[4];
-        gather4(p.cur, p.n, no, b + 128, so, endo, mo, wo);
-        gather4(p.cur, p.n, ni, b + 128, si, endi, mi, wi);
+        gather4(G.cur, mo ? ids : 0u, no, wo);
+        gather4(G.cur, mi ? ids : 0u, ni, wi);
         unsigned ro = 0, ri = 0;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
@@ -1062,8 +1155,8 @@ __device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, co
             unsigned so_[4], si_[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                so_[q] = (ro >> q) & 1u ? atomicOr(&p.mark[uo[q]], 1u) : 1u;
-                si_[q] = (ri >> q) & 1u ? atomicOr(&p.mark[ui[q]], 1u) : 1u;
+                so_[q] = (ro >> q) & 1u ? atomicOr(&G.mark[uo[q]], 1u) : 1u;
+                si_[q] = (ri >> q) & 1u ? atomicOr(&G.mark[ui[q]], 1u) : 1u;
             }
             ro = ri = 0;
 #pragma unroll
@@ -1072,10 +1165,10 @@ __device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, co
                 if (si_[q] == 0u) ri |= 1u << q;
             }
             if (keep_one(keep, &ro, uo) || keep_one(keep, &ri, ui)) {
-                if (kLeave) step_count_kept(c, word);
+                if (kLeave) step_count_kept(G.ctl, word);
                 else --*pending;  // the item being finished pays for the kept one
             }
-            step_push_mask8(c, p.q, ro, uo, ri, ui, step_tag(word));
+            step_push_mask8(G.ctl, G.q, ro, uo, ri, ui, step_tag(word));
         }
         if (!mo && !mi) break;
 #pragma unroll
@@ -1085,8 +1178,8 @@ __device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, co
             vo[q] = wo[q];
             vi[q] = wi[q];
         }
-        load_ids4(p.out_nbr, L.oo, endo, b + 256, mo, no);
-        load_ids4(p.in_nbr, L.io, endi, b + 256, mi, ni);
+        load_ids4(p.out_nbr, L.oo, L.no, b + 256, mo, no);
+        load_ids4(p.in_nbr, L.io, L.ni, b + 256, mi, ni);
         ao = mo;
         ai = mi;
     }
@@ -1096,7 +1189,7 @@ __device__ __forceinline__ int drop_pass(const Trans2Params& p, EngineCtl* c, co
 // The value of x when it fell more than kThr - 1 below cap: windows of kWin
 // values below hi, histograms in shared memory; carry_o / carry_i = counts
 // above hi.  Counts at the value found go to *c_o / *c_i.
-__device__ __forceinline__ int window_value(const Trans2Params& p, const RowLists& L, int j, int hi, int carry_o,
+__device__ __forceinline__ int window_value(const Trans2Params& p, const RowGroup& G, uint32_t ids, const RowLists& L, int j, int hi, int carry_o,
                                             int carry_i, int* ho, int* hi_, int* c_o, int* c_i, int* entries) {
     const unsigned lane = threadIdx.x & 31u;
     for (;;) {
@@ -1106,7 +1199,7 @@ __device__ __forceinline__ int window_value(const Trans2Params& p, const RowList
         hi_[lane] = 0;
         hi_[lane + 32] = 0;
         __syncwarp();
-        *entries += hist_pass2v(p.cur, p.n, p.out_nbr, L.oo, L.no, p.in_nbr, L.io, L.ni, lo, hi, p.sorted != 0, ho, hi_);
+        *entries += hist_pass2v(G.cur, ids, p.out_nbr, L.oo, L.no, p.in_nbr, L.io, L.ni, lo, hi, p.sorted != 0, ho, hi_);
         __syncwarp();
         int b0 = 2 * lane, b1 = 2 * lane + 1;
         int o0 = ho[b0], o1 = ho[b1], i0 = hi_[b0], i1 = hi_[b1];
@@ -1178,32 +1271,78 @@ static constexpr unsigned kLogChunk = 8;
 #endif
 __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans2Params p) {
     const unsigned lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
-    const unsigned gwarp = blockIdx.x * kWarpsPerBlock + wib;
-    const unsigned nwarps = gridDim.x * kWarpsPerBlock;
-    EngineCtl* c = p.ctl;
+    int gid = 0;
+    while (gid + 1 < p.n_groups && blockIdx.x >= p.first_block[gid + 1]) ++gid;
+    const unsigned block = blockIdx.x - p.first_block[gid];
+    const RowsNext next{p, gid, p.first_block[gid + 1] - p.first_block[gid]};
+    const unsigned gwarp = block * kWarpsPerBlock + wib;
+    const unsigned nwarps = next.blocks * kWarpsPerBlock;
+    const RowGroup& G = p.g[gid];
+    EngineCtl* c = G.ctl;
     __shared__ int s_ho[kWarpsPerBlock][kWin];
     __shared__ int s_hi[kWarpsPerBlock][kWin];
     __shared__ StepBlock s_step;
     const bool tracing = c->trace != nullptr;
     // failure-detection tests: this block never reports, the others' waits run out
     if (c->test_skip_block && (int)blockIdx.x == c->test_skip_block - 1) return;
-    const TransHook next;
     unsigned my_evals = 0, my_drops = 0, my_log = 0;
     unsigned long long my_entries = 0;
     unsigned ticket = kNoTicket;
+    unsigned* const log_count = p.n_groups > 1 ? &p.plan->log_count : &c->log_count;
     unsigned long long log_at = 0;  // lane 0: the records of the warp's chunk
     unsigned log_left = 0;
     step_block_init(&s_step, c);
     unsigned long long word = step_block_word(&s_step);
-    int jprev = p.preleft ? p.K0 : 0;  // row currently held in cur
-    bool seed_out = p.preleft != 0;
+    int jprev = p.K0;      // row currently held in cur
+    bool seed_out = true;  // first row of a run: members are seeded by their out-counts too
+    uint32_t ids = p.n;    // vertices with state
     for (;;) {
         const int j = step_level(word);
-        if (word == kStopWord || j > p.Kstop) break;
+        if (word == kStopWord || j == kRowsEnd) break;
         const unsigned long long tag = step_tag(word);
         if (tracing && threadIdx.x == 0) trace_wake(c, word);
         uint32_t keep = kNoKeep;
         int pending = 0;
+        if (j < 0) {
+            // between runs: the finished run's last row to the seam, then the
+            // next run's start values and counters (every value is read from
+            // row 0, a thread clears what it has copied itself)
+            const RowPlan::Own& own = p.plan->own[gid];
+            const unsigned fn = ld_vol(&own.flush_n), fo = ld_vol(&own.flush_off);
+            for (uint32_t i = block * kThreads + threadIdx.x; i < fn; i += next.blocks * kThreads)
+                p.seam[fo + i] = ld_vol(&G.cur[i]);
+            if (j == kRowsInit) {
+                jprev = ld_vol(&own.lo);
+                seed_out = true;
+                ids = __ldg(p.ck + jprev);
+                const int from = ld_vol(&own.from);
+                const int32_t* src = from < 0 ? p.row0 : p.g[from].cur;
+                for (uint32_t i = block * kThreads + threadIdx.x; i < ids; i += next.blocks * kThreads) {
+                    G.cur[i] = ld_vol(&src[i]);
+                    G.mark[i] = 0;
+                    G.stamp[i] = -1;
+                }
+            } else if (j == kRowsCount) {
+                for (uint32_t v = gwarp; v < ids; v += nwarps) {
+                    int go[1] = {0}, gi[1] = {0};
+                    const int cv = ld_vol(&G.cur[v]);
+                    if (cv >= 1) {
+                        count_pass<1>(p, G.cur, ids, row_lists(p, v), cv, go, gi);
+                        go[0] = __reduce_add_sync(0xFFFFFFFFu, go[0]);
+                        gi[0] = __reduce_add_sync(0xFFFFFFFFu, gi[0]);
+                    }
+                    if (lane == 0) {
+                        G.cnt_out[v] = go[0];
+                        G.cnt_in[v] = gi[0];
+                    }
+                }
+            }
+            __threadfence();
+            step_seeded(c, &s_step, kNoBound, false, word, tracing, next);
+            unsigned long long none;
+            if (step_take(c, G.q, &s_step, &ticket, &none, &pending, &word, next) == kTakeStop) break;
+            continue;
+        }
         // rows jprev+1 .. j-1 equal row jprev; vertices with kmax in
         // [jprev, j-1] leave now (all but those with kmax == j-1 have value 0)
         const uint32_t vj = __ldg(p.ck + j), vprev = __ldg(p.ck + jprev);
@@ -1218,8 +1357,8 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
             int al = 0;
             if (lane < share && i < vprev) {
                 xl = p.order ? __ldg(p.order + i) : i;
-                al = ld_vol(&p.cur[xl]);
-                *(volatile int32_t*)&p.cur[xl] = -1;
+                al = ld_vol(&G.cur[xl]);
+                *(volatile int32_t*)&G.cur[xl] = -1;
             }
             unsigned m = __ballot_sync(0xFFFFFFFFu, al >= 1);
             if (!m) continue;
@@ -1230,7 +1369,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 const RowLists cur_l = L;
                 m &= m - 1u;
                 if (m) L = row_lists(p, __shfl_sync(0xFFFFFFFFu, xl, __ffs(m) - 1));
-                drop_pass<true>(p, c, cur_l, 0, a, j, word, nullptr, nullptr, &keep, &pending, &bound);
+                drop_pass<true>(p, G, ids, cur_l, 0, a, j, word, nullptr, nullptr, &keep, &pending, &bound);
             }
         }
         // ---- seeds: members whose in-count at their own level is below j;
@@ -1242,18 +1381,18 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
             uint32_t v = 0;
             if (i < vj) {
                 v = p.order ? __ldg(p.order + i) : i;
-                const int cv = ld_vol(&p.cur[v]), ci = ld_vol(&p.cnt_in[v]);
-                const int co = seed_out ? ld_vol(&p.cnt_out[v]) : 0x7FFFFFFF;
+                const int cv = ld_vol(&G.cur[v]), ci = ld_vol(&G.cnt_in[v]);
+                const int co = seed_out ? ld_vol(&G.cnt_out[v]) : 0x7FFFFFFF;
                 const int km = __ldg(p.kmax + v);
                 if (cv >= 1) {
-                    if (ci < j || co < cv) req = mark_request(&p.mark[v]) ? 1u : 0u;
+                    if (ci < j || co < cv) req = mark_request(&G.mark[v]) ? 1u : 0u;
                     else bound = min(bound, min(ci, km) + 1);
                 }
             }
             if (__any_sync(0xFFFFFFFFu, req != 0u)) {
                 const uint32_t u[4] = {v, 0u, 0u, 0u};
                 if (keep_one(&keep, &req, u)) step_count_kept(c, word);
-                step_push(c, p.q, req != 0u, (unsigned long long)v | tag);
+                step_push(c, G.q, req != 0u, (unsigned long long)v | tag);
             }
         }
         step_seeded(c, &s_step, bound, false, word, tracing, next);
@@ -1268,7 +1407,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 x = keep;
                 keep = kNoKeep;
             } else {
-                state = step_take(c, p.q, &s_step, &ticket, &item, &pending, &word, next);
+                state = step_take(c, G.q, &s_step, &ticket, &item, &pending, &word, next);
                 if (state != kTakeItem) break;
                 x = (uint32_t)item;
             }
@@ -1278,17 +1417,17 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
             // between the counter snapshot and the mark only makes the counter
             // too low, which costs an evaluation
             unsigned mk = 0;
-            if (lane == 0) mk = atomicExch(&p.mark[x], 2u);
-            const int cap = ld_vol(&p.cur[x]);
-            const int s0o = ld_vol(&p.cnt_out[x]), s0i = ld_vol(&p.cnt_in[x]);
-            const int stamp = ld_vol(&p.stamp[x]);
-            const uint32_t logidx = ld_vol(&p.logidx[x]);
+            if (lane == 0) mk = atomicExch(&G.mark[x], 2u);
+            const int cap = ld_vol(&G.cur[x]);
+            const int s0o = ld_vol(&G.cnt_out[x]), s0i = ld_vol(&G.cnt_in[x]);
+            const int stamp = ld_vol(&G.stamp[x]);
+            const uint32_t logidx = ld_vol(&G.logidx[x]);
             const int km = __ldg(p.kmax + x);
             const RowLists L = row_lists(p, x);
-            if (lane == 0) used_result(mk, ld_acquire(&p.mark[x]));
+            if (lane == 0) used_result(mk, ld_acquire(&G.mark[x]));
             __syncwarp();
             if (km < j || cap < 1) {
-                if (lane == 0) atomicExch(&p.mark[x], 0u);
+                if (lane == 0) atomicExch(&G.mark[x], 0u);
                 ++pending;
                 continue;
             }
@@ -1296,7 +1435,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
             int c_o = 0, c_i = 0, nv = -1, entries;
             {
                 int go[kThr], gi[kThr];
-                entries = count_pass(p, L, cap, go, gi);
+                entries = count_pass<kThr>(p, G.cur, ids, L, cap, go, gi);
 #pragma unroll
                 for (int r = 0; r < kThr; ++r) {
                     go[r] = __reduce_add_sync(0xFFFFFFFFu, go[r]);
@@ -1311,7 +1450,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                     }
                 if (nv < 0) {
                     if (cap >= kThr) {
-                        nv = window_value(p, L, j, cap - kThr, go[kThr - 1], gi[kThr - 1], s_ho[wib], s_hi[wib], &c_o,
+                        nv = window_value(p, G, ids, L, j, cap - kThr, go[kThr - 1], gi[kThr - 1], s_ho[wib], s_hi[wib], &c_o,
                                           &c_i, &entries);
                     } else {  // unreachable for members of C_j
                         nv = 0;
@@ -1327,7 +1466,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                     const bool fresh = stamp != j;
                     if (fresh) {
                         if (!log_left) {
-                            log_at = atomicAdd(&c->log_count, kLogChunk);
+                            log_at = atomicAdd(log_count, kLogChunk);
                             log_left = kLogChunk;
                         }
                         li = log_at++;
@@ -1336,8 +1475,8 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                     }
                     if (li < p.log_cap) {
                         if (fresh) {
-                            p.stamp[x] = j;
-                            p.logidx[x] = (uint32_t)li;
+                            G.stamp[x] = j;
+                            G.logidx[x] = (uint32_t)li;
                             p.log_v[li] = x;
                             p.log_k[li] = j;
                         }
@@ -1345,7 +1484,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                     } else {
                         set_dev_error(c, DC_DEV_ERR_CAPACITY, 20);
                     }
-                    *(volatile int32_t*)&p.cur[x] = nv;
+                    *(volatile int32_t*)&G.cur[x] = nv;
                 }
                 __syncwarp();
                 __threadfence();
@@ -1354,7 +1493,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 // hold x in cnt_in, in-neighbours in cnt_out
                 c_o = 0;
                 c_i = 0;
-                entries += drop_pass<false>(p, c, L, nv, cap, j, word, &c_o, &c_i, &keep, &pending, nullptr);
+                entries += drop_pass<false>(p, G, ids, L, nv, cap, j, word, &c_o, &c_i, &keep, &pending, nullptr);
                 c_o = __reduce_add_sync(0xFFFFFFFFu, c_o);
                 c_i = __reduce_add_sync(0xFFFFFFFFu, c_i);
             }
@@ -1363,13 +1502,13 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 atomicMax(&c->trace[8 * (step_number(word) - 1) + 7], (unsigned long long)entries);
             unsigned again = 0;
             if (lane == 0) {
-                const int no = atomicAdd(&p.cnt_out[x], c_o - s0o) + (c_o - s0o);
-                const int ni = atomicAdd(&p.cnt_in[x], c_i - s0i) + (c_i - s0i);
+                const int no = atomicAdd(&G.cnt_out[x], c_o - s0o) + (c_o - s0o);
+                const int ni = atomicAdd(&G.cnt_in[x], c_i - s0i) + (c_i - s0i);
                 const bool stable = nv < 1 || (no >= nv && ni >= j);
                 // released once the counters are; requested meanwhile or
                 // unstable: evaluated again
-                if (!stable || atomicCAS(&p.mark[x], 2u, 0u) == 3u) {
-                    used_result(atomicExch(&p.mark[x], 1u));
+                if (!stable || atomicCAS(&G.mark[x], 2u, 0u) == 3u) {
+                    used_result(atomicExch(&G.mark[x], 1u));
                     again = 1u;
                 }
             }
@@ -1378,7 +1517,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                     keep = x;  // at once: still the item being finished
                     continue;
                 }
-                step_push(c, p.q, lane == 0, (unsigned long long)x | tag);
+                step_push(c, G.q, lane == 0, (unsigned long long)x | tag);
             }
             ++pending;
         }
@@ -1398,36 +1537,31 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
 }
 
 // ---------------------------------------------------------------------------
-// adjacency lists ordered by neighbour kmax, descending
+// lists of the relabeled graph, in id order
 // ---------------------------------------------------------------------------
-// With every list in this order, the neighbours inside C_j = {kmax >= j}
-// form a prefix of the list, so row-to-row evaluations read only that
-// prefix.  Short lists: one thread, insertion sort.  Medium lists: one block,
-// bitonic sort of (kmax, id) pairs in shared memory.  Long lists: one block,
-// counting sort by kmax through a scratch copy of the list.
+// New ids are positions in kmax-descending order, so a list in id order has
+// the neighbours inside C_j = {kmax >= j} as a prefix for every j (row
+// evaluations read only that) and close neighbours side by side (their values
+// share cache lines).  List i is copied from list order[i] of the handle's
+// graph with every entry renamed by pos.
 static constexpr int kSortShort = 32;
 static constexpr int kSortWarp = 256;
 static constexpr int kSortMid = 4096;
+static constexpr int kSortThreads = 256;
 
-// Where the entries of list i come from: the list itself (sorted in place),
-// or, when the relabeled graph is built, list order[i] of the handle's graph
-// with every entry renamed by pos (copy, rename and sort in one pass).
 struct ListSrc {
     const uint32_t* off;
     const uint32_t* nbr;
-    const uint32_t* order;  // nullptr: in place
+    const uint32_t* order;
     const uint32_t* pos;
 };
-__device__ __forceinline__ const uint32_t* src_list(const ListSrc& s, uint32_t i, const uint32_t* own) {
-    return s.order ? s.nbr + s.off[s.order[i]] : own;
-}
-__device__ __forceinline__ uint32_t src_id(const ListSrc& s, uint32_t u) { return s.order ? s.pos[u] : u; }
+__device__ __forceinline__ const uint32_t* src_list(const ListSrc& s, uint32_t i) { return s.nbr + s.off[s.order[i]]; }
 
 // Lists of at most kSortShort entries are sorted here, one thread each;
 // longer ones are listed for the warp sort (up to kSortWarp), the block
 // sort (up to kSortMid) or the counting sort.
-__global__ void k_sort_short(uint32_t V, const uint32_t* off, const int32_t* len, uint32_t* nbr, const int32_t* kmax,
-                             uint32_t* warp_list, uint32_t* mid_list, uint32_t* big_list, unsigned* cnt, ListSrc src) {
+__global__ void k_sort_short(uint32_t V, const uint32_t* off, const int32_t* len, uint32_t* nbr, uint32_t* warp_list,
+                             uint32_t* mid_list, uint32_t* big_list, unsigned* cnt, ListSrc src) {
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
         int n = len[v];
         if (n > kSortMid) {
@@ -1442,177 +1576,151 @@ __global__ void k_sort_short(uint32_t V, const uint32_t* off, const int32_t* len
             warp_list[atomicAdd(&cnt[0], 1u)] = (uint32_t)v;
             continue;
         }
+        if (n < 1) continue;
         uint32_t* a = nbr + off[v];
-        const uint32_t* in = src_list(src, (uint32_t)v, a);
-        if (n < 2) {
-            if (n == 1 && src.order) a[0] = src_id(src, in[0]);
-            continue;
-        }
+        const uint32_t* in = src_list(src, (uint32_t)v);
         uint32_t ids[kSortShort];
-        int ks[kSortShort];
-        for (int i = 0; i < n; ++i) {
-            ids[i] = src_id(src, in[i]);
-            ks[i] = kmax[ids[i]];
-        }
+        for (int i = 0; i < n; ++i) ids[i] = src.pos[in[i]];
         for (int i = 1; i < n; ++i) {
-            uint32_t x = ids[i];
-            int kx = ks[i];
+            const uint32_t x = ids[i];
             int jj = i - 1;
-            while (jj >= 0 && ks[jj] < kx) {
+            while (jj >= 0 && ids[jj] > x) {
                 ids[jj + 1] = ids[jj];
-                ks[jj + 1] = ks[jj];
                 --jj;
             }
             ids[jj + 1] = x;
-            ks[jj + 1] = kx;
         }
         for (int i = 0; i < n; ++i) a[i] = ids[i];
     }
 }
 
-// One warp per list of kSortShort+1 .. kSortWarp entries: the list and its
-// neighbours' kmax go to the warp's shared buffer, every entry's place is its
-// rank (entries with a larger kmax, or an equal kmax and a smaller index, go
-// before it), and the entries are written back at their places.  The list
-// count is read on the device (no host round trip).
-constexpr int kSortWarpThreads = 256;
-// Lane-strided entries i = lane + 32 t, t < T: rank among the n staged
-// entries, written to a[rank].  Staged keys are (kmax << 8) | (255 - index),
-// all distinct, so the rank (kmax descending, index ascending on ties) is the
-// number of larger keys.
+// One warp per list of kSortShort+1 .. 32 T entries: bitonic sort in
+// registers (entry 32 t + lane in k[t]; the places past the end hold the
+// largest value and stay last).  240 shuffles for 256 entries, where ranking
+// every entry against every other took 2,048 comparisons per lane.
 template <int T>
-__device__ __forceinline__ void warp_rank_place(const uint32_t* ids, const uint32_t* ks, int n, uint32_t* a) {
+__device__ __forceinline__ void warp_sort(const uint32_t* in, const uint32_t* pos, int n, uint32_t* a) {
     const unsigned lane = threadIdx.x & 31u;
-    uint32_t mk[T];
-    int rank[T];
+    uint32_t k[T];
 #pragma unroll
-    for (int t = 0; t < T; ++t) {
-        const int i = (int)lane + 32 * t;
-        mk[t] = i < n ? ks[i] : 0xFFFFFFFFu;
-        rank[t] = 0;
-    }
-    for (int j = 0; j < n; ++j) {
-        const uint32_t kj = ks[j];
+    for (int t = 0; t < T; ++t) k[t] = 32 * t + (int)lane < n ? in[32 * t + lane] : 0xFFFFFFFFu;
 #pragma unroll
-        for (int t = 0; t < T; ++t) rank[t] += kj > mk[t];
+    for (int t = 0; t < T; ++t)
+        if (32 * t + (int)lane < n) k[t] = pos[k[t]];
+#pragma unroll
+    for (int size = 2; size <= 32 * T; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride; stride >>= 1) {
+#pragma unroll
+            for (int t = 0; t < T; ++t) {
+                if (stride >= 32) {
+                    const int o = t ^ (stride >> 5);
+                    if (o > t) {
+                        const bool up = ((32 * t) & size) == 0;  // size > 32 here
+                        const uint32_t lo = min(k[t], k[o]), hi = max(k[t], k[o]);
+                        k[t] = up ? lo : hi;
+                        k[o] = up ? hi : lo;
+                    }
+                } else {
+                    const bool up = ((32 * t + (int)lane) & size) == 0;
+                    const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, k[t], stride);
+                    k[t] = ((lane & stride) == 0) == up ? min(k[t], o) : max(k[t], o);
+                }
+            }
+        }
     }
 #pragma unroll
-    for (int t = 0; t < T; ++t) {
-        const int i = (int)lane + 32 * t;
-        if (i < n) a[rank[t]] = ids[i];
-    }
+    for (int t = 0; t < T; ++t)
+        if (32 * t + (int)lane < n) a[32 * t + lane] = k[t];
 }
-__global__ void __launch_bounds__(kSortWarpThreads) k_sort_warp(const uint32_t* off, const int32_t* len,
-                                                                 uint32_t* nbr, const int32_t* kmax,
-                                                                 const uint32_t* list, const unsigned* n_list,
-                                                                 ListSrc src) {
-    constexpr int kW = kSortWarpThreads / 32;
-    static_assert(kSortWarp <= 256, "index part of the staged keys is 8 bits");
-    __shared__ uint32_t s_id[kW][kSortWarp];
-    __shared__ uint32_t s_k[kW][kSortWarp];
-    const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-    const unsigned nl = *n_list;
-    for (unsigned li = blockIdx.x * kW + w; li < nl; li += gridDim.x * kW) {
+__global__ void __launch_bounds__(kSortThreads) k_sort_warp(const uint32_t* off, const int32_t* len, uint32_t* nbr,
+                                                             const uint32_t* list, const unsigned* n_list,
+                                                             ListSrc src) {
+    static_assert(kSortWarp == 256, "eight entries per lane");
+    const unsigned nl = *n_list, nw = gridDim.x * (kSortThreads / 32);
+    for (unsigned li = blockIdx.x * (kSortThreads / 32) + (threadIdx.x >> 5); li < nl; li += nw) {
         const uint32_t v = list[li];
         const int n = len[v];
         uint32_t* a = nbr + off[v];
-        const uint32_t* in = src_list(src, v, a);
-        for (int i = lane; i < n; i += 32) {
-            const uint32_t u = src_id(src, in[i]);
-            s_id[w][i] = u;
-            s_k[w][i] = ((uint32_t)kmax[u] << 8) | (uint32_t)(255 - i);
-        }
-        __syncwarp();
-        switch ((n + 31) >> 5) {  // chunks of 32 entries (uniform over the warp)
-            case 1: warp_rank_place<1>(s_id[w], s_k[w], n, a); break;
-            case 2: warp_rank_place<2>(s_id[w], s_k[w], n, a); break;
-            case 3: warp_rank_place<3>(s_id[w], s_k[w], n, a); break;
-            case 4: warp_rank_place<4>(s_id[w], s_k[w], n, a); break;
-            case 5: warp_rank_place<5>(s_id[w], s_k[w], n, a); break;
-            case 6: warp_rank_place<6>(s_id[w], s_k[w], n, a); break;
-            case 7: warp_rank_place<7>(s_id[w], s_k[w], n, a); break;
-            default: warp_rank_place<8>(s_id[w], s_k[w], n, a); break;
-        }
-        __syncwarp();
+        const uint32_t* in = src_list(src, v);
+        if (n <= 64) warp_sort<2>(in, src.pos, n, a);
+        else if (n <= 128) warp_sort<4>(in, src.pos, n, a);
+        else warp_sort<8>(in, src.pos, n, a);
     }
 }
 
-// One block per list of kSortWarp+1 .. kSortMid entries: a counting sort by
-// neighbour kmax in shared memory (K + 1 bins, the list staged in shared
-// memory), written back in place.  Entries of equal kmax keep no particular
-// order; only the kmax order matters to the readers.  Dynamic shared memory:
-// 4 (K + 1) + 8 kSortMid bytes.
-__global__ void k_sort_mid(const uint32_t* off, const int32_t* len, uint32_t* nbr, const int32_t* kmax, int K,
-                           const uint32_t* list, unsigned n_list, ListSrc src) {
-    extern __shared__ unsigned s_mid[];
-    unsigned* bins = s_mid;                   // K + 1
-    uint32_t* ids = s_mid + (K + 1);          // kSortMid
-    int* ks = (int*)(ids + kSortMid);         // kSortMid
-    for (unsigned li = blockIdx.x; li < n_list; li += gridDim.x) {
+// One block per list of kSortWarp+1 .. kSortMid entries: bitonic sort in
+// shared memory.
+__global__ void __launch_bounds__(kSortThreads) k_sort_mid(const uint32_t* off, const int32_t* len, uint32_t* nbr,
+                                                            const uint32_t* list, const unsigned* n_list,
+                                                            ListSrc src) {
+    __shared__ uint32_t k[kSortMid];
+    const unsigned nl = *n_list;
+    for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
         const uint32_t v = list[li];
         const int n = len[v];
         uint32_t* a = nbr + off[v];
-        const uint32_t* in = src_list(src, v, a);
-        for (int i = threadIdx.x; i <= K; i += blockDim.x) bins[i] = 0;
+        const uint32_t* in = src_list(src, v);
+        int N = 2 * kSortWarp;
+        while (N < n) N <<= 1;
+        for (int i = threadIdx.x; i < N; i += kSortThreads) k[i] = i < n ? src.pos[in[i]] : 0xFFFFFFFFu;
         __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint32_t u = src_id(src, in[i]);
-            const int k = kmax[u];
-            ids[i] = u;
-            ks[i] = k;
-            atomicAdd(&bins[K - k], 1u);
-        }
+        for (int size = 2; size <= N; size <<= 1)
+            for (int stride = size >> 1; stride; stride >>= 1) {
+                for (int p = threadIdx.x; p < N / 2; p += kSortThreads) {
+                    const int i = ((p & ~(stride - 1)) << 1) | (p & (stride - 1)), o = i | stride;
+                    const uint32_t x = k[i], y = k[o];
+                    if ((x > y) == ((i & size) == 0)) {
+                        k[i] = y;
+                        k[o] = x;
+                    }
+                }
+                // pairs up to 32 apart stay within a warp's 64 entries
+                if (stride > 32) __syncthreads();
+                else __syncwarp();
+                if (stride == 1) __syncthreads();
+            }
+        for (int i = threadIdx.x; i < n; i += kSortThreads) a[i] = k[i];
         __syncthreads();
+    }
+}
+
+// One block per longer list: counting sort.  Bin of an id: its 32-id line (a
+// cache line of values) while there are bins for lines, plus K - kmax, which
+// grows with the id and keeps the classes of kmax apart; entries of a bin keep
+// no particular order.  The list fits no shared memory, so its entries are
+// renamed twice.
+static constexpr int kSortBigBins = 11264;
+__global__ void k_sort_big(const uint32_t* off, const int32_t* len, uint32_t* nbr, const int32_t* kmax, int K,
+                           const uint32_t* list, const unsigned* n_list, ListSrc src) {
+    __shared__ unsigned bins[kSortBigBins];
+    const unsigned nl = *n_list;
+    const uint32_t lines = (uint32_t)(kSortBigBins - 1 - K);
+    auto bin_of = [&](uint32_t u) { return (int)min(u >> 5, lines) + (K - kmax[u]); };
+    for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
+        const uint32_t v = list[li];
+        const int n = len[v];
+        uint32_t* a = nbr + off[v];
+        const uint32_t* in = src_list(src, v);
+        for (int i = threadIdx.x; i < kSortBigBins; i += blockDim.x) bins[i] = 0;
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&bins[bin_of(src.pos[in[i]])], 1u);
+        __syncthreads();
+        // exclusive scan of the bins, blockDim at a time
         unsigned long long carry = 0;
-        for (int b0 = 0; b0 <= K; b0 += blockDim.x) {
+        for (int b0 = 0; b0 < kSortBigBins; b0 += blockDim.x) {
             const int b = b0 + threadIdx.x;
-            const unsigned long long x = b <= K ? bins[b] : 0ull;
+            const unsigned long long x = b < kSortBigBins ? bins[b] : 0ull;
             unsigned long long tot;
             const unsigned long long ex = block_excl_scan64(x, &tot);
-            if (b <= K) bins[b] = (unsigned)(ex + carry);
-            carry += tot;
-            __syncthreads();
-        }
-        for (int i = threadIdx.x; i < n; i += blockDim.x) a[atomicAdd(&bins[K - ks[i]], 1u)] = ids[i];
-        __syncthreads();
-    }
-}
-
-// bins = K + 1 counters in shared memory (K < kSortBigBins)
-static constexpr int kSortBigBins = 11264;
-__global__ void k_sort_big(const uint32_t* off, const int32_t* len, uint32_t* nbr, uint32_t* tmp, const int32_t* kmax,
-                           int K, const uint32_t* list, unsigned n_list, ListSrc src) {
-    __shared__ unsigned bins[kSortBigBins];
-    for (unsigned li = blockIdx.x; li < n_list; li += gridDim.x) {
-        uint32_t v = list[li];
-        const int n = len[v];
-        uint32_t* a = nbr + off[v];
-        // in place: staged through tmp; from a source list: straight into a
-        uint32_t* t = src.order ? a : tmp + off[v];
-        const uint32_t* in = src_list(src, v, a);
-        for (int i = threadIdx.x; i <= K; i += blockDim.x) bins[i] = 0;
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&bins[K - kmax[src_id(src, in[i])]], 1u);
-        __syncthreads();
-        // exclusive scan of bins (K+1 values), chunked by blockDim
-        unsigned long long carry = 0;
-        for (int b0 = 0; b0 <= K; b0 += blockDim.x) {
-            int b = b0 + threadIdx.x;
-            unsigned long long x = b <= K ? bins[b] : 0ull;
-            unsigned long long tot;
-            unsigned long long ex = block_excl_scan64(x, &tot);
-            if (b <= K) bins[b] = (unsigned)(ex + carry);
+            if (b < kSortBigBins) bins[b] = (unsigned)(ex + carry);
             carry += tot;
             __syncthreads();
         }
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            uint32_t u = src_id(src, in[i]);
-            unsigned pos = atomicAdd(&bins[K - kmax[u]], 1u);
-            t[pos] = u;
+            const uint32_t u = src.pos[in[i]];
+            a[atomicAdd(&bins[bin_of(u)], 1u)] = u;
         }
-        __syncthreads();
-        if (!src.order)
-            for (int i = threadIdx.x; i < n; i += blockDim.x) a[i] = t[i];
         __syncthreads();
     }
 }
@@ -1686,52 +1794,11 @@ __global__ void k_corner_bound(uint32_t V, const int32_t* kmax, const int32_t* r
     if ((threadIdx.x & 31u) == 0) atomicAdd(acc, s);
 }
 
-// Row ranges of the segments of a split run of rows.
-struct SegBounds {
-    int32_t lo[kMaxRowSegments], hi[kMaxRowSegments];
-    int n;
-};
-// Corner bounds per segment: acc[i] = corners of rows lo[i]..hi[i] (a
-// vertex's value drops at least one per corner, so it has at most
-// min(rows it belongs to, row 0 value) of them; the first corner of a
-// segment that starts from row 0 is one of them).
-__global__ void k_corner_bounds(uint32_t V, const int32_t* kmax, const int32_t* row0, SegBounds b,
-                                unsigned long long* acc) {
-    unsigned long long t[kMaxRowSegments] = {};
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
-        const int32_t km = kmax[v], r0 = row0[v];
-#pragma unroll
-        for (int i = 0; i < kMaxRowSegments; ++i)
-            if (i < b.n) t[i] += (unsigned long long)max(0, min(min(km, b.hi[i]) - b.lo[i] + 1, r0));
-    }
-#pragma unroll
-    for (int i = 0; i < kMaxRowSegments; ++i) {
-#pragma unroll
-        for (int o = 16; o; o >>= 1) t[i] += __shfl_xor_sync(0xFFFFFFFFu, t[i], o);
-        if ((threadIdx.x & 31u) == 0 && i < b.n && t[i]) atomicAdd(&acc[i], t[i]);
-    }
-}
-
 // log entries with a negative row are void (dropped corners)
 __global__ void k_sky_count(uint32_t V, uint64_t nlog, const uint32_t* log_v, const int32_t* log_k,
                             unsigned long long* cnt) {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < nlog; i += (uint64_t)gridDim.x * blockDim.x)
         if (log_k[i] >= 0) atomicAdd(&cnt[log_v[i]], 1ull);
-}
-// A row segment that jumped from row 0 to row k logs vertex v at row k
-// whenever its value differs from row 0; the corner is void when the value
-// equals row k-1's (cur after the previous segment).  Counts the void entries.
-__global__ void k_seg_void(uint64_t n, const uint32_t* log_v, int32_t* log_k, const int32_t* log_l, int32_t k,
-                           const int32_t* cur, unsigned long long* dropped) {
-    unsigned long long t = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        if (log_k[i] == k && log_l[i] == cur[log_v[i]]) {
-            log_k[i] = -1;
-            ++t;
-        }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
-    if ((threadIdx.x & 31u) == 0 && t) atomicAdd(dropped, t);
 }
 __global__ void k_set_one(uint32_t V, unsigned long long* cnt) {
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
@@ -2010,7 +2077,6 @@ void free_scratch(dc_graph* h) {
     Scratch* s = h->scratch;
     if (!s) return;
     for (RowSegment& g : s->seg) {
-        if (g.stream) cudaStreamSynchronize(g.stream);
         dfree(h->stream, g.cur);
         dfree(h->stream, g.cnt_out);
         dfree(h->stream, g.cnt_in);
@@ -2019,9 +2085,6 @@ void free_scratch(dc_graph* h) {
         dfree(h->stream, g.logidx);
         dfree(h->stream, g.tring);
         dfree(h->stream, g.ctl);
-        if (g.stream) cudaStreamDestroy(g.stream);
-        for (auto& e : g.ev)
-            if (e) cudaEventDestroy(e);
     }
     dfree(h->stream, s->key);
     dfree(h->stream, s->cdeg);
@@ -2034,7 +2097,6 @@ void free_scratch(dc_graph* h) {
     dfree(h->stream, s->rem1);
     dfree(h->stream, s->order);
     dfree(h->stream, s->ck);
-    dfree(h->stream, s->ring);
     dfree(h->stream, s->log_v);
     dfree(h->stream, s->log_k);
     dfree(h->stream, s->log_l);
@@ -2047,12 +2109,11 @@ void free_scratch(dc_graph* h) {
     dfree(h->stream, s->rem3);
     dfree(h->stream, s->cnt_out);
     dfree(h->stream, s->tring);
-    dfree(h->stream, s->w_out_len);
-    dfree(h->stream, s->w_in_len);
-    dfree(h->stream, s->w_out_nbr);
-    dfree(h->stream, s->w_in_nbr);
     dfree(h->stream, s->kmax_old);
     dfree(h->stream, s->row0_old);
+    dfree(h->stream, s->plan);
+    dfree(h->stream, s->seam_of);
+    dfree(h->stream, s->seam);
     dfree(h->stream, s->pos);
     dfree(h->stream, s->kmax_r);
     dfree(h->stream, s->row0_r);
@@ -2071,7 +2132,7 @@ int ensure_scratch(dc_graph* h, uint32_t V) {
     if (s->cap_V >= V && s->key) return DC_OK;
     // release V-sized buffers and reallocate
     dfree(h->stream, s->key); dfree(h->stream, s->cdeg); dfree(h->stream, s->cur); dfree(h->stream, s->row0); dfree(h->stream, s->mark); dfree(h->stream, s->stamp);
-    dfree(h->stream, s->logidx); dfree(h->stream, s->rem0); dfree(h->stream, s->rem1); dfree(h->stream, s->order); dfree(h->stream, s->ring); dfree(h->stream, s->tmp64);
+    dfree(h->stream, s->logidx); dfree(h->stream, s->rem0); dfree(h->stream, s->rem1); dfree(h->stream, s->order); dfree(h->stream, s->tmp64);
     dfree(h->stream, s->partial); dfree(h->stream, s->cursor);
     dfree(h->stream, s->key2); dfree(h->stream, s->cdeg2); dfree(h->stream, s->rem2); dfree(h->stream, s->rem3); dfree(h->stream, s->cnt_out);
     uint64_t n = (uint64_t)V + 1;
@@ -2082,11 +2143,6 @@ int ensure_scratch(dc_graph* h, uint32_t V) {
         dmalloc(h->stream, &s->key2, n) || dmalloc(h->stream, &s->cdeg2, n) || dmalloc(h->stream, &s->rem2, n) || dmalloc(h->stream, &s->rem3, n) ||
         dmalloc(h->stream, &s->cnt_out, n))
         return DC_ERR_NOMEM;
-    uint64_t need = (uint64_t)V + (uint64_t)h->geom.sms * 64 * 32 + 64;
-    uint64_t rc = 1024;
-    while (rc < need) rc <<= 1;
-    if (dmalloc(h->stream, &s->ring, rc)) return DC_ERR_NOMEM;
-    s->ring_mask = (uint32_t)(rc - 1);
     s->cap_V = V;
     return DC_OK;
 }
@@ -2102,12 +2158,12 @@ uint64_t device_footprint(const dc_graph* h) {
     b += 4 * d.rows_cap;
     if (const Scratch* s = h->scratch) {
         uint64_t n = (uint64_t)s->cap_V + 1;
-        if (s->key) b += 4 * (16 * n + 1) + 8 * (n + 1) + 8 * ((uint64_t)h->geom.sms * 64 + 64) + 4ull * (s->ring_mask + 1ull);
+        if (s->key) b += 4 * (16 * n + 1) + 8 * (n + 1) + 8 * ((uint64_t)h->geom.sms * 64 + 64);
         b += 4ull * s->ck_cap + 12 * s->log_cap + 8 * s->tring_cap;
-        b += 4 * (s->w_out_cap + s->w_in_cap);
         if (s->kmax_old) b += 8 * n;
         for (const RowSegment& sg : s->seg)
             b += (sg.cur ? 24 * ((uint64_t)sg.cap_V + 1) : 0) + 8 * sg.tring_cap + (sg.ctl ? sizeof(EngineCtl) : 0);
+        b += (s->plan ? sizeof(RowPlan) : 0) + 4ull * s->seam_of_cap + 4 * s->seam_cap;
         if (s->pos) b += 4 * 7 * ((uint64_t)s->r_cap_V + 1);     // relabeled graph: ids, kmax, row 0, offsets, lengths
         if (s->r_nbr_alloc[0]) b += 2 * 4 * (s->r_cap + 7);     // its lists
     }
@@ -2169,7 +2225,6 @@ static int finish_build(dc_graph* h, uint32_t V, uint64_t E, const uint32_t* d_s
     DC_CUDA(cudaGetLastError());
     g.V = V;
     g.E = E;
-    g.sorted_kmax = false;
     return DC_OK;
 }
 
@@ -2289,14 +2344,13 @@ int ensure_tring(dc_graph* h, uint64_t need) {
 // once the queue counters sit on separate lines (the autotuner refines it).
 static constexpr int kDefaultBlocksPerSm = 2;
 
-static int persistent_grid(dc_graph* h, const void* fn, int bps, int* blocks, int share = 1) {
+static int persistent_grid(dc_graph* h, const void* fn, int bps, int* blocks) {
     int per_sm = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kThreads, 0);
     if (e != cudaSuccess || per_sm < 1)
         return set_error(DC_ERR_CUDA, "occupancy query failed (%s)", cudaGetErrorString(e));
     if (bps <= 0) bps = h->blocks_per_sm > 0 ? h->blocks_per_sm : kDefaultBlocksPerSm;
-    // launches that share the SMs get an equal part of the resident blocks each
-    *blocks = std::max(1, std::min(bps * h->geom.sms, per_sm * h->geom.sms / share));
+    *blocks = std::min(bps, per_sm) * h->geom.sms;
     return DC_OK;
 }
 
@@ -2339,22 +2393,20 @@ int persistent_enqueue(dc_graph* h, const void* fn, void** args, const char* nam
 // Initialises a control block (on stream st) and launches a persistent
 // kernel there without waiting.  The handle's own block carries the trace.
 // first: the kernel's first step (nullptr: it starts with a grid barrier);
-// share: the launch is one of that many which run at the same time.
+// grid: blocks (0: by blocks per SM).
 static int persistent_launch(dc_graph* h, const void* fn, void** args, const char* name, EngineCtl* ctl,
-                             cudaStream_t st, int bps, const FirstStep* first = nullptr, int share = 1) {
-    int blocks = 0;
-    if (int rc = persistent_grid(h, fn, bps, &blocks, share)) return rc;
+                             cudaStream_t st, int bps, const FirstStep* first = nullptr, int grid = 0) {
+    int blocks = grid;
+    if (!blocks)
+        if (int rc = persistent_grid(h, fn, bps, &blocks)) return rc;
     const bool own = ctl == h->ctl;
-    EngineCtl* initp = &h->ctl_init;
-    for (int i = 0; i < kMaxRowSegments - 1; ++i)
-        if (ctl == h->scratch->seg[i].ctl) initp = &h->ctl_init_seg[i];
-    EngineCtl& init = *initp;
+    EngineCtl& init = h->ctl_init;
     memset(&init, 0, sizeof(init));
     init.step = -1;
     init.wait_ns = h->wait_ns;
     if (first) {
         init.step = 0;
-        init.t_work = (unsigned long long)blocks << kWorkShift;
+        init.t_work = (unsigned long long)(first->blocks ? first->blocks : blocks) << kWorkShift;
         for (auto& w : init.step_word) w.v = (1ull << 32) | (unsigned long long)(uint32_t)first->level;
     }
     if (own) {
@@ -2389,14 +2441,7 @@ static int finish_persistent(dc_graph* h, EngineCtl* ctl, cudaStream_t st, const
     }
     if (rc != DC_OK) {
         Scratch* s = h->scratch;
-        unsigned long long* ring = s->tring;
-        uint64_t cap = s->tring_cap;
-        for (const RowSegment& g : s->seg)
-            if (ctl == g.ctl) {
-                ring = g.tring;
-                cap = g.tring_cap;
-            }
-        cudaMemsetAsync(ring, 0xFF, sizeof(unsigned long long) * cap, st);
+        cudaMemsetAsync(s->tring, 0xFF, sizeof(unsigned long long) * s->tring_cap, st);
         cudaStreamSynchronize(st);
     }
     return rc;
@@ -2409,22 +2454,11 @@ int run_persistent(dc_graph* h, const void* fn, void** args, const char* name, E
     return finish_persistent(h, h->ctl, h->stream, name, out);
 }
 
-// Stream, events and control block of row segment i + 1 (seg[i]).
-static int ensure_segment_stream(dc_graph* h, int i) {
-    RowSegment& g = h->scratch->seg[i];
-    if (!g.stream) {
-        DC_CUDA(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
-        for (auto& e : g.ev) DC_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
-    if (!g.ctl && dmalloc(h->stream, &g.ctl, 1)) return DC_ERR_NOMEM;
-    return DC_OK;
-}
-
-// State of row segment i + 1 for the n vertices of its first row's core (ids
-// below n of the relabeled graph), with an eighth of headroom.
+// State of row group i + 1 for the ids below n of the relabeled graph, with
+// an eighth of headroom.
 static int ensure_segment(dc_graph* h, int i, uint32_t n) {
-    if (int rc = ensure_segment_stream(h, i)) return rc;
     RowSegment& g = h->scratch->seg[i];
+    if (!g.ctl && dmalloc(h->stream, &g.ctl, 1)) return DC_ERR_NOMEM;
     if (g.cap_V < n || !g.cur) {
         dfree(h->stream, g.cur);
         dfree(h->stream, g.cnt_out);
@@ -2448,20 +2482,6 @@ static int ensure_segment(dc_graph* h, int i, uint32_t n) {
         g.tring_cap = cap;
         DC_CUDA(cudaMemsetAsync(g.tring, 0xFF, sizeof(unsigned long long) * cap, h->stream));
     }
-    return DC_OK;
-}
-
-// Creates the streams of the row segments the handle's cuts ask for (their
-// state is sized for the graph's cores by the first run that uses them).
-int prepare_row_segments(dc_graph* h) {
-    const uint32_t V = h->g.V;
-    if (!V) return DC_OK;
-    int n = 0;
-    while (n < kMaxRowSegments - 1 && h->rows_split[n] > 0) ++n;
-    if (!n) return DC_OK;
-    if (int rc = ensure_scratch(h, V)) return rc;
-    for (int i = 0; i < n; ++i)
-        if (int rc = ensure_segment_stream(h, i)) return rc;
     return DC_OK;
 }
 
@@ -2508,7 +2528,7 @@ int run_peel2(dc_graph* h, int ninst, const PeelInst* inst, int32_t* maxv) {
     void* args[] = {&p};
     EngineCtl hc;
     const void* fn = inst[0].member ? (const void*)k_peel2<true> : (const void*)k_peel2<false>;
-    const FirstStep first{0};
+    const FirstStep first{0, 0};
     if (int rc = run_persistent(h, fn, args, "peel", &hc, h->peel_bps, &first)) return rc;
     for (int i = 0; i < ninst; ++i) maxv[i] = hc.maxv[i];
     return DC_OK;
@@ -2533,34 +2553,19 @@ int run_peel(dc_graph* h, int which, const int32_t* member, int32_t k, int32_t* 
     return DC_OK;
 }
 
-// Skyline from row 0 and the corner logs of the last run of rows: the
-// first segment's nlog entries at the log's start (h->log_used of them
-// records, the others void) and the other segments' ranges (h->seg_off /
-// seg_n, void entries skipped).
+// Skyline from row 0 and the corner log of the last run of rows (nlog
+// entries, h->log_used of them records, the others void).
 int build_skyline_from_log(dc_graph* h, uint64_t nlog) {
     Scratch* s = h->scratch;
     Decomp& d = h->d;
     uint32_t V = h->g.V;
     unsigned long long* cnt = (unsigned long long*)s->tmp64;
-    uint64_t lo[kMaxRowSegments], n[kMaxRowSegments];
-    int nr = 0;
-    uint64_t total = (uint64_t)V;
-    if (nlog) {
-        lo[nr] = 0;
-        n[nr++] = nlog;
-        total += h->log_used;
-    }
-    for (int i = 0; i < h->nseg_extra; ++i)
-        if (h->seg_n[i]) {
-            lo[nr] = h->seg_off[i];
-            n[nr++] = h->seg_n[i];
-            total += h->seg_n[i] - h->seg_void[i];
-        }
+    const uint64_t total = (uint64_t)V + (nlog ? h->log_used : 0);
     ++g_launches;
     k_set_one<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, cnt);
-    for (int r = 0; r < nr; ++r) {
+    if (nlog) {
         ++g_launches;
-        k_sky_count<<<grid_for(h, n[r]), kThreads, 0, h->stream>>>(V, n[r], s->log_v + lo[r], s->log_k + lo[r], cnt);
+        k_sky_count<<<grid_for(h, nlog), kThreads, 0, h->stream>>>(V, nlog, s->log_v, s->log_k, cnt);
     }
     if (int rc = scan_tmp64(h, V)) return rc;
     if (d.corner_cap < total || !d.sky_k) {
@@ -2575,11 +2580,10 @@ int build_skyline_from_log(dc_graph* h, uint64_t nlog) {
     if (!d.sky_off && dmalloc(h->stream, &d.sky_off, (uint64_t)V + 1)) return DC_ERR_NOMEM;
     ++g_launches;
     k_sky_fill_row0<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, cnt, s->row0, d.sky_k, d.sky_l, s->cursor);
-    for (int r = 0; r < nr; ++r) {
+    if (nlog) {
         ++g_launches;
-        k_sky_fill_log<<<grid_for(h, n[r]), kThreads, 0, h->stream>>>(n[r], s->log_v + lo[r], s->log_k + lo[r],
-                                                                      s->log_l + lo[r], cnt, d.sky_k, d.sky_l,
-                                                                      s->cursor);
+        k_sky_fill_log<<<grid_for(h, nlog), kThreads, 0, h->stream>>>(nlog, s->log_v, s->log_k, s->log_l, cnt, d.sky_k,
+                                                                      d.sky_l, s->cursor);
     }
     ++g_launches;
     k_sky_sort<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, cnt, d.sky_k, d.sky_l, d.sky_off);
@@ -2613,72 +2617,20 @@ int expand_rows(dc_graph* h, uint32_t k0, uint32_t n, int32_t* d_dst) {
     return DC_OK;
 }
 
-// Orders every adjacency list by neighbour kmax, descending.  *sorted = 0
-// when kmax is too large for the long-list counting sort (lists then stay
-// in arbitrary order and evaluations read them whole).
-// Orders every list of one side by neighbour kmax, descending (kmax[u] of
-// each entry u of the graph the lists belong to).  cap = entries the lists'
-// array spans (the long-list sort stages through a scratch copy that size).
+// The lists of one side of the relabeled graph from the handle's lists.
 static int sort_side(dc_graph* h, int32_t K, uint32_t V, const uint32_t* off, const int32_t* len, uint32_t* nbr,
-                     uint64_t cap, const int32_t* kmax, int side, ListSrc src) {
+                     const int32_t* kmax, ListSrc src) {
     Scratch* s = h->scratch;
     unsigned* cnt = s->cursor;
     DC_CUDA(cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned), h->stream));
-    ++g_launches;
-    k_sort_short<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, off, len, nbr, kmax, s->rem0, s->rem2, s->rem1, cnt,
-                                                              src);
-    // most lists go to the warp sort, which reads its count on the device
-    ++g_launches;
-    k_sort_warp<<<h->geom.sms * 8, kSortWarpThreads, 0, h->stream>>>(off, len, nbr, kmax, s->rem0, &cnt[0], src);
-    unsigned hc[3] = {0, 0, 0};
-    DC_CUDA(cudaMemcpyAsync(hc, cnt, sizeof(hc), cudaMemcpyDeviceToHost, h->stream));
-    DC_CUDA(cudaStreamSynchronize(h->stream));
-    if (hc[1]) {
-        const size_t shm = 4ull * (K + 1) + 8ull * kSortMid;
-        // the kernel's limit is set to its largest need, the same value on
-        // every call: handles sorting on other threads at the same time
-        // (the serving loop) must never see it lowered below their launch
-        constexpr size_t kMidMax = 4ull * kSortBigBins + 8ull * kSortMid;
-        static_assert(kMidMax <= 227ull * 1024, "mid-list sort shared memory");
-        DC_CUDA(cudaFuncSetAttribute(k_sort_mid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMidMax));
-        int blocks = (int)std::min<unsigned>(hc[1], (unsigned)h->geom.sms * 8);
-        ++g_launches;
-        k_sort_mid<<<blocks, 256, shm, h->stream>>>(off, len, nbr, kmax, K, s->rem2, hc[1], src);
-    }
-    if (hc[2]) {
-        uint32_t*& tmp = side == 0 ? s->w_out_nbr : s->w_in_nbr;
-        uint64_t& tcap = side == 0 ? s->w_out_cap : s->w_in_cap;
-        if (!src.order && (tcap < cap || !tmp)) {  // in place: staging copy of the lists' span
-            dfree(h->stream, tmp);
-            if (dmalloc(h->stream, &tmp, cap)) return DC_ERR_NOMEM;
-            tcap = cap;
-        }
-        int blocks = (int)std::min<unsigned>(hc[2], (unsigned)h->geom.sms * 2);
-        ++g_launches;
-        k_sort_big<<<blocks, 512, 0, h->stream>>>(off, len, nbr, tmp, kmax, K, s->rem1, hc[2], src);
-    }
+    // most lists go to the short and the warp sort; the others read their
+    // counts on the device
+    g_launches += 4;
+    k_sort_short<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, off, len, nbr, s->rem0, s->rem2, s->rem1, cnt, src);
+    k_sort_warp<<<h->geom.sms * 8, kSortThreads, 0, h->stream>>>(off, len, nbr, s->rem0, &cnt[0], src);
+    k_sort_mid<<<h->geom.sms * 8, kSortThreads, 0, h->stream>>>(off, len, nbr, s->rem2, &cnt[1], src);
+    k_sort_big<<<h->geom.sms * 2, 512, 0, h->stream>>>(off, len, nbr, kmax, K, s->rem1, &cnt[2], src);
     DC_CUDA(cudaGetLastError());
-    return DC_OK;
-}
-
-// Orders every adjacency list of the graph by neighbour kmax, descending.
-// *sorted = 0 when kmax is too large for the long-list counting sort (lists
-// then stay in arbitrary order and evaluations read them whole).
-static int sort_lists_by_kmax(dc_graph* h, int32_t K, int* sorted) {
-    DevGraph& g = h->g;
-    *sorted = 0;
-    if (g.sorted_kmax) {
-        *sorted = 1;
-        return DC_OK;
-    }
-    if (K + 1 > kSortBigBins) return DC_OK;
-    for (int side = 0; side < 2; ++side)
-        if (int rc = sort_side(h, K, g.V, side == 0 ? g.out_off : g.in_off, side == 0 ? g.out_len : g.in_len,
-                               side == 0 ? g.out_nbr : g.in_nbr, side == 0 ? g.out_cap : g.in_cap, h->d.kmax_v, side,
-                               ListSrc{nullptr, nullptr, nullptr, nullptr}))
-            return rc;
-    g.sorted_kmax = true;
-    *sorted = 1;
     return DC_OK;
 }
 
@@ -2708,10 +2660,82 @@ __global__ void k_len_to_u64e(uint32_t V, const int32_t* len, unsigned long long
         out[i] = (unsigned long long)len[i];
 }
 
-// corner records of the relabeled run back to original ids (void ones hold none)
-__global__ void k_unlabel_log(uint64_t n, const uint32_t* order, uint32_t* log_v, const int32_t* log_k) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        if (log_k[i] >= 0) log_v[i] = order[log_v[i]];
+// Corner records of the relabeled run back to original ids.  A run that
+// jumped from row 0 to row k logs vertex v at row k whenever its value differs
+// from row 0; where another run computed row k - 1 the corner is void when the
+// value equals that row's (in the seam array).  *n: records in the log.
+__global__ void k_log_finish(const unsigned* n, unsigned long long cap, const uint32_t* order, uint32_t* log_v,
+                             int32_t* log_k, const int32_t* log_l, const uint32_t* seam_of, const int32_t* seam,
+                             unsigned long long* voids) {
+    const uint64_t m = min((unsigned long long)*n, cap);
+    unsigned t = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
+        const int32_t k = log_k[i];
+        if (k < 0) continue;
+        const uint32_t v = log_v[i];
+        const uint32_t at = seam_of ? seam_of[k] : 0u;
+        if (at && log_l[i] == seam[at - 1u + v]) {
+            log_k[i] = -1;
+            ++t;
+        } else {
+            log_v[i] = order[v];
+        }
+    }
+    t = __reduce_add_sync(0xFFFFFFFFu, t);
+    if ((threadIdx.x & 31u) == 0 && t) atomicAdd(voids, (unsigned long long)t);
+}
+
+// Control blocks of the groups after the first (group 0's is the handle's own,
+// initialised by its launch) and the plan's runs.
+struct RowsStart {
+    int n_groups;
+    EngineCtl* ctl[kRowGroups];
+    unsigned blocks[kRowGroups];
+    unsigned long long span[kRowGroups];
+    uint32_t seam_row[kRowGroups], seam_at[kRowGroups];  // first rows of the runs after the first, their seams
+    unsigned seam_tail;
+    unsigned long long wait_ns;
+};
+__global__ void k_rows_start(RowsStart r, RowPlan* plan, uint32_t* seam_of, uint32_t n_seam_of) {
+    // one block: clear, then set
+    for (uint32_t i = threadIdx.x; i < sizeof(RowPlan) / 4; i += blockDim.x) reinterpret_cast<uint32_t*>(plan)[i] = 0;
+    for (uint32_t i = threadIdx.x; i < n_seam_of; i += blockDim.x) seam_of[i] = 0;
+    for (int g = 1; g < r.n_groups; ++g)
+        for (uint32_t i = threadIdx.x; i < sizeof(EngineCtl) / 4; i += blockDim.x)
+            reinterpret_cast<uint32_t*>(r.ctl[g])[i] = 0;
+    __syncthreads();
+    if (threadIdx.x < (unsigned)r.n_groups) {
+        const int g = threadIdx.x;
+        plan->span[g].v = r.span[g];
+        plan->own[g].lo = (int)(uint32_t)r.span[g];
+        plan->own[g].from = -1;
+        plan->own[g].ready = g == 0;
+        if (r.seam_row[g]) seam_of[r.seam_row[g]] = r.seam_at[g] + 1u;
+        if (g) {
+            EngineCtl* c = r.ctl[g];
+            // a group with a run starts it, one without looks for one
+            const int level = r.span[g] ? kRowsInit : kRowsWait;
+            for (int i = 0; i < kStepWords; ++i) c->step_word[i].v = (1ull << 32) | (unsigned long long)(uint32_t)level;
+            c->t_work = (unsigned long long)r.blocks[g] << kWorkShift;
+            c->wait_ns = r.wait_ns;
+        }
+    }
+    if (threadIdx.x == 0) plan->seam_tail = r.seam_tail;
+}
+// The groups' status and statistics into group 0's control block.
+__global__ void k_rows_collect(RowsStart r, const RowPlan* plan) {
+    EngineCtl* c0 = r.ctl[0];
+    for (int g = 1; g < r.n_groups; ++g) {
+        const EngineCtl* c = r.ctl[g];
+        if (c->error && !c0->error) c0->err_where = c->err_where;
+        c0->error |= c->error;
+        c0->log_used += c->log_used;
+        c0->evals += c->evals;
+        c0->drops += c->drops;
+        c0->edges_scanned += c->edges_scanned;
+    }
+    c0->log_count = plan->log_count;
+    c0->pushes = plan->voids;
 }
 
 // Builds the relabeled graph (s->order must hold the kmax order of the
@@ -2768,8 +2792,7 @@ static int build_relabeled(dc_graph* h, int32_t K) {
     // sorted by neighbour kmax in one pass
     for (int side = 0; side < 2; ++side) {
         const ListSrc src{side == 0 ? g.out_off : g.in_off, side == 0 ? g.out_nbr : g.in_nbr, s->order, s->pos};
-        if (int rc = sort_side(h, K, V, s->r_off[side], s->r_len[side], s->r_nbr[side], s->r_cap, s->kmax_r, side, src))
-            return rc;
+        if (int rc = sort_side(h, K, V, s->r_off[side], s->r_len[side], s->r_nbr[side], s->kmax_r, src)) return rc;
     }
     return DC_OK;
 }
@@ -2779,15 +2802,13 @@ static int build_relabeled(dc_graph* h, int32_t K) {
 // row-to-row kernel.  Corners of rows 1..Kstop are left in the scratch log
 // (*nlog entries).  allow_sort: order adjacency lists by neighbour kmax
 // first (otherwise lists are read whole).
-int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint64_t* nlog_out, int32_t K0,
-                   bool allow_relabel) {
+int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint64_t* nlog_out, int32_t K0) {
     DevGraph& g = h->g;
     Decomp& d = h->d;
     Scratch* s = h->scratch;
     const uint32_t V = g.V;
     *nlog_out = 0;
     h->log_used = 0;
-    h->nseg_extra = 0;
     cudaEventRecord(h->ev[2], h->stream);
     if (s->ck_cap < (uint32_t)K + 2) {
         dfree(h->stream, s->ck);
@@ -2824,71 +2845,69 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     // relabeled in kmax order with kmax-sorted lists (C_k a prefix of the
     // ids); else the handle's own lists (kmax-sorted when they still are from
     // an earlier run) with C_k listed by `order`.
-    const bool relabel = allow_sort && allow_relabel && K + 1 <= kSortBigBins;
-    // a run from row 1 on the relabeled graph (a full decomposition, or rows
-    // 1..R of a maintenance batch) may be split in row segments run concurrently: segment 0 (rows
-    // 1..cut[0]) on the handle's stream, segment i (rows cut[i-1]+1..cut[i],
-    // starting there from row 0) on seg[i-1]'s stream, each with its own
-    // state (for the vertices of its first row's core: the ids below |C_a|)
-    // and its own range of the corner log; runs of fewer than kMinSplitRows
-    // rows stay whole
+    const bool relabel = allow_sort && K + 1 <= kSortBigBins;
+    // A run from row 1 on the relabeled graph (a full decomposition, or rows
+    // 1..R of a maintenance batch) may be cut in runs of rows that groups of
+    // blocks work on at the same time: group 0 starts at row 1, a run starting
+    // at row a starts from row 0 inside C_a, with state for the ids below
+    // |C_a|.  Groups whose run is over take over rows of others (RowsNext).
     const int32_t k0 = std::max(1, K0);
-    int32_t cut[kMaxRowSegments];
-    int nseg = 1;
+    int32_t first_row[kRowGroups] = {k0};  // of each run, ascending
+    int nrun = 1, ngroups = 1;
+    int32_t run_min = Kstop + 1;
+    uint32_t n_state = 0;  // vertices every group after the first has state for
     if (relabel && k0 == 1 && Kstop >= kMinSplitRows) {
-        int32_t split[kMaxRowSegments - 1] = {};
-        for (int i = 0; i < kMaxRowSegments - 1; ++i)
-            split[i] = (int32_t)((int64_t)K * (h->auto_cuts ? (i + 1) * 1000 / kMaxRowSegments : h->rows_split[i]) / 1000);
         if (h->auto_cuts) {
-            // Cuts of a handle whose launch shapes were never set: equal runs
-            // of rows, where the core a run starts from is small.  A run's
-            // start costs a pass over its first core's lists and a refinement
-            // from row 0 there: with skewed degrees (|C_k| a few per cent of
-            // |C_1| at the first cut) eight runs at a time take the rows from
-            // 3.46 / 8.92 / 34.2 ms to 1.30 / 3.66 / 19.6 (R-MAT 17 / 18 / 22,
-            // the best of 13 sets of cuts 1.27 / 3.23 / 18.1); where every
-            // vertex is in almost every core (ER, 100 edges per vertex) the
-            // same cuts take them from 3.6 to 11.0 ms.  Hence a quarter of
-            // |C_1| at most for a run's core, half of it for all together
-            // (which also bounds the runs' state).
-            uint64_t sum = 0;
-            for (int i = kMaxRowSegments - 2; i >= 0; --i) {
-                const uint64_t m = split[i] >= 1 && split[i] < Kstop ? ck[split[i] + 1] : 0;
-                if (4 * m > ck[1] || 2 * (sum + m) > ck[1]) split[i] = 0;
-                else sum += m;
+            // A handle whose launch shapes were never set is cut where the
+            // core a run starts from is small: a start costs a pass over its
+            // core's lists and a refinement from row 0 there.  With skewed
+            // degrees (|C_k| a few per cent of |C_1| after a tenth of the
+            // rows) eight runs at a time take the rows from 3.4 / 8.9 / 15.6 /
+            // 44 ms to 1.3 / 3.5 / 7.8 / 19 (ragged R-MAT 17, R-MAT 18 / 20 /
+            // 22) with fixed cuts; where every vertex is in almost every core
+            // (ER, 100 edges per vertex) they take them from 3.6 to 11.0 ms.
+            // Hence an eighth of |C_1| at most (a quarter up to 65,536
+            // vertices), which also bounds the groups' state, and no cut
+            // where that leaves more than half of the rows to the first run.
+            n_state = std::max(ck[1] / 8, std::min(ck[1] / 4, 65536u));
+            run_min = 2;
+            while (run_min <= Kstop && ck[run_min] > n_state) ++run_min;
+            // Groups: eight small ones hide each other's latency best until the
+            // rows are heavy enough to want more warps each (8 / 6 / 5 / 4
+            // groups: R-MAT 18, 3.9 M edges 2.1 / 2.5 / 2.7 / 3.0 ms; R-MAT 20,
+            // 16 M 5.4 / 4.9 / 5.9 / 6.5; R-MAT 22, 65 M 19.9 / 14.8 / 14.8 /
+            // 19.0; 2^21 vertices, 45 M edges 18.9 / 16.7 / 16.2 / 15.3).
+            const int most = std::min<int>(kRowGroups, g.E < (8ull << 20) ? 8 : g.E < (32ull << 20) ? 6 : 5);
+            if (2 * (run_min - 1) <= Kstop) {
+                const int32_t rows = Kstop - run_min + 1, runs = std::min<int32_t>(most - 1, rows / 2);
+                for (int32_t i = 0; i < runs; ++i) first_row[nrun++] = run_min + (int32_t)((int64_t)rows * i / runs);
+                n_state = ck[run_min];
+                ngroups = nrun > 1 ? most : 1;
+            }
+        } else {
+            for (int i = 0; i < kMaxRowSegments - 1 && nrun < kRowGroups; ++i) {
+                const int32_t c = (int32_t)((int64_t)K * h->rows_split[i] / 1000);
+                if (c >= 1 && c < Kstop && c + 1 > first_row[nrun - 1]) first_row[nrun++] = c + 1;
+            }
+            if (nrun > 1) {
+                run_min = first_row[1];
+                n_state = ck[run_min];
+                ngroups = nrun;
             }
         }
-        for (int i = 0; i < kMaxRowSegments - 1; ++i) {
-            const int32_t c = split[i];
-            if (c >= 1 && c < Kstop && (nseg == 1 || c > cut[nseg - 2])) cut[nseg++ - 1] = c;
-        }
     }
-    cut[nseg - 1] = Kstop;
-    // log ranges: [off[i], off[i] + cap[i]) per segment
-    uint64_t off[kMaxRowSegments] = {}, capn[kMaxRowSegments] = {};
-    // records every warp of the largest grid may leave unused in its last chunk
-    const uint64_t spare = (uint64_t)kLogChunk * kWarpsPerBlock * 8 * h->geom.sms / nseg;
-    uint64_t lc = bound + 1 + spare;
-    if (nseg > 1) {
-        SegBounds sb;
-        sb.n = nseg;
-        for (int i = 0; i < nseg; ++i) {
-            sb.lo[i] = i == 0 ? k0 : cut[i - 1] + 1;
-            sb.hi[i] = cut[i];
-        }
-        DC_CUDA(cudaMemsetAsync(acc, 0, nseg * sizeof(unsigned long long), h->stream));
-        ++g_launches;
-        k_corner_bounds<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, d.kmax_v, s->row0, sb, acc);
-        unsigned long long bs[kMaxRowSegments] = {};
-        DC_CUDA(cudaMemcpyAsync(bs, acc, nseg * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
-        DC_CUDA(cudaStreamSynchronize(h->stream));
-        lc = 0;
-        for (int i = 0; i < nseg; ++i) {
-            off[i] = lc;
-            capn[i] = bs[i] + 1 + spare;
-            lc += capn[i];
-        }
-    }
+    // blocks: what fits at the same time, the first run of an uncut handle
+    // (the one with the large cores) twice the others' share
+    int grid = 0;
+    if (int rc = persistent_grid(h, (const void*)k_trans2, ngroups > 1 ? 8 : h->rows_bps, &grid)) return rc;
+    if (ngroups > 1 && h->rows_bps > 0) grid = std::min(grid, h->rows_bps * ngroups * h->geom.sms);
+    const uint64_t spare = (uint64_t)kLogChunk * kWarpsPerBlock * grid;  // records left over in the warps' chunks
+    // seams: the values of row a - 1 in C_a for every run that starts at a,
+    // with room for rows taken over (a void record each at most)
+    uint64_t seam_cap = 0;
+    for (int i = 1; i < nrun; ++i) seam_cap += ck[first_row[i]];
+    if (nrun > 1) seam_cap = std::min<uint64_t>(seam_cap + 8ull * n_state, 0xFFFFFFF0ull);
+    const uint64_t lc = bound + 1 + spare + seam_cap;
     if (s->log_cap < lc) {
         // a quarter of headroom: later runs (maintenance batches) rarely grow it again
         const uint64_t cap = lc + lc / 4;
@@ -2899,7 +2918,6 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
         if (dmalloc(h->stream, &s->log_v, cap) || dmalloc(h->stream, &s->log_k, cap) || dmalloc(h->stream, &s->log_l, cap)) return DC_ERR_NOMEM;
         s->log_cap = cap;
     }
-    if (nseg == 1) capn[0] = s->log_cap;
     int sorted = 0;
     const uint32_t *G_out_off = g.out_off, *G_in_off = g.in_off, *G_order = s->order;
     int32_t *G_out_len = g.out_len, *G_in_len = g.in_len;
@@ -2917,160 +2935,126 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
         G_kmax = s->kmax_r;
         G_row0 = s->row0_r;
         G_order = nullptr;
-    } else if (allow_sort || g.sorted_kmax) {
-        if (int rc = sort_lists_by_kmax(h, K, &sorted)) return rc;
     }
-    // starting values and counters of a run that starts at row a: row 0
-    // inside C_a with the vertices outside already left (for a = 1 those of
-    // kmax 0), so the run's first step has no leaving pass
-    auto start_state = [&](cudaStream_t st, int32_t a, int32_t* cur, int32_t* co, int32_t* ci, uint32_t* mark,
-                           uint64_t n_mark, int32_t* stamp) -> int {
-        const uint32_t n = relabel ? ck[std::min(a, K + 1)] : V;
-        DC_CUDA(cudaMemsetAsync(mark, 0, sizeof(uint32_t) * n_mark, st));
-        if (!n) return DC_OK;
+    // starting values and counters of the first run: row 0 inside C_k0 with
+    // the vertices outside already left (for k0 = 1 those of kmax 0), so its
+    // first step has no leaving pass; the marks of all V vertices, because the
+    // local core update expects them clear
+    const uint32_t n0 = relabel ? ck[std::min(k0, K + 1)] : V;
+    if (int rc = ensure_tring(h, 2ull * V + (uint64_t)h->geom.sms * 64 + 4096)) return rc;
+    Trans2Params tp;
+    memset(&tp, 0, sizeof(tp));
+    tp.out_off = G_out_off; tp.out_len = G_out_len; tp.out_nbr = G_out_nbr;
+    tp.in_off = G_in_off; tp.in_len = G_in_len; tp.in_nbr = G_in_nbr;
+    tp.kmax = G_kmax;
+    tp.row0 = G_row0;
+    tp.K = K;
+    tp.K0 = k0;
+    tp.Kstop = Kstop;
+    tp.n = n0;
+    tp.sorted = sorted;
+    tp.order = G_order;
+    tp.ck = s->ck;
+    tp.log_v = s->log_v;
+    tp.log_k = s->log_k;
+    tp.log_l = s->log_l;
+    tp.log_cap = s->log_cap;
+    tp.n_groups = ngroups;
+    tp.g[0] = RowGroup{s->cur, s->cnt_out, s->key, s->mark, s->stamp, s->logidx,
+                       TicketQueue{s->tring, (unsigned)(s->tring_cap - 1)}, h->ctl};
+    DC_CUDA(cudaMemsetAsync(s->mark, 0, sizeof(uint32_t) * V, h->stream));
+    if (n0) {
         if (relabel) {
-            DC_CUDA(cudaMemcpyAsync(cur, G_row0, 4ull * n, cudaMemcpyDeviceToDevice, st));
+            DC_CUDA(cudaMemcpyAsync(s->cur, G_row0, 4ull * n0, cudaMemcpyDeviceToDevice, h->stream));
         } else {
             ++g_launches;
-            k_preleft_cur<<<grid_for(h, n), kThreads, 0, st>>>(n, G_kmax, G_row0, a, cur);
+            k_preleft_cur<<<grid_for(h, n0), kThreads, 0, h->stream>>>(n0, G_kmax, G_row0, k0, s->cur);
         }
         ++g_launches;
-        k_counters_init<<<grid_for(h, (uint64_t)n * 32), kThreads, 0, st>>>(
-            n, G_out_off, G_out_len, G_out_nbr, G_in_off, G_in_len, G_in_nbr, cur, co, ci, sorted);
-        DC_CUDA(cudaMemsetAsync(stamp, 0xFF, sizeof(int32_t) * n, st));
-        return DC_OK;
-    };
-    if (int rc = start_state(h->stream, k0, s->cur, s->cnt_out, s->key, s->mark, V, s->stamp))
-        return rc;  // (the marks of all V vertices: the local core update expects them clear)
-    if (int rc = ensure_tring(h, 2ull * V + (uint64_t)h->geom.sms * 64 + 4096)) return rc;
-    Trans2Params tp[kMaxRowSegments];
-    tp[0].n = relabel ? ck[std::min(k0, K + 1)] : V;
-    tp[0].out_off = G_out_off; tp[0].out_len = G_out_len; tp[0].out_nbr = G_out_nbr;
-    tp[0].in_off = G_in_off; tp[0].in_len = G_in_len; tp[0].in_nbr = G_in_nbr;
-    tp[0].kmax = G_kmax;
-    tp[0].K = K;
-    tp[0].K0 = k0;
-    tp[0].preleft = 1;
-    tp[0].Kstop = cut[0];
-    tp[0].sorted = sorted;
-    tp[0].order = G_order;
-    tp[0].ck = s->ck;
-    tp[0].cur = s->cur;
-    tp[0].cnt_out = s->cnt_out;
-    tp[0].cnt_in = s->key;
-    tp[0].mark = s->mark;
-    tp[0].stamp = s->stamp;
-    tp[0].logidx = s->logidx;
-    tp[0].log_v = s->log_v;
-    tp[0].log_k = s->log_k;
-    tp[0].log_l = s->log_l;
-    tp[0].log_cap = capn[0];
-    tp[0].q.slots = s->tring;
-    tp[0].q.mask = (unsigned)(s->tring_cap - 1);
-    tp[0].ctl = h->ctl;
-    for (int i = 1; i < nseg; ++i)
-        if (int rc = ensure_segment(h, i - 1, ck[cut[i - 1] + 1])) return rc;
-    if (nseg > 1) {
-        // the other segments start once the shared preparation is done
-        DC_CUDA(cudaEventRecord(s->seg[0].ev[0], h->stream));
-        for (int i = 1; i < nseg; ++i) {
-            RowSegment& sg = s->seg[i - 1];
-            DC_CUDA(cudaStreamWaitEvent(sg.stream, s->seg[0].ev[0], 0));
-            const uint32_t t_n = ck[cut[i - 1] + 1];
-            if (int rc = start_state(sg.stream, cut[i - 1] + 1, sg.cur, sg.cnt_out, sg.cnt_in, sg.mark, t_n, sg.stamp))
-                return rc;
-            Trans2Params& t = tp[i];
-            t = tp[0];
-            t.n = t_n;
-            t.K0 = cut[i - 1] + 1;
-            t.preleft = 1;
-            t.Kstop = cut[i];
-            t.cur = sg.cur;
-            t.cnt_out = sg.cnt_out;
-            t.cnt_in = sg.cnt_in;
-            t.mark = sg.mark;
-            t.stamp = sg.stamp;
-            t.logidx = sg.logidx;
-            t.log_v = s->log_v + off[i];
-            t.log_k = s->log_k + off[i];
-            t.log_l = s->log_l + off[i];
-            t.log_cap = capn[i];
-            t.q.slots = sg.tring;
-            t.q.mask = (unsigned)(sg.tring_cap - 1);
-            t.ctl = sg.ctl;
+        k_counters_init<<<grid_for(h, (uint64_t)n0 * 32), kThreads, 0, h->stream>>>(tp);
+        DC_CUDA(cudaMemsetAsync(s->stamp, 0xFF, sizeof(int32_t) * n0, h->stream));
+    }
+    RowsStart rs;
+    memset(&rs, 0, sizeof(rs));
+    if (ngroups > 1) {
+        const int shares = ngroups + (h->auto_cuts ? 1 : 0);
+        tp.first_block[0] = 0;
+        for (int i = 0; i < ngroups; ++i)
+            tp.first_block[i + 1] = (unsigned)((int64_t)grid * (i + 1 + (h->auto_cuts ? 1 : 0)) / shares);
+        for (int i = 1; i < ngroups; ++i) {
+            if (int rc = ensure_segment(h, i - 1, n_state)) return rc;
+            const RowSegment& sg = s->seg[i - 1];
+            tp.g[i] = RowGroup{sg.cur, sg.cnt_out, sg.cnt_in, sg.mark, sg.stamp, sg.logidx,
+                               TicketQueue{sg.tring, (unsigned)(sg.tring_cap - 1)}, sg.ctl};
         }
+        if (!s->plan && dmalloc(h->stream, &s->plan, 1)) return DC_ERR_NOMEM;
+        if (s->seam_of_cap < (uint32_t)K + 2 || !s->seam_of) {
+            dfree(h->stream, s->seam_of);
+            s->seam_of_cap = 0;
+            if (dmalloc(h->stream, &s->seam_of, (uint64_t)K + 2)) return DC_ERR_NOMEM;
+            s->seam_of_cap = (uint32_t)K + 2;
+        }
+        if (s->seam_cap < seam_cap || !s->seam) {
+            dfree(h->stream, s->seam);
+            s->seam_cap = 0;
+            const uint64_t want = seam_cap + seam_cap / 8;
+            if (dmalloc(h->stream, &s->seam, want)) return DC_ERR_NOMEM;
+            s->seam_cap = want;
+        }
+        tp.plan = s->plan;
+        tp.run_min = run_min;
+        tp.seam_of = s->seam_of;
+        tp.seam = s->seam;
+        tp.seam_cap = (unsigned)seam_cap;
+        rs.n_groups = ngroups;
+        rs.wait_ns = h->wait_ns;
+        for (int i = 0; i < ngroups; ++i) {
+            rs.ctl[i] = tp.g[i].ctl;
+            rs.blocks[i] = tp.first_block[i + 1] - tp.first_block[i];
+            if (i >= nrun) continue;
+            const int32_t last = i + 1 < nrun ? first_row[i + 1] - 1 : Kstop;
+            rs.span[i] = ((unsigned long long)last << 32) | (unsigned long long)first_row[i];
+            if (i) {
+                rs.seam_row[i] = (uint32_t)first_row[i];
+                rs.seam_at[i] = rs.seam_tail;
+                rs.seam_tail += ck[first_row[i]];
+            }
+        }
+        ++g_launches;
+        k_rows_start<<<1, 512, 0, h->stream>>>(rs, s->plan, s->seam_of, (uint32_t)K + 2);
+    } else {
+        tp.first_block[1] = (unsigned)grid;
     }
     uint64_t nlog = 0;
-    uint64_t nseg_log[kMaxRowSegments] = {}, nseg_used[kMaxRowSegments] = {};
-    unsigned long long voids[kMaxRowSegments] = {};
     cudaEventRecord(h->ev[3], h->stream);
-    if (tp[0].Kstop >= tp[0].K0) {
-        static const char* const kNames[8] = {"transitions",           "transitions (segment 2)",
-                                              "transitions (segment 3)", "transitions (segment 4)",
-                                              "transitions (segment 5)", "transitions (segment 6)",
-                                              "transitions (segment 7)", "transitions (segment 8)"};
-        static_assert(kMaxRowSegments <= 8, "one name per segment");
-        void* args[kMaxRowSegments][1];
-        int launched = 0, rc = DC_OK;
-        for (int i = 0; i < nseg && rc == DC_OK; ++i) {
-            args[i][0] = &tp[i];
-            EngineCtl* ctl = i == 0 ? h->ctl : s->seg[i - 1].ctl;
-            cudaStream_t st = i == 0 ? h->stream : s->seg[i - 1].stream;
-            const FirstStep first{tp[i].K0};
-            rc = persistent_launch(h, (const void*)k_trans2, args[i], kNames[i], ctl, st, h->rows_bps, &first, nseg);
-            if (rc == DC_OK) ++launched;
+    if (Kstop >= k0) {
+        void* args[] = {&tp};
+        const FirstStep first{k0, (int)(tp.first_block[1] - tp.first_block[0])};
+        if (int rc = persistent_launch(h, (const void*)k_trans2, args, "transitions", h->ctl, h->stream, 0, &first, grid))
+            return rc;
+        if (ngroups > 1) {
+            ++g_launches;
+            k_rows_collect<<<1, 1, 0, h->stream>>>(rs, s->plan);
         }
-        h->stat_evals = h->stat_drops = h->stat_entries = 0;
-        for (int i = 0; i < launched; ++i) {
-            EngineCtl hc;
-            EngineCtl* ctl = i == 0 ? h->ctl : s->seg[i - 1].ctl;
-            cudaStream_t st = i == 0 ? h->stream : s->seg[i - 1].stream;
-            const int r = finish_persistent(h, ctl, st, kNames[i], &hc);
-            if (r != DC_OK) {
-                if (rc == DC_OK) rc = r;
-                continue;
-            }
-            nseg_log[i] = hc.log_count;
-            nseg_used[i] = hc.log_used;
-            h->stat_evals += hc.evals;
-            h->stat_drops += hc.drops;
-            h->stat_entries += hc.edges_scanned;
+        if (relabel) {
+            ++g_launches;
+            k_log_finish<<<grid_for(h, lc / 4), kThreads, 0, h->stream>>>(
+                &h->ctl->log_count, s->log_cap, s->order, s->log_v, s->log_k, s->log_l,
+                ngroups > 1 ? s->seam_of : nullptr, s->seam, &h->ctl->pushes);
         }
-        if (rc) return rc;
-        nlog = nseg_log[0];
-        h->log_used = nseg_used[0];
-        if (nseg > 1) {
-            DC_CUDA(cudaMemsetAsync(acc, 0, nseg * sizeof(unsigned long long), h->stream));
-            for (int i = 1; i < nseg; ++i) {
-                RowSegment& sg = s->seg[i - 1];
-                DC_CUDA(cudaEventRecord(sg.ev[1], sg.stream));
-                DC_CUDA(cudaStreamWaitEvent(h->stream, sg.ev[1], 0));
-                if (!nseg_log[i]) continue;
-                // a corner at the segment's first row is void where the value
-                // equals the previous segment's last row
-                const int32_t* prev = i == 1 ? s->cur : s->seg[i - 2].cur;
-                ++g_launches;
-                k_seg_void<<<grid_for(h, nseg_log[i]), kThreads, 0, h->stream>>>(
-                    nseg_log[i], s->log_v + off[i], s->log_k + off[i], s->log_l + off[i], cut[i - 1] + 1, prev,
-                    acc + i);
-            }
-            DC_CUDA(cudaMemcpyAsync(voids, acc, nseg * sizeof(unsigned long long), cudaMemcpyDeviceToHost, h->stream));
-            DC_CUDA(cudaStreamSynchronize(h->stream));
-            h->nseg_extra = nseg - 1;
-            for (int i = 1; i < nseg; ++i) {
-                h->seg_off[i - 1] = off[i];
-                h->seg_n[i - 1] = nseg_log[i];
-                h->seg_void[i - 1] = nseg_log[i] - nseg_used[i] + voids[i];
-            }
+        EngineCtl hc;
+        const int rc = finish_persistent(h, h->ctl, h->stream, "transitions", &hc);
+        if (rc != DC_OK) {
+            for (RowSegment& sg : s->seg)
+                if (sg.tring) cudaMemsetAsync(sg.tring, 0xFF, sizeof(unsigned long long) * sg.tring_cap, h->stream);
+            cudaStreamSynchronize(h->stream);
+            return rc;
         }
-        if (relabel)  // corner records back to original ids (the seam check above compares relabeled state)
-            for (int i = 0; i < nseg; ++i)
-                if (nseg_log[i]) {
-                    ++g_launches;
-                    k_unlabel_log<<<grid_for(h, nseg_log[i]), kThreads, 0, h->stream>>>(nseg_log[i], s->order,
-                                                                                       s->log_v + off[i],
-                                                                                       s->log_k + off[i]);
-                }
+        nlog = hc.log_count;
+        h->log_used = hc.log_used - hc.pushes;
+        h->stat_evals = hc.evals;
+        h->stat_drops = hc.drops;
+        h->stat_entries = hc.edges_scanned;
     }
     cudaEventRecord(h->ev[4], h->stream);
     *nlog_out = nlog;

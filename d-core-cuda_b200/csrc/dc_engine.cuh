@@ -6,9 +6,10 @@
 
 namespace dc {
 
-// One row segment after the first: rows split over concurrent launches,
-// each segment with its own values, counters, marks, ticket ring, control
-// block and stream.
+struct RowPlan;
+
+// State of one group of blocks after the first that works on a run of rows:
+// its own values, counters, marks, ticket ring and control block.
 struct RowSegment {
     uint32_t cap_V = 0;
     int32_t* cur = nullptr;
@@ -20,13 +21,12 @@ struct RowSegment {
     unsigned long long* tring = nullptr;
     uint64_t tring_cap = 0;
     EngineCtl* ctl = nullptr;
-    cudaStream_t stream = nullptr;
-    cudaEvent_t ev[2] = {nullptr, nullptr};
 };
 
 // First step of a kernel whose steps advance without a barrier.
 struct FirstStep {
     int level;
+    int blocks;  // that work on it (0: the grid)
 };
 
 struct Scratch {
@@ -43,8 +43,6 @@ struct Scratch {
     uint32_t* order = nullptr;   // [V] vertices by kmax descending
     uint32_t* ck = nullptr;      // [kmax+2] |C_k|
     uint32_t ck_cap = 0;
-    uint32_t* ring = nullptr;    // ring queue slots
-    uint32_t ring_mask = 0;
     uint32_t* log_v = nullptr;
     int32_t* log_k = nullptr;
     int32_t* log_l = nullptr;
@@ -61,17 +59,16 @@ struct Scratch {
     // ticket-queue ring
     unsigned long long* tring = nullptr;
     uint64_t tring_cap = 0;
-    // prunable working copies of the adjacency
-    int32_t* w_out_len = nullptr;
-    int32_t* w_in_len = nullptr;
-    uint32_t* w_out_nbr = nullptr;
-    uint32_t* w_in_nbr = nullptr;
-    uint64_t w_out_cap = 0, w_in_cap = 0;
     // maintenance
     int32_t* kmax_old = nullptr;  // [V]
     int32_t* row0_old = nullptr;  // [V]
-    // row segments after the first (rows split over concurrent launches)
-    RowSegment seg[kMaxRowSegments - 1];
+    // row groups after the first, and what the groups share
+    RowSegment seg[kRowGroups - 1];
+    RowPlan* plan = nullptr;
+    uint32_t* seam_of = nullptr;
+    uint32_t seam_of_cap = 0;
+    int32_t* seam = nullptr;
+    uint64_t seam_cap = 0;
     // the graph relabeled in kmax-descending order for the row kernel:
     // new id = position in `order`; lists of new ids sorted by neighbour kmax
     uint32_t* pos = nullptr;                    // [V] new id of each vertex
@@ -158,11 +155,9 @@ int decompose(dc_graph* h, int method, int materialize_rows);
 // step is the fixpoint of row K0 below row 0, so the corners it logs at K0
 // are relative to row 0 and rows 1..K0-1 of the resulting skyline are not
 // meaningful.
-// allow_relabel: with sorting allowed, run on the graph relabeled in kmax
-// order (whole decompositions and row ranges); else sort the handle's lists
-// in place (maintenance recomputations, whose graph changes every batch).
-int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint64_t* nlog_out, int32_t K0 = 1,
-                   bool allow_relabel = true);
+// allow_sort: run on the graph relabeled in kmax order with its lists in id
+// order (runs of many rows), else on the handle's lists as they are.
+int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint64_t* nlog_out, int32_t K0 = 1);
 // kmax and row 0 (fused peel) when k_first <= 0 or not current, then rows
 // max(k_first, 1)..min(k_last, kmax) only; the decomposition then holds row 0
 // and that range.
@@ -199,7 +194,6 @@ int scan_tmp64(dc_graph* h, uint64_t n);
 // Skyline from row 0 and the corner log: entries [0, nlog) and, when a second
 // row segment ran, [off2, off2 + n2).
 int build_skyline_from_log(dc_graph* h, uint64_t nlog);
-int prepare_row_segments(dc_graph* h);
 // Spare skyline buffers (slot 0 or 1): take hands over the slot's buffers with
 // room for at least n corners and V + 1 offsets (allocated or grown with a
 // quarter of headroom; the slot is left empty); put returns buffers to a slot

@@ -39,7 +39,6 @@ struct DevGraph {
     // 16-byte boundary inside them: the row kernel reads ids 16 bytes at a time)
     uint32_t* out_nbr_alloc = nullptr;
     uint32_t* in_nbr_alloc = nullptr;
-    bool sorted_kmax = false;  // lists ordered by neighbour kmax of the current graph
 };
 
 // Persistent-kernel launch geometry for the current device.
@@ -124,12 +123,7 @@ struct dc_graph {
     // each nonzero entry (ascending), segments run concurrently
     int rows_split[dc::kMaxRowSegments - 1] = {};
     bool auto_cuts = true;  // launch shapes never set: cuts by the rule in rows_from_row0
-    // corner logs of the segments after the first from the last run:
-    // [seg_off[i], seg_off[i] + seg_n[i]), seg_void[i] entries voided (row k < 0)
-    int nseg_extra = 0;
-    uint64_t log_used = 0;  // records of the first segment's log (its other entries are void)
-    uint64_t seg_off[dc::kMaxRowSegments - 1] = {}, seg_n[dc::kMaxRowSegments - 1] = {},
-             seg_void[dc::kMaxRowSegments - 1] = {};
+    uint64_t log_used = 0;  // records in the last run's corner log (its other entries are void)
     uint64_t stat_evals = 0, stat_drops = 0, stat_entries = 0;
     uint64_t full_work = 0;  // sum over vertices of degree x kmax at the last full decomposition
     float full_rows_ms = 0;  // rows phase (rows 1..kmax) of the last full decomposition
@@ -146,7 +140,6 @@ struct dc_graph {
     uint64_t cb_words = 0;                 // capacity of cb_host / cb_dev in words (status excluded)
     cudaGraphExec_t cb_exec[2] = {};       // deletion / insertion batch graphs (updated per batch)
     dc::EngineCtl ctl_init{};
-    dc::EngineCtl ctl_init_seg[dc::kMaxRowSegments - 1] = {};  // the other row segments'
     // optional per-step trace of persistent kernels (diagnostics)
     unsigned long long* trace_dev = nullptr;
     unsigned long long* trace_host = nullptr;

@@ -938,7 +938,6 @@ static int apply_deletions(dc_graph* h, const NetBatch& nb) {
     rc = check_ctl(h, &hc, "dc_maintain: deletion apply");
     if (rc != DC_OK) return rc;
     g.E -= nb.n_del;
-    g.sorted_kmax = false;
     return DC_OK;
 }
 
@@ -1020,7 +1019,6 @@ static int apply_insertions(dc_graph* h, const NetBatch& nb, uint32_t** d_iu_out
         mt_free(h->stream, iu); mt_free(h->stream, iv);
         return rc;
     }
-    g.sorted_kmax = false;
     *d_iu_out = iu;
     *d_iv_out = iv;
     return DC_OK;
@@ -1449,7 +1447,6 @@ static int maintain_captured(dc_graph* h, const NetBatch& nb, int rmode, dc_main
     }
     if (a.ins) g.E += nb.n_ins;
     else g.E -= nb.n_del;
-    g.sorted_kmax = false;
     st->method = DC_MAINT_LOCAL;
     st->region = r.region + (a.ins ? 0 : 2ull * a.n);
     st->rows_recomputed = r.R + 1;

@@ -91,25 +91,25 @@ namespace {
 
 // Upper bound on the device bytes a handle of V vertices and E edges can
 // hold, transients of maintenance included: slack adjacency under the
-// rebuild rule (len + len/8 + 2 per list) with its kmax-sort working copies,
-// offsets and lengths, kmax/row 0, the skyline twice (old and merged during a
-// batch), per-vertex scratch, the vertex ring and ticket ring (powers of two),
-// the corner log (at most E + V corners) and rebuild staging.
+// rebuild rule (len + len/8 + 2 per list), offsets and lengths, kmax/row 0,
+// the skyline twice (old and merged during a batch), per-vertex scratch, the
+// ticket ring (a power of two), the corner log (at most E + V corners) and
+// rebuild staging.
 uint64_t footprint_bound(uint64_t V, uint64_t E, uint64_t sms) {
     const uint64_t cap = E + E / 8 + 2 * V + 64;
-    uint64_t b = 2 * 4 * cap * 2;
+    uint64_t b = 2 * 4 * cap;
     b += 4 * 4 * (V + 1);
     b += 4 * 3 * (V + 1) + 3 * (8 * (E + 2 * V) + 4 * (V + 1));  // skyline and its two spares
     b += 4 * 20 * (V + 2) + 8 * (V + 2) + 8 * (sms * 64 + 64);
-    b += 8 * (V + sms * 64 * 32 + 64);
     b += 12 * (E + V + 1);
     b += 16 * (2 * V + 2 * cap / 32 + sms * 64 + 4096);
     b += 8 * E + 2 * 4 * cap;
     b += 4 * 7 * (V + 1) + 2 * 4 * ((E + 8) + (E + 8) / 8 + 7);  // the row kernel's relabeled graph
-    // row segments: state of at most V / 2 vertices together (27 bytes each)
-    // and their ticket rings (powers of two), control blocks, the log's spare
-    // records
-    b += 30 * V + (3ull << 20);
+    // row groups: state (24 bytes and an eighth), ticket rings (powers of two)
+    // and seams (with their void records) for an eighth of the vertices, a
+    // quarter up to 65,536; control blocks and the log's spare records
+    const uint64_t n = std::max<uint64_t>(V / 8, std::min<uint64_t>(V / 4, 65536));
+    b += 7 * (27 * n + 8 * (4 * n + 32768)) + 18 * 16 * n + (2ull << 20);
     return b + (1ull << 20);
 }
 
