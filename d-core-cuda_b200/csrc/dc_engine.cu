@@ -163,16 +163,51 @@ __global__ void k_scan_coop(unsigned long long* data, uint64_t n, unsigned long 
 // ---------------------------------------------------------------------------
 // graph build
 // ---------------------------------------------------------------------------
+// Edge lists usually come grouped by source (files, generators, a rebuilt
+// store): a warp takes 128 consecutive edges, and each run of equal sources in
+// a row of 32 is one atomic.  Bound by L2 atomics (65 M edges: one per edge and
+// side took 1.0 ms to count and 2.2 ms to place); ungrouped edges form runs
+// of one.
+// Lane's place in its run of equal x and the run's length; lanes of a run are
+// consecutive.
+__device__ __forceinline__ void warp_run(uint32_t x, unsigned* first, unsigned* length) {
+    const unsigned lane = threadIdx.x & 31u;
+    const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, x, 1);
+    const unsigned heads = __ballot_sync(0xFFFFFFFFu, lane == 0 || x != prev);
+    *first = 31u - __clz(heads & (0xFFFFFFFFu >> (31u - lane)));
+    const unsigned after = lane == 31 ? 0u : heads & (0xFFFFFFFFu << (lane + 1u));
+    *length = (after ? __ffs(after) - 1u : 32u) - *first;
+}
+
 __global__ void k_count_degrees(uint32_t V, uint64_t E, const uint32_t* src, const uint32_t* dst, int32_t* out_len,
                                 int32_t* in_len, EngineCtl* c) {
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t s = src[e], d = dst[e];
-        if (s >= V || d >= V) {
-            set_dev_error(c, DC_DEV_ERR_BADID, 10);
-            continue;
+    const unsigned lane = threadIdx.x & 31u;
+    const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t b = gw * 128; b < E; b += nw * 128) {
+        uint32_t s[4], d[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const uint64_t e = b + 32 * r + lane;
+            s[r] = d[r] = 0xFFFFFFFFu;
+            if (e < E) {
+                s[r] = src[e];
+                d[r] = dst[e];
+                if (s[r] >= V || d[r] >= V) {
+                    set_dev_error(c, DC_DEV_ERR_BADID, 10);
+                    s[r] = d[r] = 0xFFFFFFFFu;
+                }
+            }
         }
-        atomicAdd(&out_len[s], 1);
-        atomicAdd(&in_len[d], 1);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            unsigned first, length;
+            warp_run(s[r], &first, &length);
+            if (s[r] != 0xFFFFFFFFu) {
+                if (first == lane) atomicAdd(&out_len[s[r]], (int)length);
+                atomicAdd(&in_len[d[r]], 1);
+            }
+        }
     }
 }
 
@@ -194,12 +229,40 @@ __global__ void k_off_to_u32(uint32_t V, const unsigned long long* in, uint32_t*
 __global__ void k_scatter_edges(uint64_t E, const uint32_t* src, const uint32_t* dst, const uint32_t* out_off,
                                 int32_t* out_fill, uint32_t* out_nbr, const uint32_t* in_off, int32_t* in_fill,
                                 uint32_t* in_nbr) {
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < E; e += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t s = src[e], d = dst[e];
-        int po = atomicAdd(&out_fill[s], 1);
-        out_nbr[out_off[s] + po] = d;
-        int pi = atomicAdd(&in_fill[d], 1);
-        in_nbr[in_off[d] + pi] = s;
+    const unsigned lane = threadIdx.x & 31u;
+    const uint64_t gw = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t b = gw * 128; b < E; b += nw * 128) {
+        uint32_t s[4], d[4], oo[4], io[4];
+        unsigned first[4];
+        int po[4], pi[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const uint64_t e = b + 32 * r + lane;
+            s[r] = e < E ? src[e] : 0xFFFFFFFFu;
+            d[r] = e < E ? dst[e] : 0xFFFFFFFFu;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            unsigned length;
+            warp_run(s[r], &first[r], &length);
+            po[r] = pi[r] = 0;
+            oo[r] = io[r] = 0;
+            if (s[r] != 0xFFFFFFFFu) {
+                if (first[r] == lane) po[r] = atomicAdd(&out_fill[s[r]], (int)length);
+                pi[r] = atomicAdd(&in_fill[d[r]], 1);
+                oo[r] = out_off[s[r]];
+                io[r] = in_off[d[r]];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int at = __shfl_sync(0xFFFFFFFFu, po[r], first[r]) + (int)(lane - first[r]);
+            if (s[r] != 0xFFFFFFFFu) {
+                out_nbr[oo[r] + (uint32_t)at] = d[r];
+                in_nbr[io[r] + (uint32_t)pi[r]] = s[r];
+            }
+        }
     }
 }
 
@@ -1594,44 +1657,50 @@ __global__ void k_sort_short(uint32_t V, const uint32_t* off, const int32_t* len
     }
 }
 
-// One warp per list of kSortShort+1 .. 32 T entries: bitonic sort in
-// registers (entry 32 t + lane in k[t]; the places past the end hold the
-// largest value and stay last).  240 shuffles for 256 entries, where ranking
-// every entry against every other took 2,048 comparisons per lane.
+// Bitonic stages size (compile time, > 1) with strides from..1 on 32 T
+// entries in registers, entry 32 t + lane in k[t]; `at` = index of the first
+// entry in the whole list (a multiple of 32 T).
 template <int T>
-__device__ __forceinline__ void warp_sort(const uint32_t* in, const uint32_t* pos, int n, uint32_t* a) {
-    const unsigned lane = threadIdx.x & 31u;
-    uint32_t k[T];
+__device__ __forceinline__ void warp_stages(uint32_t k[T], int size, int from, int at) {
+    const int lane = (int)(threadIdx.x & 31u);
 #pragma unroll
-    for (int t = 0; t < T; ++t) k[t] = 32 * t + (int)lane < n ? in[32 * t + lane] : 0xFFFFFFFFu;
+    for (int stride = 16 * T; stride; stride >>= 1) {
+        if (stride > from) continue;
 #pragma unroll
-    for (int t = 0; t < T; ++t)
-        if (32 * t + (int)lane < n) k[t] = pos[k[t]];
-#pragma unroll
-    for (int size = 2; size <= 32 * T; size <<= 1) {
-#pragma unroll
-        for (int stride = size >> 1; stride; stride >>= 1) {
-#pragma unroll
-            for (int t = 0; t < T; ++t) {
-                if (stride >= 32) {
-                    const int o = t ^ (stride >> 5);
-                    if (o > t) {
-                        const bool up = ((32 * t) & size) == 0;  // size > 32 here
-                        const uint32_t lo = min(k[t], k[o]), hi = max(k[t], k[o]);
-                        k[t] = up ? lo : hi;
-                        k[o] = up ? hi : lo;
-                    }
-                } else {
-                    const bool up = ((32 * t + (int)lane) & size) == 0;
-                    const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, k[t], stride);
-                    k[t] = ((lane & stride) == 0) == up ? min(k[t], o) : max(k[t], o);
+        for (int t = 0; t < T; ++t) {
+            const bool up = ((at + 32 * t + lane) & size) == 0;
+            if (stride >= 32) {
+                const int o = t ^ (stride >> 5);
+                if (o > t) {
+                    const uint32_t lo = min(k[t], k[o]), hi = max(k[t], k[o]);
+                    k[t] = up ? lo : hi;
+                    k[o] = up ? hi : lo;
                 }
+            } else {
+                const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, k[t], stride);
+                k[t] = ((lane & stride) == 0) == up ? min(k[t], o) : max(k[t], o);
             }
         }
     }
+}
+// One warp per list of kSortShort+1 .. 32 T entries: bitonic sort in
+// registers (the places past the end hold the largest value and stay last).
+// 240 shuffles for 256 entries, where ranking every entry against every other
+// took 2,048 comparisons per lane.
+template <int T>
+__device__ __forceinline__ void warp_sort(const uint32_t* in, const uint32_t* pos, int n, uint32_t* a) {
+    const int lane = (int)(threadIdx.x & 31u);
+    uint32_t k[T];
+#pragma unroll
+    for (int t = 0; t < T; ++t) k[t] = 32 * t + lane < n ? in[32 * t + lane] : 0xFFFFFFFFu;
 #pragma unroll
     for (int t = 0; t < T; ++t)
-        if (32 * t + (int)lane < n) a[32 * t + lane] = k[t];
+        if (32 * t + lane < n) k[t] = pos[k[t]];
+#pragma unroll
+    for (int size = 2; size <= 32 * T; size <<= 1) warp_stages<T>(k, size, size >> 1, 0);
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+        if (32 * t + lane < n) a[32 * t + lane] = k[t];
 }
 __global__ void __launch_bounds__(kSortThreads) k_sort_warp(const uint32_t* off, const int32_t* len, uint32_t* nbr,
                                                              const uint32_t* list, const unsigned* n_list,
@@ -1649,39 +1718,64 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_warp(const uint32_t* off,
     }
 }
 
-// One block per list of kSortWarp+1 .. kSortMid entries: bitonic sort in
-// shared memory.
+// One block per list of kSortWarp+1 .. kSortMid entries: bitonic sort.  Runs of
+// 256 entries are sorted in registers by a warp each; of the later stages only
+// the strides of 256 and more go through shared memory (10 block-wide passes
+// for 4,096 entries instead of 78).
 __global__ void __launch_bounds__(kSortThreads) k_sort_mid(const uint32_t* off, const int32_t* len, uint32_t* nbr,
                                                             const uint32_t* list, const unsigned* n_list,
                                                             ListSrc src) {
-    __shared__ uint32_t k[kSortMid];
+    __shared__ uint32_t s[kSortMid];
+    const int lane = (int)(threadIdx.x & 31u), w = (int)(threadIdx.x >> 5);
     const unsigned nl = *n_list;
     for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
         const uint32_t v = list[li];
         const int n = len[v];
         uint32_t* a = nbr + off[v];
         const uint32_t* in = src_list(src, v);
-        int N = 2 * kSortWarp;
+        int N = 512;
         while (N < n) N <<= 1;
-        for (int i = threadIdx.x; i < N; i += kSortThreads) k[i] = i < n ? src.pos[in[i]] : 0xFFFFFFFFu;
+        for (int c = 256 * w; c < N; c += 8 * kSortThreads) {  // one run per warp and turn
+            uint32_t k[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) k[t] = c + 32 * t + lane < n ? in[c + 32 * t + lane] : 0xFFFFFFFFu;
+#pragma unroll
+            for (int t = 0; t < 8; ++t)
+                if (c + 32 * t + lane < n) k[t] = src.pos[k[t]];
+#pragma unroll
+            for (int size = 2; size <= 256; size <<= 1) warp_stages<8>(k, size, size >> 1, c);
+#pragma unroll
+            for (int t = 0; t < 8; ++t) s[c + 32 * t + lane] = k[t];
+        }
         __syncthreads();
-        for (int size = 2; size <= N; size <<= 1)
-            for (int stride = size >> 1; stride; stride >>= 1) {
+        for (int size = 512; size <= N; size <<= 1) {
+            for (int stride = size >> 1; stride >= 256; stride >>= 1) {
                 for (int p = threadIdx.x; p < N / 2; p += kSortThreads) {
                     const int i = ((p & ~(stride - 1)) << 1) | (p & (stride - 1)), o = i | stride;
-                    const uint32_t x = k[i], y = k[o];
+                    const uint32_t x = s[i], y = s[o];
                     if ((x > y) == ((i & size) == 0)) {
-                        k[i] = y;
-                        k[o] = x;
+                        s[i] = y;
+                        s[o] = x;
                     }
                 }
-                // pairs up to 32 apart stay within a warp's 64 entries
-                if (stride > 32) __syncthreads();
-                else __syncwarp();
-                if (stride == 1) __syncthreads();
+                __syncthreads();
             }
-        for (int i = threadIdx.x; i < n; i += kSortThreads) a[i] = k[i];
-        __syncthreads();
+            for (int c = 256 * w; c < N; c += 8 * kSortThreads) {
+                uint32_t k[8];
+#pragma unroll
+                for (int t = 0; t < 8; ++t) k[t] = s[c + 32 * t + lane];
+                warp_stages<8>(k, size, 128, c);
+                if (size < N) {
+#pragma unroll
+                    for (int t = 0; t < 8; ++t) s[c + 32 * t + lane] = k[t];
+                } else {
+#pragma unroll
+                    for (int t = 0; t < 8; ++t)
+                        if (c + 32 * t + lane < n) a[c + 32 * t + lane] = k[t];
+                }
+            }
+            __syncthreads();
+        }
     }
 }
 
@@ -1704,7 +1798,21 @@ __global__ void k_sort_big(const uint32_t* off, const int32_t* len, uint32_t* nb
         const uint32_t* in = src_list(src, v);
         for (int i = threadIdx.x; i < kSortBigBins; i += blockDim.x) bins[i] = 0;
         __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) atomicAdd(&bins[bin_of(src.pos[in[i]])], 1u);
+        // four entries in flight per thread (three dependent loads each)
+        for (int i0 = threadIdx.x; i0 < n; i0 += 4 * blockDim.x) {
+            uint32_t u[4];
+            int b[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) u[q] = i0 + q * (int)blockDim.x < n ? in[i0 + q * blockDim.x] : 0xFFFFFFFFu;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (u[q] != 0xFFFFFFFFu) u[q] = src.pos[u[q]];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) b[q] = u[q] != 0xFFFFFFFFu ? bin_of(u[q]) : -1;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (b[q] >= 0) atomicAdd(&bins[b[q]], 1u);
+        }
         __syncthreads();
         // exclusive scan of the bins, blockDim at a time
         unsigned long long carry = 0;
@@ -1717,9 +1825,19 @@ __global__ void k_sort_big(const uint32_t* off, const int32_t* len, uint32_t* nb
             carry += tot;
             __syncthreads();
         }
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint32_t u = src.pos[in[i]];
-            a[atomicAdd(&bins[bin_of(u)], 1u)] = u;
+        for (int i0 = threadIdx.x; i0 < n; i0 += 4 * blockDim.x) {
+            uint32_t u[4];
+            int b[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) u[q] = i0 + q * (int)blockDim.x < n ? in[i0 + q * blockDim.x] : 0xFFFFFFFFu;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (u[q] != 0xFFFFFFFFu) u[q] = src.pos[u[q]];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) b[q] = u[q] != 0xFFFFFFFFu ? bin_of(u[q]) : -1;
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (b[q] >= 0) a[atomicAdd(&bins[b[q]], 1u)] = u[q];
         }
         __syncthreads();
     }

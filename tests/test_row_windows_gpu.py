@@ -59,3 +59,33 @@ def test_many_leavers(dc, orc, gpu):
         g.decompose()
         assert np.array_equal(g.kmaxes(), okmaxes)
         assert np.array_equal(g.rows(), orows)
+
+
+def test_list_sizes(dc, orc, gpu):
+    """Out-lists and in-lists of every size where the list sorts change method
+    or padding, over neighbours of many different kmax; the edges given grouped
+    by source, shuffled, and with parallel edges."""
+    rng = np.random.default_rng(11)
+    sizes = [1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1025, 2047, 2049, 4095, 4096,
+             4097, 9000]
+    V0 = 9500
+    V = V0 + 2 * len(sizes)
+    e = [rng.integers(0, 60, (2500, 2)), rng.integers(0, 700, (14000, 2)), rng.integers(0, V0, (30000, 2))]
+    for i, n in enumerate(sizes):
+        pick = rng.permutation(V0)[:n]
+        e.append(np.stack([np.full(n, V0 + 2 * i), pick], 1))
+        e.append(np.stack([pick[::-1], np.full(n, V0 + 2 * i + 1)], 1))
+        e.append(np.array([[V0 + 2 * i + 1, V0 + 2 * i], [pick[0], V0 + 2 * i]]))
+    e = np.unique(np.concatenate(e), axis=0)
+    e = e[e[:, 0] != e[:, 1]].astype(np.uint32)
+    doubled = np.concatenate([e, e[::50], e[::50]])
+    for edges in (e, e[rng.permutation(len(e))], doubled[rng.permutation(len(doubled))]):
+        s, d = np.ascontiguousarray(edges[:, 0]), np.ascontiguousarray(edges[:, 1])
+        _, _, okmaxes, orows = orc.dcore(V, s, d)
+        with dc.Graph.from_edges(V, s, d) as g:
+            g.decompose()
+            assert np.array_equal(g.kmaxes(), okmaxes)
+            assert np.array_equal(g.rows(), orows)
+            gs, gd = g.edges()
+            o, q = np.lexsort((d, s)), np.lexsort((gd, gs))
+            assert np.array_equal(gs[q], s[o]) and np.array_equal(gd[q], d[o])
