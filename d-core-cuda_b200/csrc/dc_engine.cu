@@ -2277,7 +2277,7 @@ uint64_t device_footprint(const dc_graph* h) {
     if (const Scratch* s = h->scratch) {
         uint64_t n = (uint64_t)s->cap_V + 1;
         if (s->key) b += 4 * (16 * n + 1) + 8 * (n + 1) + 8 * ((uint64_t)h->geom.sms * 64 + 64);
-        b += 4ull * s->ck_cap + 12 * s->log_cap + 8 * s->tring_cap;
+        b += 8ull * s->ck_cap + 12 * s->log_cap + 8 * s->tring_cap;
         if (s->kmax_old) b += 8 * n;
         for (const RowSegment& sg : s->seg)
             b += (sg.cur ? 24 * ((uint64_t)sg.cap_V + 1) : 0) + 8 * sg.tring_cap + (sg.ctl ? sizeof(EngineCtl) : 0);
@@ -2930,10 +2930,11 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     cudaEventRecord(h->ev[2], h->stream);
     if (s->ck_cap < (uint32_t)K + 2) {
         dfree(h->stream, s->ck);
-        if (dmalloc(h->stream, &s->ck, (uint64_t)K + 2)) return DC_ERR_NOMEM;
+        s->ck_cap = 0;
+        if (dmalloc(h->stream, &s->ck, 2 * ((uint64_t)K + 2))) return DC_ERR_NOMEM;
         s->ck_cap = K + 2;
     }
-    uint32_t* hist = s->cursor;
+    uint32_t* hist = s->ck + s->ck_cap;  // K exceeds V where edges are parallel: no vertex-sized array holds it
     DC_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * ((uint64_t)K + 2), h->stream));
     ++g_launches;
     k_kmax_hist<<<grid_for(h, V), kThreads, K + 1 <= kHistShared ? 4 * (K + 1) : 0, h->stream>>>(V, d.kmax_v, hist, K);
