@@ -31,6 +31,7 @@
 
 #include "dc_engine.cuh"
 #include "dc_internal.h"
+#include "dc_netbatch.cuh"
 
 namespace dc {
 
@@ -746,15 +747,23 @@ struct NetBatch {
     uint64_t n_del = 0, n_ins = 0;
 };
 
+static int bad_id(uint32_t V, const uint32_t* pairs, uint64_t i) {
+    return set_error(DC_ERR_INVALID, "dc_maintain: edge %llu (%u, %u) has a vertex id >= V=%u", (unsigned long long)i,
+                     pairs[2 * i], pairs[2 * i + 1], V);
+}
+
+// Batches of at least this many updates are reduced on the device where the
+// full path takes them: 4,096 updates cost the host 0.5 ms (sort, groups) and
+// the device 0.4.
+static constexpr uint64_t kDeviceNetMin = 4096;
+
 // Net effect of a batch under sequential semantics: per distinct (u, v),
 // occurrences inserted minus occurrences deleted.
 static int net_batch(uint32_t V, const uint32_t* pairs, const uint8_t* is_del, uint64_t b, NetBatch& nb) {
     std::vector<uint64_t> key(b);
     for (uint64_t i = 0; i < b; ++i) {
         uint32_t u = pairs[2 * i], v = pairs[2 * i + 1];
-        if (u >= V || v >= V)
-            return set_error(DC_ERR_INVALID, "dc_maintain: edge %llu (%u, %u) has a vertex id >= V=%u",
-                             (unsigned long long)i, u, v, V);
+        if (u >= V || v >= V) return bad_id(V, pairs, i);
         key[i] = ((uint64_t)u << 32) | v;
     }
     std::vector<uint64_t> idx(b);
@@ -879,65 +888,69 @@ static void group_by(const std::vector<uint32_t>& key, const std::vector<uint32_
     goff.push_back((uint32_t)gnbr.size());
 }
 
-// Applies the validated deletions to both adjacency sides.
-static int apply_deletions(dc_graph* h, const NetBatch& nb) {
+// Applies grouped deletions to both adjacency sides, once all of them are in
+// the graph.
+static int apply_deletions(dc_graph* h, DeviceBatch& d) {
     DevGraph& g = h->g;
-    if (nb.del_u.empty()) return DC_OK;
     int rc = DC_OK;
-    uint32_t *du = nullptr, *dv = nullptr;
-    int32_t* dn = nullptr;
-    if ((rc = upload(h, &du, nb.del_u)) || (rc = upload(h, &dv, nb.del_v)) || (rc = upload(h, &dn, nb.del_n))) {
-        mt_free(h->stream, du); mt_free(h->stream, dv); mt_free(h->stream, dn);
-        return rc;
-    }
     MT_CUDA(cudaMemsetAsync(h->ctl, 0, sizeof(EngineCtl), h->stream));
     if (h->wait_ns)
         MT_CUDA(cudaMemcpyAsync(&h->ctl->wait_ns, &h->wait_ns, sizeof(h->wait_ns), cudaMemcpyHostToDevice, h->stream));
     ++g_launches;
-    k_del_validate<<<mgrid(h, nb.del_u.size() * 32), kMThreads, 0, h->stream>>>(
-        (uint32_t)nb.del_u.size(), du, dv, dn, g.out_off, g.out_len, g.out_nbr, h->ctl);
+    k_del_validate<<<mgrid(h, d.n_pairs * 32ull), kMThreads, 0, h->stream>>>(d.n_pairs, d.del_u, d.del_v, d.del_n,
+                                                                             g.out_off, g.out_len, g.out_nbr, h->ctl);
     EngineCtl hc;
     rc = check_ctl(h, &hc, "dc_maintain: deletion check");
-    mt_free(h->stream, du);
-    mt_free(h->stream, dv);
-    mt_free(h->stream, dn);
     if (rc != DC_OK) {
         if (hc.error & DC_DEV_ERR_NOTFOUND)
             return set_error(DC_ERR_NOT_FOUND, "dc_maintain: a deleted edge is not in the graph (batch not applied)");
         return rc;
     }
+    uint32_t* pos = nullptr;
+    if ((rc = mt_malloc(h->stream, &pos, d.n_del))) return rc;
     for (int side = 0; side < 2; ++side) {
-        std::vector<uint32_t> gvert, goff, gnbr;
-        if (side == 0) group_by(nb.del_u, nb.del_v, nb.del_n, gvert, goff, gnbr);
-        else group_by(nb.del_v, nb.del_u, nb.del_n, gvert, goff, gnbr);
-        std::vector<uint32_t> gof(gnbr.size());
-        for (size_t q = 0; q + 1 < goff.size(); ++q)
-            for (uint32_t t = goff[q]; t < goff[q + 1]; ++t) gof[t] = gvert[q];
-        uint32_t *d_gv = nullptr, *d_go = nullptr, *d_gn = nullptr, *d_gof = nullptr, *d_pos = nullptr;
-        auto release = [&]() {
-            mt_free(h->stream, d_gv); mt_free(h->stream, d_go); mt_free(h->stream, d_gn);
-            mt_free(h->stream, d_gof); mt_free(h->stream, d_pos);
-        };
-        if ((rc = upload(h, &d_gv, gvert)) || (rc = upload(h, &d_go, goff)) || (rc = upload(h, &d_gn, gnbr)) ||
-            (rc = upload(h, &d_gof, gof)) || (rc = mt_malloc(h->stream, &d_pos, gnbr.size()))) {
-            release();
-            return rc;
-        }
         const uint32_t* off = side == 0 ? g.out_off : g.in_off;
         int32_t* len = side == 0 ? g.out_len : g.in_len;
         uint32_t* nbr = side == 0 ? g.out_nbr : g.in_nbr;
         g_launches += 2;
-        k_del_find<<<mgrid(h, gnbr.size() * 32), kMThreads, 0, h->stream>>>((uint32_t)gnbr.size(), d_gof, d_gn, off,
-                                                                            len, nbr, d_pos, h->ctl);
-        k_del_close<<<mgrid(h, gvert.size() * 32), kMThreads, 0, h->stream>>>(
-            (uint32_t)gvert.size(), d_gv, d_go, d_gn, off, len, nbr, d_pos, h->ctl);
-        cudaError_t e = cudaStreamSynchronize(h->stream);
-        release();
-        if (e != cudaSuccess) return set_error(DC_ERR_CUDA, "deletion apply: %s", cudaGetErrorString(e));
+        k_del_find<<<mgrid(h, d.n_del * 32ull), kMThreads, 0, h->stream>>>(d.n_del, d.gof[side], d.gnbr[side], off, len,
+                                                                          nbr, pos, h->ctl);
+        k_del_close<<<mgrid(h, d.ngroups[side] * 32ull), kMThreads, 0, h->stream>>>(
+            d.ngroups[side], d.gvert[side], d.goff[side], d.gnbr[side], off, len, nbr, pos, h->ctl);
     }
+    mt_free(h->stream, pos);
     rc = check_ctl(h, &hc, "dc_maintain: deletion apply");
     if (rc != DC_OK) return rc;
-    g.E -= nb.n_del;
+    g.E -= d.n_del;
+    return DC_OK;
+}
+
+// The host's net batch in device memory.
+static int upload_batch(dc_graph* h, const NetBatch& nb, DeviceBatch* d) {
+    d->n_pairs = (uint32_t)nb.del_u.size();
+    d->n_del = (uint32_t)nb.n_del;
+    d->n_ins = (uint32_t)nb.ins_u.size();
+    int rc = DC_OK;
+    if (d->n_pairs) {
+        if ((rc = upload(h, &d->del_u, nb.del_u)) || (rc = upload(h, &d->del_v, nb.del_v)) ||
+            (rc = upload(h, &d->del_n, nb.del_n)))
+            return rc;
+        for (int side = 0; side < 2; ++side) {
+            std::vector<uint32_t> gvert, goff, gnbr;
+            if (side == 0) group_by(nb.del_u, nb.del_v, nb.del_n, gvert, goff, gnbr);
+            else group_by(nb.del_v, nb.del_u, nb.del_n, gvert, goff, gnbr);
+            std::vector<uint32_t> gof(gnbr.size());
+            for (size_t q = 0; q + 1 < goff.size(); ++q)
+                for (uint32_t t = goff[q]; t < goff[q + 1]; ++t) gof[t] = gvert[q];
+            d->ngroups[side] = (uint32_t)gvert.size();
+            if ((rc = upload(h, &d->gvert[side], gvert)) || (rc = upload(h, &d->goff[side], goff)) ||
+                (rc = upload(h, &d->gnbr[side], gnbr)) || (rc = upload(h, &d->gof[side], gof)))
+                return rc;
+            MT_CUDA(cudaStreamSynchronize(h->stream));  // the host arrays end here
+        }
+    }
+    if (d->n_ins)
+        if ((rc = upload(h, &d->ins_u, nb.ins_u)) || (rc = upload(h, &d->ins_v, nb.ins_v))) return rc;
     return DC_OK;
 }
 
@@ -967,7 +980,14 @@ static int rebuild_store(dc_graph* h, const uint32_t* d_iu, const uint32_t* d_iv
     Decomp keep = h->d;
     h->d = Decomp();
     uint32_t gm = h->gap_min, gd = h->gap_div;
-    h->gap_min = std::max<uint32_t>(gm, 2);
+    // free slots per list (2 to 8) that a batch like this one is not expected
+    // to outgrow: with lambda = insertions per vertex, fewer than one list in
+    // twenty batches receives more (Poisson).  With two, batches of 250,000
+    // updates rebuilt the store every time (R-MAT 22, 15-20 ms).
+    uint32_t slots = 2;
+    const double lambda = (double)n_ins / std::max<uint32_t>(V, 1);
+    for (double p = lambda * lambda * lambda / 6.0; slots < 8 && p * V > 0.05; p *= lambda / (slots + 1)) ++slots;
+    h->gap_min = std::max<uint32_t>(gm, slots);
     h->gap_div = gd ? std::min<uint32_t>(gd, 8) : 8;
     int rc = build_from_device_edges(h, V, E, src, dst);
     cudaStreamSynchronize(h->stream);
@@ -979,20 +999,13 @@ static int rebuild_store(dc_graph* h, const uint32_t* d_iu, const uint32_t* d_iv
 }
 
 // Inserts the net insertions; returns 1 in *rebuilt when the store grew.
-static int apply_insertions(dc_graph* h, const NetBatch& nb, uint32_t** d_iu_out, uint32_t** d_iv_out, int* rebuilt) {
+static int apply_insertions(dc_graph* h, const DeviceBatch& d, int* rebuilt) {
     DevGraph& g = h->g;
     Scratch* s = h->scratch;
-    const uint32_t V = g.V;
+    const uint32_t V = g.V, n = d.n_ins;
+    const uint32_t *iu = d.ins_u, *iv = d.ins_v;
     *rebuilt = 0;
-    *d_iu_out = *d_iv_out = nullptr;
-    if (nb.ins_u.empty()) return DC_OK;
-    uint32_t *iu = nullptr, *iv = nullptr;
     int rc = DC_OK;
-    if ((rc = upload(h, &iu, nb.ins_u)) || (rc = upload(h, &iv, nb.ins_v))) {
-        mt_free(h->stream, iu); mt_free(h->stream, iv);
-        return rc;
-    }
-    const uint32_t n = (uint32_t)nb.ins_u.size();
     MT_CUDA(cudaMemsetAsync(s->key2, 0, 4ull * V, h->stream));
     MT_CUDA(cudaMemsetAsync(s->cdeg2, 0, 4ull * V, h->stream));
     MT_CUDA(cudaMemsetAsync(h->ctl, 0, sizeof(EngineCtl), h->stream));
@@ -1015,13 +1028,7 @@ static int apply_insertions(dc_graph* h, const NetBatch& nb, uint32_t** d_iu_out
                                                               g.in_len, g.in_nbr, nullptr);
         g.E += n;
     }
-    if (rc != DC_OK) {
-        mt_free(h->stream, iu); mt_free(h->stream, iv);
-        return rc;
-    }
-    *d_iu_out = iu;
-    *d_iv_out = iv;
-    return DC_OK;
+    return rc;
 }
 
 // Parameters of one local core update.  which: 0 = kmax (count list =
@@ -1527,7 +1534,32 @@ static int maintain_impl(dc_graph* h, const uint32_t* pairs, const uint8_t* is_d
     if (!d.full())
         if (int rc = decompose(h, 0, 0)) return rc;
     NetBatch nb;
-    if (int rc = net_batch(V, pairs, is_del, b, nb)) return rc;
+    DeviceBatch db;
+    struct Release {
+        dc_graph* h;
+        DeviceBatch* d;
+        ~Release() { device_batch_free(h, d); }
+    } release{h, &db};
+    // A large batch that will take the full path (re-peel, rows recomputed)
+    // and needs no features is reduced to its net effect on the device.
+    bool on_device = false;
+    const int rm0 = repair_mode >= 0 ? repair_mode : h->row_repair;
+    if (!nested && b >= kDeviceNetMin && b < (1ull << 30) && rm0 <= 1 && !h->log_maint &&
+        (method == DC_MAINT_REPEEL || (method == DC_MAINT_AUTO && !h->sched))) {
+        for (uint64_t i = 0; i < b; ++i)
+            if (pairs[2 * i] >= V || pairs[2 * i + 1] >= V) return bad_id(V, pairs, i);
+        const int rc = net_batch_device(h, pairs, is_del, b, &db);
+        if (rc != DC_OK && rc != DC_ERR_NOMEM) return rc;  // without room for it the host does it
+        on_device = rc == DC_OK && (uint64_t)db.n_ins + db.n_del > kRuleRepairMax;
+        if (on_device) {
+            nb.n_ins = db.n_ins;
+            nb.n_del = db.n_del;
+        } else {
+            device_batch_free(h, &db);
+        }
+    }
+    if (!on_device)
+        if (int rc = net_batch(V, pairs, is_del, b, nb)) return rc;
     // features of the batch against the decomposition before it
     float feat[16];
     const bool want_feat = !nested && (h->log_maint || (method == DC_MAINT_AUTO && h->sched));
@@ -1562,8 +1594,9 @@ static int maintain_impl(dc_graph* h, const uint32_t* pairs, const uint8_t* is_d
     if (rmode == 1 && nb.n_ins + nb.n_del > kRuleRepairMax) rmode = 0;
     // ---- one kind of update, local method, rows in place: one graph launch
     const uint64_t n_one = nb.del_u.empty() ? nb.ins_u.size() : nb.del_u.size();
-    if (h->captured_batches && method == DC_MAINT_LOCAL && rmode != 0 && nb.del_u.empty() != nb.ins_u.empty() &&
-        n_one <= kCapturedMax && !h->trace_dev && h->barrier_fault_block < 0 && d.kmax_v && d.sky_off) {
+    if (!on_device && h->captured_batches && method == DC_MAINT_LOCAL && rmode != 0 &&
+        nb.del_u.empty() != nb.ins_u.empty() && n_one <= kCapturedMax && !h->trace_dev && h->barrier_fault_block < 0 &&
+        d.kmax_v && d.sky_off) {
         bool handled = false;
         st->deleted = nb.n_del;
         st->inserted = nb.n_ins;
@@ -1645,32 +1678,30 @@ static int maintain_impl(dc_graph* h, const uint32_t* pairs, const uint8_t* is_d
         return DC_ERR_NOMEM;
     // values before the batch (for the row bound) and row 0 in scratch
     MT_CUDA(cudaMemcpyAsync(s->kmax_old, d.kmax_v, 4ull * V, cudaMemcpyDeviceToDevice, h->stream));
-    uint32_t *d_du = nullptr, *d_dv = nullptr, *d_iu = nullptr, *d_iv = nullptr;
     int rc = DC_OK;
     int rebuilt = 0;
     uint64_t region = 0;
+    if (!on_device && (rc = upload_batch(h, nb, &db))) goto out;
     // ---- deletions
-    if (!nb.del_u.empty()) {
-        if ((rc = apply_deletions(h, nb))) return rc;
-        std::vector<uint32_t> heads(nb.del_v), tails(nb.del_u);
-        if ((rc = upload(h, &d_dv, heads)) || (rc = upload(h, &d_du, tails))) goto out;
+    if (db.n_pairs) {
+        if ((rc = apply_deletions(h, db))) return rc;
         if (method == DC_MAINT_LOCAL) {
             MT_CUDA(cudaMemcpyAsync(s->row0_old, d.row0, 4ull * V, cudaMemcpyDeviceToDevice, h->stream));
-            if ((rc = core_local(h, 0, d.kmax_v, s->kmax_old, d_dv, (uint32_t)heads.size(), 0, 0, &region))) goto out;
-            if ((rc = core_local(h, 1, d.row0, s->row0_old, d_du, (uint32_t)tails.size(), 0, 0, &region))) goto out;
+            if ((rc = core_local(h, 0, d.kmax_v, s->kmax_old, db.del_v, db.n_pairs, 0, 0, &region))) goto out;
+            if ((rc = core_local(h, 1, d.row0, s->row0_old, db.del_u, db.n_pairs, 0, 0, &region))) goto out;
         }
     }
     // ---- insertions
-    if (!nb.ins_u.empty()) {
-        if ((rc = apply_insertions(h, nb, &d_iu, &d_iv, &rebuilt))) goto out;
+    if (db.n_ins) {
+        if ((rc = apply_insertions(h, db, &rebuilt))) goto out;
         if (method == DC_MAINT_LOCAL) {
             int32_t bb = (int32_t)std::min<uint64_t>(nb.n_ins, 0x3FFFFFFF);
             int32_t* old_k = s->cdeg2;  // values before the insertions
             int32_t* old_r = s->key2;
             MT_CUDA(cudaMemcpyAsync(old_k, d.kmax_v, 4ull * V, cudaMemcpyDeviceToDevice, h->stream));
             MT_CUDA(cudaMemcpyAsync(old_r, d.row0, 4ull * V, cudaMemcpyDeviceToDevice, h->stream));
-            if ((rc = core_local(h, 0, d.kmax_v, old_k, d_iv, (uint32_t)nb.ins_u.size(), 1, bb, &region))) goto out;
-            if ((rc = core_local(h, 1, d.row0, old_r, d_iu, (uint32_t)nb.ins_u.size(), 1, bb, &region))) goto out;
+            if ((rc = core_local(h, 0, d.kmax_v, old_k, db.ins_v, db.n_ins, 1, bb, &region))) goto out;
+            if ((rc = core_local(h, 1, d.row0, old_r, db.ins_u, db.n_ins, 1, bb, &region))) goto out;
         }
     }
     cudaEventRecord(ev[1], h->stream);
@@ -1687,15 +1718,15 @@ static int maintain_impl(dc_graph* h, const uint32_t* pairs, const uint8_t* is_d
         int* dbuf = (int*)s->cursor;  // [0] = R, [1] = new kmax, [2] = new lmax
         int init[3] = {-1, 0, 0};
         MT_CUDA(cudaMemcpyAsync(dbuf, init, sizeof(init), cudaMemcpyHostToDevice, h->stream));
-        if (!nb.del_u.empty()) {
+        if (db.n_pairs) {
             ++g_launches;
-            k_rows_bound_edges<<<mgrid(h, nb.del_u.size()), kMThreads, 0, h->stream>>>(
-                (uint32_t)nb.del_u.size(), d_du, d_dv, s->kmax_old, d.kmax_v, dbuf);
+            k_rows_bound_edges<<<mgrid(h, db.n_pairs), kMThreads, 0, h->stream>>>(db.n_pairs, db.del_u, db.del_v,
+                                                                                  s->kmax_old, d.kmax_v, dbuf);
         }
-        if (!nb.ins_u.empty()) {
+        if (db.n_ins) {
             ++g_launches;
-            k_rows_bound_edges<<<mgrid(h, nb.ins_u.size()), kMThreads, 0, h->stream>>>(
-                (uint32_t)nb.ins_u.size(), d_iu, d_iv, s->kmax_old, d.kmax_v, dbuf);
+            k_rows_bound_edges<<<mgrid(h, db.n_ins), kMThreads, 0, h->stream>>>(db.n_ins, db.ins_u, db.ins_v,
+                                                                                s->kmax_old, d.kmax_v, dbuf);
         }
         ++g_launches;
         k_rows_bound_changed<<<mgrid(h, V), kMThreads, 0, h->stream>>>(V, s->kmax_old, d.kmax_v, dbuf, dbuf + 1);
@@ -1731,10 +1762,10 @@ static int maintain_impl(dc_graph* h, const uint32_t* pairs, const uint8_t* is_d
             }
         }
         // ---- deletions only: repair rows 1..R in place
-        if (repair_del && nb.ins_u.empty()) {
+        if (repair_del && !db.n_ins) {
             bool applied = false;
             cudaEventRecord(ev[4], h->stream);
-            if ((rc = rows_repair(h, R, d_du, d_dv, (uint32_t)nb.del_u.size(), repair_deadline_ns(h, R, rmode),
+            if ((rc = rows_repair(h, R, db.del_u, db.del_v, db.n_pairs, repair_deadline_ns(h, R, rmode),
                                   &applied)))
                 goto out;
             cudaEventRecord(ev[5], h->stream);
@@ -1752,11 +1783,11 @@ static int maintain_impl(dc_graph* h, const uint32_t* pairs, const uint8_t* is_d
             }
         }
         // ---- insertions only: repair rows 1..R in place
-        if (repair_ins && nb.del_u.empty()) {
+        if (repair_ins && !db.n_pairs) {
             bool applied = false;
             unsigned long long scanned = 0;
             cudaEventRecord(ev[4], h->stream);
-            if ((rc = rows_repair_ins(h, R, d_iu, d_iv, (uint32_t)nb.ins_u.size(), repair_deadline_ns(h, R, rmode), &applied,
+            if ((rc = rows_repair_ins(h, R, db.ins_u, db.ins_v, db.n_ins, repair_deadline_ns(h, R, rmode), &applied,
                                       &scanned)))
                 goto out;
             cudaEventRecord(ev[5], h->stream);
@@ -1798,10 +1829,6 @@ timing:
     st->lmax = d.lmax;
     if (h->log_maint && want_feat) log_batch(h, feat, st);
 out:
-    mt_free(h->stream, d_du);
-    mt_free(h->stream, d_dv);
-    mt_free(h->stream, d_iu);
-    mt_free(h->stream, d_iv);
     if (rc != DC_OK) {
         d.valid = false;
         d.peel_valid = false;

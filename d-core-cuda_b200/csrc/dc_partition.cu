@@ -25,6 +25,7 @@
 
 #include "dc_engine.cuh"
 #include "dc_internal.h"
+#include "dc_netbatch.cuh"
 
 namespace dc {
 extern std::atomic<unsigned long long> g_launches;
@@ -220,6 +221,21 @@ int pt_alloc(cudaStream_t st, T** p, uint64_t n) {
 
 }  // namespace
 
+uint64_t radix_count_words(uint64_t n) { return (uint64_t)kDigits * ((n + kPTile - 1) / kPTile) + 1; }
+
+void radix_sort_pairs(cudaStream_t st, uint64_t n, int bits, uint32_t** key, uint32_t** val, uint32_t** key2,
+                      uint32_t** val2, uint32_t* cnt) {
+    const unsigned nblk = (unsigned)((n + kPTile - 1) / kPTile);
+    for (int shift = 0; shift < bits; shift += kDigitBits) {
+        g_launches += 3;
+        k_pt_digit_count<<<nblk, kPT, 0, st>>>(n, *key, shift, cnt);
+        k_pt_scan_one_block<<<1, kPT, 0, st>>>(cnt, (uint64_t)kDigits * nblk);
+        k_pt_digit_scatter<<<nblk, kPT, 0, st>>>(n, *key, *val, *key2, *val2, shift, cnt);
+        std::swap(*key, *key2);
+        std::swap(*val, *val2);
+    }
+}
+
 int kmax_edge_batches_device(dc_graph* h, uint64_t B, const uint32_t* d_from, const uint32_t* d_to,
                              int64_t* d_batch_of, int64_t* n_batches) {
     *n_batches = 0;
@@ -264,17 +280,7 @@ int kmax_edge_batches_device(dc_graph* h, uint64_t B, const uint32_t* d_from, co
         if ((rc = launched("roots"))) break;
         // stable LSD radix sort of the edge indices by root
         const int bits = V > 1 ? 32 - __builtin_clz(V - 1) : 0;
-        for (int shift = 0; shift < bits; shift += kDigitBits) {
-            k_pt_digit_count<<<(unsigned)nblk, kPT, 0, st>>>(B, key0, shift, cnt);
-            if ((rc = launched("digit count"))) break;
-            k_pt_scan_one_block<<<1, kPT, 0, st>>>(cnt, kDigits * nblk);
-            if ((rc = launched("digit scan"))) break;
-            k_pt_digit_scatter<<<(unsigned)nblk, kPT, 0, st>>>(B, key0, val0, key1, val1, shift, cnt);
-            if ((rc = launched("digit scatter"))) break;
-            std::swap(key0, key1);
-            std::swap(val0, val1);
-        }
-        if (rc) break;
+        radix_sort_pairs(st, B, bits, &key0, &val0, &key1, &val1, cnt);
         // occurrence of every edge's root so far (input order), passes per root kmax
         k_pt_run_flags<<<(unsigned)nblk, kPT, 0, st>>>(B, key0, f, part);
         if ((rc = launched("run flags"))) break;

@@ -91,12 +91,12 @@ namespace {
 
 // Upper bound on the device bytes a handle of V vertices and E edges can
 // hold, transients of maintenance included: slack adjacency under the
-// rebuild rule (len + len/8 + 2 per list), offsets and lengths, kmax/row 0,
+// rebuild rule (len + len/8 + 8 per list), offsets and lengths, kmax/row 0,
 // the skyline twice (old and merged during a batch), per-vertex scratch, the
 // ticket ring (a power of two), the corner log (at most E + V corners) and
 // rebuild staging.
 uint64_t footprint_bound(uint64_t V, uint64_t E, uint64_t sms) {
-    const uint64_t cap = E + E / 8 + 2 * V + 64;
+    const uint64_t cap = E + E / 8 + 8 * V + 64;
     uint64_t b = 2 * 4 * cap;
     b += 4 * 4 * (V + 1);
     b += 4 * 3 * (V + 1) + 3 * (8 * (E + 2 * V) + 4 * (V + 1));  // skyline and its two spares
