@@ -2974,6 +2974,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     int32_t first_row[kRowGroups] = {k0};  // of each run, ascending
     int nrun = 1, ngroups = 1;
     int32_t run_min = Kstop + 1;
+    int first_share = 1;   // blocks of the first run, in shares of the others'
     uint32_t n_state = 0;  // vertices every group after the first has state for
     if (relabel && k0 == 1 && Kstop >= kMinSplitRows) {
         if (h->auto_cuts) {
@@ -2991,17 +2992,29 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
             n_state = std::max(ck[1] / 8, std::min(ck[1] / 4, 65536u));
             run_min = 2;
             while (run_min <= Kstop && ck[run_min] > n_state) ++run_min;
-            // Groups: eight small ones hide each other's latency best until the
-            // rows are heavy enough to want more warps each (8 / 6 / 5 / 4
-            // groups: R-MAT 18, 3.9 M edges 2.1 / 2.5 / 2.7 / 3.0 ms; R-MAT 20,
-            // 16 M 5.4 / 4.9 / 5.9 / 6.5; R-MAT 22, 65 M 19.9 / 14.8 / 14.8 /
-            // 19.0; 2^21 vertices, 45 M edges 18.9 / 16.7 / 16.2 / 15.3).
-            const int most = std::min<int>(kRowGroups, g.E < (8ull << 20) ? 8 : g.E < (32ull << 20) ? 6 : 5);
+            // Small graphs: eight groups hide each other's latency best, equal
+            // runs (8 / 6 / 5 / 4 groups: R-MAT 18, 3.9 M edges 2.1 / 2.5 /
+            // 2.7 / 3.0 ms).  From 8 M edges on the rows want more warps each
+            // and the cores are large for longer: five groups, first rows at
+            // 0.6, 0.3, 0.15 and 0.075 of the rows, which took the rows of
+            // nine R-MAT graphs of 2^19 to 2^22 vertices from 6.5 / 11.1 /
+            // 21.4 ms (five or six equal runs, 16 / 32 / 64 M edges) to 5.9 /
+            // 10.0 / 18.6, between 17 % less and 3 % more.
+            first_share = g.E < (8ull << 20) ? 2 : 1;
             if (2 * (run_min - 1) <= Kstop) {
-                const int32_t rows = Kstop - run_min + 1, runs = std::min<int32_t>(most - 1, rows / 2);
-                for (int32_t i = 0; i < runs; ++i) first_row[nrun++] = run_min + (int32_t)((int64_t)rows * i / runs);
+                const int32_t rows = Kstop - run_min + 1, runs = std::min<int32_t>(kRowGroups - 1, rows / 2);
+                if (first_share == 2) {
+                    for (int32_t i = 0; i < runs; ++i) first_row[nrun++] = run_min + (int32_t)((int64_t)rows * i / runs);
+                } else {
+                    for (int64_t f : {75, 150, 300, 600}) {
+                        const int32_t c = (int32_t)(Kstop * f / 1000);
+                        if (c >= run_min && c > first_row[nrun - 1]) first_row[nrun++] = c;
+                    }
+                    if (nrun == 1) first_row[nrun++] = run_min;
+                    run_min = first_row[1];
+                }
                 n_state = ck[run_min];
-                ngroups = nrun > 1 ? most : 1;
+                ngroups = nrun == 1 ? 1 : first_share == 2 ? kRowGroups : 5;
             }
         } else {
             for (int i = 0; i < kMaxRowSegments - 1 && nrun < kRowGroups; ++i) {
@@ -3015,8 +3028,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
             }
         }
     }
-    // blocks: what fits at the same time, the first run of an uncut handle
-    // (the one with the large cores) twice the others' share
+    // blocks: what fits at the same time
     int grid = 0;
     if (int rc = persistent_grid(h, (const void*)k_trans2, ngroups > 1 ? 8 : h->rows_bps, &grid)) return rc;
     if (ngroups > 1 && h->rows_bps > 0) grid = std::min(grid, h->rows_bps * ngroups * h->geom.sms);
@@ -3096,10 +3108,10 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     RowsStart rs;
     memset(&rs, 0, sizeof(rs));
     if (ngroups > 1) {
-        const int shares = ngroups + (h->auto_cuts ? 1 : 0);
+        const int shares = ngroups + first_share - 1;
         tp.first_block[0] = 0;
         for (int i = 0; i < ngroups; ++i)
-            tp.first_block[i + 1] = (unsigned)((int64_t)grid * (i + 1 + (h->auto_cuts ? 1 : 0)) / shares);
+            tp.first_block[i + 1] = (unsigned)((int64_t)grid * (i + first_share) / shares);
         for (int i = 1; i < ngroups; ++i) {
             if (int rc = ensure_segment(h, i - 1, n_state)) return rc;
             const RowSegment& sg = s->seg[i - 1];

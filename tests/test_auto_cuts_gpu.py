@@ -49,3 +49,25 @@ def test_maintenance_on_a_fresh_handle(dc, orc, gpu):
             assert (st["kmax"], st["lmax"]) == (okm, olm)
             assert np.array_equal(g.kmaxes(), okmaxes)
             assert np.array_equal(g.rows(), orows)
+
+
+@pytest.mark.parametrize("skew", [True, False])
+@pytest.mark.parametrize("E", [(8 << 20) - 1, 8 << 20])
+def test_cut_rule_by_edges(dc, gpu, skew, E):
+    """Both sides of the rule's line at 8 M edges, with every cut allowed
+    (skewed degrees) and with the lower ones inside too large a core (a small
+    dense part on 12 random edges per vertex)."""
+    if skew:
+        V, s, d = dc.gen_rmat(19, 18, 41)
+    else:
+        V, (a, b) = 1 << 19, dc.gen_er(1 << 19, 6 << 20, 42)
+        _, u, v = dc.gen_rmat(15, 128, 43)
+        s, d = np.concatenate([a, u]), np.concatenate([b, v])
+    assert len(s) >= E
+    keep = np.random.default_rng(44).permutation(len(s))[:E]
+    s, d = np.ascontiguousarray(s[keep]), np.ascontiguousarray(d[keep])
+    with dc.Graph.from_edges(V, s, d) as a, dc.Graph.from_edges(V, s, d) as b:
+        b.set_tuning(2, 2, 64, ())
+        assert a.decompose() == b.decompose()
+        assert np.array_equal(a.kmaxes(), b.kmaxes())
+        assert all(np.array_equal(x, y) for x, y in zip(a.skyline(), b.skyline()))
