@@ -120,44 +120,88 @@ __device__ __forceinline__ unsigned block_append(unsigned* ctr, bool pred) {
 }
 
 // ---------------------------------------------------------------------------
-// cooperative exclusive scan (u64), n elements in place; out[n] = total
+// exclusive prefix sums of one or two arrays, n elements each
 // ---------------------------------------------------------------------------
-__global__ void k_scan_coop(unsigned long long* data, uint64_t n, unsigned long long* partial, EngineCtl* c) {
-    const uint64_t nb = gridDim.x;
-    const uint64_t per = (n + nb - 1) / nb;
-    const uint64_t lo = min(n, per * blockIdx.x), hi = min(n, lo + per);
-    // phase 1: block sums
-    unsigned long long s = 0;
-    for (uint64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) s += data[i];
-    unsigned long long tot;
+// Two plain launches: every block sums its range (the last one to finish
+// scans the sums), then every block writes its range.  A grid of small arrays
+// is bound by launches and round trips: 10,000 elements took 14 us in one
+// cooperative launch with two grid barriers, plus 6 us in the kernels that
+// widened and narrowed the values around it, once per side; these take 6 us
+// for both sides.  Long arrays are bound by memory, read twice.
+constexpr int kScanThreads = 256, kScanTile = 4 * kScanThreads;
+struct WordsInPlace {  // data[0 .. n] becomes the sums, data[n] the total
+    unsigned long long* data;
+    __device__ unsigned long long get(int, uint64_t i) const { return data[i]; }
+    __device__ void put(int, uint64_t i, unsigned long long x) const { data[i] = x; }
+};
+struct ListStarts {  // starts of lists with room for max(gap_min, len / gap_div) more entries each
+    const int32_t* len[2];
+    uint32_t* off[2];
+    uint32_t gap_min, gap_div;
+    __device__ unsigned long long get(int side, uint64_t i) const {
+        const uint32_t l = (uint32_t)len[side][i];
+        return (unsigned long long)l + (gap_div ? max(gap_min, l / gap_div) : gap_min);
+    }
+    __device__ void put(int side, uint64_t i, unsigned long long x) const { off[side][i] = (uint32_t)x; }
+};
+__device__ __forceinline__ uint64_t scan_range(uint64_t n) {  // elements per block
+    const uint64_t per = (n + gridDim.x - 1) / gridDim.x;
+    return (per + kScanTile - 1) / kScanTile * kScanTile;
+}
+// part: gridDim.x + 1 words per side; *ticket is 0 before and after.
+// total (optional): one word per side.
+template <class A>
+__global__ void __launch_bounds__(kScanThreads) k_scan_sums(A a, uint64_t n, unsigned long long* part, unsigned* ticket,
+                                                            unsigned long long* total) {
+    __shared__ bool s_last;
+    const uint64_t per = scan_range(n), lo = min(n, per * blockIdx.x), hi = min(n, lo + per);
+    unsigned long long s = 0, tot;
+    for (uint64_t i = lo + threadIdx.x; i < hi; i += kScanThreads) s += a.get(blockIdx.y, i);
     block_excl_scan64(s, &tot);
-    if (threadIdx.x == 0) partial[blockIdx.x] = tot;
-    if (!grid_sync(c)) return;
-    // phase 2: block 0 scans the partials
-    if (blockIdx.x == 0) {
+    if (threadIdx.x == 0) {
+        part[blockIdx.y * (gridDim.x + 1) + blockIdx.x] = tot;
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x * gridDim.y - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    for (unsigned side = 0; side < gridDim.y; ++side) {
+        volatile unsigned long long* q = part + side * (gridDim.x + 1);
         unsigned long long carry = 0;
-        for (uint64_t b0 = 0; b0 < nb; b0 += blockDim.x) {
-            uint64_t b = b0 + threadIdx.x;
-            unsigned long long v = b < nb ? partial[b] : 0ull;
-            unsigned long long t2;
-            unsigned long long ex = block_excl_scan64(v, &t2);
-            if (b < nb) partial[b] = ex + carry;
-            carry += t2;
-            __syncthreads();
+        for (unsigned b0 = 0; b0 < gridDim.x; b0 += kScanThreads) {
+            const unsigned b = b0 + threadIdx.x;
+            const unsigned long long x = b < gridDim.x ? q[b] : 0ull;
+            const unsigned long long ex = block_excl_scan64(x, &tot);
+            if (b < gridDim.x) q[b] = ex + carry;
+            carry += tot;
         }
-        if (threadIdx.x == 0) data[n] = carry;
+        if (threadIdx.x == 0) {
+            q[gridDim.x] = carry;
+            if (total) total[side] = carry;
+        }
     }
-    if (!grid_sync(c)) return;
-    // phase 3: scan own range
-    unsigned long long carry = partial[blockIdx.x];
-    for (uint64_t b0 = lo; b0 < hi; b0 += blockDim.x) {
-        uint64_t i = b0 + threadIdx.x;
-        unsigned long long v = i < hi ? data[i] : 0ull;
-        unsigned long long t2;
-        unsigned long long ex = block_excl_scan64(v, &t2);
-        if (i < hi) data[i] = ex + carry;
-        carry += t2;
+    if (threadIdx.x == 0) *ticket = 0;
+}
+template <class A>
+__global__ void __launch_bounds__(kScanThreads) k_scan_apply(A a, uint64_t n, const unsigned long long* part) {
+    const uint64_t per = scan_range(n), lo = min(n, per * blockIdx.x), hi = min(n, lo + per);
+    const unsigned long long* q = part + blockIdx.y * (gridDim.x + 1);
+    unsigned long long carry = q[blockIdx.x];
+    for (uint64_t b0 = lo; b0 < hi; b0 += kScanTile) {
+        const uint64_t i0 = b0 + 4 * threadIdx.x;
+        unsigned long long x[4], tot;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) x[j] = i0 + j < hi ? a.get(blockIdx.y, i0 + j) : 0ull;
+        unsigned long long at = carry + block_excl_scan64(x[0] + x[1] + x[2] + x[3], &tot);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (i0 + j < hi) a.put(blockIdx.y, i0 + j, at);
+            at += x[j];
+        }
+        carry += tot;
     }
+    if (blockIdx.x == 0 && threadIdx.x == 0) a.put(blockIdx.y, n, q[gridDim.x]);
 }
 
 // ---------------------------------------------------------------------------
@@ -209,21 +253,6 @@ __global__ void k_count_degrees(uint32_t V, uint64_t E, const uint32_t* src, con
             }
         }
     }
-}
-
-// capacity of v's list = len + max(gap_min, len / gap_div)
-__global__ void k_capacity(uint32_t V, const int32_t* len, uint32_t gap_min, uint32_t gap_div, unsigned long long* cap) {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t l = (uint32_t)len[v];
-        uint32_t g = gap_min;
-        if (gap_div) g = max(g, l / gap_div);
-        cap[v] = (unsigned long long)l + g;
-    }
-}
-
-__global__ void k_off_to_u32(uint32_t V, const unsigned long long* in, uint32_t* out) {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v <= V; v += (uint64_t)gridDim.x * blockDim.x)
-        out[v] = (uint32_t)in[v];
 }
 
 __global__ void k_scatter_edges(uint64_t E, const uint32_t* src, const uint32_t* dst, const uint32_t* out_off,
@@ -1619,24 +1648,41 @@ struct ListSrc {
     const uint32_t* pos;
 };
 __device__ __forceinline__ const uint32_t* src_list(const ListSrc& s, uint32_t i) { return s.nbr + s.off[s.order[i]]; }
+// Both sides of the relabeled graph in one launch (blockIdx.y), of its lists
+// those for the warp, block and counting sort listed by the first one.
+struct SortArgs {
+    const uint32_t* off[2];
+    const int32_t* len[2];
+    uint32_t* nbr[2];
+    ListSrc src[2];
+    uint32_t* list[2][3];
+    unsigned* cnt;  // [6], zero before
+    const int32_t* kmax;
+    int K;
+};
 
 // Lists of at most kSortShort entries are sorted here, one thread each;
 // longer ones are listed for the warp sort (up to kSortWarp), the block
 // sort (up to kSortMid) or the counting sort.
-__global__ void k_sort_short(uint32_t V, const uint32_t* off, const int32_t* len, uint32_t* nbr, uint32_t* warp_list,
-                             uint32_t* mid_list, uint32_t* big_list, unsigned* cnt, ListSrc src) {
+__global__ void k_sort_short(uint32_t V, SortArgs p) {
+    const uint32_t* off = p.off[blockIdx.y];
+    const int32_t* len = p.len[blockIdx.y];
+    uint32_t* nbr = p.nbr[blockIdx.y];
+    uint32_t* const* lists = p.list[blockIdx.y];
+    unsigned* cnt = p.cnt + 3 * blockIdx.y;
+    const ListSrc src = p.src[blockIdx.y];
     for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
         int n = len[v];
         if (n > kSortMid) {
-            big_list[atomicAdd(&cnt[2], 1u)] = (uint32_t)v;
+            lists[2][atomicAdd(&cnt[2], 1u)] = (uint32_t)v;
             continue;
         }
         if (n > kSortWarp) {
-            mid_list[atomicAdd(&cnt[1], 1u)] = (uint32_t)v;
+            lists[1][atomicAdd(&cnt[1], 1u)] = (uint32_t)v;
             continue;
         }
         if (n > kSortShort) {
-            warp_list[atomicAdd(&cnt[0], 1u)] = (uint32_t)v;
+            lists[0][atomicAdd(&cnt[0], 1u)] = (uint32_t)v;
             continue;
         }
         if (n < 1) continue;
@@ -1702,11 +1748,14 @@ __device__ __forceinline__ void warp_sort(const uint32_t* in, const uint32_t* po
     for (int t = 0; t < T; ++t)
         if (32 * t + lane < n) a[32 * t + lane] = k[t];
 }
-__global__ void __launch_bounds__(kSortThreads) k_sort_warp(const uint32_t* off, const int32_t* len, uint32_t* nbr,
-                                                             const uint32_t* list, const unsigned* n_list,
-                                                             ListSrc src) {
+__global__ void __launch_bounds__(kSortThreads) k_sort_warp(SortArgs p) {
+    const uint32_t* off = p.off[blockIdx.y];
+    const int32_t* len = p.len[blockIdx.y];
+    uint32_t* nbr = p.nbr[blockIdx.y];
+    const uint32_t* list = p.list[blockIdx.y][0];
+    const ListSrc src = p.src[blockIdx.y];
     static_assert(kSortWarp == 256, "eight entries per lane");
-    const unsigned nl = *n_list, nw = gridDim.x * (kSortThreads / 32);
+    const unsigned nl = p.cnt[3 * blockIdx.y], nw = gridDim.x * (kSortThreads / 32);
     for (unsigned li = blockIdx.x * (kSortThreads / 32) + (threadIdx.x >> 5); li < nl; li += nw) {
         const uint32_t v = list[li];
         const int n = len[v];
@@ -1722,12 +1771,15 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_warp(const uint32_t* off,
 // 256 entries are sorted in registers by a warp each; of the later stages only
 // the strides of 256 and more go through shared memory (10 block-wide passes
 // for 4,096 entries instead of 78).
-__global__ void __launch_bounds__(kSortThreads) k_sort_mid(const uint32_t* off, const int32_t* len, uint32_t* nbr,
-                                                            const uint32_t* list, const unsigned* n_list,
-                                                            ListSrc src) {
+__global__ void __launch_bounds__(kSortThreads) k_sort_mid(SortArgs p) {
+    const uint32_t* off = p.off[blockIdx.y];
+    const int32_t* len = p.len[blockIdx.y];
+    uint32_t* nbr = p.nbr[blockIdx.y];
+    const uint32_t* list = p.list[blockIdx.y][1];
+    const ListSrc src = p.src[blockIdx.y];
     __shared__ uint32_t s[kSortMid];
     const int lane = (int)(threadIdx.x & 31u), w = (int)(threadIdx.x >> 5);
-    const unsigned nl = *n_list;
+    const unsigned nl = p.cnt[3 * blockIdx.y + 1];
     for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
         const uint32_t v = list[li];
         const int n = len[v];
@@ -1750,8 +1802,8 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_mid(const uint32_t* off, 
         __syncthreads();
         for (int size = 512; size <= N; size <<= 1) {
             for (int stride = size >> 1; stride >= 256; stride >>= 1) {
-                for (int p = threadIdx.x; p < N / 2; p += kSortThreads) {
-                    const int i = ((p & ~(stride - 1)) << 1) | (p & (stride - 1)), o = i | stride;
+                for (int q = threadIdx.x; q < N / 2; q += kSortThreads) {
+                    const int i = ((q & ~(stride - 1)) << 1) | (q & (stride - 1)), o = i | stride;
                     const uint32_t x = s[i], y = s[o];
                     if ((x > y) == ((i & size) == 0)) {
                         s[i] = y;
@@ -1785,10 +1837,16 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_mid(const uint32_t* off, 
 // no particular order.  The list fits no shared memory, so its entries are
 // renamed twice.
 static constexpr int kSortBigBins = 11264;
-__global__ void k_sort_big(const uint32_t* off, const int32_t* len, uint32_t* nbr, const int32_t* kmax, int K,
-                           const uint32_t* list, const unsigned* n_list, ListSrc src) {
+__global__ void k_sort_big(SortArgs p) {
+    const uint32_t* off = p.off[blockIdx.y];
+    const int32_t* len = p.len[blockIdx.y];
+    uint32_t* nbr = p.nbr[blockIdx.y];
+    const uint32_t* list = p.list[blockIdx.y][2];
+    const ListSrc src = p.src[blockIdx.y];
+    const int32_t* kmax = p.kmax;
+    const int K = p.K;
     __shared__ unsigned bins[kSortBigBins];
-    const unsigned nl = *n_list;
+    const unsigned nl = p.cnt[3 * blockIdx.y + 2];
     const uint32_t lines = (uint32_t)(kSortBigBins - 1 - K);
     auto bin_of = [&](uint32_t u) { return (int)min(u >> 5, lines) + (K - kmax[u]); };
     for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
@@ -1846,17 +1904,37 @@ __global__ void k_sort_big(const uint32_t* off, const int32_t* len, uint32_t* nb
 // ---------------------------------------------------------------------------
 // order by kmax, skyline assembly, expansion
 // ---------------------------------------------------------------------------
-// Counts per kmax value.  Most vertices share a few small values, so the
-// counts go to per-block shared bins first (when kmax + 1 <= kHistShared).
+// One pass over the vertices: counts per kmax value, the number of corners rows
+// 1.. can have (min(kmax, row 0) each: *corners) and sum of (in + out degree) x
+// kmax, the list entries a pass over rows 1..kmax scans, a deterministic
+// measure of a graph's row work (*work).  Most vertices share a few small kmax
+// values, so the counts go to per-block shared bins first (when kmax + 1 <=
+// kHistShared).  Three kernels, each with its own read-back, took 30 us more.
 constexpr int kHistShared = 8192;
-__global__ void k_kmax_hist(uint32_t V, const int32_t* kmax, uint32_t* hist, int32_t K) {
+__global__ void k_row_stats(uint32_t V, const int32_t* kmax, const int32_t* row0, const int32_t* in_len,
+                            const int32_t* out_len, uint32_t* hist, int32_t K, unsigned long long* corners,
+                            unsigned long long* work) {
     extern __shared__ uint32_t sh[];
     const bool shared = K + 1 <= kHistShared;
     if (shared)
         for (int i = threadIdx.x; i <= K; i += blockDim.x) sh[i] = 0;
     __syncthreads();
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
-        atomicAdd(shared ? &sh[kmax[v]] : &hist[kmax[v]], 1u);
+    unsigned long long c = 0, w = 0;
+    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
+        const int k = kmax[v];
+        atomicAdd(shared ? &sh[k] : &hist[k], 1u);
+        c += (unsigned long long)min(k, row0[v]);
+        w += (unsigned long long)(in_len[v] + out_len[v]) * (unsigned long long)k;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
+        w += __shfl_xor_sync(0xFFFFFFFFu, w, o);
+    }
+    if ((threadIdx.x & 31u) == 0) {
+        atomicAdd(corners, c);
+        atomicAdd(work, w);
+    }
     __syncthreads();
     if (shared)
         for (int i = threadIdx.x; i <= K; i += blockDim.x)
@@ -1900,16 +1978,6 @@ __global__ void k_order_scatter(uint32_t V, const int32_t* kmax, uint32_t* curso
         p0 = __shfl_sync(0xFFFFFFFFu, p0, leader);
         if (ok) order[p0 + __popc(peers & ((1u << lane) - 1u))] = (uint32_t)v;
     }
-}
-
-// corner bound per vertex: min(kmax, row0) + 1
-__global__ void k_corner_bound(uint32_t V, const int32_t* kmax, const int32_t* row0, unsigned long long* acc) {
-    unsigned long long s = 0;
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
-        s += (unsigned long long)min(kmax[v], row0[v]);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-    if ((threadIdx.x & 31u) == 0) atomicAdd(acc, s);
 }
 
 // log entries with a negative row are void (dropped corners)
@@ -2129,12 +2197,10 @@ int init_handle(dc_graph* h) {
 void free_graph_arrays(DevGraph& g, cudaStream_t st) {
     dfree(st, g.out_off);
     dfree(st, g.out_len);
-    dfree(st, g.out_nbr_alloc);
-    g.out_nbr = nullptr;
+    dfree(st, g.out_nbr);
     dfree(st, g.in_off);
     dfree(st, g.in_len);
-    dfree(st, g.in_nbr_alloc);
-    g.in_nbr = nullptr;
+    dfree(st, g.in_nbr);
     g.out_cap = g.in_cap = 0;
 }
 
@@ -2238,11 +2304,14 @@ void free_scratch(dc_graph* h) {
     for (int i = 0; i < 2; ++i) {
         dfree(h->stream, s->r_off[i]);
         dfree(h->stream, s->r_len[i]);
-        dfree(h->stream, s->r_nbr_alloc[i]);
+        dfree(h->stream, s->r_nbr[i]);
     }
     delete s;
     h->scratch = nullptr;
 }
+
+static uint64_t scan_words(const dc_graph* h) { return (uint64_t)h->geom.sms * 64 + 64; }
+static unsigned* scan_ticket(dc_graph* h) { return (unsigned*)(h->scratch->partial + scan_words(h) - 1); }
 
 int ensure_scratch(dc_graph* h, uint32_t V) {
     if (!h->scratch) h->scratch = new Scratch();
@@ -2257,10 +2326,11 @@ int ensure_scratch(dc_graph* h, uint32_t V) {
     if (dmalloc(h->stream, &s->key, n) || dmalloc(h->stream, &s->cdeg, n) || dmalloc(h->stream, &s->cur, n) || dmalloc(h->stream, &s->row0, n) ||
         dmalloc(h->stream, &s->mark, n) || dmalloc(h->stream, &s->stamp, n) || dmalloc(h->stream, &s->logidx, n) || dmalloc(h->stream, &s->rem0, n) ||
         dmalloc(h->stream, &s->rem1, n) || dmalloc(h->stream, &s->order, n) || dmalloc(h->stream, &s->tmp64, n + 1) ||
-        dmalloc(h->stream, &s->partial, (uint64_t)h->geom.sms * 64 + 64) || dmalloc(h->stream, &s->cursor, n + 1) ||
+        dmalloc(h->stream, &s->partial, scan_words(h)) || dmalloc(h->stream, &s->cursor, n + 1) ||
         dmalloc(h->stream, &s->key2, n) || dmalloc(h->stream, &s->cdeg2, n) || dmalloc(h->stream, &s->rem2, n) || dmalloc(h->stream, &s->rem3, n) ||
         dmalloc(h->stream, &s->cnt_out, n))
         return DC_ERR_NOMEM;
+    DC_CUDA(cudaMemsetAsync(scan_ticket(h), 0, sizeof(unsigned), h->stream));
     s->cap_V = V;
     return DC_OK;
 }
@@ -2283,66 +2353,36 @@ uint64_t device_footprint(const dc_graph* h) {
             b += (sg.cur ? 24 * ((uint64_t)sg.cap_V + 1) : 0) + 8 * sg.tring_cap + (sg.ctl ? sizeof(EngineCtl) : 0);
         b += (s->plan ? sizeof(RowPlan) : 0) + 4ull * s->seam_of_cap + 4 * s->seam_cap;
         if (s->pos) b += 4 * 7 * ((uint64_t)s->r_cap_V + 1);     // relabeled graph: ids, kmax, row 0, offsets, lengths
-        if (s->r_nbr_alloc[0]) b += 2 * 4 * (s->r_cap + 7);     // its lists
+        if (s->r_nbr[0]) b += 2 * 4 * s->r_cap;     // its lists
     }
     return b;
 }
 
-// Exclusive scan of n u64 values in s->tmp64 (tmp64[n] receives the total).
-int scan_tmp64(dc_graph* h, uint64_t n) {
-    Scratch* s = h->scratch;
-    unsigned long long* data = (unsigned long long*)s->tmp64;
-    unsigned long long* part = (unsigned long long*)s->partial;
-    void* args[] = {&data, &n, &part, &h->ctl};
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)k_scan_coop, 256, 0);
-    per_sm = std::max(1, std::min(per_sm, 8));
-    DC_CUDA(cudaMemsetAsync(h->ctl, 0, sizeof(EngineCtl), h->stream));
-    ++g_launches;
-    cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_scan_coop, dim3(per_sm * h->geom.sms), dim3(256), args,
-                                                0, h->stream);
-    if (e != cudaSuccess) return set_error(DC_ERR_CUDA, "scan launch failed: %s", cudaGetErrorString(e));
-    return DC_OK;
+// Grid of the prefix sums over n elements: at most 16 blocks per SM (two sides'
+// sums fit s->partial), a tile each at least.
+static unsigned scan_blocks(const dc_graph* h, uint64_t n) {
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + kScanTile - 1) / kScanTile, 16ull * h->geom.sms));
 }
 
-static int finish_build(dc_graph* h, uint32_t V, uint64_t E, const uint32_t* d_src, const uint32_t* d_dst) {
-    DevGraph& g = h->g;
-    Scratch* s = h->scratch;
-    // capacities -> offsets (out)
-    for (int side = 0; side < 2; ++side) {
-        int32_t* len = side == 0 ? g.out_len : g.in_len;
-        ++g_launches;
-        k_capacity<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, len, h->gap_min, h->gap_div,
-                                                               (unsigned long long*)s->tmp64);
-        if (int rc = scan_tmp64(h, V)) return rc;
-        unsigned long long total = 0;
-        DC_CUDA(cudaMemcpyAsync(&total, s->tmp64 + V, sizeof(total), cudaMemcpyDeviceToHost, h->stream));
-        DC_CUDA(cudaStreamSynchronize(h->stream));
-        if (total >= 0xFFFFFFFFull)
-            return set_error(DC_ERR_CAPACITY, "adjacency with slack exceeds 2^32 entries (u32 offsets)");
-        uint32_t** off = side == 0 ? &g.out_off : &g.in_off;
-        uint32_t** nbr = side == 0 ? &g.out_nbr : &g.in_nbr;
-        uint32_t** alloc = side == 0 ? &g.out_nbr_alloc : &g.in_nbr_alloc;
-        // the row kernel reads ids in aligned 16-byte groups: the lists
-        // start at a 16-byte boundary (three spare entries in front cover
-        // any alignment of the allocation) and four spare entries at the end
-        // cover the last group of the last list
-        if (dmalloc(h->stream, off, (uint64_t)V + 1) || dmalloc(h->stream, alloc, total + 7)) return DC_ERR_NOMEM;
-        *nbr = (uint32_t*)(((uintptr_t)*alloc + 15u) & ~(uintptr_t)15u);
-        ++g_launches;
-        k_off_to_u32<<<grid_for(h, (uint64_t)V + 1), kThreads, 0, h->stream>>>(V, (unsigned long long*)s->tmp64, *off);
-        if (side == 0) g.out_cap = total;
-        else g.in_cap = total;
-    }
-    DC_CUDA(cudaMemsetAsync(g.out_len, 0, sizeof(int32_t) * V, h->stream));
-    DC_CUDA(cudaMemsetAsync(g.in_len, 0, sizeof(int32_t) * V, h->stream));
-    if (E)
-        ++g_launches;
-        k_scatter_edges<<<grid_for(h, E), kThreads, 0, h->stream>>>(E, d_src, d_dst, g.out_off, g.out_len, g.out_nbr,
-                                                                     g.in_off, g.in_len, g.in_nbr);
+template <class A>
+static void scan_sums(dc_graph* h, const A& a, int sides, uint64_t n, unsigned long long* total = nullptr) {
+    ++g_launches;
+    k_scan_sums<A><<<dim3(scan_blocks(h, n), sides), kScanThreads, 0, h->stream>>>(
+        a, n, (unsigned long long*)h->scratch->partial, scan_ticket(h), total);
+}
+template <class A>
+static void scan_apply(dc_graph* h, const A& a, int sides, uint64_t n) {
+    ++g_launches;
+    k_scan_apply<A><<<dim3(scan_blocks(h, n), sides), kScanThreads, 0, h->stream>>>(
+        a, n, (const unsigned long long*)h->scratch->partial);
+}
+
+// Exclusive scan of n u64 values in s->tmp64 (tmp64[n] receives the total).
+int scan_tmp64(dc_graph* h, uint64_t n) {
+    const WordsInPlace a{(unsigned long long*)h->scratch->tmp64};
+    scan_sums(h, a, 1, n);
+    scan_apply(h, a, 1, n);
     DC_CUDA(cudaGetLastError());
-    g.V = V;
-    g.E = E;
     return DC_OK;
 }
 
@@ -2355,10 +2395,37 @@ int build_from_device_edges(dc_graph* h, uint32_t V, uint64_t E, const uint32_t*
     DC_CUDA(cudaMemsetAsync(g.out_len, 0, sizeof(int32_t) * ((uint64_t)V + 1), h->stream));
     DC_CUDA(cudaMemsetAsync(g.in_len, 0, sizeof(int32_t) * ((uint64_t)V + 1), h->stream));
     DC_CUDA(cudaMemsetAsync(h->ctl, 0, sizeof(EngineCtl), h->stream));
-    if (E) k_count_degrees<<<grid_for(h, E), kThreads, 0, h->stream>>>(V, E, d_src, d_dst, g.out_len, g.in_len, h->ctl);
+    if (E) {
+        ++g_launches;
+        k_count_degrees<<<grid_for(h, E), kThreads, 0, h->stream>>>(V, E, d_src, d_dst, g.out_len, g.in_len, h->ctl);
+    }
+    // list starts; the totals come back with the status of the count
+    ListStarts ls{{g.out_len, g.in_len}, {nullptr, nullptr}, h->gap_min, h->gap_div};
+    static_assert(offsetof(EngineCtl, drops) == offsetof(EngineCtl, evals) + 8, "two totals side by side");
+    scan_sums(h, ls, 2, V, &h->ctl->evals);
     EngineCtl hc;
     if (int rc = check_ctl(h, &hc, "graph build")) return rc;
-    return finish_build(h, V, E, d_src, d_dst);
+    if (hc.evals >= 0xFFFFFFFFull || hc.drops >= 0xFFFFFFFFull)
+        return set_error(DC_ERR_CAPACITY, "adjacency with slack exceeds 2^32 entries (u32 offsets)");
+    if (dmalloc(h->stream, &g.out_off, (uint64_t)V + 1) || dmalloc(h->stream, &g.out_nbr, hc.evals) ||
+        dmalloc(h->stream, &g.in_off, (uint64_t)V + 1) || dmalloc(h->stream, &g.in_nbr, hc.drops))
+        return DC_ERR_NOMEM;
+    g.out_cap = hc.evals;
+    g.in_cap = hc.drops;
+    ls.off[0] = g.out_off;
+    ls.off[1] = g.in_off;
+    scan_apply(h, ls, 2, V);
+    DC_CUDA(cudaMemsetAsync(g.out_len, 0, sizeof(int32_t) * V, h->stream));
+    DC_CUDA(cudaMemsetAsync(g.in_len, 0, sizeof(int32_t) * V, h->stream));
+    if (E) {
+        ++g_launches;
+        k_scatter_edges<<<grid_for(h, E), kThreads, 0, h->stream>>>(E, d_src, d_dst, g.out_off, g.out_len, g.out_nbr,
+                                                                     g.in_off, g.in_len, g.in_nbr);
+    }
+    DC_CUDA(cudaGetLastError());
+    g.V = V;
+    g.E = E;
+    return DC_OK;
 }
 
 __global__ void k_host_csr_len(uint32_t V, const int32_t* deg, int32_t* len) {
@@ -2735,23 +2802,6 @@ int expand_rows(dc_graph* h, uint32_t k0, uint32_t n, int32_t* d_dst) {
     return DC_OK;
 }
 
-// The lists of one side of the relabeled graph from the handle's lists.
-static int sort_side(dc_graph* h, int32_t K, uint32_t V, const uint32_t* off, const int32_t* len, uint32_t* nbr,
-                     const int32_t* kmax, ListSrc src) {
-    Scratch* s = h->scratch;
-    unsigned* cnt = s->cursor;
-    DC_CUDA(cudaMemsetAsync(cnt, 0, 3 * sizeof(unsigned), h->stream));
-    // most lists go to the short and the warp sort; the others read their
-    // counts on the device
-    g_launches += 4;
-    k_sort_short<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, off, len, nbr, s->rem0, s->rem2, s->rem1, cnt, src);
-    k_sort_warp<<<h->geom.sms * 8, kSortThreads, 0, h->stream>>>(off, len, nbr, s->rem0, &cnt[0], src);
-    k_sort_mid<<<h->geom.sms * 8, kSortThreads, 0, h->stream>>>(off, len, nbr, s->rem2, &cnt[1], src);
-    k_sort_big<<<h->geom.sms * 2, 512, 0, h->stream>>>(off, len, nbr, kmax, K, s->rem1, &cnt[2], src);
-    DC_CUDA(cudaGetLastError());
-    return DC_OK;
-}
-
 // ---------------------------------------------------------------------------
 // the graph relabeled in kmax order for the row kernel
 // ---------------------------------------------------------------------------
@@ -2771,11 +2821,6 @@ __global__ void k_relabel_gather(uint32_t V, const uint32_t* order, const int32_
         len_o[i] = out_len[v];
         len_i[i] = in_len[v];
     }
-}
-
-__global__ void k_len_to_u64e(uint32_t V, const int32_t* len, unsigned long long* out) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < V; i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = (unsigned long long)len[i];
 }
 
 // Corner records of the relabeled run back to original ids.  A run that
@@ -2859,7 +2904,7 @@ __global__ void k_rows_collect(RowsStart r, const RowPlan* plan) {
 // Builds the relabeled graph (s->order must hold the kmax order of the
 // current kmax) with its lists sorted by neighbour kmax, plus kmax and row 0
 // by new id.
-static int build_relabeled(dc_graph* h, int32_t K) {
+static int build_relabeled(dc_graph* h, int32_t K, unsigned* sort_cnt) {
     DevGraph& g = h->g;
     Scratch* s = h->scratch;
     const uint32_t V = g.V;
@@ -2879,19 +2924,15 @@ static int build_relabeled(dc_graph* h, int32_t K) {
             return DC_ERR_NOMEM;
         s->r_cap_V = V;
     }
-    // list arrays: three spare entries in front for the 16-byte alignment of
-    // the array start, four at the end for the last 16-byte id group
-    const uint64_t cap = g.E + 8;
-    if (s->r_cap < cap || !s->r_nbr_alloc[0]) {
+    const uint64_t cap = g.E + 1;
+    if (s->r_cap < cap || !s->r_nbr[0]) {
         for (int i = 0; i < 2; ++i) {
-            dfree(h->stream, s->r_nbr_alloc[i]);
-            s->r_nbr[i] = nullptr;
+            dfree(h->stream, s->r_nbr[i]);
         }
         s->r_cap = 0;
         const uint64_t want = cap + cap / 8;  // headroom for later, larger graphs of the handle
         for (int i = 0; i < 2; ++i) {
-            if (dmalloc(h->stream, &s->r_nbr_alloc[i], want + 7)) return DC_ERR_NOMEM;
-            s->r_nbr[i] = (uint32_t*)(((uintptr_t)s->r_nbr_alloc[i] + 15u) & ~(uintptr_t)15u);
+            if (dmalloc(h->stream, &s->r_nbr[i], want)) return DC_ERR_NOMEM;
         }
         s->r_cap = want;
     }
@@ -2899,19 +2940,26 @@ static int build_relabeled(dc_graph* h, int32_t K) {
     k_relabel_gather<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, s->order, h->d.kmax_v, s->row0, g.out_len,
                                                                   g.in_len, s->pos, s->kmax_r, s->row0_r, s->r_len[0],
                                                                   s->r_len[1]);
-    for (int side = 0; side < 2; ++side) {
-        ++g_launches;
-        k_len_to_u64e<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, s->r_len[side], (unsigned long long*)s->tmp64);
-        if (int rc = scan_tmp64(h, V)) return rc;
-        ++g_launches;
-        k_off_to_u32<<<grid_for(h, n), kThreads, 0, h->stream>>>(V, (unsigned long long*)s->tmp64, s->r_off[side]);
-    }
+    const ListStarts ls{{s->r_len[0], s->r_len[1]}, {s->r_off[0], s->r_off[1]}, 0, 0};
+    scan_sums(h, ls, 2, V);
+    scan_apply(h, ls, 2, V);
     // every relabeled list is read from its original list, renamed and
-    // sorted by neighbour kmax in one pass
-    for (int side = 0; side < 2; ++side) {
-        const ListSrc src{side == 0 ? g.out_off : g.in_off, side == 0 ? g.out_nbr : g.in_nbr, s->order, s->pos};
-        if (int rc = sort_side(h, K, V, s->r_off[side], s->r_len[side], s->r_nbr[side], s->kmax_r, src)) return rc;
-    }
+    // sorted in one pass; most lists go to the short and the warp sort, the
+    // others read their counts on the device
+    const SortArgs so{{s->r_off[0], s->r_off[1]},
+                      {s->r_len[0], s->r_len[1]},
+                      {s->r_nbr[0], s->r_nbr[1]},
+                      {{g.out_off, g.out_nbr, s->order, s->pos}, {g.in_off, g.in_nbr, s->order, s->pos}},
+                      {{s->rem0, s->rem2, s->rem1}, {s->rem3, (uint32_t*)s->cdeg, (uint32_t*)s->cdeg2}},
+                      sort_cnt,
+                      s->kmax_r,
+                      K};
+    g_launches += 4;
+    k_sort_short<<<dim3(grid_for(h, V), 2), kThreads, 0, h->stream>>>(V, so);
+    k_sort_warp<<<dim3(h->geom.sms * 8, 2), kSortThreads, 0, h->stream>>>(so);
+    k_sort_mid<<<dim3(h->geom.sms * 8, 2), kSortThreads, 0, h->stream>>>(so);
+    k_sort_big<<<dim3(h->geom.sms * 2, 2), 512, 0, h->stream>>>(so);
+    DC_CUDA(cudaGetLastError());
     return DC_OK;
 }
 
@@ -2928,36 +2976,43 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     *nlog_out = 0;
     h->log_used = 0;
     cudaEventRecord(h->ev[2], h->stream);
-    if (s->ck_cap < (uint32_t)K + 2) {
+    // |C_k| and first positions by kmax (K + 2 words each, sized by kmax: it
+    // exceeds V where edges are parallel), two sums, the sorts' counters
+    const uint64_t nk = (uint64_t)K + 2;
+    if (s->ck_cap < nk) {
         dfree(h->stream, s->ck);
         s->ck_cap = 0;
-        if (dmalloc(h->stream, &s->ck, 2 * ((uint64_t)K + 2))) return DC_ERR_NOMEM;
-        s->ck_cap = K + 2;
+        if (dmalloc(h->stream, &s->ck, 2 * nk + kRowPrepWords)) return DC_ERR_NOMEM;
+        s->ck_cap = (uint32_t)nk;
     }
-    uint32_t* hist = s->ck + s->ck_cap;  // K exceeds V where edges are parallel: no vertex-sized array holds it
-    DC_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * ((uint64_t)K + 2), h->stream));
+    unsigned long long* sums = (unsigned long long*)s->ck;  // corners, row work
+    unsigned* sort_cnt = s->ck + 4;
+    uint32_t* d_ck = s->ck + kRowPrepWords;
+    uint32_t* hist = d_ck + nk;
+    static_assert(kRowPrepWords >= 4 + 6, "two sums, six counters");
+    DC_CUDA(cudaMemsetAsync(s->ck, 0, sizeof(uint32_t) * (2 * nk + kRowPrepWords), h->stream));
     ++g_launches;
-    k_kmax_hist<<<grid_for(h, V), kThreads, K + 1 <= kHistShared ? 4 * (K + 1) : 0, h->stream>>>(V, d.kmax_v, hist, K);
-    std::vector<uint32_t> hh((size_t)K + 2), ck((size_t)K + 2), start((size_t)K + 2);
-    DC_CUDA(cudaMemcpyAsync(hh.data(), hist, sizeof(uint32_t) * ((size_t)K + 2), cudaMemcpyDeviceToHost, h->stream));
-    unsigned long long* acc = (unsigned long long*)s->tmp64;
-    DC_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long), h->stream));
-    ++g_launches;
-    k_corner_bound<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, d.kmax_v, s->row0, acc);
-    unsigned long long bound = 0;
-    DC_CUDA(cudaMemcpyAsync(&bound, acc, sizeof(bound), cudaMemcpyDeviceToHost, h->stream));
+    k_row_stats<<<grid_for(h, V), kThreads, K + 1 <= kHistShared ? 4 * (K + 1) : 0, h->stream>>>(
+        V, d.kmax_v, s->row0, g.in_len, g.out_len, hist, K, sums, sums + 1);
+    std::vector<uint32_t> host(2 * nk + kRowPrepWords);
+    DC_CUDA(cudaMemcpyAsync(host.data(), s->ck, sizeof(uint32_t) * host.size(), cudaMemcpyDeviceToHost, h->stream));
     DC_CUDA(cudaStreamSynchronize(h->stream));
+    unsigned long long bound = 0;
+    memcpy(&bound, host.data(), sizeof(bound));
+    memcpy(&h->row_work, host.data() + 2, sizeof(h->row_work));
+    uint32_t* ck = host.data() + kRowPrepWords;
     {
-        uint64_t run = 0;
+        uint32_t* start = ck + nk;  // counts, then first positions
+        uint32_t run = 0;
         ck[K + 1] = 0;
         for (int32_t k = K; k >= 0; --k) {
-            start[k] = (uint32_t)run;
-            run += hh[k];
-            ck[k] = (uint32_t)run;
+            const uint32_t c = start[k];
+            start[k] = run;
+            run += c;
+            ck[k] = run;
         }
     }
-    DC_CUDA(cudaMemcpyAsync(s->ck, ck.data(), sizeof(uint32_t) * ((size_t)K + 2), cudaMemcpyHostToDevice, h->stream));
-    DC_CUDA(cudaMemcpyAsync(hist, start.data(), sizeof(uint32_t) * ((size_t)K + 2), cudaMemcpyHostToDevice, h->stream));
+    DC_CUDA(cudaMemcpyAsync(d_ck, ck, sizeof(uint32_t) * 2 * nk, cudaMemcpyHostToDevice, h->stream));
     ++g_launches;
     k_order_scatter<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, d.kmax_v, hist, s->order);
     // The graph the row kernel reads: where sorting is allowed, the graph
@@ -3055,7 +3110,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     uint32_t *G_out_nbr = g.out_nbr, *G_in_nbr = g.in_nbr;
     const int32_t *G_kmax = d.kmax_v, *G_row0 = s->row0;
     if (relabel) {
-        if (int rc = build_relabeled(h, K)) return rc;
+        if (int rc = build_relabeled(h, K, sort_cnt)) return rc;
         sorted = 1;
         G_out_off = s->r_off[0];
         G_in_off = s->r_off[1];
@@ -3085,7 +3140,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     tp.n = n0;
     tp.sorted = sorted;
     tp.order = G_order;
-    tp.ck = s->ck;
+    tp.ck = d_ck;
     tp.log_v = s->log_v;
     tp.log_k = s->log_k;
     tp.log_l = s->log_l;
@@ -3284,7 +3339,7 @@ int decompose(dc_graph* h, int method, int materialize_rows) {
     // ---- method 0: rows 1..K derived row to row
     uint64_t nlog = 0;
     if (int rc = rows_from_row0(h, K, K, true, &nlog)) return rc;
-    if (int rc = degree_kmax_sum(h, &h->full_work)) return rc;
+    h->full_work = h->row_work;
     if (int rc = build_skyline_from_log(h, nlog)) return rc;
     cudaEventRecord(h->ev[5], h->stream);
     d.valid = true;
@@ -3334,8 +3389,7 @@ int row_weights(dc_graph* h, uint64_t* out) {
     return DC_OK;
 }
 
-// sum over vertices of (in + out degree) x kmax: the list entries a per-row
-// pass over rows 1..kmax scans, a deterministic measure of a graph's row work
+// the row work alone (k_row_stats)
 __global__ void k_deg_kmax_sum(uint32_t V, const int32_t* kmax, const int32_t* in_len, const int32_t* out_len,
                                unsigned long long* acc) {
     unsigned long long w = 0;

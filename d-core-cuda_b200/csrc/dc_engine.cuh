@@ -29,6 +29,7 @@ struct FirstStep {
     int blocks;  // that work on it (0: the grid)
 };
 
+constexpr int kRowPrepWords = 16;
 struct Scratch {
     uint32_t cap_V = 0;
     int32_t* key = nullptr;      // [V] peeling degree / cnt_in
@@ -41,14 +42,14 @@ struct Scratch {
     uint32_t* rem0 = nullptr;    // [V]
     uint32_t* rem1 = nullptr;    // [V]
     uint32_t* order = nullptr;   // [V] vertices by kmax descending
-    uint32_t* ck = nullptr;      // [kmax+2] |C_k|
+    uint32_t* ck = nullptr;      // [kRowPrepWords + 2 (kmax+2)] row preparation: sums, counters, |C_k|, first positions
     uint32_t ck_cap = 0;
     uint32_t* log_v = nullptr;
     int32_t* log_k = nullptr;
     int32_t* log_l = nullptr;
     uint64_t log_cap = 0;
     uint64_t* tmp64 = nullptr;   // [V+1] scan scratch
-    uint64_t* partial = nullptr; // [blocks] scan scratch
+    uint64_t* partial = nullptr; // block sums of the scans; the last word is their ticket
     uint32_t* cursor = nullptr;  // [V+1]
     // second peel instance
     int32_t* key2 = nullptr;
@@ -76,8 +77,7 @@ struct Scratch {
     int32_t* row0_r = nullptr;                  // [V] row 0 by new id
     uint32_t* r_off[2] = {nullptr, nullptr};    // out / in list starts [V+1]
     int32_t* r_len[2] = {nullptr, nullptr};     // [V]
-    uint32_t* r_nbr_alloc[2] = {nullptr, nullptr};
-    uint32_t* r_nbr[2] = {nullptr, nullptr};    // 16-byte aligned inside r_nbr_alloc
+    uint32_t* r_nbr[2] = {nullptr, nullptr};    // their lists
     uint32_t r_cap_V = 0;
     uint64_t r_cap = 0;                         // list entries per side
 };

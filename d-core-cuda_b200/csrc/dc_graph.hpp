@@ -35,10 +35,6 @@ struct DevGraph {
     int32_t* in_len = nullptr;
     uint32_t* in_nbr = nullptr;
     uint64_t out_cap = 0, in_cap = 0;
-    // allocations behind out_nbr / in_nbr (the lists start at the first
-    // 16-byte boundary inside them: the row kernel reads ids 16 bytes at a time)
-    uint32_t* out_nbr_alloc = nullptr;
-    uint32_t* in_nbr_alloc = nullptr;
 };
 
 // Persistent-kernel launch geometry for the current device.
@@ -126,6 +122,7 @@ struct dc_graph {
     uint64_t log_used = 0;  // records in the last run's corner log (its other entries are void)
     uint64_t stat_evals = 0, stat_drops = 0, stat_entries = 0;
     uint64_t full_work = 0;  // sum over vertices of degree x kmax at the last full decomposition
+    uint64_t row_work = 0;   // the same at the last preparation of rows
     float full_rows_ms = 0;  // rows phase (rows 1..kmax) of the last full decomposition
     // limit of one bounded device wait in ns (0: the default, dc::kWaitNs)
     uint64_t wait_ns = 0;
