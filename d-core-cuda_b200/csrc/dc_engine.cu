@@ -87,7 +87,7 @@ __device__ __forceinline__ unsigned long long warp_incl_scan64(unsigned long lon
 // Block-wide exclusive scan of one 64-bit value per thread; returns the block
 // total through *total.
 __device__ unsigned long long block_excl_scan64(unsigned long long x, unsigned long long* total) {
-    __shared__ unsigned long long s_w[32];
+    __shared__ unsigned long long s_w[33];  // exclusive sums of up to 32 warps, total
     const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     unsigned long long inc = warp_incl_scan64(x);
     if (lane == 31) s_w[w] = inc;
@@ -97,11 +97,11 @@ __device__ unsigned long long block_excl_scan64(unsigned long long x, unsigned l
         unsigned long long v = lane < nw ? s_w[lane] : 0ull;
         unsigned long long vi = warp_incl_scan64(v);
         if (lane < nw) s_w[lane] = vi - v;
-        if (lane == nw - 1) s_w[31] = vi;
+        if (lane == nw - 1) s_w[32] = vi;
     }
     __syncthreads();
     unsigned long long res = inc - x + s_w[w];
-    *total = s_w[31];
+    *total = s_w[32];
     __syncthreads();
     return res;
 }
@@ -1168,7 +1168,8 @@ __device__ __forceinline__ int count_pass(const Trans2Params& p, const int32_t* 
     return entries;
 }
 
-// Counters of the first run's vertices against every neighbour, at the
+// Counters of the first run's vertices on the handle's own graph (the sorts
+// count those of the relabeled one) against every neighbour, at the
 // vertex's starting value in group 0's cur (vertices with a value below 1 get
 // zero counts: they are never evaluated and no counter includes them).
 __global__ void k_counters_init(Trans2Params p) {
@@ -1641,65 +1642,100 @@ static constexpr int kSortWarp = 256;
 static constexpr int kSortMid = 4096;
 static constexpr int kSortThreads = 256;
 
-struct ListSrc {
-    const uint32_t* off;
-    const uint32_t* nbr;
-    const uint32_t* order;
-    const uint32_t* pos;
+// Both sides of the relabeled graph in one launch (blockIdx.y).  Along with its
+// list every vertex gets its support count on that side at its row 0: the
+// neighbours below n0 (|C_k0|) whose row 0 is no smaller.  The entries are in
+// registers here; a pass of its own over both sides took 0.43 ms of R-MAT 20.
+struct SortSide {
+    const uint32_t* off;    // starts and lengths of the new lists
+    const int32_t* len;
+    uint32_t* nbr;
+    const uint32_t* src;    // the handle's lists, and where each list starts there
+    const uint32_t* start;
+    uint32_t* list[3];      // longer lists: for the warp, the block and the counting sort
+    int32_t* support;
 };
-__device__ __forceinline__ const uint32_t* src_list(const ListSrc& s, uint32_t i) { return s.nbr + s.off[s.order[i]]; }
-// Both sides of the relabeled graph in one launch (blockIdx.y), of its lists
-// those for the warp, block and counting sort listed by the first one.
 struct SortArgs {
-    const uint32_t* off[2];
-    const int32_t* len[2];
-    uint32_t* nbr[2];
-    ListSrc src[2];
-    uint32_t* list[2][3];
-    unsigned* cnt;  // [6], zero before
-    const int32_t* kmax;
+    SortSide side[2];
+    unsigned* cnt;        // [6] longer lists by side and sort, zero before
+    const uint2* pos;     // new id and row 0 by the handle's id: one gather per entry
+    const int32_t* kmax;  // by new id
+    const int32_t* row0;
+    uint32_t n0;
     int K;
 };
+// Least value that supports v (0x7FFFFFFF: v is never evaluated, no counts).
+__device__ __forceinline__ int support_level(const SortArgs& p, uint32_t v) {
+    const int r = v < p.n0 ? p.row0[v] : 0;
+    return r >= 1 ? r : 0x7FFFFFFF;
+}
+// Entry u renamed; *sup counts it if it supports.
+__device__ __forceinline__ uint32_t rename(const SortArgs& p, uint32_t u, int level, int* sup) {
+    const uint2 x = __ldg(p.pos + u);
+    *sup += x.x < p.n0 && (int)x.y >= level;
+    return x.x;
+}
 
-// Lists of at most kSortShort entries are sorted here, one thread each;
-// longer ones are listed for the warp sort (up to kSortWarp), the block
-// sort (up to kSortMid) or the counting sort.
-__global__ void k_sort_short(uint32_t V, SortArgs p) {
-    const uint32_t* off = p.off[blockIdx.y];
-    const int32_t* len = p.len[blockIdx.y];
-    uint32_t* nbr = p.nbr[blockIdx.y];
-    uint32_t* const* lists = p.list[blockIdx.y];
-    unsigned* cnt = p.cnt + 3 * blockIdx.y;
-    const ListSrc src = p.src[blockIdx.y];
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x) {
-        int n = len[v];
-        if (n > kSortMid) {
-            lists[2][atomicAdd(&cnt[2], 1u)] = (uint32_t)v;
-            continue;
-        }
-        if (n > kSortWarp) {
-            lists[1][atomicAdd(&cnt[1], 1u)] = (uint32_t)v;
-            continue;
-        }
-        if (n > kSortShort) {
-            lists[0][atomicAdd(&cnt[0], 1u)] = (uint32_t)v;
-            continue;
-        }
-        if (n < 1) continue;
-        uint32_t* a = nbr + off[v];
-        const uint32_t* in = src_list(src, (uint32_t)v);
-        uint32_t ids[kSortShort];
-        for (int i = 0; i < n; ++i) ids[i] = src.pos[in[i]];
-        for (int i = 1; i < n; ++i) {
-            const uint32_t x = ids[i];
-            int jj = i - 1;
-            while (jj >= 0 && ids[jj] > x) {
-                ids[jj + 1] = ids[jj];
-                --jj;
+// Lists of at most kSortShort entries, eight lanes each with T entries per
+// lane (entry 8 t + lane in k[t], bitonic as below): four lists per warp, their
+// entries read and written side by side.  Bound by the latency of the two
+// dependent loads (entry, new id).  One thread per list, an insertion
+// sort in local memory and the list found through two more loads took 148 us
+// of R-MAT 20 and 23 us of 10,000 vertices (both sides, no counts).
+template <int T>
+__device__ __forceinline__ void oct_sort(const SortArgs& p, const uint32_t* in, int n, int level, uint32_t* a, int* sup) {
+    const int sl = (int)(threadIdx.x & 7u);
+    uint32_t k[T];
+    int c = 0;
+#pragma unroll
+    for (int t = 0; t < T; ++t) k[t] = 8 * t + sl < n ? in[8 * t + sl] : 0xFFFFFFFFu;
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+        if (8 * t + sl < n) k[t] = rename(p, k[t], level, &c);
+#pragma unroll
+    for (int size = 2; size <= 8 * T; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride; stride >>= 1) {
+#pragma unroll
+            for (int t = 0; t < T; ++t) {
+                const bool up = ((8 * t + sl) & size) == 0;
+                if (stride >= 8) {
+                    const int o = t ^ (stride >> 3);
+                    if (o > t) {
+                        const uint32_t lo = min(k[t], k[o]), hi = max(k[t], k[o]);
+                        k[t] = up ? lo : hi;
+                        k[o] = up ? hi : lo;
+                    }
+                } else {
+                    const uint32_t o = __shfl_xor_sync(0xFFFFFFFFu, k[t], stride);
+                    k[t] = ((sl & stride) == 0) == up ? min(k[t], o) : max(k[t], o);
+                }
             }
-            ids[jj + 1] = x;
         }
-        for (int i = 0; i < n; ++i) a[i] = ids[i];
+    }
+#pragma unroll
+    for (int t = 0; t < T; ++t)
+        if (8 * t + sl < n) a[8 * t + sl] = k[t];
+    c += __shfl_xor_sync(0xFFFFFFFFu, c, 4);
+    c += __shfl_xor_sync(0xFFFFFFFFu, c, 2);
+    *sup = c + __shfl_xor_sync(0xFFFFFFFFu, c, 1);
+}
+__global__ void k_sort_short(uint32_t V, SortArgs p) {
+    const SortSide& S = p.side[blockIdx.y];
+    const unsigned lane = threadIdx.x & 31u;
+    const uint64_t stride = (((uint64_t)gridDim.x * blockDim.x) >> 5) * 4;
+    for (uint64_t b = ((blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5) * 4; b < V; b += stride) {
+        const uint64_t i = b + (lane >> 3);
+        const int len = i < V ? S.len[i] : 0, n = len <= kSortShort ? len : 0;
+        const uint32_t v = i < V ? (uint32_t)i : 0u;
+        const uint32_t* in = S.src + S.start[v];
+        uint32_t* a = S.nbr + S.off[v];
+        const int level = support_level(p, v), most = (int)__reduce_max_sync(0xFFFFFFFFu, (unsigned)n);
+        int sup = 0;
+        if (most > 16) oct_sort<4>(p, in, n, level, a, &sup);
+        else if (most > 8) oct_sort<2>(p, in, n, level, a, &sup);
+        else if (most) oct_sort<1>(p, in, n, level, a, &sup);
+        if ((lane & 7u) == 0 && i < p.n0 && len <= kSortShort) S.support[i] = sup;
     }
 }
 
@@ -1732,38 +1768,37 @@ __device__ __forceinline__ void warp_stages(uint32_t k[T], int size, int from, i
 // One warp per list of kSortShort+1 .. 32 T entries: bitonic sort in
 // registers (the places past the end hold the largest value and stay last).
 // 240 shuffles for 256 entries, where ranking every entry against every other
-// took 2,048 comparisons per lane.
+// took 2,048 comparisons per lane.  Returns the support count.
 template <int T>
-__device__ __forceinline__ void warp_sort(const uint32_t* in, const uint32_t* pos, int n, uint32_t* a) {
+__device__ __forceinline__ int warp_sort(const SortArgs& p, const uint32_t* in, int n, int level, uint32_t* a) {
     const int lane = (int)(threadIdx.x & 31u);
     uint32_t k[T];
+    int c = 0;
 #pragma unroll
     for (int t = 0; t < T; ++t) k[t] = 32 * t + lane < n ? in[32 * t + lane] : 0xFFFFFFFFu;
 #pragma unroll
     for (int t = 0; t < T; ++t)
-        if (32 * t + lane < n) k[t] = pos[k[t]];
+        if (32 * t + lane < n) k[t] = rename(p, k[t], level, &c);
 #pragma unroll
     for (int size = 2; size <= 32 * T; size <<= 1) warp_stages<T>(k, size, size >> 1, 0);
 #pragma unroll
     for (int t = 0; t < T; ++t)
         if (32 * t + lane < n) a[32 * t + lane] = k[t];
+    return __reduce_add_sync(0xFFFFFFFFu, c);
 }
 __global__ void __launch_bounds__(kSortThreads) k_sort_warp(SortArgs p) {
-    const uint32_t* off = p.off[blockIdx.y];
-    const int32_t* len = p.len[blockIdx.y];
-    uint32_t* nbr = p.nbr[blockIdx.y];
-    const uint32_t* list = p.list[blockIdx.y][0];
-    const ListSrc src = p.src[blockIdx.y];
     static_assert(kSortWarp == 256, "eight entries per lane");
+    const SortSide& S = p.side[blockIdx.y];
     const unsigned nl = p.cnt[3 * blockIdx.y], nw = gridDim.x * (kSortThreads / 32);
     for (unsigned li = blockIdx.x * (kSortThreads / 32) + (threadIdx.x >> 5); li < nl; li += nw) {
-        const uint32_t v = list[li];
-        const int n = len[v];
-        uint32_t* a = nbr + off[v];
-        const uint32_t* in = src_list(src, v);
-        if (n <= 64) warp_sort<2>(in, src.pos, n, a);
-        else if (n <= 128) warp_sort<4>(in, src.pos, n, a);
-        else warp_sort<8>(in, src.pos, n, a);
+        const uint32_t v = S.list[0][li];
+        const int n = S.len[v], level = support_level(p, v);
+        uint32_t* a = S.nbr + S.off[v];
+        const uint32_t* in = S.src + S.start[v];
+        const int sup = n <= 64    ? warp_sort<2>(p, in, n, level, a)
+                        : n <= 128 ? warp_sort<4>(p, in, n, level, a)
+                                   : warp_sort<8>(p, in, n, level, a);
+        if ((threadIdx.x & 31u) == 0 && v < p.n0) S.support[v] = sup;
     }
 }
 
@@ -1772,19 +1807,19 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_warp(SortArgs p) {
 // the strides of 256 and more go through shared memory (10 block-wide passes
 // for 4,096 entries instead of 78).
 __global__ void __launch_bounds__(kSortThreads) k_sort_mid(SortArgs p) {
-    const uint32_t* off = p.off[blockIdx.y];
-    const int32_t* len = p.len[blockIdx.y];
-    uint32_t* nbr = p.nbr[blockIdx.y];
-    const uint32_t* list = p.list[blockIdx.y][1];
-    const ListSrc src = p.src[blockIdx.y];
     __shared__ uint32_t s[kSortMid];
+    __shared__ int s_sup;
+    const SortSide& S = p.side[blockIdx.y];
     const int lane = (int)(threadIdx.x & 31u), w = (int)(threadIdx.x >> 5);
     const unsigned nl = p.cnt[3 * blockIdx.y + 1];
+    if (threadIdx.x == 0) s_sup = 0;
+    __syncthreads();
     for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
-        const uint32_t v = list[li];
-        const int n = len[v];
-        uint32_t* a = nbr + off[v];
-        const uint32_t* in = src_list(src, v);
+        const uint32_t v = S.list[1][li];
+        const int n = S.len[v], level = support_level(p, v);
+        uint32_t* a = S.nbr + S.off[v];
+        const uint32_t* in = S.src + S.start[v];
+        int sup = 0;
         int N = 512;
         while (N < n) N <<= 1;
         for (int c = 256 * w; c < N; c += 8 * kSortThreads) {  // one run per warp and turn
@@ -1793,13 +1828,19 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_mid(SortArgs p) {
             for (int t = 0; t < 8; ++t) k[t] = c + 32 * t + lane < n ? in[c + 32 * t + lane] : 0xFFFFFFFFu;
 #pragma unroll
             for (int t = 0; t < 8; ++t)
-                if (c + 32 * t + lane < n) k[t] = src.pos[k[t]];
+                if (c + 32 * t + lane < n) k[t] = rename(p, k[t], level, &sup);
 #pragma unroll
             for (int size = 2; size <= 256; size <<= 1) warp_stages<8>(k, size, size >> 1, c);
 #pragma unroll
             for (int t = 0; t < 8; ++t) s[c + 32 * t + lane] = k[t];
         }
+        sup = __reduce_add_sync(0xFFFFFFFFu, sup);
+        if (lane == 0 && sup) atomicAdd(&s_sup, sup);
         __syncthreads();
+        if (threadIdx.x == 0) {
+            if (v < p.n0) S.support[v] = s_sup;
+            s_sup = 0;
+        }
         for (int size = 512; size <= N; size <<= 1) {
             for (int stride = size >> 1; stride >= 256; stride >>= 1) {
                 for (int q = threadIdx.x; q < N / 2; q += kSortThreads) {
@@ -1835,25 +1876,23 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_mid(SortArgs p) {
 // cache line of values) while there are bins for lines, plus K - kmax, which
 // grows with the id and keeps the classes of kmax apart; entries of a bin keep
 // no particular order.  The list fits no shared memory, so its entries are
-// renamed twice.
+// renamed twice.  Bound by the longest list: 1,024 threads, four entries each.
 static constexpr int kSortBigBins = 11264;
-__global__ void k_sort_big(SortArgs p) {
-    const uint32_t* off = p.off[blockIdx.y];
-    const int32_t* len = p.len[blockIdx.y];
-    uint32_t* nbr = p.nbr[blockIdx.y];
-    const uint32_t* list = p.list[blockIdx.y][2];
-    const ListSrc src = p.src[blockIdx.y];
-    const int32_t* kmax = p.kmax;
-    const int K = p.K;
+__global__ void __launch_bounds__(1024) k_sort_big(SortArgs p) {
     __shared__ unsigned bins[kSortBigBins];
+    __shared__ int s_sup;
+    const SortSide& S = p.side[blockIdx.y];
     const unsigned nl = p.cnt[3 * blockIdx.y + 2];
+    const int K = p.K;
     const uint32_t lines = (uint32_t)(kSortBigBins - 1 - K);
-    auto bin_of = [&](uint32_t u) { return (int)min(u >> 5, lines) + (K - kmax[u]); };
+    auto bin_of = [&](uint32_t u) { return (int)min(u >> 5, lines) + (K - p.kmax[u]); };
     for (unsigned li = blockIdx.x; li < nl; li += gridDim.x) {
-        const uint32_t v = list[li];
-        const int n = len[v];
-        uint32_t* a = nbr + off[v];
-        const uint32_t* in = src_list(src, v);
+        const uint32_t v = S.list[2][li];
+        const int n = S.len[v], level = support_level(p, v);
+        uint32_t* a = S.nbr + S.off[v];
+        const uint32_t* in = S.src + S.start[v];
+        int sup = 0;
+        if (threadIdx.x == 0) s_sup = 0;
         for (int i = threadIdx.x; i < kSortBigBins; i += blockDim.x) bins[i] = 0;
         __syncthreads();
         // four entries in flight per thread (three dependent loads each)
@@ -1864,14 +1903,16 @@ __global__ void k_sort_big(SortArgs p) {
             for (int q = 0; q < 4; ++q) u[q] = i0 + q * (int)blockDim.x < n ? in[i0 + q * blockDim.x] : 0xFFFFFFFFu;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                if (u[q] != 0xFFFFFFFFu) u[q] = src.pos[u[q]];
+                if (u[q] != 0xFFFFFFFFu) u[q] = rename(p, u[q], level, &sup);
 #pragma unroll
             for (int q = 0; q < 4; ++q) b[q] = u[q] != 0xFFFFFFFFu ? bin_of(u[q]) : -1;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
                 if (b[q] >= 0) atomicAdd(&bins[b[q]], 1u);
         }
+        if (sup) atomicAdd(&s_sup, sup);
         __syncthreads();
+        if (threadIdx.x == 0 && v < p.n0) S.support[v] = s_sup;
         // exclusive scan of the bins, blockDim at a time
         unsigned long long carry = 0;
         for (int b0 = 0; b0 < kSortBigBins; b0 += blockDim.x) {
@@ -1890,7 +1931,7 @@ __global__ void k_sort_big(SortArgs p) {
             for (int q = 0; q < 4; ++q) u[q] = i0 + q * (int)blockDim.x < n ? in[i0 + q * blockDim.x] : 0xFFFFFFFFu;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                if (u[q] != 0xFFFFFFFFu) u[q] = src.pos[u[q]];
+                if (u[q] != 0xFFFFFFFFu) u[q] = __ldg(p.pos + u[q]).x;
 #pragma unroll
             for (int q = 0; q < 4; ++q) b[q] = u[q] != 0xFFFFFFFFu ? bin_of(u[q]) : -1;
 #pragma unroll
@@ -1961,22 +2002,45 @@ __global__ void k_kmax_degree_hist(uint32_t V, const int32_t* kmax, const int32_
             if (sw[i]) atomicAdd(&w[i], sw[i]);
 }
 
-// cursor[k] = first position of bucket k in descending-kmax order
-// Warp-aggregated: lanes holding the same kmax take their positions with one
-// atomic (the leader's) instead of one each.
-__global__ void k_order_scatter(uint32_t V, const int32_t* kmax, uint32_t* cursor, uint32_t* order) {
-    const unsigned lane = threadIdx.x & 31u;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t base = (blockIdx.x * (uint64_t)blockDim.x) & ~31ull; base < V; base += stride) {
-        const uint64_t v = base + (threadIdx.x & ~31u) % blockDim.x + lane;
-        const bool ok = v < V;
-        const int key = ok ? kmax[v] : -1;
-        const unsigned peers = __match_any_sync(0xFFFFFFFFu, key);
-        const unsigned leader = __ffs(peers) - 1;
-        unsigned p0 = 0;
-        if (ok && lane == leader) p0 = atomicAdd(&cursor[key], (unsigned)__popc(peers));
-        p0 = __shfl_sync(0xFFFFFFFFu, p0, leader);
-        if (ok) order[p0 + __popc(peers & ((1u << lane) - 1u))] = (uint32_t)v;
+// cursor[k] = first position of bucket k in descending-kmax order.  Most
+// vertices share a few small kmax values, whose cursors bound the pass: the
+// lanes of a warp that hold the same kmax count as one in the block's bins,
+// and a block takes the positions of a bin's vertices with one atomic (one
+// per warp and value: 73 us of R-MAT 20).  Values past the bins go to the
+// cursor one warp at a time.
+constexpr int kOrderBins = 1024, kOrderItems = 8;
+__global__ void __launch_bounds__(kThreads) k_order_scatter(uint32_t V, const int32_t* kmax, int K, uint32_t* cursor,
+                                                            uint32_t* order) {
+    __shared__ uint32_t bin[kOrderBins];
+    const unsigned lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    const int bins = min(K + 1, kOrderBins);
+    for (uint64_t b = (uint64_t)blockIdx.x * kThreads * kOrderItems; b < V; b += (uint64_t)gridDim.x * kThreads * kOrderItems) {
+        int key[kOrderItems];
+        uint32_t at[kOrderItems];
+        for (int i = threadIdx.x; i < bins; i += kThreads) bin[i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kOrderItems; ++q) {
+            const uint64_t v = b + q * kThreads + threadIdx.x;
+            key[q] = v < V ? kmax[v] : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < kOrderItems; ++q) {
+            const unsigned peers = __match_any_sync(0xFFFFFFFFu, key[q]), leader = __ffs(peers) - 1;
+            uint32_t p0 = 0;
+            if (key[q] >= 0 && lane == leader)
+                p0 = atomicAdd(key[q] < bins ? &bin[key[q]] : &cursor[key[q]], (unsigned)__popc(peers));
+            at[q] = __shfl_sync(0xFFFFFFFFu, p0, leader) + __popc(peers & below);
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < bins; i += kThreads)
+            if (bin[i]) bin[i] = atomicAdd(&cursor[i], bin[i]);
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kOrderItems; ++q)
+            if (key[q] >= 0)
+                order[at[q] + (key[q] < bins ? bin[key[q]] : 0u)] = (uint32_t)(b + q * kThreads + threadIdx.x);
+        __syncthreads();
     }
 }
 
@@ -2352,7 +2416,7 @@ uint64_t device_footprint(const dc_graph* h) {
         for (const RowSegment& sg : s->seg)
             b += (sg.cur ? 24 * ((uint64_t)sg.cap_V + 1) : 0) + 8 * sg.tring_cap + (sg.ctl ? sizeof(EngineCtl) : 0);
         b += (s->plan ? sizeof(RowPlan) : 0) + 4ull * s->seam_of_cap + 4 * s->seam_cap;
-        if (s->pos) b += 4 * 7 * ((uint64_t)s->r_cap_V + 1);     // relabeled graph: ids, kmax, row 0, offsets, lengths
+        if (s->pos) b += 4 * 8 * ((uint64_t)s->r_cap_V + 1);     // relabeled graph: ids, kmax, row 0, offsets, lengths
         if (s->r_nbr[0]) b += 2 * 4 * s->r_cap;     // its lists
     }
     return b;
@@ -2810,16 +2874,48 @@ int expand_rows(dc_graph* h, uint32_t k0, uint32_t n, int32_t* d_dst) {
 // of C_k read its state contiguously, and the dense core's state (the
 // vertices of the heavy rows) packs into a small range that stays in the
 // SMs' caches.  Lists hold new ids, ordered by neighbour kmax.
+// Starts and lengths of both lists go along, and the lists too long for
+// k_sort_short are listed for the other sorts (one atomic per warp and sort).
+struct GatherSide {
+    const uint32_t* off;
+    const int32_t* len;
+    uint32_t* start;
+    int32_t* len_r;
+    uint32_t* list[3];
+};
 __global__ void k_relabel_gather(uint32_t V, const uint32_t* order, const int32_t* kmax, const int32_t* row0,
-                                 const int32_t* out_len, const int32_t* in_len, uint32_t* pos, int32_t* kmax_r,
-                                 int32_t* row0_r, int32_t* len_o, int32_t* len_i) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < V; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = order[i];
-        pos[v] = (uint32_t)i;
-        kmax_r[i] = kmax[v];
-        row0_r[i] = row0[v];
-        len_o[i] = out_len[v];
-        len_i[i] = in_len[v];
+                                 uint2* pos, int32_t* kmax_r, int32_t* row0_r, GatherSide out, GatherSide in,
+                                 unsigned* cnt) {
+    const unsigned lane = threadIdx.x & 31u;
+    for (uint64_t b = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) & ~31ull; b < V;
+         b += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = b + lane;
+        int n[2] = {0, 0};
+        if (i < V) {
+            const uint32_t v = order[i];
+            const int r0 = row0[v];
+            pos[v] = make_uint2((uint32_t)i, (uint32_t)r0);
+            kmax_r[i] = kmax[v];
+            row0_r[i] = r0;
+            out.start[i] = out.off[v];
+            in.start[i] = in.off[v];
+            out.len_r[i] = n[0] = out.len[v];
+            in.len_r[i] = n[1] = in.len[v];
+        }
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const GatherSide& S = side == 0 ? out : in;
+            const int to = n[side] > kSortMid ? 2 : n[side] > kSortWarp ? 1 : n[side] > kSortShort ? 0 : -1;
+#pragma unroll
+            for (int l = 0; l < 3; ++l) {
+                const unsigned m = __ballot_sync(0xFFFFFFFFu, to == l);
+                if (!m) continue;
+                unsigned at = 0;
+                if (lane == 0) at = atomicAdd(&cnt[3 * side + l], (unsigned)__popc(m));
+                at = __shfl_sync(0xFFFFFFFFu, at, 0);
+                if (to == l) S.list[l][at + __popc(m & ((1u << lane) - 1u))] = (uint32_t)i;
+            }
+        }
     }
 }
 
@@ -2904,7 +3000,7 @@ __global__ void k_rows_collect(RowsStart r, const RowPlan* plan) {
 // Builds the relabeled graph (s->order must hold the kmax order of the
 // current kmax) with its lists sorted by neighbour kmax, plus kmax and row 0
 // by new id.
-static int build_relabeled(dc_graph* h, int32_t K, unsigned* sort_cnt) {
+static int build_relabeled(dc_graph* h, int32_t K, uint32_t n0, unsigned* sort_cnt) {
     DevGraph& g = h->g;
     Scratch* s = h->scratch;
     const uint32_t V = g.V;
@@ -2936,29 +3032,37 @@ static int build_relabeled(dc_graph* h, int32_t K, unsigned* sort_cnt) {
         }
         s->r_cap = want;
     }
+    uint32_t* start = (uint32_t*)s->tmp64;  // of every list in the handle's, out then in
+    SortArgs so;
+    so.side[0] = SortSide{s->r_off[0], s->r_len[0], s->r_nbr[0], g.out_nbr, start, {s->rem0, s->rem2, s->rem1}, s->cnt_out};
+    so.side[1] = SortSide{s->r_off[1], s->r_len[1], s->r_nbr[1], g.in_nbr, start + n,
+                          {s->rem3, (uint32_t*)s->cdeg, (uint32_t*)s->cdeg2}, s->key};
+    so.cnt = sort_cnt;
+    so.pos = s->pos;
+    so.kmax = s->kmax_r;
+    so.row0 = s->row0_r;
+    so.n0 = n0;
+    so.K = K;
+    GatherSide gs[2];
+    for (int side = 0; side < 2; ++side) {
+        gs[side] = GatherSide{side == 0 ? g.out_off : g.in_off, side == 0 ? g.out_len : g.in_len, start + side * n,
+                              s->r_len[side], {}};
+        for (int l = 0; l < 3; ++l) gs[side].list[l] = so.side[side].list[l];
+    }
     ++g_launches;
-    k_relabel_gather<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, s->order, h->d.kmax_v, s->row0, g.out_len,
-                                                                  g.in_len, s->pos, s->kmax_r, s->row0_r, s->r_len[0],
-                                                                  s->r_len[1]);
+    k_relabel_gather<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, s->order, h->d.kmax_v, s->row0, s->pos, s->kmax_r,
+                                                                  s->row0_r, gs[0], gs[1], sort_cnt);
     const ListStarts ls{{s->r_len[0], s->r_len[1]}, {s->r_off[0], s->r_off[1]}, 0, 0};
     scan_sums(h, ls, 2, V);
     scan_apply(h, ls, 2, V);
     // every relabeled list is read from its original list, renamed and
     // sorted in one pass; most lists go to the short and the warp sort, the
     // others read their counts on the device
-    const SortArgs so{{s->r_off[0], s->r_off[1]},
-                      {s->r_len[0], s->r_len[1]},
-                      {s->r_nbr[0], s->r_nbr[1]},
-                      {{g.out_off, g.out_nbr, s->order, s->pos}, {g.in_off, g.in_nbr, s->order, s->pos}},
-                      {{s->rem0, s->rem2, s->rem1}, {s->rem3, (uint32_t*)s->cdeg, (uint32_t*)s->cdeg2}},
-                      sort_cnt,
-                      s->kmax_r,
-                      K};
     g_launches += 4;
-    k_sort_short<<<dim3(grid_for(h, V), 2), kThreads, 0, h->stream>>>(V, so);
+    k_sort_short<<<dim3(grid_for(h, 8ull * V), 2), kThreads, 0, h->stream>>>(V, so);
     k_sort_warp<<<dim3(h->geom.sms * 8, 2), kSortThreads, 0, h->stream>>>(so);
     k_sort_mid<<<dim3(h->geom.sms * 8, 2), kSortThreads, 0, h->stream>>>(so);
-    k_sort_big<<<dim3(h->geom.sms * 2, 2), 512, 0, h->stream>>>(so);
+    k_sort_big<<<dim3(h->geom.sms, 2), 1024, 0, h->stream>>>(so);
     DC_CUDA(cudaGetLastError());
     return DC_OK;
 }
@@ -3014,7 +3118,8 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     }
     DC_CUDA(cudaMemcpyAsync(d_ck, ck, sizeof(uint32_t) * 2 * nk, cudaMemcpyHostToDevice, h->stream));
     ++g_launches;
-    k_order_scatter<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, d.kmax_v, hist, s->order);
+    k_order_scatter<<<grid_for(h, ((uint64_t)V + kOrderItems - 1) / kOrderItems), kThreads, 0, h->stream>>>(
+        V, d.kmax_v, K, hist, s->order);
     // The graph the row kernel reads: where sorting is allowed, the graph
     // relabeled in kmax order with kmax-sorted lists (C_k a prefix of the
     // ids); else the handle's own lists (kmax-sorted when they still are from
@@ -3104,13 +3209,14 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
         if (dmalloc(h->stream, &s->log_v, cap) || dmalloc(h->stream, &s->log_k, cap) || dmalloc(h->stream, &s->log_l, cap)) return DC_ERR_NOMEM;
         s->log_cap = cap;
     }
+    const uint32_t n0 = relabel ? ck[std::min(k0, K + 1)] : V;
     int sorted = 0;
     const uint32_t *G_out_off = g.out_off, *G_in_off = g.in_off, *G_order = s->order;
     int32_t *G_out_len = g.out_len, *G_in_len = g.in_len;
     uint32_t *G_out_nbr = g.out_nbr, *G_in_nbr = g.in_nbr;
     const int32_t *G_kmax = d.kmax_v, *G_row0 = s->row0;
     if (relabel) {
-        if (int rc = build_relabeled(h, K, sort_cnt)) return rc;
+        if (int rc = build_relabeled(h, K, n0, sort_cnt)) return rc;
         sorted = 1;
         G_out_off = s->r_off[0];
         G_in_off = s->r_off[1];
@@ -3126,7 +3232,6 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     // the vertices outside already left (for k0 = 1 those of kmax 0), so its
     // first step has no leaving pass; the marks of all V vertices, because the
     // local core update expects them clear
-    const uint32_t n0 = relabel ? ck[std::min(k0, K + 1)] : V;
     if (int rc = ensure_tring(h, 2ull * V + (uint64_t)h->geom.sms * 64 + 4096)) return rc;
     Trans2Params tp;
     memset(&tp, 0, sizeof(tp));
@@ -3153,11 +3258,10 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
         if (relabel) {
             DC_CUDA(cudaMemcpyAsync(s->cur, G_row0, 4ull * n0, cudaMemcpyDeviceToDevice, h->stream));
         } else {
-            ++g_launches;
+            g_launches += 2;
             k_preleft_cur<<<grid_for(h, n0), kThreads, 0, h->stream>>>(n0, G_kmax, G_row0, k0, s->cur);
+            k_counters_init<<<grid_for(h, (uint64_t)n0 * 32), kThreads, 0, h->stream>>>(tp);
         }
-        ++g_launches;
-        k_counters_init<<<grid_for(h, (uint64_t)n0 * 32), kThreads, 0, h->stream>>>(tp);
         DC_CUDA(cudaMemsetAsync(s->stamp, 0xFF, sizeof(int32_t) * n0, h->stream));
     }
     RowsStart rs;

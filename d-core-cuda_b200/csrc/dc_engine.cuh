@@ -72,7 +72,7 @@ struct Scratch {
     uint64_t seam_cap = 0;
     // the graph relabeled in kmax-descending order for the row kernel:
     // new id = position in `order`; lists of new ids sorted by neighbour kmax
-    uint32_t* pos = nullptr;                    // [V] new id of each vertex
+    uint2* pos = nullptr;                       // [V] new id and row 0 of each vertex
     int32_t* kmax_r = nullptr;                  // [V] kmax by new id
     int32_t* row0_r = nullptr;                  // [V] row 0 by new id
     uint32_t* r_off[2] = {nullptr, nullptr};    // out / in list starts [V+1]

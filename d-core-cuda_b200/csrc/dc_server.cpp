@@ -104,7 +104,7 @@ uint64_t footprint_bound(uint64_t V, uint64_t E, uint64_t sms) {
     b += 12 * (E + V + 1);
     b += 16 * (2 * V + 2 * cap / 32 + sms * 64 + 4096);
     b += 8 * E + 2 * 4 * cap;
-    b += 4 * 7 * (V + 1) + 2 * 4 * ((E + 8) + (E + 8) / 8 + 7);  // the row kernel's relabeled graph
+    b += 4 * 8 * (V + 1) + 2 * 4 * ((E + 8) + (E + 8) / 8 + 7);  // the row kernel's relabeled graph
     // row groups: state (24 bytes and an eighth), ticket rings (powers of two)
     // and seams (with their void records) for an eighth of the vertices, a
     // quarter up to 65,536; control blocks and the log's spare records
