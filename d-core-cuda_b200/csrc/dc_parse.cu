@@ -17,13 +17,14 @@
 // vertex its row values 0..kmax[v] separated by spaces, a newline after every
 // vertex but the last.  Each vertex's line is formatted from its skyline
 // corners (a run of equal values per corner), line lengths are scanned, the
-// text is written on the device and copied to the host once.
+// text is written on the device and copied to the host a piece at a time.
 #include <algorithm>
 #include <atomic>
 #include <cerrno>
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <vector>
 
 #include "dc_engine.cuh"
 #include "dc_internal.h"
@@ -38,6 +39,7 @@ namespace {
 constexpr int kFT = 256;                // threads per block
 constexpr int kFBytes = 16;             // bytes (or items) per thread and tile
 constexpr int kFTile = kFT * kFBytes;   // per block tile
+constexpr uint64_t kFileChunk = 1u << 20;  // bytes read or written at a time
 constexpr int kMaxLine = 511;           // host parser's fgets buffer minus the terminator
 
 __device__ __forceinline__ unsigned long long block_excl_scan_u64(unsigned long long x, unsigned long long* total) {
@@ -144,6 +146,7 @@ __device__ bool parse_u(const char* b, uint64_t* p, uint64_t e, unsigned long lo
 __global__ void k_f_parse_lines(const char* b, uint64_t nbytes, const uint64_t* start, uint64_t nlines, uint32_t* src,
                                 uint32_t* dst, uint8_t* kind, unsigned long long* bad_line, unsigned* maxid,
                                 unsigned long long* header_v) {
+    unsigned most = 0;
     for (uint64_t l = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; l < nlines; l += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t s = start[l];
         uint64_t e = l + 1 < nlines ? start[l + 1] - 1 : nbytes;  // before the newline
@@ -169,12 +172,14 @@ __global__ void k_f_parse_lines(const char* b, uint64_t nbytes, const uint64_t* 
                     k = 1;
                     src[l] = (uint32_t)a;
                     dst[l] = (uint32_t)c;
-                    atomicMax(maxid, (unsigned)max(a, c));
+                    most = max(most, (unsigned)max(a, c));
                 }
             }
         }
         kind[l] = k;
     }
+    most = __reduce_max_sync(0xFFFFFFFFu, most);
+    if ((threadIdx.x & 31u) == 0 && most) atomicMax(maxid, most);
 }
 
 struct IsEdge {
@@ -301,18 +306,6 @@ int parse_text_graph_device(const char* path, int prune, cudaStream_t st, int sm
         return set_error(DC_ERR_INVALID, "'%s': empty file (no header line)", path);
     }
     const uint64_t nb = (uint64_t)size;
-    char* hbuf = nullptr;
-    if (cudaMallocHost((void**)&hbuf, nb) != cudaSuccess) {
-        cudaGetLastError();
-        fclose(f);
-        return set_error(DC_ERR_NOMEM, "pinned host buffer of %llu bytes", (unsigned long long)nb);
-    }
-    const bool read_ok = fread(hbuf, 1, nb, f) == nb;
-    fclose(f);
-    if (!read_ok) {
-        cudaFreeHost(hbuf);
-        return set_error(DC_ERR_IO, "short read of '%s'", path);
-    }
     int rc = DC_OK;
     char* d_b = nullptr;
     uint64_t* start = nullptr;
@@ -326,14 +319,24 @@ int parse_text_graph_device(const char* path, int prune, cudaStream_t st, int sm
         return e == cudaSuccess ? DC_OK : set_error(DC_ERR_CUDA, "text parse: %s: %s", what, cudaGetErrorString(e));
     };
     uint64_t nlines = 0, E = 0, V = 0;
+    char last = 0;
     do {
         const uint64_t ntile = (nb + kFTile - 1) / kFTile;
         if ((rc = f_alloc(st, &d_b, nb)) || (rc = f_alloc(st, &part, ntile + 1)) || (rc = f_alloc(st, &misc, 4)))
             break;
-        if (cudaMemcpyAsync(d_b, hbuf, nb, cudaMemcpyHostToDevice, st) != cudaSuccess) {
-            rc = set_error(DC_ERR_CUDA, "text parse: upload failed");
-            break;
+        // the file passes through a small buffer that stays in the CPU's
+        // caches: page-locking one of the file's size took 2 to 6 ms for 5 MB
+        // and its release 0.7, reading and copying take 0.8
+        std::vector<char> chunk(std::min<uint64_t>(nb, kFileChunk));
+        for (uint64_t at = 0; at < nb && !rc; at += chunk.size()) {
+            const uint64_t m = std::min<uint64_t>(chunk.size(), nb - at);
+            if (fread(chunk.data(), 1, m, f) != m) rc = set_error(DC_ERR_IO, "short read of '%s'", path);
+            else if (cudaMemcpyAsync(d_b + at, chunk.data(), m, cudaMemcpyHostToDevice, st) != cudaSuccess ||
+                     cudaStreamSynchronize(st) != cudaSuccess)
+                rc = set_error(DC_ERR_CUDA, "text parse: upload failed");
+            last = chunk[m - 1];
         }
+        if (rc) break;
         // line starts
         IsNewline isnl{d_b};
         k_f_tile_count<<<(unsigned)ntile, kFT, 0, st>>>(nb, isnl, part);
@@ -347,7 +350,7 @@ int parse_text_graph_device(const char* path, int prune, cudaStream_t st, int sm
             break;
         }
         // a last line without a newline counts too
-        nlines = nnl + (hbuf[nb - 1] != '\n' ? 1 : 0);
+        nlines = nnl + (last != '\n' ? 1 : 0);
         if ((rc = f_alloc(st, &start, nlines + 1))) break;
         const uint64_t zero = 0;
         if (cudaMemcpyAsync(start, &zero, 8, cudaMemcpyHostToDevice, st) != cudaSuccess) {
@@ -445,7 +448,7 @@ int parse_text_graph_device(const char* path, int prune, cudaStream_t st, int sm
                     (void*)used, (void*)map})
         if (p) cudaFreeAsync(p, st);
     cudaStreamSynchronize(st);
-    cudaFreeHost(hbuf);
+    fclose(f);
     if (rc) {
         if (src) cudaFreeAsync(src, st);
         if (dst) cudaFreeAsync(dst, st);
@@ -467,18 +470,16 @@ int write_decomp_cpu_device(dc_graph* h, const char* path) {
     char head[16];
     const int hn = snprintf(head, sizeof(head), "%u\n", V);
     int rc = DC_OK;
-    unsigned long long* len = nullptr;
     char* d_out = nullptr;
-    char* hbuf = nullptr;
     unsigned long long total = 0;
     const int grid = h->geom.sms * 8;
     do {
         if (V) {
-            if ((rc = f_alloc(st, &len, (uint64_t)V + 1))) break;
+            if ((rc = ensure_scratch(h, V))) break;
+            unsigned long long* len = (unsigned long long*)h->scratch->tmp64;
             ++g_launches;
             k_f_line_len<<<grid, kFT, 0, st>>>(V, d.kmax_v, d.sky_off, d.sky_k, d.sky_l, len);
-            ++g_launches;
-            k_f_scan_one_block<<<1, kFT, 0, st>>>(len, V);
+            if ((rc = scan_tmp64(h, V))) break;
             if (cudaMemcpyAsync(&total, len + V, 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                 cudaStreamSynchronize(st) != cudaSuccess) {
                 rc = set_error(DC_ERR_CUDA, "decompCPU: %s", cudaGetErrorString(cudaGetLastError()));
@@ -487,13 +488,7 @@ int write_decomp_cpu_device(dc_graph* h, const char* path) {
             if ((rc = f_alloc(st, &d_out, total))) break;
             ++g_launches;
             k_f_write_lines<<<grid, kFT, 0, st>>>(V, d.kmax_v, d.sky_off, d.sky_k, d.sky_l, len, d_out);
-            if (cudaMallocHost((void**)&hbuf, std::max<unsigned long long>(total, 1)) != cudaSuccess) {
-                cudaGetLastError();
-                rc = set_error(DC_ERR_NOMEM, "pinned host buffer of %llu bytes", total);
-                break;
-            }
-            if (cudaMemcpyAsync(hbuf, d_out, total, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-                cudaStreamSynchronize(st) != cudaSuccess) {
+            if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {
                 rc = set_error(DC_ERR_CUDA, "decompCPU: %s", cudaGetErrorString(cudaGetLastError()));
                 break;
             }
@@ -504,14 +499,20 @@ int write_decomp_cpu_device(dc_graph* h, const char* path) {
             break;
         }
         bool ok = fwrite(head, 1, (size_t)hn, f) == (size_t)hn;
-        if (ok && total) ok = fwrite(hbuf, 1, total, f) == total;
+        std::vector<char> chunk(std::min<uint64_t>(total, kFileChunk));
+        for (uint64_t at = 0; at < total && ok && !rc; at += chunk.size()) {
+            const uint64_t m = std::min<uint64_t>(chunk.size(), total - at);
+            if (cudaMemcpyAsync(chunk.data(), d_out + at, m, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaStreamSynchronize(st) != cudaSuccess)
+                rc = set_error(DC_ERR_CUDA, "decompCPU: %s", cudaGetErrorString(cudaGetLastError()));
+            else ok = fwrite(chunk.data(), 1, m, f) == m;
+        }
         if (fclose(f) != 0) ok = false;
+        if (rc) break;
         if (!ok) rc = set_error(DC_ERR_IO, "short write to '%s'", path);
     } while (0);
-    if (len) cudaFreeAsync(len, st);
     if (d_out) cudaFreeAsync(d_out, st);
     cudaStreamSynchronize(st);
-    if (hbuf) cudaFreeHost(hbuf);
     return rc;
 }
 
