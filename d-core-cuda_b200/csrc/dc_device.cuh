@@ -616,7 +616,7 @@ __device__ __forceinline__ unsigned long long step_block_word(const StepBlock* b
 
 // One thread: n producers or items of step `word` are finished; the last one
 // advances the step.  next(c, level, worked, bound): the next level;
-// next.blocks: the blocks that work on the steps.
+// next.begin(step): the blocks that seed that step, before it is published.
 template <typename Next>
 __device__ __forceinline__ void step_finish(EngineCtl* c, int n, unsigned long long word, const Next& next) {
     const unsigned long long old = atomicAdd(&c->t_work, 0ull - ((unsigned long long)n << kWorkShift));
@@ -643,7 +643,7 @@ __device__ __forceinline__ void step_finish(EngineCtl* c, int n, unsigned long l
     }
     c->step = (int)step;
     c->trace_tail0 = tail;
-    atomicAdd(&c->t_work, (unsigned long long)next.blocks << kWorkShift);
+    atomicAdd(&c->t_work, (unsigned long long)next.begin(step + 1) << kWorkShift);
     __threadfence();
     const unsigned long long w = ((unsigned long long)(step + 1) << 32) | (unsigned long long)(uint32_t)level;
 #pragma unroll

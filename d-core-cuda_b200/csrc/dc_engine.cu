@@ -361,6 +361,7 @@ __device__ __forceinline__ unsigned peel_unit(unsigned chunk, unsigned len) {
 struct PeelHook {
     int ninst;
     unsigned blocks;
+    __device__ unsigned begin(unsigned) const { return blocks; }
     __device__ __forceinline__ int operator()(EngineCtl* c, int level, bool worked, int bound) const {
         for (int i = 0; i < ninst; ++i) {
             unsigned n = ld_vol(&c->rc_cur[i]);
@@ -814,6 +815,10 @@ struct RowPlan {
         int from;                     // group whose values the run to start begins with (-1: row 0)
         unsigned ready;               // the group's values belong to its run
         unsigned readers;             // groups about to copy its values
+        unsigned members;             // blocks of the group, those that joined included
+        unsigned long long step_blocks;  // (step << 32) | blocks that seed it: members 0 .. blocks - 1
+        int prev;                     // row before the current one (the current one if it is the run's first)
+        int join;                     // group that this one's blocks go to
     } own[kRowGroups];
     alignas(128) unsigned seam_tail;
     alignas(128) unsigned log_count;
@@ -856,6 +861,7 @@ constexpr int kRowsEnd = 0x7FFFFFFF;  // the group leaves
 constexpr int kRowsInit = -1;         // start values of the group's next run
 constexpr int kRowsCount = -2;        // its counters
 constexpr int kRowsWait = -3;         // nothing to take over yet
+constexpr int kRowsJoin = -4;         // the group is over, its blocks go on in another one
 
 // Next step of a group (run by the warp that finished the step).  After a row
 // that needed no work the run jumps to the first row whose leaving set or
@@ -867,10 +873,27 @@ constexpr int kRowsWait = -3;         // nothing to take over yet
 // other group's values as they are: values only fall, within a row and from
 // row to row, so any of them bounds the later row's from above (from row 0
 // the first row of such a run took up to 8 ms).
+// When no group has rows worth taking over, the group's blocks join the one
+// with the most left for good: they take items of its current row at once and
+// seed with its own blocks from the next step on.  The last rows below a cliff
+// of |C_k| are the heaviest and cannot be cut any more: one group's blocks
+// alone took the last 30 % of the rows of R-MAT 20 and 22 for them (joining,
+// and counts in shared memory instead of spilled registers, took the rows from
+// 5.7 and 17.7 ms to 5.0 and 15.8).  A group that others join has a run at
+// that time, a finished group's run is cleared before it looks for one to
+// join, and it never gets another: no two groups join each other.
 struct RowsNext {
     const Trans2Params& p;
     int gid;
-    unsigned blocks;
+    unsigned blocks;  // of a launch without groups
+
+    __device__ unsigned begin(unsigned step) const {
+        if (p.n_groups == 1) return blocks;
+        RowPlan::Own& own = p.plan->own[gid];
+        const unsigned b = ld_vol(&own.members);
+        *(volatile unsigned long long*)&own.step_blocks = ((unsigned long long)step << 32) | b;
+        return b;
+    }
 
     __device__ int operator()(EngineCtl*, int level, bool worked, int bound) const {
         const int r = worked ? level + 1 : max(level + 1, bound);
@@ -888,7 +911,9 @@ struct RowsNext {
             own.row_ns = 0;
             __threadfence();
             *(volatile unsigned*)&own.ready = 1u;
-            return ld_vol(&own.lo);
+            const int lo = ld_vol(&own.lo);
+            *(volatile int*)&own.prev = lo;
+            return lo;
         }
         bool flush = false;
         if (level > 0) {
@@ -905,6 +930,7 @@ struct RowsNext {
                     const unsigned long long t = *(volatile unsigned long long*)&own.t_row;
                     if (t) *(volatile unsigned*)&own.row_ns = (unsigned)min(now - t, 0xFFFFFFFFull);
                     *(volatile unsigned long long*)&own.t_row = now;
+                    *(volatile int*)&own.prev = level;
                     return r;
                 }
                 // the run is over: the run that starts at stop + 1 needs its last row's values
@@ -920,7 +946,7 @@ struct RowsNext {
         } else {
             own.flush_n = 0;
         }
-        bool any = false;
+        bool any = false, wanted = false;
         // (a group that others still copy from keeps its values)
         const bool busy = ld_acquire(&own.readers) != 0u;
         for (int attempt = 0; attempt < 4; ++attempt) {
@@ -951,6 +977,7 @@ struct RowsNext {
                     best_score = score;
                 }
             }
+            wanted = best >= 0;
             if (best < 0 || busy) break;
             const unsigned n = __ldg(p.ck + best_start);
             if (own.spare_n < n) {
@@ -990,6 +1017,24 @@ struct RowsNext {
         for (int h = 0; h < p.n_groups; ++h)
             if (ld_vol(&p.g[h].ctl->error)) any = false;
         if (!any) return kRowsEnd;
+        if (!wanted) {
+            int to = -1;
+            unsigned long long most = 0;
+            for (int h = 0; h < p.n_groups; ++h) {
+                const unsigned long long s = h == gid ? 0ull : ld_acquire(&pl->span[h].v);
+                if (!s) continue;
+                const unsigned long long t = *(volatile unsigned long long*)&pl->own[h].t_row;
+                const unsigned long long ns = max((unsigned long long)ld_vol(&pl->own[h].row_ns), t && now > t ? now - t : 0ull);
+                const unsigned long long left = (s >> 32) - (uint32_t)s + 1ull, score = left * (ns + 1ull);
+                if (score > most) {
+                    most = score;
+                    to = h;
+                }
+            }
+            if (to < 0) return kRowsWait;  // the last run ended meanwhile
+            *(volatile int*)&own.join = to;
+            return kRowsJoin;
+        }
         __nanosleep(10000);
         return kRowsWait;
     }
@@ -1362,60 +1407,90 @@ static constexpr unsigned kLogChunk = 8;
 #ifndef DC_TRANS2_MIN_BLOCKS
 #define DC_TRANS2_MIN_BLOCKS 3
 #endif
+struct RowWarp {
+    unsigned long long entries, log_at;
+    unsigned evals, drops, log, log_left;
+};
+// kGroups: several groups of blocks (RowPlan); else one run, no plan.
+template <bool kGroups>
 __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans2Params p) {
     const unsigned lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
     int gid = 0;
-    while (gid + 1 < p.n_groups && blockIdx.x >= p.first_block[gid + 1]) ++gid;
-    const unsigned block = blockIdx.x - p.first_block[gid];
-    const RowsNext next{p, gid, p.first_block[gid + 1] - p.first_block[gid]};
-    const unsigned gwarp = block * kWarpsPerBlock + wib;
-    const unsigned nwarps = next.blocks * kWarpsPerBlock;
-    const RowGroup& G = p.g[gid];
-    EngineCtl* c = G.ctl;
+    while (kGroups && gid + 1 < p.n_groups && blockIdx.x >= p.first_block[gid + 1]) ++gid;
+    unsigned block = blockIdx.x - p.first_block[gid];  // number within the group
+    EngineCtl* c = p.g[gid].ctl;
     __shared__ int s_ho[kWarpsPerBlock][kWin];
     __shared__ int s_hi[kWarpsPerBlock][kWin];
     __shared__ StepBlock s_step;
-    const bool tracing = c->trace != nullptr;
+    __shared__ unsigned s_member;
+    bool tracing = c->trace != nullptr;
     // failure-detection tests: this block never reports, the others' waits run out
     if (c->test_skip_block && (int)blockIdx.x == c->test_skip_block - 1) return;
-    unsigned my_evals = 0, my_drops = 0, my_log = 0;
-    unsigned long long my_entries = 0;
+    // lane 0's counts of its warp and the records left in its log chunk: in
+    // shared memory, the loop has no registers to spare
+    __shared__ RowWarp s_warp[kWarpsPerBlock];
+    RowWarp& my = s_warp[wib];
+    if (lane == 0) my = RowWarp{0ull, 0ull, 0u, 0u, 0u, 0u};
     unsigned ticket = kNoTicket;
-    unsigned* const log_count = p.n_groups > 1 ? &p.plan->log_count : &c->log_count;
-    unsigned long long log_at = 0;  // lane 0: the records of the warp's chunk
-    unsigned log_left = 0;
+    unsigned* const log_count = kGroups ? &p.plan->log_count : &c->log_count;
     step_block_init(&s_step, c);
     unsigned long long word = step_block_word(&s_step);
-    int jprev = p.K0;      // row currently held in cur
-    bool seed_out = true;  // first row of a run: members are seeded by their out-counts too
-    uint32_t ids = p.n;    // vertices with state
+    int jprev = p.K0;    // row before this step's (the row itself: the first of its run)
+    uint32_t ids = p.n;  // vertices with state
     for (;;) {
         const int j = step_level(word);
         if (word == kStopWord || j == kRowsEnd) break;
+        if (kGroups && j == kRowsJoin) {
+            // the whole block goes over: a new number, the other group's word
+            // (which every warp reads before one of them can replace it)
+            gid = ld_vol(&p.plan->own[gid].join);
+            c = p.g[gid].ctl;
+            tracing = c->trace != nullptr;
+            __syncthreads();
+            if (threadIdx.x == 0) s_member = atomicAdd(&p.plan->own[gid].members, 1u);
+            step_block_init(&s_step, c);
+            word = step_block_word(&s_step);
+            block = s_member;
+            __syncthreads();
+            ticket = kNoTicket;
+            continue;
+        }
+        const RowGroup& G = p.g[gid];
+        const RowPlan::Own* own = kGroups ? &p.plan->own[gid] : nullptr;
+        unsigned blocks = gridDim.x;
+        bool seeds = true;  // the block has a share of this step's seeding
+        if (kGroups) {
+            const unsigned long long sb = *(const volatile unsigned long long*)&own->step_blocks;
+            blocks = (unsigned)sb;
+            // (another step's number: this one is over)
+            seeds = (unsigned)(sb >> 32) == step_number(word) && block < blocks;
+            ids = __ldg(p.ck + ld_vol(&own->lo));
+            jprev = ld_vol(&own->prev);
+        }
+        const bool seed_out = jprev == j;  // first row of a run: members are seeded by their out-counts too
+        const RowsNext next{p, gid, blocks};
+        const unsigned gwarp = block * kWarpsPerBlock + wib;
+        const unsigned nwarps = blocks * kWarpsPerBlock;
         const unsigned long long tag = step_tag(word);
         if (tracing && threadIdx.x == 0) trace_wake(c, word);
         uint32_t keep = kNoKeep;
         int pending = 0;
-        if (j < 0) {
+        if (kGroups && j < 0) {
             // between runs: the finished run's last row to the seam, then the
             // next run's start values and counters (every value is read from
             // row 0, a thread clears what it has copied itself)
-            const RowPlan::Own& own = p.plan->own[gid];
-            const unsigned fn = ld_vol(&own.flush_n), fo = ld_vol(&own.flush_off);
-            for (uint32_t i = block * kThreads + threadIdx.x; i < fn; i += next.blocks * kThreads)
+            const unsigned fn = seeds ? ld_vol(&own->flush_n) : 0u, fo = ld_vol(&own->flush_off);
+            for (uint32_t i = block * kThreads + threadIdx.x; i < fn; i += blocks * kThreads)
                 p.seam[fo + i] = ld_vol(&G.cur[i]);
-            if (j == kRowsInit) {
-                jprev = ld_vol(&own.lo);
-                seed_out = true;
-                ids = __ldg(p.ck + jprev);
-                const int from = ld_vol(&own.from);
+            if (j == kRowsInit && seeds) {
+                const int from = ld_vol(&own->from);
                 const int32_t* src = from < 0 ? p.row0 : p.g[from].cur;
-                for (uint32_t i = block * kThreads + threadIdx.x; i < ids; i += next.blocks * kThreads) {
+                for (uint32_t i = block * kThreads + threadIdx.x; i < ids; i += blocks * kThreads) {
                     G.cur[i] = ld_vol(&src[i]);
                     G.mark[i] = 0;
                     G.stamp[i] = -1;
                 }
-            } else if (j == kRowsCount) {
+            } else if (j == kRowsCount && seeds) {
                 for (uint32_t v = gwarp; v < ids; v += nwarps) {
                     int go[1] = {0}, gi[1] = {0};
                     const int cv = ld_vol(&G.cur[v]);
@@ -1431,14 +1506,14 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 }
             }
             __threadfence();
-            step_seeded(c, &s_step, kNoBound, false, word, tracing, next);
+            if (seeds) step_seeded(c, &s_step, kNoBound, false, word, tracing, next);
             unsigned long long none;
             if (step_take(c, G.q, &s_step, &ticket, &none, &pending, &word, next) == kTakeStop) break;
             continue;
         }
         // rows jprev+1 .. j-1 equal row jprev; vertices with kmax in
         // [jprev, j-1] leave now (all but those with kmax == j-1 have value 0)
-        const uint32_t vj = __ldg(p.ck + j), vprev = __ldg(p.ck + jprev);
+        const uint32_t vj = seeds ? __ldg(p.ck + j) : 0u, vprev = seeds ? __ldg(p.ck + jprev) : 0u;
         // ---- vertices leaving C_j: value -1; neighbours they supported lose one count
         int bound = kNoBound;  // on the next row that can need work
         // spread over all warps; a warp's share (up to 32 at a time) is cleared
@@ -1488,7 +1563,7 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 step_push(c, G.q, req != 0u, (unsigned long long)v | tag);
             }
         }
-        step_seeded(c, &s_step, bound, false, word, tracing, next);
+        if (seeds) step_seeded(c, &s_step, bound, false, word, tracing, next);
 
         // ---- drain: the warp's kept item first, else the queue; finished
         // items are counted off in batches (before the warp waits)
@@ -1550,21 +1625,20 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                     }
                 }
             }
-            ++my_evals;
             if (nv < cap) {
-                ++my_drops;
                 if (lane == 0) {
+                    ++my.drops;
                     // the value and its corner record
                     unsigned long long li = logidx;
                     const bool fresh = stamp != j;
                     if (fresh) {
-                        if (!log_left) {
-                            log_at = atomicAdd(log_count, kLogChunk);
-                            log_left = kLogChunk;
+                        if (!my.log_left) {
+                            my.log_at = atomicAdd(log_count, kLogChunk);
+                            my.log_left = kLogChunk;
                         }
-                        li = log_at++;
-                        --log_left;
-                        ++my_log;
+                        li = my.log_at++;
+                        --my.log_left;
+                        ++my.log;
                     }
                     if (li < p.log_cap) {
                         if (fresh) {
@@ -1590,7 +1664,10 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 c_o = __reduce_add_sync(0xFFFFFFFFu, c_o);
                 c_i = __reduce_add_sync(0xFFFFFFFFu, c_i);
             }
-            my_entries += (unsigned)entries;
+            if (lane == 0) {
+                ++my.evals;
+                my.entries += (unsigned)entries;
+            }
             if (tracing && lane == 0 && step_number(word) - 1 < c->trace_cap)
                 atomicMax(&c->trace[8 * (step_number(word) - 1) + 7], (unsigned long long)entries);
             unsigned again = 0;
@@ -1615,17 +1692,16 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
             ++pending;
         }
         if (state == kTakeStop) break;
-        jprev = j;
-        seed_out = false;
+        if (!kGroups) jprev = j;
     }
     if (lane == 0) {
         // unused records of the last chunk are void
-        for (; log_left; --log_left, ++log_at)
-            if (log_at < p.log_cap) p.log_k[log_at] = -1;
-        atomicAdd(&c->log_used, my_log);
-        atomicAdd(&c->evals, (unsigned long long)my_evals);
-        atomicAdd(&c->drops, (unsigned long long)my_drops);
-        atomicAdd(&c->edges_scanned, my_entries);
+        for (; my.log_left; --my.log_left, ++my.log_at)
+            if (my.log_at < p.log_cap) p.log_k[my.log_at] = -1;
+        atomicAdd(&c->log_used, my.log);
+        atomicAdd(&c->evals, (unsigned long long)my.evals);
+        atomicAdd(&c->drops, (unsigned long long)my.drops);
+        atomicAdd(&c->edges_scanned, my.entries);
     }
 }
 
@@ -2966,7 +3042,9 @@ __global__ void k_rows_start(RowsStart r, RowPlan* plan, uint32_t* seam_of, uint
     if (threadIdx.x < (unsigned)r.n_groups) {
         const int g = threadIdx.x;
         plan->span[g].v = r.span[g];
-        plan->own[g].lo = (int)(uint32_t)r.span[g];
+        plan->own[g].lo = plan->own[g].prev = (int)(uint32_t)r.span[g];
+        plan->own[g].members = r.blocks[g];
+        plan->own[g].step_blocks = (1ull << 32) | r.blocks[g];
         plan->own[g].from = -1;
         plan->own[g].ready = g == 0;
         if (r.seam_row[g]) seam_of[r.seam_row[g]] = r.seam_at[g] + 1u;
@@ -3189,8 +3267,9 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
         }
     }
     // blocks: what fits at the same time
+    const void* rows_fn = ngroups > 1 ? (const void*)k_trans2<true> : (const void*)k_trans2<false>;
     int grid = 0;
-    if (int rc = persistent_grid(h, (const void*)k_trans2, ngroups > 1 ? 8 : h->rows_bps, &grid)) return rc;
+    if (int rc = persistent_grid(h, rows_fn, ngroups > 1 ? 8 : h->rows_bps, &grid)) return rc;
     if (ngroups > 1 && h->rows_bps > 0) grid = std::min(grid, h->rows_bps * ngroups * h->geom.sms);
     const uint64_t spare = (uint64_t)kLogChunk * kWarpsPerBlock * grid;  // records left over in the warps' chunks
     // seams: the values of row a - 1 in C_a for every run that starts at a,
@@ -3320,7 +3399,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     if (Kstop >= k0) {
         void* args[] = {&tp};
         const FirstStep first{k0, (int)(tp.first_block[1] - tp.first_block[0])};
-        if (int rc = persistent_launch(h, (const void*)k_trans2, args, "transitions", h->ctl, h->stream, 0, &first, grid))
+        if (int rc = persistent_launch(h, rows_fn, args, "transitions", h->ctl, h->stream, 0, &first, grid))
             return rc;
         if (ngroups > 1) {
             ++g_launches;
