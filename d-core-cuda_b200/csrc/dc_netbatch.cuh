@@ -29,7 +29,8 @@ void device_batch_free(dc_graph* h, DeviceBatch* d);
 
 // Stable sort of (key, val) by the low `bits` bits of key on stream st
 // (dc_partition.cu); the sorted arrays end up in *key, *val (the pairs of
-// pointers are exchanged as needed); cnt holds radix_count_words(n) words.
+// pointers are exchanged as needed); cnt holds radix_count_words(m) words of
+// some m >= n.
 void radix_sort_pairs(cudaStream_t st, uint64_t n, int bits, uint32_t** key, uint32_t** val, uint32_t** key2,
                       uint32_t** val2, uint32_t* cnt);
 uint64_t radix_count_words(uint64_t n);

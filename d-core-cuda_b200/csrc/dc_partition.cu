@@ -87,12 +87,13 @@ __global__ void k_pt_roots(uint64_t B, uint32_t V, const uint32_t* from, const u
 }
 
 // digit counts of one tile per block: cnt[d * nblk + blk]
+template <int kItems>
 __global__ void k_pt_digit_count(uint64_t n, const uint32_t* key, int shift, uint32_t* cnt) {
     __shared__ uint32_t s_c[kDigits];
     if (threadIdx.x < kDigits) s_c[threadIdx.x] = 0;
     __syncthreads();
-    const uint64_t t0 = (uint64_t)blockIdx.x * kPTile;
-    for (int r = 0; r < kPItems; ++r) {
+    const uint64_t t0 = (uint64_t)blockIdx.x * kPT * kItems;
+    for (int r = 0; r < kItems; ++r) {
         const uint64_t i = t0 + (uint64_t)r * kPT + threadIdx.x;
         if (i < n) atomicAdd(&s_c[(key[i] >> shift) & (kDigits - 1)], 1u);
     }
@@ -118,14 +119,15 @@ __global__ void k_pt_scan_one_block(uint32_t* a, uint64_t n) {
 // index order, 256 at a time; equal digits are ranked inside each warp
 // (match) and across the block's warps (shared counts), on top of the
 // tile's base for the digit
+template <int kItems>
 __global__ void k_pt_digit_scatter(uint64_t n, const uint32_t* key_in, const uint32_t* val_in, uint32_t* key_out,
                                    uint32_t* val_out, int shift, const uint32_t* off) {
     __shared__ uint32_t s_base[kDigits];
     __shared__ uint32_t s_wc[kPT / 32][kDigits];
     const unsigned lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
     if (threadIdx.x < kDigits) s_base[threadIdx.x] = off[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x];
-    const uint64_t t0 = (uint64_t)blockIdx.x * kPTile;
-    for (int r = 0; r < kPItems; ++r) {
+    const uint64_t t0 = (uint64_t)blockIdx.x * kPT * kItems;
+    for (int r = 0; r < kItems; ++r) {
         for (int j = threadIdx.x; j < (kPT / 32) * kDigits; j += kPT) (&s_wc[0][0])[j] = 0;
         __syncthreads();
         const uint64_t i = t0 + (uint64_t)r * kPT + threadIdx.x;
@@ -221,16 +223,34 @@ int pt_alloc(cudaStream_t st, T** p, uint64_t n) {
 
 }  // namespace
 
-uint64_t radix_count_words(uint64_t n) { return (uint64_t)kDigits * ((n + kPTile - 1) / kPTile) + 1; }
+// Tiles of the sort: a block visits its tile 256 elements at a time, so up to
+// a million elements small tiles are faster (10,000: 39 us per digit with
+// tiles of 4,096, three blocks, 17 with tiles of 1,024); beyond that the one
+// block that scans the tiles' counts would be what bounds it.
+constexpr uint64_t kRadixSmall = 1u << 20;
+constexpr int kRadixSmallItems = 4;
+
+// enough for any sort of at most n elements
+uint64_t radix_count_words(uint64_t n) {
+    auto tiles = [](uint64_t m, int items) { return (m + kPT * items - 1) / (kPT * items); };
+    return (uint64_t)kDigits * std::max(tiles(n, kPItems), tiles(std::min(n, kRadixSmall), kRadixSmallItems)) + 1;
+}
+
+template <int kItems>
+static void radix_pass(cudaStream_t st, uint64_t n, int shift, const uint32_t* key, const uint32_t* val, uint32_t* key2,
+                       uint32_t* val2, uint32_t* cnt) {
+    const unsigned nblk = (unsigned)((n + kPT * kItems - 1) / (kPT * kItems));
+    g_launches += 3;
+    k_pt_digit_count<kItems><<<nblk, kPT, 0, st>>>(n, key, shift, cnt);
+    k_pt_scan_one_block<<<1, kPT, 0, st>>>(cnt, (uint64_t)kDigits * nblk);
+    k_pt_digit_scatter<kItems><<<nblk, kPT, 0, st>>>(n, key, val, key2, val2, shift, cnt);
+}
 
 void radix_sort_pairs(cudaStream_t st, uint64_t n, int bits, uint32_t** key, uint32_t** val, uint32_t** key2,
                       uint32_t** val2, uint32_t* cnt) {
-    const unsigned nblk = (unsigned)((n + kPTile - 1) / kPTile);
     for (int shift = 0; shift < bits; shift += kDigitBits) {
-        g_launches += 3;
-        k_pt_digit_count<<<nblk, kPT, 0, st>>>(n, *key, shift, cnt);
-        k_pt_scan_one_block<<<1, kPT, 0, st>>>(cnt, (uint64_t)kDigits * nblk);
-        k_pt_digit_scatter<<<nblk, kPT, 0, st>>>(n, *key, *val, *key2, *val2, shift, cnt);
+        if (n <= kRadixSmall) radix_pass<kRadixSmallItems>(st, n, shift, *key, *val, *key2, *val2, cnt);
+        else radix_pass<kPItems>(st, n, shift, *key, *val, *key2, *val2, cnt);
         std::swap(*key, *key2);
         std::swap(*val, *val2);
     }
@@ -257,7 +277,7 @@ int kmax_edge_batches_device(dc_graph* h, uint64_t B, const uint32_t* d_from, co
             if (p) cudaFreeAsync(p, st);
     };
     if ((rc = pt_alloc(st, &key0, B)) || (rc = pt_alloc(st, &val0, B)) || (rc = pt_alloc(st, &key1, B)) ||
-        (rc = pt_alloc(st, &val1, B)) || (rc = pt_alloc(st, &cnt, kDigits * nblk + 1)) ||
+        (rc = pt_alloc(st, &val1, B)) || (rc = pt_alloc(st, &cnt, radix_count_words(B))) ||
         (rc = pt_alloc(st, &f, B)) || (rc = pt_alloc(st, &part, nblk + 1)) || (rc = pt_alloc(st, &run, B)) ||
         (rc = pt_alloc(st, &start, B)) || (rc = pt_alloc(st, &occ, B)) ||
         (rc = pt_alloc(st, &passes, (uint64_t)K + 2)) || (rc = pt_alloc(st, &rk, B)) || (rc = pt_alloc(st, &bad, 1))) {

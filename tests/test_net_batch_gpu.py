@@ -77,3 +77,32 @@ def test_refused_batches(dc, gpu, b):
         g.maintain(np.r_[u[:half], u[:half]], np.r_[v[:half], v[:half]],
                    np.r_[np.zeros(half, np.uint8), np.ones(half, np.uint8)], 2)
         assert np.array_equal(np.stack(g.edges()), before) and np.array_equal(g.kmaxes(), km)
+
+
+@pytest.mark.parametrize("b", [1 << 20, (1 << 20) + 1, (1 << 20) + 4097])
+def test_large_batches(dc, gpu, b):
+    """Around a million updates, where the sort's tiles change; few of them
+    are left after the others cancel."""
+    rng = np.random.default_rng(b)
+    V, E = 5000, 30000
+    s, d = rng.integers(0, V, E).astype(np.uint32), rng.integers(0, V, E).astype(np.uint32)
+    gone = rng.permutation(E)[:300]
+    n_ins = 200 + (b - 500) % 2
+    n = (b - 300 - n_ins) // 2
+    t, ins = rng.integers(0, V, (n, 2)), rng.integers(0, V, (n_ins, 2))
+    pairs = np.concatenate([t, np.stack([s[gone], d[gone]], 1), ins, t]).astype(np.uint32)
+    flag = np.concatenate([np.zeros(n), np.ones(300), np.zeros(n_ins), np.ones(n)]).astype(np.uint8)
+    o = rng.permutation(len(pairs))
+    assert len(pairs) == b
+    with dc.Graph.from_edges(V, s, d) as g:
+        g.decompose()
+        st = g.maintain(pairs[o, 0], pairs[o, 1], flag[o], 2)
+        both = Counter(map(tuple, pairs[n:n + 300].tolist())) & Counter(map(tuple, ins.tolist()))
+        assert st["deleted"] == 300 - sum(both.values()) and st["inserted"] == n_ins - sum(both.values())
+        keep = np.ones(E, bool)
+        keep[gone] = False
+        es = np.concatenate([s[keep], ins[:, 0].astype(np.uint32)])
+        ed = np.concatenate([d[keep], ins[:, 1].astype(np.uint32)])
+        gs, gd = g.edges()
+        x, y = np.lexsort((gd, gs)), np.lexsort((ed, es))
+        assert np.array_equal(gs[x], es[y]) and np.array_equal(gd[x], ed[y])
