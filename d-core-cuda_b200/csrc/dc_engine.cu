@@ -2665,8 +2665,8 @@ int ensure_tring(dc_graph* h, uint64_t need) {
     return DC_OK;
 }
 
-// Two 256-thread blocks per SM: measured best or near it from R-MAT 19 to 22
-// once the queue counters sit on separate lines (the autotuner refines it).
+// Two 256-thread blocks per SM where nothing better is known (the autotuner
+// refines it).
 static constexpr int kDefaultBlocksPerSm = 2;
 
 static int persistent_grid(dc_graph* h, const void* fn, int bps, int* blocks) {
@@ -2853,8 +2853,16 @@ int run_peel2(dc_graph* h, int ninst, const PeelInst* inst, int32_t* maxv) {
     void* args[] = {&p};
     EngineCtl hc;
     const void* fn = inst[0].member ? (const void*)k_peel2<true> : (const void*)k_peel2<false>;
+    // Blocks on a handle that was not told: every block adds about 9 ns to a
+    // light level, and large levels want more warps.  1 / 2 / 3 blocks per SM:
+    // R-MAT 13 0.95 / 1.01 / 1.08 ms, R-MAT 15 1.11 / 1.19 / 1.29, ER of 10,000
+    // 0.20 / 0.21 / 0.23, of 60,000 (60 edges per vertex) 0.45 / 0.43 / 0.45,
+    // of 100,000 0.30 / 0.27 / 0.28, R-MAT 20 4.03 / 3.83 / 4.00, R-MAT 21 6.0 /
+    // 5.4 / 5.5, R-MAT 22 9.4 / 7.84 / 7.78, ER of 3 M 2.95 / 1.74 / 1.35.
+    int bps = h->peel_bps;
+    if (bps <= 0 && h->blocks_per_sm <= 0 && !inst[0].member) bps = g.V <= 50000u ? 1 : g.V >= 3000000u ? 3 : 2;
     const FirstStep first{0, 0};
-    if (int rc = run_persistent(h, fn, args, "peel", &hc, h->peel_bps, &first)) return rc;
+    if (int rc = run_persistent(h, fn, args, "peel", &hc, bps, &first)) return rc;
     for (int i = 0; i < ninst; ++i) maxv[i] = hc.maxv[i];
     return DC_OK;
 }
