@@ -1,8 +1,7 @@
 // Device-side building blocks shared by the persistent engine kernels:
 //   - EngineCtl: counters, error word and grid-barrier state in device memory
 //   - grid_sync: software grid barrier with a bounded wait (cooperative launch)
-//   - work queue: ring of vertex ids with claim / done counters and a
-//     termination test, so cascades run without per-round barriers
+//   - ticket queue, and steps on it that follow one another without a barrier
 //   - warp-aggregated append
 // Every spin in here is bounded by the control block's wait limit
 // (EngineCtl::wait_ns, kWaitNs when 0) of %globaltimer time; on expiry the
@@ -15,7 +14,6 @@
 namespace dc {
 
 constexpr unsigned DC_DEV_ERR_TIMEOUT = 1u;   // a bounded wait ran out
-constexpr unsigned DC_DEV_ERR_QUEUE = 2u;     // queue capacity exceeded
 constexpr unsigned DC_DEV_ERR_BADID = 4u;     // vertex id out of range
 constexpr unsigned DC_DEV_ERR_CAPACITY = 8u;  // a log or list buffer overflowed
 constexpr unsigned DC_DEV_ERR_NOTFOUND = 16u; // delete of an absent edge
@@ -49,19 +47,8 @@ struct EngineCtl {
     unsigned worked;               // last step of which an item was kept by the warp that found it
     unsigned log_used;             // corner records written (the log's ranges have holes)
     unsigned phase_done;    // set by whoever brings outstanding to 0
-    // work queue (monotone within one phase)
-    alignas(128) unsigned q_head;
-    unsigned q_tail;
-    unsigned q_done;
-    unsigned pad0;
-    // per-step counters, rotated over three slots
-    unsigned producers[3];
-    unsigned rcount[3];
     // results / statistics
-    int maxval;
-    int steps;
     alignas(128) unsigned log_count;
-    unsigned pad1;
     unsigned long long evals;
     unsigned long long drops;
     unsigned long long pushes;
@@ -81,8 +68,7 @@ struct EngineCtl {
     PadU rc_next[2];        // next level's remaining-list sizes (appended by every warp)
     int maxv[2];            // largest value per peel instance
     int step;               // level / transition index
-    unsigned nworkers;      // producers per phase (warps in the grid)
-    int level;              // current level / row of the persistent loop
+    int level;              // row repair: last row taken
     // optional per-step timing trace: 8 words per step
     //   [0] %globaltimer at step start, [1] when its work ran out,
     //   [2] queue items of the step, [3] %globaltimer at the closing barrier,
@@ -234,86 +220,6 @@ __device__ __forceinline__ unsigned warp_append(unsigned* counter, bool pred, un
     return base + __popc(mask & ((1u << lane) - 1u));
 }
 
-// Ring of vertex ids.  Producers reserve slots with q_tail and store the id;
-// a consumer claims [h, h+n) by CAS on q_head, waits for each slot to be
-// filled, resets it to kEmptySlot and, after its work (including its own
-// pushes) is visible, adds n to q_done.  The phase is over when every
-// producer has finished its seeding share and q_done == q_tail.
-struct RingQueue {
-    uint32_t* slots;
-    unsigned mask;
-};
-
-// Converged-warp push of v for lanes with pred.
-__device__ __forceinline__ void q_push_warp(EngineCtl* c, RingQueue q, bool pred, uint32_t v) {
-    unsigned pos = warp_append(&c->q_tail, pred);
-    if (pred) {
-        atomicExch(&q.slots[pos & q.mask], v);
-    }
-}
-
-// Single-thread push (divergent contexts).
-__device__ __forceinline__ void q_push_one(EngineCtl* c, RingQueue q, uint32_t v) {
-    unsigned pos = atomicAdd(&c->q_tail, 1u);
-    atomicExch(&q.slots[pos & q.mask], v);
-}
-
-// Lane 0 of a converged warp tries to claim up to maxn items.  Returns the
-// claimed count (broadcast) and the first index in *first.  0 with
-// *finished = true means the phase is complete; 0 with *finished = false
-// means nothing to claim right now.
-__device__ __forceinline__ unsigned q_claim_warp(EngineCtl* c, unsigned maxn, unsigned total_producers,
-                                                 unsigned* producers, unsigned* first, bool* finished) {
-    const unsigned lane = threadIdx.x & 31u;
-    unsigned n = 0, h = 0, fin = 0;
-    if (lane == 0) {
-        h = ld_vol(&c->q_head);
-        unsigned t = ld_vol(&c->q_tail);
-        if (h < t) {
-            unsigned want = min(maxn, t - h);
-            if (atomicCAS(&c->q_head, h, h + want) == h) n = want;
-        } else {
-            unsigned p = ld_vol(producers);
-            __threadfence();
-            unsigned d = ld_vol(&c->q_done);
-            __threadfence();
-            unsigned t2 = ld_vol(&c->q_tail);
-            if (p == total_producers && d == t2) fin = 1;
-        }
-    }
-    n = __shfl_sync(0xFFFFFFFFu, n, 0);
-    h = __shfl_sync(0xFFFFFFFFu, h, 0);
-    fin = __shfl_sync(0xFFFFFFFFu, fin, 0);
-    *first = h;
-    *finished = fin != 0;
-    return n;
-}
-
-// Reads a claimed slot, waiting (bounded) for its producer's store.
-__device__ __forceinline__ uint32_t q_take(EngineCtl* c, RingQueue q, unsigned idx) {
-    uint32_t* s = &q.slots[idx & q.mask];
-    uint32_t v = atomicExch(s, kEmptySlot);
-    if (v != kEmptySlot) return v;
-    const unsigned long long t0 = gtimer(), lim = wait_limit(c);
-    for (;;) {
-        v = atomicExch(s, kEmptySlot);
-        if (v != kEmptySlot) return v;
-        if (ld_vol(&c->error)) return kEmptySlot;
-        if (gtimer() - t0 > lim) {
-            set_dev_error(c, DC_DEV_ERR_TIMEOUT, 2);
-            return kEmptySlot;
-        }
-        __nanosleep(16);
-    }
-}
-
-// Marks n claimed items as done after the calling warp's writes are visible.
-__device__ __forceinline__ void q_done_warp(EngineCtl* c, unsigned n) {
-    __threadfence();
-    __syncwarp();
-    if ((threadIdx.x & 31u) == 0 && n) atomicAdd(&c->q_done, n);
-}
-
 // ---------------------------------------------------------------------------
 // Ticket queue.  Items are 64-bit words in a ring of slots (kEmptyItem =
 // free).  A consumer warp takes a ticket with one atomicAdd on t_head and
@@ -339,22 +245,6 @@ __device__ __forceinline__ void tq_finish(EngineCtl* c, int n) {
         atomicExch(&c->phase_done, 1u);
         if (c->trace && (unsigned)c->step < c->trace_cap) c->trace[8 * c->step + 1] = gtimer();
     }
-}
-
-// Called by the last block of a phase-ending barrier: closes the step's
-// trace record and opens the next one.
-__device__ __forceinline__ void trace_step_end(EngineCtl* c) {
-    unsigned long long now = gtimer();
-    if (c->trace && c->step >= 0 && (unsigned)c->step < c->trace_cap) {
-        c->trace[8 * c->step + 2] = c->t_tail - c->trace_tail0;
-        c->trace[8 * c->step + 3] = now;
-    }
-    c->step++;
-    if (c->trace && (unsigned)c->step < c->trace_cap) {
-        c->trace[8 * c->step] = now;
-        c->trace[8 * c->step + 6] = ~0ull;
-    }
-    c->trace_tail0 = c->t_tail;
 }
 
 // Converged warp: lanes with pred push `cnt` consecutive items item0,
@@ -397,33 +287,6 @@ __device__ __forceinline__ void tq_push_warp(EngineCtl* c, TicketQueue q, bool p
         __threadfence();
         volatile unsigned long long* s = &q.slots[(base + __popc(m & ((1u << lane) - 1u))) & q.mask];
         *s = item;
-    }
-}
-
-// Converged warp: each lane pushes its first cnt (<= 4) entries of items[].
-__device__ __forceinline__ void tq_push_warp4(EngineCtl* c, TicketQueue q, unsigned cnt, const uint32_t* items) {
-    const unsigned lane = threadIdx.x & 31u;
-    unsigned x = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        unsigned y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-        if (lane >= (unsigned)o) x += y;
-    }
-    unsigned total = __shfl_sync(0xFFFFFFFFu, x, 31);
-    if (total == 0) return;
-    unsigned base = 0;
-    if (lane == 0) {
-        atomicAdd(&c->outstanding, (int)total);
-        base = atomicAdd(&c->t_tail, total);
-    }
-    base = __shfl_sync(0xFFFFFFFFu, base, 0) + (x - cnt);
-    if (cnt) __threadfence();
-#pragma unroll
-    for (unsigned i = 0; i < 4; ++i) {
-        if (i < cnt) {
-            volatile unsigned long long* s = &q.slots[(base + i) & q.mask];
-            *s = (unsigned long long)items[i];
-        }
     }
 }
 
@@ -516,25 +379,6 @@ __device__ __forceinline__ bool tq_take_warp(EngineCtl* c, TicketQueue q, unsign
     __threadfence();
     *item = it;
     return state == 1;
-}
-
-// tq_take_warp with lazily counted finishes: *pending (lane 0's count of
-// items this warp finished but has not yet subtracted from `outstanding`) is
-// subtracted in one atomic when the warp's slot is not filled at once, i.e.
-// before the warp can wait; a warp that keeps finding items never touches
-// `outstanding` for them until then.  On a false return *pending is 0.
-__device__ __forceinline__ bool tq_take_warp_lazy(EngineCtl* c, TicketQueue q, unsigned* ticket,
-                                                  unsigned long long* item, unsigned* pending) {
-    const unsigned lane = threadIdx.x & 31u;
-    if (lane == 0) {
-        if (*ticket == kNoTicket) *ticket = atomicAdd(&c->t_head, 1u);
-        volatile unsigned long long* s = &q.slots[*ticket & q.mask];
-        if (*s == kEmptyItem && *pending) {
-            tq_finish(c, (int)*pending);
-            *pending = 0;
-        }
-    }
-    return tq_take_warp(c, q, ticket, item);
 }
 
 // ---------------------------------------------------------------------------
@@ -787,30 +631,5 @@ __device__ __forceinline__ int step_take(EngineCtl* c, TicketQueue q, StepBlock*
     *word = w;
     return state;
 }
-
-// Idle-wait helper for the drain loops: returns false once the phase has made
-// no progress for the wait limit (error recorded).
-struct IdleClock {
-    unsigned long long t0;
-    unsigned last_done;
-    __device__ __forceinline__ void start(EngineCtl* c) {
-        t0 = gtimer();
-        last_done = ld_vol(&c->q_done);
-    }
-    __device__ __forceinline__ bool tick(EngineCtl* c) {
-        unsigned d = ld_vol(&c->q_done);
-        if (d != last_done) {
-            last_done = d;
-            t0 = gtimer();
-            return true;
-        }
-        if (gtimer() - t0 > wait_limit(c)) {
-            set_dev_error(c, DC_DEV_ERR_TIMEOUT, 3);
-            return false;
-        }
-        __nanosleep(64);
-        return true;
-    }
-};
 
 }  // namespace dc

@@ -8,10 +8,10 @@
 //   decomposition     dcore, main.cu:197-262 (kmax via swapInOut, then one
 //                     pass per k = 0..kmax)
 // The engine computes the same numbers with a different schedule: one
-// persistent cooperative kernel per pass (software grid barrier per level, a
-// device work queue for cascades, no host round trip per level), and rows
-// k >= 1 derived from row k-1 by h-index refinement instead of one fresh
-// peel per row (see k_transitions).
+// persistent cooperative kernel per pass (levels and rows follow one another
+// without a barrier, a device work queue for cascades, no host round trip per
+// level), and rows k >= 1 derived from row k-1 by h-index refinement instead
+// of one fresh peel per row (see k_trans2).
 #include <atomic>
 #include <algorithm>
 #include <cstdio>
@@ -2261,15 +2261,6 @@ __global__ void k_rows_corner_fill(uint32_t V, const int32_t* kmax, const int32_
     }
 }
 
-__global__ void k_max_reduce(uint64_t n, const int32_t* a, int* out) {
-    int m = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        m = max(m, a[i]);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-    if ((threadIdx.x & 31u) == 0) atomicMax(out, m);
-}
-
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -2566,11 +2557,6 @@ int build_from_device_edges(dc_graph* h, uint32_t V, uint64_t E, const uint32_t*
     g.V = V;
     g.E = E;
     return DC_OK;
-}
-
-__global__ void k_host_csr_len(uint32_t V, const int32_t* deg, int32_t* len) {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < V; v += (uint64_t)gridDim.x * blockDim.x)
-        len[v] = deg[v];
 }
 
 // Expands a CSR with arbitrary per-list slots into an edge list on device.

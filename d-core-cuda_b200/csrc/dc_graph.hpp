@@ -111,12 +111,12 @@ struct dc_graph {
     uint32_t gap_div = 0;      // extra slack = len / gap_div (0 = none)
     int method = 0;            // 0 = incremental rows, 1 = per-row peel
     int blocks_per_sm = 0;     // persistent-kernel blocks per SM (0 = default)
-    int peel_bps = 0;          // the fused peel's blocks per SM (0 = blocks_per_sm)
+    int peel_bps = 0;          // the fused peel's blocks per SM (0 = blocks_per_sm, or by vertices)
     int rows_bps = 0;          // the row kernel's blocks per SM (0 = blocks_per_sm)
     unsigned peel_chunk = 64;  // adjacency entries per peel work item
     int row_repair = 1;        // deletions: repair rows locally instead of recomputing
     // full decompositions: rows cut after kmax * rows_split[i] / 1000 for
-    // each nonzero entry (ascending), segments run concurrently
+    // each nonzero entry (ascending), groups of blocks work on the segments
     int rows_split[dc::kMaxRowSegments - 1] = {};
     bool auto_cuts = true;  // launch shapes never set: cuts by the rule in rows_from_row0
     uint64_t log_used = 0;  // records in the last run's corner log (its other entries are void)

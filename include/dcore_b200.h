@@ -440,13 +440,13 @@ typedef struct dc_tuning {
     int32_t peel_chunk;         /* power of two, 16..4096: a list of more than four
                                    chunks is split into items of four */
     /* Row segments of a full decomposition: each nonzero s cuts rows 1..kmax
-     * after row kmax*s/1000, and the segments run as concurrent launches
-     * (each one after the first starts from row 0 inside its first row's
-     * core).  Nonzero entries are strictly ascending in 1..999 and precede
-     * the zeros; all zero = one launch.  (On a handle whose shapes were never
-     * set the engine cuts into up to eight equal runs where the cores shrink
-     * fast enough for that to pay.)  Segments share the SMs: each gets
-     * at most 1/n of the row kernel's resident blocks. */
+     * after row kmax*s/1000, and groups of blocks of one launch work on the
+     * segments at the same time (each one after the first starts from row 0
+     * inside its first row's core; a group that is done takes over rows of
+     * another one or joins it).  Nonzero entries are strictly ascending in
+     * 1..999 and precede the zeros; all zero = one segment.  (On a handle
+     * whose shapes were never set the engine chooses cuts itself where the
+     * cores shrink fast enough for that to pay.) */
     int32_t rows_split_permille[7];
 } dc_tuning;
 int dc_get_tuning(dc_graph* g, dc_tuning* t);
