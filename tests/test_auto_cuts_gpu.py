@@ -71,3 +71,17 @@ def test_cut_rule_by_edges(dc, gpu, skew, E):
         assert a.decompose() == b.decompose()
         assert np.array_equal(a.kmaxes(), b.kmaxes())
         assert all(np.array_equal(x, y) for x, y in zip(a.skyline(), b.skyline()))
+
+
+@pytest.mark.parametrize("E", [299999, 300000, 1499999, 1500000])
+def test_blocks_by_edges(dc, gpu, E):
+    """Both sides of the lines between 1, 2 and more blocks per SM for the rows."""
+    V, s, d = dc.gen_rmat(16, 32, 45)
+    keep = np.random.default_rng(46).permutation(len(s))[:E]
+    assert len(keep) == E
+    s, d = np.ascontiguousarray(s[keep]), np.ascontiguousarray(d[keep])
+    with dc.Graph.from_edges(V, s, d) as a, dc.Graph.from_edges(V, s, d) as b:
+        b.set_tuning(2, 2, 64, ())
+        assert a.decompose() == b.decompose()
+        assert np.array_equal(a.kmaxes(), b.kmaxes())
+        assert all(np.array_equal(x, y) for x, y in zip(a.skyline(), b.skyline()))
