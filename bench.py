@@ -1037,7 +1037,7 @@ def run_decomposition(args, w, rank, world, local, dist):
                 "unit": "GB/s", "frac": kernels[dom]["frac"], "peak_source": peak_kind,
                 "traffic": kernel_traffic(dom, args.workload),
                 "timing": "CUDA events on the graph's stream around each phase inside dc_decompose; the rows "
-                          "phase spans all k_trans2 launches (row segments on concurrent streams joined back)",
+                          "phase spans the k_trans2 launch and the collection of its groups' corner records",
                 "kernels": kernels,
                 "decomposition": {"alg_bytes": b_alg, "ms": ms_per_step,
                                   "achieved_gbs": b_alg / (ms_per_step / 1000.0) / 1e9,
