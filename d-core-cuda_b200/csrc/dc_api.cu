@@ -254,6 +254,7 @@ extern "C" int dc_set_trace(dc_graph* h, uint32_t max_steps, dc_trace_fn fn, voi
 
 extern "C" int dc_graph_free(dc_graph* h) {
     if (!h) return DC_OK;
+    if (h->side_stream) cudaStreamSynchronize(h->side_stream);
     if (h->stream) cudaStreamSynchronize(h->stream);
     dc_set_trace(h, 0, nullptr, nullptr);
     free_graph_arrays(h->g, h->stream);
@@ -264,6 +265,9 @@ extern "C" int dc_graph_free(dc_graph* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (auto& e : h->ev)
         if (e) cudaEventDestroy(e);
+    for (auto& e : h->side_ev)
+        if (e) cudaEventDestroy(e);
+    if (h->side_stream) cudaStreamDestroy(h->side_stream);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return DC_OK;

@@ -107,6 +107,8 @@ struct dc_graph {
     bool log_maint = false;                // record features and timings of each batch
     std::vector<dc::MaintLogRec> maint_log;
     cudaEvent_t ev[8] = {};
+    cudaStream_t side_stream = nullptr;  // the long lists' sort, beside the others (made when first used)
+    cudaEvent_t side_ev[2] = {};
     uint32_t gap_min = 1;      // minimum free slots per list
     uint32_t gap_div = 0;      // extra slack = len / gap_div (0 = none)
     int method = 0;            // 0 = incremental rows, 1 = per-row peel
