@@ -787,6 +787,132 @@ __global__ void __launch_bounds__(kThreads, DC_PEEL_MIN_BLOCKS) k_peel2(Peel2Par
     }
 }
 
+// The peels of a small graph, one block each: degrees and the removed vertices
+// in shared memory, a level's removals in rounds with a block barrier between
+// them (a vertex is listed once, when it is removed, so the list never exceeds
+// V entries).  The grid's version spends 8 to 10 us on an empty level and about
+// 1.2 us on every link of a chain of removals, here they take about 1 us and
+// 0.5; what bounds it is the entries one SM can take (shared-memory atomics,
+// about 2,000 per us), and the other SMs are free for other handles.
+struct SmallPeel {
+    PeelInst in[2];
+    uint32_t V;
+    EngineCtl* ctl;
+};
+constexpr int kSmallPeelThreads = 1024;
+constexpr uint32_t kSmallPeelV = 36000;           // 6 bytes of shared memory per vertex
+// Faster than the grid's kernel, small / grid in ms: R-MAT 12 0.20 / 0.65,
+// 13 (24 edges per vertex) 0.39 / 0.95, 14 (40) 0.73 / 1.36, 15 (32) 1.08 /
+// 1.56; ER 1,000 0.045 / 0.125, 10,000 (20) 0.14 / 0.20, 10,000 (60) 0.23 /
+// 0.26, but 20,000 (20) 0.22 / 0.21 and 30,000 (50) 0.49 / 0.31: where all
+// degrees are alike the removals are a few wide cascades, which want the
+// chip's atomics.  Hence by the longest list, as it was when the lists were
+// built (any choice gives the same result).
+static bool peel_fits_block(const DevGraph& g) {
+    const bool skewed = g.max_len >= 8 * (g.E / std::max<uint32_t>(g.V, 1) + 4);
+    return g.V >= 1 && (skewed ? g.V <= kSmallPeelV && g.E <= 2000000u : g.V <= 16384 && g.E <= 500000u);
+}
+// longest list of either side
+__global__ void k_max_len(uint32_t V, const int32_t* a, const int32_t* b, int* out) {
+    int m = 0;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) m = max(m, max(a[v], b[v]));
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    if ((threadIdx.x & 31u) == 0) atomicMax(out, m);
+}
+constexpr int kSmallPeelGone = 1 << 30;           // taken from the degree of a removed vertex
+constexpr unsigned kSmallPeelLong = 256, kSmallPeelLongs = 64;  // lists that the whole block reads
+__global__ void __launch_bounds__(kSmallPeelThreads, 1) k_peel_small(SmallPeel p) {
+    extern __shared__ int s_key[];
+    uint16_t* s_list = reinterpret_cast<uint16_t*>(s_key + p.V);
+    __shared__ unsigned s_tail, s_longs, s_long[kSmallPeelLongs];
+    __shared__ int s_min;
+    const PeelInst& I = p.in[blockIdx.x];
+    const unsigned t = threadIdx.x, lane = t & 31u, V = p.V;
+    for (unsigned v = t; v < V; v += kSmallPeelThreads) s_key[v] = __ldg(I.a_len + v);
+    if (t == 0) s_tail = s_longs = 0;
+    int level = 0;
+    unsigned head = 0;
+    // an entry of a removed vertex's list: one from the neighbour's degree
+    auto entry = [&](uint32_t u) {
+        if (atomicSub(&s_key[u], 1) == level + 1) {
+            atomicSub(&s_key[u], kSmallPeelGone);
+            I.val[u] = level;
+            s_list[atomicAdd(&s_tail, 1u)] = (uint16_t)u;
+        }
+    };
+    while (head < V) {
+        // the next level: the least degree left
+        __syncthreads();
+        if (t == 0) s_min = 0x7FFFFFFF;
+        __syncthreads();
+        int m = 0x7FFFFFFF;
+        for (unsigned v = t; v < V; v += kSmallPeelThreads) {
+            const int k = s_key[v];
+            if (k >= 0) m = min(m, k);
+        }
+        m = __reduce_min_sync(0xFFFFFFFFu, m);
+        if (lane == 0) atomicMin(&s_min, m);
+        __syncthreads();
+        level = s_min;
+        if (level == 0x7FFFFFFF) break;  // (no vertex left: head is V)
+        for (unsigned b = t - lane; b < V; b += kSmallPeelThreads) {
+            const unsigned v = b + lane;
+            const int k = v < V ? s_key[v] : -1;
+            const bool gone = k >= 0 && k <= level;
+            const unsigned mask = __ballot_sync(0xFFFFFFFFu, gone);
+            if (!mask) continue;
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(&s_tail, (unsigned)__popc(mask));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (gone) {
+                s_key[v] = k - kSmallPeelGone;
+                I.val[v] = level;
+                s_list[at + __popc(mask & ((1u << lane) - 1u))] = (uint16_t)v;
+            }
+        }
+        __syncthreads();
+        unsigned tail = s_tail;
+        __syncthreads();
+        while (head < tail) {
+            // eight lanes per vertex, four entries in flight each
+            for (unsigned i = head + (t >> 3); i < tail; i += kSmallPeelThreads / 8) {
+                const uint32_t v = s_list[i], off = __ldg(I.b_off + v);
+                const unsigned n = (unsigned)__ldg(I.b_len + v);
+                if (n > kSmallPeelLong) {
+                    unsigned at = kSmallPeelLongs;
+                    if ((t & 7u) == 0) at = atomicAdd(&s_longs, 1u);
+                    at = __shfl_sync(0xFFu << (lane & ~7u), at, lane & ~7u);
+                    if (at < kSmallPeelLongs) {
+                        if ((t & 7u) == 0) s_long[at] = v;
+                        continue;
+                    }
+                }
+                for (unsigned e = t & 7u; e < n; e += 32) {
+                    uint32_t u[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) u[q] = e + 8 * q < n ? __ldg(I.b_nbr + off + e + 8 * q) : 0xFFFFFFFFu;
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        if (u[q] != 0xFFFFFFFFu) entry(u[q]);
+                }
+            }
+            __syncthreads();
+            const unsigned longs = min(s_longs, kSmallPeelLongs);
+            for (unsigned i = 0; i < longs; ++i) {
+                const uint32_t v = s_long[i], off = __ldg(I.b_off + v);
+                const unsigned n = (unsigned)__ldg(I.b_len + v);
+                for (unsigned e = t; e < n; e += kSmallPeelThreads) entry(__ldg(I.b_nbr + off + e));
+            }
+            __syncthreads();
+            head = tail;
+            tail = s_tail;
+            if (t == 0) s_longs = 0;
+            __syncthreads();
+        }
+    }
+    if (t == 0) p.ctl->maxv[blockIdx.x] = level;
+}
+
 // ---------------------------------------------------------------------------
 // incremental rows with exact support counters
 // ---------------------------------------------------------------------------
@@ -2534,8 +2660,13 @@ int build_from_device_edges(dc_graph* h, uint32_t V, uint64_t E, const uint32_t*
     ListStarts ls{{g.out_len, g.in_len}, {nullptr, nullptr}, h->gap_min, h->gap_div};
     static_assert(offsetof(EngineCtl, drops) == offsetof(EngineCtl, evals) + 8, "two totals side by side");
     scan_sums(h, ls, 2, V, &h->ctl->evals);
+    if (V <= kSmallPeelV) {  // (other peels do not ask)
+        ++g_launches;
+        k_max_len<<<grid_for(h, V), kThreads, 0, h->stream>>>(V, g.out_len, g.in_len, &h->ctl->maxv[0]);
+    }
     EngineCtl hc;
     if (int rc = check_ctl(h, &hc, "graph build")) return rc;
+    g.max_len = (uint32_t)hc.maxv[0];
     if (hc.evals >= 0xFFFFFFFFull || hc.drops >= 0xFFFFFFFFull)
         return set_error(DC_ERR_CAPACITY, "adjacency with slack exceeds 2^32 entries (u32 offsets)");
     if (dmalloc(h->stream, &g.out_off, (uint64_t)V + 1) || dmalloc(h->stream, &g.out_nbr, hc.evals) ||
@@ -2822,6 +2953,27 @@ PeelInst make_inst(dc_graph* h, int which, const int32_t* member, int32_t k, int
 int run_peel2(dc_graph* h, int ninst, const PeelInst* inst, int32_t* maxv) {
     Scratch* s = h->scratch;
     DevGraph& g = h->g;
+    // one block per peel where the shapes were never set (a trace or a barrier
+    // test wants the grid's kernel)
+    if (h->peel_bps <= 0 && h->blocks_per_sm <= 0 && !inst[0].member && peel_fits_block(g) && !h->trace_dev &&
+        h->barrier_fault_block < 0) {
+        SmallPeel sp;
+        sp.in[0] = inst[0];
+        sp.in[1] = ninst > 1 ? inst[1] : inst[0];
+        sp.V = g.V;
+        sp.ctl = h->ctl;
+        const int shm = (int)(6u * g.V + 8u);
+        DC_CUDA(cudaFuncSetAttribute((const void*)k_peel_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(6u * kSmallPeelV + 8u)));
+        DC_CUDA(cudaMemsetAsync(h->ctl, 0, sizeof(EngineCtl), h->stream));
+        ++g_launches;
+        k_peel_small<<<ninst, kSmallPeelThreads, shm, h->stream>>>(sp);
+        DC_CUDA(cudaGetLastError());
+        EngineCtl hc;
+        if (int rc = check_ctl(h, &hc, "peel")) return rc;
+        for (int i = 0; i < ninst; ++i) maxv[i] = hc.maxv[i];
+        return DC_OK;
+    }
     const unsigned chunk = h->peel_chunk ? h->peel_chunk : 64;
     // bags (at least 8 of the 2 V vertices each) and pieces of long lists
     uint64_t need = 2ull * g.V + 2ull * (g.out_cap + g.in_cap) / (4ull * chunk) + (uint64_t)h->geom.sms * 64 + 4096;

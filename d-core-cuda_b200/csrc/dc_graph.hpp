@@ -35,6 +35,7 @@ struct DevGraph {
     int32_t* in_len = nullptr;
     uint32_t* in_nbr = nullptr;
     uint64_t out_cap = 0, in_cap = 0;
+    uint32_t max_len = 0;  // longest list when the lists were built (small graphs, else 0)
 };
 
 // Persistent-kernel launch geometry for the current device.
