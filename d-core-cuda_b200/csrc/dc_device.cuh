@@ -401,12 +401,17 @@ __device__ __forceinline__ bool tq_take_warp(EngineCtl* c, TicketQueue q, unsign
 //     one warp while another advances the step would lose an item), and items
 //     carry their step: a warp that finds an item of a newer step in its slot
 //     has not started that step yet and leaves the item there until it has
-// Memory order: acquire loads and acquire atomics cost no more than relaxed
-// ones here (327 and 528 clocks), a fence costs 280-900 clocks, so readers
-// acquire, and a writer fences once, between its value and whatever makes
-// another warp look at it.  Counters are only changed by atomics whose result
-// is used: they are performed in L2, where every reader reads, before
-// anything that follows from the result.
+// Memory order: atomics on different addresses are not ordered by themselves,
+// not even by a result that was waited for.  Whatever a warp did in a step is
+// released by the subtraction on t_work that reports it; the one that ends the
+// step acquires all of it with a fence, reads the step's counters, and releases
+// the next step with the fence before its words; the polling warp acquires the
+// word and hands it on inside the block with fences of the block's scope.
+// (Without the release the end of a step could be seen before its bound, and a
+// peel ended early or a row was jumped, about once in 5,000 decompositions
+// while other kernels kept L2 busy.)  Acquire loads cost no more than relaxed
+// ones here (327 clocks), a fence 280-900, so readers acquire, and a writer
+// fences once, between its value and whatever makes another warp look at it.
 // ---------------------------------------------------------------------------
 constexpr int kWorkShift = 33;
 
@@ -418,6 +423,15 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+// Atomic addition after everything this thread wrote, or saw from its warp or
+// block through their barriers, is performed.
+__device__ __forceinline__ unsigned long long add_release(unsigned long long* p, unsigned long long x) {
+    unsigned long long v;
+    asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;" : "=l"(v) : "l"(p), "l"(x) : "memory");
     return v;
 }
 
@@ -458,13 +472,14 @@ __device__ __forceinline__ unsigned long long step_block_word(const StepBlock* b
     return *reinterpret_cast<const volatile unsigned long long*>(&b->word);
 }
 
-// One thread: n producers or items of step `word` are finished; the last one
-// advances the step.  next(c, level, worked, bound): the next level;
+// One thread (after a warp barrier): n producers or items of step `word` are
+// finished; the last one advances the step.  next(c, level, worked, bound): the next level;
 // next.begin(step): the blocks that seed that step, before it is published.
 template <typename Next>
 __device__ __forceinline__ void step_finish(EngineCtl* c, int n, unsigned long long word, const Next& next) {
-    const unsigned long long old = atomicAdd(&c->t_work, 0ull - ((unsigned long long)n << kWorkShift));
+    const unsigned long long old = add_release(&c->t_work, 0ull - ((unsigned long long)n << kWorkShift));
     if ((old >> kWorkShift) != (unsigned long long)n) return;
+    fence_acq_rel();
     const unsigned step = step_number(word);
     const unsigned tail = (unsigned)old;
     const unsigned tail0 = ld_vol(&c->trace_tail0);
@@ -502,6 +517,7 @@ template <typename Next>
 __device__ __forceinline__ void step_seeded(EngineCtl* c, StepBlock* b, int bound, bool worked,
                                             unsigned long long word, bool tracing, const Next& next) {
     bound = __reduce_min_sync(0xFFFFFFFFu, bound);
+    __syncwarp();
     if ((threadIdx.x & 31u) == 0) {
         if (bound != kNoBound) atomicMin(&b->bound, bound);
         if (worked) atomicOr(&b->worked, 1u);
@@ -511,14 +527,12 @@ __device__ __forceinline__ void step_seeded(EngineCtl* c, StepBlock* b, int boun
             __threadfence_block();
             const int m = atomicExch(&b->bound, kNoBound);
             const unsigned step = step_number(word);
-            unsigned long long r = 0;
-            if (atomicExch(&b->worked, 0u)) r = atomicMax(&c->worked, step);
+            if (atomicExch(&b->worked, 0u)) atomicMax(&c->worked, step);
             for (int i = 0; i < 2; ++i)
-                if (const unsigned k = atomicExch(&b->count[i], 0u)) r += atomicAdd(&c->removed[i], k);
+                if (const unsigned k = atomicExch(&b->count[i], 0u)) atomicAdd(&c->removed[i], k);
             if (tracing && step - 1 < c->trace_cap) atomicMax(&c->trace[8 * (step - 1) + 5], gtimer());
             if (m != kNoBound)
-                r += atomicMax(&c->next_low, ((unsigned long long)step << 32) | (unsigned long long)(kNoBound - m));
-            used_result(r);
+                atomicMax(&c->next_low, ((unsigned long long)step << 32) | (unsigned long long)(kNoBound - m));
             step_finish(c, 1, word, next);
         }
     }
@@ -526,12 +540,12 @@ __device__ __forceinline__ void step_seeded(EngineCtl* c, StepBlock* b, int boun
 }
 
 // Converged warp, while the step is being seeded: an item kept by the warp
-// counts like a queued one, and the step has work.
-__device__ __forceinline__ void step_count_kept(EngineCtl* c, unsigned long long word) {
+// counts like a queued one (before the block's report, which another warp may
+// make).  The warp reports work with its share (step_seeded).
+__device__ __forceinline__ void step_count_kept(EngineCtl* c) {
     if ((threadIdx.x & 31u) == 0) {
-        const unsigned long long a = atomicAdd(&c->t_work, 1ull << kWorkShift);
-        const unsigned o = atomicMax(&c->worked, step_number(word));
-        used_result(a, o);
+        atomicAdd(&c->t_work, 1ull << kWorkShift);
+        fence_acq_rel();
     }
     __syncwarp();
 }
@@ -577,6 +591,7 @@ __device__ __forceinline__ int step_take(EngineCtl* c, TicketQueue q, StepBlock*
     const unsigned lane = threadIdx.x & 31u;
     unsigned long long it = kEmptyItem, w = *word;
     int state = 0;
+    __syncwarp();
     if (lane == 0) {
         const bool poller = threadIdx.x == 0;
         if (*ticket == kNoTicket) *ticket = atomicAdd(&c->t_head, 1u);
@@ -607,7 +622,10 @@ __device__ __forceinline__ int step_take(EngineCtl* c, TicketQueue q, StepBlock*
                         w = kStopWord;
                     }
                 }
-                if (w != *word) *reinterpret_cast<volatile unsigned long long*>(&b->word) = w;
+                if (w != *word) {
+                    __threadfence_block();
+                    *reinterpret_cast<volatile unsigned long long*>(&b->word) = w;
+                }
             } else {
                 w = step_block_word(b);
                 ++spins;
@@ -621,9 +639,11 @@ __device__ __forceinline__ int step_take(EngineCtl* c, TicketQueue q, StepBlock*
             *ticket = kNoTicket;
             state = kTakeItem;
         } else {
+            __threadfence_block();
             state = w == kStopWord ? kTakeStop : kTakeStep;
         }
     }
+    __syncwarp();
     state = __shfl_sync(0xFFFFFFFFu, state, 0);
     if (state == kTakeItem) it = __shfl_sync(0xFFFFFFFFu, it, 0);
     else w = __shfl_sync(0xFFFFFFFFu, w, 0);

@@ -1429,7 +1429,7 @@ __device__ __forceinline__ int drop_pass(const Trans2Params& p, const RowGroup& 
                 if (si_[q] == 0u) ri |= 1u << q;
             }
             if (keep_one(keep, &ro, uo) || keep_one(keep, &ri, ui)) {
-                if (kLeave) step_count_kept(G.ctl, word);
+                if (kLeave) step_count_kept(G.ctl);
                 else --*pending;  // the item being finished pays for the kept one
             }
             step_push_mask8(G.ctl, G.q, ro, uo, ri, ui, step_tag(word));
@@ -1685,11 +1685,11 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
             }
             if (__any_sync(0xFFFFFFFFu, req != 0u)) {
                 const uint32_t u[4] = {v, 0u, 0u, 0u};
-                if (keep_one(&keep, &req, u)) step_count_kept(c, word);
+                if (keep_one(&keep, &req, u)) step_count_kept(c);
                 step_push(c, G.q, req != 0u, (unsigned long long)v | tag);
             }
         }
-        if (seeds) step_seeded(c, &s_step, bound, false, word, tracing, next);
+        if (seeds) step_seeded(c, &s_step, bound, keep != kNoKeep, word, tracing, next);
 
         // ---- drain: the warp's kept item first, else the queue; finished
         // items are counted off in batches (before the warp waits)

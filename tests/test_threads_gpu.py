@@ -1,0 +1,72 @@
+"""Several threads decompose their own handles at the same time: other
+kernels' traffic delays every memory access of a decomposition, and whatever
+is not ordered shows.  Each result equals the one of the handle alone, which
+equals the oracle's.  4 x 150 decompositions per case: an error of one in 100
+is met in all but 0.3 % of the runs, one in 5,000 (what a missing wait gave
+once) in 11 %; the wide margins are for runs of many repeats."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# above 36,000 vertices, where the peel takes the whole chip
+GRAPHS = [("rmat", 16, 8, 3), ("rmat", 16, 16, 4), ("rmat", 17, 8, 5), ("er", 60_000, 600_000, 6)]
+
+
+def graph(dc, kind, a, b, seed):
+    if kind == "rmat":
+        return dc.gen_rmat(a, b, seed)
+    s, d = dc.gen_er(a, b, seed)
+    return a, s, d
+
+
+def result(g):
+    return [g.kmaxes().copy()] + [np.array(x) for x in g.skyline()]
+
+
+def run_threads(dc, jobs, repeats):
+    """jobs: (graph, settings, expected); one thread each, a new handle every
+    third decomposition."""
+    wrong, start = [], threading.Barrier(len(jobs))
+
+    def work(i, g, settings, want):
+        start.wait()
+        try:
+            for turn in range(0, repeats, 3):
+                with dc.Graph.from_edges(*g) as h:
+                    if settings is not None:
+                        h.set_tuning(*settings)
+                    for again in range(3):
+                        h.decompose()
+                        got = result(h)
+                        bad = [p for p, (x, y) in enumerate(zip(got, want)) if not np.array_equal(x, y)]
+                        if bad:
+                            wrong.append((i, turn + again, bad))
+        except Exception as e:  # a failed call, not a wrong result
+            wrong.append((i, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(i, *j)) for i, j in enumerate(jobs)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    return wrong
+
+
+@pytest.fixture(scope="module")
+def alone(dc, orc, gpu):
+    out = []
+    for spec in GRAPHS:
+        V, s, d = graph(dc, *spec)
+        km, lm, kmaxes, rows = orc.dcore(V, s, d)
+        with dc.Graph.from_edges(V, s, d) as g:
+            assert g.decompose() == (km, lm)
+            assert np.array_equal(g.kmaxes(), kmaxes) and np.array_equal(g.rows(), rows)
+            out.append(((V, s, d), result(g)))
+    return out
+
+
+def test_own_handles_engine_shapes(dc, alone):
+    assert run_threads(dc, [(g, None, want) for g, want in alone], 150) == []
