@@ -1705,21 +1705,31 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 if (state != kTakeItem) break;
                 x = (uint32_t)item;
             }
-            // the mark says "being evaluated" before any neighbour is read (a
+            // The mark says "being evaluated" before any neighbour is read (a
             // request made before it belongs to a drop that is seen below, one
-            // made after it has x evaluated again); a decrement that lands
-            // between the counter snapshot and the mark only makes the counter
-            // too low, which costs an evaluation
-            unsigned mk = 0;
-            if (lane == 0) mk = atomicExch(&G.mark[x], 2u);
-            const int cap = ld_vol(&G.cur[x]);
-            const int s0o = ld_vol(&G.cnt_out[x]), s0i = ld_vol(&G.cnt_in[x]);
-            const int stamp = ld_vol(&G.stamp[x]);
-            const uint32_t logidx = ld_vol(&G.logidx[x]);
+            // made after it has x evaluated again), and so is the snapshot of
+            // the counters: one read after a neighbour's decrement, beside that
+            // neighbour's value from before it, would leave the counter too
+            // high for good, and a later drop unseen.  (A decrement that lands
+            // after the snapshot, beside the neighbour's new value, only makes
+            // the counter too low, which costs an evaluation.)  So all of x's
+            // state is read by acquire loads, a word per lane, in one latency;
+            // lane 0's load of the mark returns after its exchange.
+            if (lane == 0) atomicExch(&G.mark[x], 2u);
             const int km = __ldg(p.kmax + x);
             const RowLists L = row_lists(p, x);
-            if (lane == 0) used_result(mk, ld_acquire(&G.mark[x]));
+            const void* at = lane == 0   ? (const void*)G.mark
+                             : lane == 1 ? (const void*)G.cnt_out
+                             : lane == 2 ? (const void*)G.cnt_in
+                             : lane == 3 ? (const void*)G.cur
+                             : lane == 4 ? (const void*)G.stamp
+                                         : (const void*)G.logidx;
+            const unsigned state_word = ld_acquire((const unsigned*)at + x);
             __syncwarp();
+            const int s0o = (int)__shfl_sync(0xFFFFFFFFu, state_word, 1), s0i = (int)__shfl_sync(0xFFFFFFFFu, state_word, 2);
+            const int cap = (int)__shfl_sync(0xFFFFFFFFu, state_word, 3);
+            const int stamp = (int)__shfl_sync(0xFFFFFFFFu, state_word, 4);
+            const uint32_t logidx = __shfl_sync(0xFFFFFFFFu, state_word, 5);
             if (km < j || cap < 1) {
                 if (lane == 0) atomicExch(&G.mark[x], 0u);
                 ++pending;

@@ -70,3 +70,8 @@ def alone(dc, orc, gpu):
 
 def test_own_handles_engine_shapes(dc, alone):
     assert run_threads(dc, [(g, None, want) for g, want in alone], 150) == []
+
+
+def test_own_handles_one_run(dc, alone):
+    # rows as one run: every evaluation meets those of the whole chip
+    assert run_threads(dc, [(g, (2, 2, 64, ()), want) for g, want in alone], 150) == []
