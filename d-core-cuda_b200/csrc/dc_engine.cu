@@ -1811,10 +1811,15 @@ __global__ void __launch_bounds__(kThreads, DC_TRANS2_MIN_BLOCKS) k_trans2(Trans
                 const int no = atomicAdd(&G.cnt_out[x], c_o - s0o) + (c_o - s0o);
                 const int ni = atomicAdd(&G.cnt_in[x], c_i - s0i) + (c_i - s0i);
                 const bool stable = nv < 1 || (no >= nv && ni >= j);
-                // released once the counters are; requested meanwhile or
-                // unstable: evaluated again
+                // released once the counters are performed everywhere;
+                // requested meanwhile or unstable: evaluated again, and the
+                // mark says so before another warp can take the item (an
+                // exchange that came after the taker's would leave the mark
+                // set with nobody queued, and drop every later request)
+                fence_acq_rel();
                 if (!stable || atomicCAS(&G.mark[x], 2u, 0u) == 3u) {
-                    used_result(atomicExch(&G.mark[x], 1u));
+                    atomicExch(&G.mark[x], 1u);
+                    fence_acq_rel();
                     again = 1u;
                 }
             }

@@ -75,3 +75,8 @@ def test_own_handles_engine_shapes(dc, alone):
 def test_own_handles_one_run(dc, alone):
     # rows as one run: every evaluation meets those of the whole chip
     assert run_threads(dc, [(g, (2, 2, 64, ()), want) for g, want in alone], 150) == []
+
+
+def test_own_handles_cut_rows(dc, alone):
+    # three groups of blocks per handle, twelve at a time on the chip
+    assert run_threads(dc, [(g, (2, 2, 64, (200, 500)), want) for g, want in alone], 150) == []
