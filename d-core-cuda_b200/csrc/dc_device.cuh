@@ -435,11 +435,6 @@ __device__ __forceinline__ unsigned long long add_release(unsigned long long* p,
     return v;
 }
 
-// Makes the program wait for an atomic's result: it is performed then.
-__device__ __forceinline__ void used_result(unsigned long long a, unsigned long long b = 0) {
-    asm volatile("{ .reg .b64 t; add.s64 t, %0, %1; }" ::"l"(a), "l"(b) : "memory");
-}
-
 __device__ __forceinline__ int step_level(unsigned long long w) { return (int)(uint32_t)w; }
 __device__ __forceinline__ unsigned step_number(unsigned long long w) { return (unsigned)(w >> 32); }
 // 9 bits above 32 bits of payload and 22 of detail; the top bit stays 0, so

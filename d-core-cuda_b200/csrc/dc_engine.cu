@@ -1029,7 +1029,10 @@ struct RowsNext {
         const unsigned long long now = gtimer();
         if (level == kRowsInit) {  // the values are copied
             own.flush_n = 0;
-            if (own.from >= 0) used_result(atomicSub(&pl->own[own.from].readers, 1u));
+            if (own.from >= 0) {
+                __threadfence();  // the copies are made before the other group may overwrite what they read
+                atomicSub(&pl->own[own.from].readers, 1u);
+            }
             return kRowsCount;
         }
         if (level == kRowsCount) {
@@ -1116,9 +1119,11 @@ struct RowsNext {
                 own.spare_n = n;
             }
             // the seam is there, and the other group knows that its values
-            // are wanted, before its run is shortened
+            // are wanted, before its run is shortened (its last step reads
+            // both after the exchange on its span that ends the run, with a
+            // fence between)
             if (atomicCAS(p.seam_of + best_start, 0u, own.spare_off + 1u) != 0u) continue;
-            used_result(atomicAdd(&pl->own[best].readers, 1u));
+            atomicAdd(&pl->own[best].readers, 1u);
             __threadfence();
             const unsigned long long stop = best_s >> 32;
             for (int again = 0; again < 8; ++again) {  // the other group may move on meanwhile
@@ -1126,7 +1131,7 @@ struct RowsNext {
                     &pl->span[best].v, best_s, ((unsigned long long)(best_start - 1) << 32) | (best_s & 0xFFFFFFFFull));
                 if (o == best_s) {
                     own.from = ld_acquire(&pl->own[best].ready) ? best : -1;
-                    if (own.from < 0) used_result(atomicSub(&pl->own[best].readers, 1u));
+                    if (own.from < 0) atomicSub(&pl->own[best].readers, 1u);
                     own.spare_n = 0;
                     own.lo = best_start;
                     *(volatile unsigned long long*)&pl->span[gid].v = (stop << 32) | (unsigned)best_start;
@@ -1135,8 +1140,8 @@ struct RowsNext {
                 if ((o >> 32) != stop || (int)(uint32_t)o >= best_start) break;
                 best_s = o;
             }
-            used_result(atomicExch(p.seam_of + best_start, 0u));
-            used_result(atomicSub(&pl->own[best].readers, 1u));
+            atomicExch(p.seam_of + best_start, 0u);
+            atomicSub(&pl->own[best].readers, 1u);
         }
         if (flush) return kRowsWait;  // leaves the values first
         // nothing to wait for, or a group that stopped on an error

@@ -80,3 +80,17 @@ def test_own_handles_one_run(dc, alone):
 def test_own_handles_cut_rows(dc, alone):
     # three groups of blocks per handle, twelve at a time on the chip
     assert run_threads(dc, [(g, (2, 2, 64, (200, 500)), want) for g, want in alone], 150) == []
+
+
+def test_own_handles_groups_join(dc, orc, gpu):
+    # eight groups with a few rows each: rows change hands and groups join all
+    # the time, and a group copies the values of one that goes on or ends
+    jobs = []
+    for seed in (51, 52, 53, 54):
+        V, s, d = dc.gen_rmat(13, 32, seed)
+        km, lm, kmaxes, rows = orc.dcore(V, s, d)
+        with dc.Graph.from_edges(V, s, d) as g:
+            assert g.decompose() == (km, lm)
+            assert np.array_equal(g.kmaxes(), kmaxes) and np.array_equal(g.rows(), rows)
+            jobs.append(((V, s, d), (2, 2, 64, (10, 20, 30, 40, 50, 60, 70)), result(g)))
+    assert run_threads(dc, jobs, 300) == []
