@@ -62,7 +62,9 @@ struct EngineCtl {
     alignas(128) unsigned bag_tail;            // fused peel: vertices put into bags
     int peel_list[2];       // per peel: remaining vertices in rem0 / rem1, or all (-1)
     int peel_compact[2];    // the level writes the list anew
-    unsigned removed[2];    // removed since it was written
+    unsigned removed[2];    // removed so far
+    unsigned removed_at[2]; // removed when the list was written
+    unsigned members[2];    // vertices to remove
     alignas(128) unsigned long long next_low;  // (step << 32) | (2^31 - 1 - least next level)
     alignas(128) unsigned rc_cur[2];  // remaining-list sizes per peel instance
     PadU rc_next[2];        // next level's remaining-list sizes (appended by every warp)

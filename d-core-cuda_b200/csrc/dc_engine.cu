@@ -370,11 +370,11 @@ struct PeelHook {
                 c->rc_cur[i] = n;
                 c->rc_next[i].v = 0;
                 c->peel_list[i] = ld_vol(&c->peel_list[i]) == 0 ? 1 : 0;
-                c->removed[i] = 0;
+                c->removed_at[i] = ld_vol(&c->removed[i]);
                 c->peel_compact[i] = 0;
             } else {
                 // the list is written anew once a quarter of it is gone
-                c->peel_compact[i] = 4ull * ld_vol(&c->removed[i]) > n;
+                c->peel_compact[i] = 4ull * (ld_vol(&c->removed[i]) - ld_vol(&c->removed_at[i])) > n;
             }
         }
         // a level whose scan found nothing to remove changed no degree: the
@@ -389,7 +389,7 @@ struct PeelStart {
     bool member;
     __device__ void operator()(EngineCtl* c) const {
         for (int i = 0; i < ninst; ++i) {
-            c->rc_cur[i] = member ? c->rc_next[i].v : V;
+            c->rc_cur[i] = c->members[i] = member ? c->rc_next[i].v : V;
             c->rc_next[i].v = 0;
             c->peel_list[i] = member ? 0 : -1;
             c->peel_compact[i] = 1;
@@ -910,7 +910,11 @@ __global__ void __launch_bounds__(kSmallPeelThreads, 1) k_peel_small(SmallPeel p
             __syncthreads();
         }
     }
-    if (t == 0) p.ctl->maxv[blockIdx.x] = level;
+    if (t == 0) {
+        p.ctl->maxv[blockIdx.x] = level;
+        p.ctl->removed[blockIdx.x] = head;
+        p.ctl->members[blockIdx.x] = V;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2969,6 +2973,18 @@ PeelInst make_inst(dc_graph* h, int which, const int32_t* member, int32_t k, int
     return I;
 }
 
+// A peel is over when every vertex is removed (the last level's scan reports
+// what its warps removed before); a vertex left would go into the rows with
+// -1 for its kmax, an index there.
+static int peel_status(const EngineCtl& c, int ninst, int32_t* maxv) {
+    for (int i = 0; i < ninst; ++i) {
+        if (c.removed[i] != c.members[i])
+            return set_error(DC_ERR_CUDA, "peel: ended with %u of %u vertices removed", c.removed[i], c.members[i]);
+        maxv[i] = c.maxv[i];
+    }
+    return DC_OK;
+}
+
 // Runs one or two peels in one persistent launch; maxv[i] = largest value.
 int run_peel2(dc_graph* h, int ninst, const PeelInst* inst, int32_t* maxv) {
     Scratch* s = h->scratch;
@@ -2991,8 +3007,7 @@ int run_peel2(dc_graph* h, int ninst, const PeelInst* inst, int32_t* maxv) {
         DC_CUDA(cudaGetLastError());
         EngineCtl hc;
         if (int rc = check_ctl(h, &hc, "peel")) return rc;
-        for (int i = 0; i < ninst; ++i) maxv[i] = hc.maxv[i];
-        return DC_OK;
+        return peel_status(hc, ninst, maxv);
     }
     const unsigned chunk = h->peel_chunk ? h->peel_chunk : 64;
     // bags (at least 8 of the 2 V vertices each) and pieces of long lists
@@ -3021,8 +3036,7 @@ int run_peel2(dc_graph* h, int ninst, const PeelInst* inst, int32_t* maxv) {
     if (bps <= 0 && h->blocks_per_sm <= 0 && !inst[0].member) bps = g.V <= 50000u ? 1 : g.V >= 3000000u ? 3 : 2;
     const FirstStep first{0, 0};
     if (int rc = run_persistent(h, fn, args, "peel", &hc, bps, &first)) return rc;
-    for (int i = 0; i < ninst; ++i) maxv[i] = hc.maxv[i];
-    return DC_OK;
+    return peel_status(hc, ninst, maxv);
 }
 
 int peel_kmax_row0(dc_graph* h, int32_t* kmax, int32_t* lmax) {
