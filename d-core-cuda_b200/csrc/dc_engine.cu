@@ -3468,9 +3468,13 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     // (engine's cuts, 1 / 2 / 3 blocks per SM: 53,000 edges 0.41 / 0.43 / 0.47
     // ms, 175,000 0.47 / 0.50 / 0.52, 470,000 0.69 / 0.62 / 0.62, 1.0 M 0.90 /
     // 0.85 / 0.88, 1.9 M 1.39 / 1.26 / 1.23, 3.9 M 2.36 / 2.10 / 1.89)
-    const int most_bps = !h->auto_cuts || h->blocks_per_sm > 0 ? 8 : g.E < 300000u ? 1 : g.E < 1500000u ? 2 : 8;
+    const int most_bps = !h->auto_cuts ? 8
+                         : h->blocks_per_sm > 0 ? h->blocks_per_sm  // dc_set_launch bounds the launch
+                         : g.E < 300000u ? 1 : g.E < 1500000u ? 2 : 8;
     if (int rc = persistent_grid(h, rows_fn, ngroups > 1 ? most_bps : h->rows_bps, &grid)) return rc;
-    if (ngroups > 1 && h->rows_bps > 0) grid = std::min(grid, h->rows_bps * ngroups * h->geom.sms);
+    // (cuts of the caller's: blocks per SM for every run, as for separate launches)
+    const int run_bps = h->rows_bps > 0 ? h->rows_bps : h->blocks_per_sm;
+    if (ngroups > 1 && !h->auto_cuts && run_bps > 0) grid = std::min(grid, run_bps * ngroups * h->geom.sms);
     const uint64_t spare = (uint64_t)kLogChunk * kWarpsPerBlock * grid;  // records left over in the warps' chunks
     // seams: the values of row a - 1 in C_a for every run that starts at a,
     // with room for rows taken over (a void record each at most)

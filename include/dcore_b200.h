@@ -426,8 +426,10 @@ int dc_server_set_row_repair(dc_server* s, int on);
  * tracing off. */
 typedef void (*dc_trace_fn)(const char* phase, const unsigned long long* rec, unsigned steps, void* user);
 int dc_set_trace(dc_graph* g, uint32_t max_steps, dc_trace_fn fn, void* user);
-/* Persistent-kernel blocks per SM for every persistent kernel (0 = the
- * default, 2; dc_set_tuning sets the peel and row kernels separately). */
+/* Persistent-kernel blocks per SM for every persistent kernel, also where the
+ * engine cuts the rows itself (0 = the engine's choice by the graph's size
+ * where shapes were never set, else 2; dc_set_tuning sets the peel and row
+ * kernels separately). */
 int dc_set_launch(dc_graph* g, int blocks_per_sm);
 
 /* Launch shapes of the persistent kernels: blocks per SM of the fused peel
@@ -449,6 +451,10 @@ typedef struct dc_tuning {
      * cores shrink fast enough for that to pay.) */
     int32_t rows_split_permille[7];
 } dc_tuning;
+/* On a handle whose shapes were never set dc_get_tuning reports 2 blocks per
+ * SM, chunks of 64 and no cuts, what a handle tuned to these values has; the
+ * engine's own choices are not among them.  dc_set_tuning, with any values,
+ * ends those choices for the handle. */
 int dc_get_tuning(dc_graph* g, dc_tuning* t);
 int dc_set_tuning(dc_graph* g, const dc_tuning* t);
 /* Autotuner: times the decomposition of this graph under candidate launch
