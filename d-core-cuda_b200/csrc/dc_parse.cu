@@ -17,7 +17,7 @@
 // vertex its row values 0..kmax[v] separated by spaces, a newline after every
 // vertex but the last.  Each vertex's line is formatted from its skyline
 // corners (a run of equal values per corner), line lengths are scanned, the
-// text is written on the device and copied to the host a piece at a time.
+// text is written on the device, copied to the host and then to the file.
 #include <algorithm>
 #include <atomic>
 #include <cerrno>
@@ -28,6 +28,7 @@
 
 #include "dc_engine.cuh"
 #include "dc_internal.h"
+#include "dc_textout.hpp"
 
 namespace dc {
 extern std::atomic<unsigned long long> g_launches;
@@ -39,7 +40,7 @@ namespace {
 constexpr int kFT = 256;                // threads per block
 constexpr int kFBytes = 16;             // bytes (or items) per thread and tile
 constexpr int kFTile = kFT * kFBytes;   // per block tile
-constexpr uint64_t kFileChunk = 1u << 20;  // bytes read or written at a time
+constexpr uint64_t kFileChunk = 1u << 20;  // bytes read at a time
 constexpr int kMaxLine = 511;           // host parser's fgets buffer minus the terminator
 
 __device__ __forceinline__ unsigned long long block_excl_scan_u64(unsigned long long x, unsigned long long* total) {
@@ -493,23 +494,13 @@ int write_decomp_cpu_device(dc_graph* h, const char* path) {
                 break;
             }
         }
-        FILE* f = fopen(path, "wb");
-        if (!f) {
-            rc = set_error(DC_ERR_IO, "cannot write '%s': %s", path, strerror(errno));
-            break;
-        }
-        bool ok = fwrite(head, 1, (size_t)hn, f) == (size_t)hn;
-        std::vector<char> chunk(std::min<uint64_t>(total, kFileChunk));
-        for (uint64_t at = 0; at < total && ok && !rc; at += chunk.size()) {
-            const uint64_t m = std::min<uint64_t>(chunk.size(), total - at);
-            if (cudaMemcpyAsync(chunk.data(), d_out + at, m, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        // (ordinary memory: see the reader)
+        rc = write_fetched(path, head, (size_t)hn, total, [&](char* to) {
+            if (cudaMemcpyAsync(to, d_out, total, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
                 cudaStreamSynchronize(st) != cudaSuccess)
-                rc = set_error(DC_ERR_CUDA, "decompCPU: %s", cudaGetErrorString(cudaGetLastError()));
-            else ok = fwrite(chunk.data(), 1, m, f) == m;
-        }
-        if (fclose(f) != 0) ok = false;
-        if (rc) break;
-        if (!ok) rc = set_error(DC_ERR_IO, "short write to '%s'", path);
+                return set_error(DC_ERR_CUDA, "decompCPU: %s", cudaGetErrorString(cudaGetLastError()));
+            return DC_OK;
+        });
     } while (0);
     if (d_out) cudaFreeAsync(d_out, st);
     cudaStreamSynchronize(st);
