@@ -1,7 +1,10 @@
 """Peels in which most of a wave of removals falls to one warp, which keeps at
 most 16 vertices while others wait: grids and layered graphs (waves of a few
-to thousands of vertices, one to eight entries each) and a chain, both kinds of
-instance, against the oracle."""
+to thousands of vertices, one to eight entries each); and chains of single
+removals, which a warp works off an entry per lane up to 32 entries: lists of
+31 to 33, of one side (leaves along the chain) and of both (a chain that falls
+out of a row because its end left the core).  Both kinds of instance, against
+the oracle."""
 import numpy as np
 import pytest
 
@@ -19,8 +22,29 @@ def layers(width, deg, count):
     return width * count, s, (s // width + 1) * width + rng.integers(0, width, len(s))
 
 
+def leaves(n, deg):
+    i = np.arange(n)
+    s, d = [i[:-1], i.repeat(deg)], [i[1:], n + np.arange(n * deg)]
+    return n * (deg + 1), np.concatenate(s), np.concatenate(d)
+
+
+def row_chain(n, K):
+    """A clique of K + 1, a path into it whose vertices have K in-edges from it,
+    the last one two fewer."""
+    a, b = np.divmod(np.arange((K + 1) ** 2), K + 1)
+    p = np.arange(n) + K + 1
+    s, d = [a[a != b], p], [b[a != b], np.append(p[1:], 0)]
+    for j in range(K):
+        q = p if j < K - 2 else p[:-1]
+        s.append(np.full(len(q), j))
+        d.append(q)
+    return n + K + 1, np.concatenate(s), np.concatenate(d)
+
+
 CASES = [(grid, (2, 30)), (grid, (15, 40)), (grid, (16, 16)), (grid, (17, 33)), (grid, (300, 300)), (layers, (15, 3, 50)),
-         (layers, (17, 1, 200)), (layers, (500, 4, 80)), (layers, (3000, 8, 20)), (grid, (1, 3000))]
+         (layers, (17, 1, 200)), (layers, (500, 4, 80)), (layers, (3000, 8, 20)), (grid, (1, 3000)),
+         (leaves, (400, 30)), (leaves, (400, 31)), (leaves, (400, 32)), (row_chain, (300, 4)), (row_chain, (300, 29)),
+         (row_chain, (300, 30)), (row_chain, (300, 31))]
 
 
 @pytest.mark.parametrize("make,args", CASES)
