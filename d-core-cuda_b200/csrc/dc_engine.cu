@@ -2572,10 +2572,12 @@ void free_decomp(Decomp& d, cudaStream_t st) {
     d.rows_valid = false;
 }
 
-void free_scratch(dc_graph* h) {
+// The row groups' state; returns whether there was any.
+static bool free_groups(dc_graph* h) {
     Scratch* s = h->scratch;
-    if (!s) return;
+    bool any = s->seam != nullptr;
     for (RowSegment& g : s->seg) {
+        any = any || g.cur || g.tring;
         dfree(h->stream, g.cur);
         dfree(h->stream, g.cnt_out);
         dfree(h->stream, g.cnt_in);
@@ -2584,7 +2586,20 @@ void free_scratch(dc_graph* h) {
         dfree(h->stream, g.logidx);
         dfree(h->stream, g.tring);
         dfree(h->stream, g.ctl);
+        g.cap_V = 0;
+        g.tring_cap = 0;
     }
+    dfree(h->stream, s->seam_of);
+    dfree(h->stream, s->seam);
+    s->seam_of_cap = 0;
+    s->seam_cap = 0;
+    return any;
+}
+
+void free_scratch(dc_graph* h) {
+    Scratch* s = h->scratch;
+    if (!s) return;
+    free_groups(h);
     dfree(h->stream, s->key);
     dfree(h->stream, s->cdeg);
     dfree(h->stream, s->cur);
@@ -2611,8 +2626,6 @@ void free_scratch(dc_graph* h) {
     dfree(h->stream, s->kmax_old);
     dfree(h->stream, s->row0_old);
     dfree(h->stream, s->plan);
-    dfree(h->stream, s->seam_of);
-    dfree(h->stream, s->seam);
     dfree(h->stream, s->pos);
     dfree(h->stream, s->kmax_r);
     dfree(h->stream, s->row0_r);
@@ -3113,7 +3126,10 @@ int build_skyline_from_log(dc_graph* h, uint64_t nlog) {
         dfree(h->stream, d.sky_l);
         d.corner_cap = 0;
         const uint64_t want = total + total / 4 + 1;
-        if (dmalloc(h->stream, &d.sky_k, want) || dmalloc(h->stream, &d.sky_l, want)) return DC_ERR_NOMEM;
+        if (dmalloc(h->stream, &d.sky_k, want) || dmalloc(h->stream, &d.sky_l, want)) {
+            dfree(h->stream, d.sky_k);
+            if (!free_groups(h) || dmalloc(h->stream, &d.sky_k, want) || dmalloc(h->stream, &d.sky_l, want)) return DC_ERR_NOMEM;
+        }
         d.corner_cap = want;
     }
     if (!d.sky_off && dmalloc(h->stream, &d.sky_off, (uint64_t)V + 1)) return DC_ERR_NOMEM;
@@ -3136,7 +3152,8 @@ static int ensure_rows(dc_graph* h, uint64_t elems) {
     if (d.rows_cap >= elems && d.rows) return DC_OK;
     dfree(h->stream, d.rows);
     d.rows_cap = 0;
-    if (dmalloc(h->stream, &d.rows, elems)) return DC_ERR_NOMEM;
+    if (dmalloc(h->stream, &d.rows, elems) && !(free_groups(h) && dmalloc(h->stream, &d.rows, elems) == DC_OK))
+        return DC_ERR_NOMEM;
     d.rows_cap = elems;
     return DC_OK;
 }
@@ -3380,7 +3397,8 @@ static int build_relabeled(dc_graph* h, int32_t K, uint32_t n0, unsigned* sort_c
 // row-to-row kernel.  Corners of rows 1..Kstop are left in the scratch log
 // (*nlog entries).  allow_sort: order adjacency lists by neighbour kmax
 // first (otherwise lists are read whole).
-int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint64_t* nlog_out, int32_t K0) {
+// cut: the engine may cut the rows by itself.
+static int rows_run(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint64_t* nlog_out, int32_t K0, bool cut) {
     DevGraph& g = h->g;
     Decomp& d = h->d;
     Scratch* s = h->scratch;
@@ -3444,7 +3462,7 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     int32_t run_min = Kstop + 1;
     int first_share = 1;   // blocks of the first run, in shares of the others'
     uint32_t n_state = 0;  // vertices every group after the first has state for
-    if (relabel && k0 == 1 && Kstop >= kMinSplitRows) {
+    if (relabel && k0 == 1 && Kstop >= kMinSplitRows && (cut || !h->auto_cuts)) {
         if (h->auto_cuts) {
             // A handle whose launch shapes were never set is cut where the
             // core a run starts from is small: a start costs a pass over its
@@ -3666,6 +3684,14 @@ int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint6
     cudaEventRecord(h->ev[4], h->stream);
     *nlog_out = nlog;
     return DC_OK;
+}
+
+int rows_from_row0(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint64_t* nlog_out, int32_t K0) {
+    const int rc = rows_run(h, K, Kstop, allow_sort, nlog_out, K0, true);
+    // cuts of the engine's own choice are not worth a refusal: one run needs
+    // no groups (all memory is taken before the kernel starts)
+    if (rc != DC_ERR_NOMEM || !h->auto_cuts || !free_groups(h)) return rc;
+    return rows_run(h, K, Kstop, allow_sort, nlog_out, K0, false);
 }
 
 int decompose(dc_graph* h, int method, int materialize_rows) {
