@@ -390,7 +390,7 @@ __device__ __forceinline__ bool tq_take_warp(EngineCtl* c, TicketQueue q, unsign
 // publishes it in step_word, and the others, which wait for items, see the
 // word change and start it.  Nothing arrives at a barrier: a grid barrier per
 // step cost its arrival and release round trips on top of the queue's own
-// termination (an empty step took 16-17 us with 296 blocks).
+// termination (an empty step took 16-17 us with 296 blocks, 10 this way).
 //   - t_work holds the queue's tail (low 33 bits) and the number of unfinished
 //     producers and items (high 31 bits) in one word: a push is one atomic,
 //     and the count can never lag behind the items it covers

@@ -824,9 +824,8 @@ __global__ void __launch_bounds__(kThreads, DC_PEEL_MIN_BLOCKS) k_peel2(Peel2Par
 // The peels of a small graph, one block each: degrees and the removed vertices
 // in shared memory, a level's removals in rounds with a block barrier between
 // them (a vertex is listed once, when it is removed, so the list never exceeds
-// V entries).  The grid's version spends 8 to 10 us on an empty level and about
-// 1.2 us on every link of a chain of removals, here they take about 1 us and
-// 0.5; what bounds it is the entries one SM can take (shared-memory atomics,
+// V entries).  The grid's version spends about 10 us on an empty level and 1.2
+// us on every link of a chain of removals, here they take about 1 us and 0.5; what bounds it is the entries one SM can take (shared-memory atomics,
 // about 2,000 per us), and the other SMs are free for other handles.
 struct SmallPeel {
     PeelInst in[2];
@@ -835,10 +834,10 @@ struct SmallPeel {
 };
 constexpr int kSmallPeelThreads = 1024;
 constexpr uint32_t kSmallPeelV = 36000;           // 6 bytes of shared memory per vertex
-// Faster than the grid's kernel, small / grid in ms: R-MAT 12 0.20 / 0.65,
-// 13 (24 edges per vertex) 0.39 / 0.95, 14 (40) 0.73 / 1.36, 15 (32) 1.08 /
-// 1.56; ER 1,000 0.045 / 0.125, 10,000 (20) 0.14 / 0.20, 10,000 (60) 0.23 /
-// 0.26, but 20,000 (20) 0.22 / 0.21 and 30,000 (50) 0.49 / 0.31: where all
+// Faster than the grid's kernel, small / grid in ms: R-MAT 12 0.21 / 0.71,
+// 13 (24 edges per vertex) 0.39 / 1.04, 14 (40) 0.75 / 1.45, 15 (32) 1.09 /
+// 1.73; ER 1,000 0.05 / 0.15, 10,000 (20) 0.14 / 0.19, but (when the line was
+// drawn) 20,000 (20) 0.22 / 0.21 and 30,000 (50) 0.49 / 0.31: where all
 // degrees are alike the removals are a few wide cascades, which want the
 // chip's atomics.  Hence by the longest list, as it was when the lists were
 // built (any choice gives the same result).
@@ -1042,8 +1041,8 @@ constexpr int kRowsJoin = -4;         // the group is over, its blocks go on in 
 // seed with its own blocks from the next step on.  The last rows below a cliff
 // of |C_k| are the heaviest and cannot be cut any more: one group's blocks
 // alone took the last 30 % of the rows of R-MAT 20 and 22 for them (joining,
-// and counts in shared memory instead of spilled registers, took the rows from
-// 5.7 and 17.7 ms to 5.0 and 15.8).  A group that others join has a run at
+// with counts in shared memory instead of spilled registers, saves a tenth of
+// the rows).  A group that others join has a run at
 // that time, a finished group's run is cleared before it looks for one to
 // join, and it never gets another: no two groups join each other.
 struct RowsNext {
@@ -1560,19 +1559,19 @@ __device__ __forceinline__ int window_value(const Trans2Params& p, const RowGrou
 // Corner records a warp takes from the log at a time.
 static constexpr unsigned kLogChunk = 8;
 
-// Latency-bound: a row's changes run through dependent evaluations (one row
-// of R-MAT 20 takes 480 us for 178 evaluations), so what counts is the number
-// of memory round trips and fences from one vertex's drop to the next one's
-// evaluation.  Hence: the static data of a vertex is loaded while its mark is
-// set, its value and counters come with it, the new value is found with
-// register counters at the four highest candidates (the shared-memory
-// histogram only for larger drops), a corner record's place is in hand before
-// the drop, one fence stands between the new value (with its record) and the
-// neighbours' values, a request is one atomicOr, a warp keeps one of the items
-// it requests, and rows advance without a grid barrier.  Together: rows
-// 1..kmax of R-MAT 18 / 20 / 22 in one launch 16.5 / 25.8 / 53.5 -> 9.6 / 17.6 /
-// 38.5 ms, ER 10,000 / 100,000 0.71 -> 0.39 ms.  80 registers for three
-// blocks per SM (64 spill); one to four blocks measure within 7 %.
+// Latency-bound: a row's changes run through dependent evaluations (a chain of
+// 20,000 takes 4.9 us per link, 7.8 with two more fences and a queue item per
+// link), so what counts is the number of memory round trips and fences from
+// one vertex's drop to the next one's evaluation.  Hence: the static data of a
+// vertex is loaded while its mark is set, its value and counters come with it,
+// the new value is found with register counters at the four highest candidates
+// (the shared-memory histogram only for larger drops), a corner record's place
+// is in hand before the drop, one fence stands between the new value (with its
+// record) and the neighbours' values and one before the vertex is released, a
+// request is one atomicOr, a warp keeps one of the items it requests, and rows
+// advance without a grid barrier.  Rows 1..kmax as one run, R-MAT 18 / 20 / 22
+// and ER of 10,000: 9.7 / 14.4 / 35.4 / 0.47 ms; in groups (RowsNext) 2.3 / 5.2 /
+// 19.0 ms.  80 registers for three blocks per SM (64 spill).
 #ifndef DC_TRANS2_MIN_BLOCKS
 #define DC_TRANS2_MIN_BLOCKS 3
 #endif
@@ -3075,10 +3074,10 @@ int run_peel2(dc_graph* h, int ninst, const PeelInst* inst, int32_t* maxv) {
     const void* fn = inst[0].member ? (const void*)k_peel2<true> : (const void*)k_peel2<false>;
     // Blocks on a handle that was not told: every block adds about 9 ns to a
     // light level, and large levels want more warps.  1 / 2 / 3 blocks per SM:
-    // R-MAT 13 0.95 / 1.01 / 1.08 ms, R-MAT 15 1.11 / 1.19 / 1.29, ER of 10,000
-    // 0.20 / 0.21 / 0.23, of 60,000 (60 edges per vertex) 0.45 / 0.43 / 0.45,
-    // of 100,000 0.30 / 0.27 / 0.28, R-MAT 20 4.03 / 3.83 / 4.00, R-MAT 21 6.0 /
-    // 5.4 / 5.5, R-MAT 22 9.4 / 7.84 / 7.78, ER of 3 M 2.95 / 1.74 / 1.35.
+    // R-MAT 13 0.87 / 0.91 / 0.99 ms, R-MAT 15 1.15 / 1.23 / 1.32, ER of 10,000
+    // 0.19 / 0.20 / 0.22, of 60,000 (60 edges per vertex) 0.47 / 0.43 / 0.45,
+    // of 100,000 0.23 / 0.22 / 0.22, R-MAT 20 4.5 / 4.4 / 4.6, R-MAT 21 6.3 /
+    // 5.7 / 5.9, R-MAT 22 10.0 / 8.5 / 8.6, ER of 3 M 2.99 / 1.79 / 1.42.
     int bps = h->peel_bps;
     if (bps <= 0 && h->blocks_per_sm <= 0 && !inst[0].member) bps = g.V <= 50000u ? 1 : g.V >= 3000000u ? 3 : 2;
     const FirstStep first{0, 0};
@@ -3468,10 +3467,10 @@ static int rows_run(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint
             // core a run starts from is small: a start costs a pass over its
             // core's lists and a refinement from row 0 there.  With skewed
             // degrees (|C_k| a few per cent of |C_1| after a tenth of the
-            // rows) eight runs at a time take the rows from 3.4 / 8.9 / 15.6 /
-            // 44 ms to 1.3 / 3.5 / 7.8 / 19 (ragged R-MAT 17, R-MAT 18 / 20 /
-            // 22) with fixed cuts; where every vertex is in almost every core
-            // (ER, 100 edges per vertex) they take them from 3.6 to 11.0 ms.
+            // rows) they take the rows from 3.0 / 9.7 / 14.4 / 35 ms to 0.7 /
+            // 2.3 / 5.2 / 19 (ragged R-MAT 17, R-MAT 18 / 20 / 22); where every
+            // vertex is in almost every core (ER, 100 edges per vertex) fixed
+            // cuts took them from 3.6 to 11.0 ms.
             // Hence an eighth of |C_1| at most (a quarter up to 65,536
             // vertices), which also bounds the groups' state, and no cut
             // where that leaves more than half of the rows to the first run.
@@ -3517,9 +3516,9 @@ static int rows_run(dc_graph* h, int32_t K, int32_t Kstop, bool allow_sort, uint
     // blocks: what fits at the same time
     const void* rows_fn = ngroups > 1 ? (const void*)k_trans2<true> : (const void*)k_trans2<false>;
     int grid = 0;
-    // (engine's cuts, 1 / 2 / 3 blocks per SM: 53,000 edges 0.41 / 0.43 / 0.47
-    // ms, 175,000 0.47 / 0.50 / 0.52, 470,000 0.69 / 0.62 / 0.62, 1.0 M 0.90 /
-    // 0.85 / 0.88, 1.9 M 1.39 / 1.26 / 1.23, 3.9 M 2.36 / 2.10 / 1.89)
+    // (engine's cuts, 1 / 2 / 3 blocks per SM: 53,000 edges 0.39 / 0.42 / 0.45
+    // ms, 228,000 0.55 / 0.53 / 0.56, 518,000 0.93 / 0.99 / 1.03, 0.96 M 1.10 /
+    // 1.00 / 1.01, 1.9 M 1.67 / 1.44 / 1.38, 3.9 M 3.2 / 2.4 / 2.3)
     const int most_bps = !h->auto_cuts ? 8
                          : h->blocks_per_sm > 0 ? h->blocks_per_sm  // dc_set_launch bounds the launch
                          : g.E < 300000u ? 1 : g.E < 1500000u ? 2 : 8;

@@ -136,7 +136,9 @@ int dc_reserve_device_memory(int device, uint64_t bytes);
  * allocateDeviceGraphMemory / moveGraphToDevice (src/cuda_memory.h:5-41). */
 int dc_graph_create(uint32_t V, uint64_t E, const uint32_t* src, const uint32_t* dst,
                     const dc_graph_opts* opts, dc_graph** out);
-/* Same from device-resident edge arrays (no host copy). */
+/* Same from device-resident edge arrays (no host copy).  The arrays are
+ * complete when the call is made: the handle reads them on a stream of its
+ * own, twice. */
 int dc_graph_create_device(uint32_t V, uint64_t E, const uint32_t* d_src, const uint32_t* d_dst,
                            const dc_graph_opts* opts, dc_graph** out);
 /* Graph(const string&) (src/graph.cpp:381-395): reads "<path>-binary-g=<gap>"
